@@ -17,22 +17,26 @@ _tensors_created = 0
 
 class Tensor:
     """src/model/autograd.ts:20-51. `data`/`grad` are host f32 arrays; with a device backend they are
-    stale until `sync()` copies them back."""
+    stale until `sync()` copies them back. Most tensors of a graph live and die on the device, so a host array that starts
+    at zero is only allocated when someone looks at it: cleared up front, the arrays of one eager forward of 15 layers at
+    512 rows (and their page faults) cost more host time than all of its launches."""
 
-    __slots__ = ("data", "grad", "shape", "requiresGrad", "_backward", "_prev", "seq", "__weakref__")
+    __slots__ = ("_data", "_grad", "size", "shape", "requiresGrad", "_backward", "_prev", "seq", "__weakref__")
 
-    def __init__(self, data: np.ndarray, shape: Sequence[int], requiresGrad: bool = False):
+    def __init__(self, data: Optional[np.ndarray], shape: Sequence[int], requiresGrad: bool = False):
         global _tensors_created
-        data = np.ascontiguousarray(data, dtype=np.float32).reshape(-1)
         n = 1
         for s in shape:
             n *= int(s)
-        if data.size != n:
-            raise ValueError(f"data length {data.size} != shape {list(shape)}")
-        self.data = data
+        if data is not None:
+            data = np.ascontiguousarray(data, dtype=np.float32).reshape(-1)
+            if data.size != n:
+                raise ValueError(f"data length {data.size} != shape {list(shape)}")
+        self._data = data
+        self._grad = None
+        self.size = n
         self.shape = [int(s) for s in shape]
         self.requiresGrad = requiresGrad
-        self.grad = np.zeros(n, dtype=np.float32)
         self._backward: Callable[[], None] = _noop
         self._prev: List["Tensor"] = []
         self.seq = _tensors_created
@@ -40,17 +44,42 @@ class Tensor:
 
     @staticmethod
     def zeros(shape: Sequence[int], requiresGrad: bool = False) -> "Tensor":
-        n = 1
-        for s in shape:
-            n *= int(s)
-        return Tensor(np.zeros(n, dtype=np.float32), shape, requiresGrad)
-
-    def zeroGrad(self):
-        self.grad.fill(0)
+        return Tensor(None, shape, requiresGrad)
 
     @property
-    def size(self) -> int:
-        return self.data.size
+    def data(self) -> np.ndarray:
+        if self._data is None:
+            self._data = np.zeros(self.size, dtype=np.float32)
+        return self._data
+
+    @data.setter
+    def data(self, a: np.ndarray):
+        self._data = a
+
+    @property
+    def grad(self) -> np.ndarray:
+        if self._grad is None:
+            self._grad = np.zeros(self.size, dtype=np.float32)
+        return self._grad
+
+    @grad.setter
+    def grad(self, a: np.ndarray):
+        self._grad = a
+
+    def dataForReading(self) -> np.ndarray:
+        """`data` for a caller that overwrites all of it (a read back from the device)."""
+        if self._data is None:
+            self._data = np.empty(self.size, dtype=np.float32)
+        return self._data
+
+    def gradForReading(self) -> np.ndarray:
+        if self._grad is None:
+            self._grad = np.empty(self.size, dtype=np.float32)
+        return self._grad
+
+    def zeroGrad(self):
+        if self._grad is not None:
+            self._grad.fill(0)
 
 
 def _noop():

@@ -650,7 +650,7 @@ class CudaBackend:
                 continue
             if e.lazy is not None:
                 self._materializeLazy(e)
-            self._read(e.data, t.data)
+            self._read(e.data, t.dataForReading())
         for t in list(self._touched.values()):
             e = self._entries.get(t)
             if e is None:
@@ -661,7 +661,7 @@ class CudaBackend:
                     self._check(self.lib.gt_zero(self.ctx, e.grad, e.bytes))
                     self.gradClearsIssued += 1
                 if t not in self._keptOnDevice:
-                    self._read(e.grad, t.grad)
+                    self._read(e.grad, t.gradForReading())
             e.gradLive = False   # the next graph's first writer overwrites (the deferred clear)
         self._check(self.lib.gt_sync(self.ctx))
         self.lastSyncReadbackBytes = self._readback
