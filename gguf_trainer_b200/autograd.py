@@ -21,7 +21,9 @@ class Tensor:
     at zero is only allocated when someone looks at it: cleared up front, the arrays of one eager forward of 15 layers at
     512 rows (and their page faults) cost more host time than all of its launches."""
 
-    __slots__ = ("_data", "_grad", "size", "shape", "requiresGrad", "_backward", "_prev", "seq", "__weakref__")
+    # `_dev`: the device entry a backend keeps for this tensor (its latest one); `_needs`: for an op's output, whether a
+    # gradient can flow through it to anything trainable.
+    __slots__ = ("_data", "_grad", "size", "shape", "requiresGrad", "_backward", "_prev", "seq", "_dev", "_needs", "__weakref__")
 
     def __init__(self, data: Optional[np.ndarray], shape: Sequence[int], requiresGrad: bool = False):
         global _tensors_created
@@ -39,8 +41,25 @@ class Tensor:
         self.requiresGrad = requiresGrad
         self._backward: Callable[[], None] = _noop
         self._prev: List["Tensor"] = []
+        self._dev = None
+        self._needs = False
         self.seq = _tensors_created
         _tensors_created += 1
+
+    @staticmethod
+    def output(shape: List[int], size: int, prev: List["Tensor"]) -> "Tensor":
+        """The output of a backend's op: `zeros(shape)` recorded on `prev`, for a backend that has the element count."""
+        global _tensors_created
+        t = Tensor.__new__(Tensor)
+        t._data = t._grad = t._dev = None
+        t.size = size
+        t.shape = shape
+        t.requiresGrad = t._needs = False
+        t._backward = _noop
+        t._prev = prev
+        t.seq = _tensors_created
+        _tensors_created += 1
+        return t
 
     @staticmethod
     def zeros(shape: Sequence[int], requiresGrad: bool = False) -> "Tensor":

@@ -17,6 +17,7 @@ Differences that are deliberate:
 from __future__ import annotations
 
 import ctypes as C
+import itertools
 import weakref
 from typing import Dict, List, Optional, Sequence
 
@@ -31,13 +32,20 @@ _KIND = {"NT": 0, "NN": 1, "TN": 2}
 PRECISION = {"fp32": 0, "tf32": 1}   # (the C ABI reserves 2 for BF16 and refuses it: there are no BF16 kernels)
 
 
+_I32 = [None] + [C.c_int32 * n for n in range(1, 9)]     # argument arrays of the grouped launches
+_U64 = [None] + [C.c_uint64 * n for n in range(1, 9)]
+
+
 class _Entry:
-    __slots__ = ("data", "grad", "bytes", "external", "gradLive", "size", "pendingDx", "copyFrom", "pendingDw", "pendingFwd",
+    __slots__ = ("owner", "needs", "region", "data", "grad", "bytes", "external", "gradLive", "size", "pendingDx", "copyFrom", "pendingDw", "pendingFwd",
                  "lazy", "ropeOf", "ropeFused")
 
-    def __init__(self, data: int, grad: int, nbytes: int, external: bool, size: int):
+    def __init__(self, owner: int, data: int, grad: int, nbytes: int, external: bool, size: int):
+        self.owner = owner        # `_uid` of the backend
         self.data = data
-        self.grad = grad          # 0 for a frozen external (webgpu.ts frozenGradStub)
+        self.grad = grad          # 0 for a frozen external (webgpu.ts frozenGradStub), and for an op's output until written
+        self.needs = grad != 0    # an op's output: does a gradient flow through it? (an external: does it have a buffer)
+        self.region = 0           # the recompute region it was made in (0: none): how long a gradient buffer must live
         self.bytes = nbytes
         self.external = external
         self.gradLive = False     # has anything been written to grad in the current graph?
@@ -96,8 +104,8 @@ class CapturedGraph:
         g = self.gpu
         for h in self.handles:
             g._check(g.lib.gt_graph_destroy(g.ctx, h))
-        for addr, _size in self.owned:
-            g._check(g.lib.gt_free(g.ctx, addr))
+        for addr, size in self.owned:
+            g._release(addr, size)
         self.owned = []
 
 
@@ -163,6 +171,30 @@ class _ProfilingLib:
         return timed
 
 
+class _Entries:
+    """`backend._entries[tensor]`: the device entry of a tensor."""
+
+    __slots__ = ("_gpu",)
+
+    def __init__(self, gpu):
+        self._gpu = gpu
+
+    def get(self, t):
+        return self._gpu._find(t)
+
+    def __getitem__(self, t):
+        e = self._gpu._find(t)
+        if e is None:
+            raise KeyError(t)
+        return e
+
+    def __contains__(self, t):
+        return self._gpu._find(t) is not None
+
+
+_uids = itertools.count(1)
+
+
 class CudaBackend:
     def __init__(self, device: int = 0, precision: str = "fp32"):
         self.lib = _lib.load()
@@ -180,11 +212,19 @@ class CudaBackend:
         self.gradClearsIssued = 0
         self.precision = precision
         self._check(self.lib.gt_set_precision(self.ctx, PRECISION[precision]))
-        self._entries: "weakref.WeakKeyDictionary[Tensor, _Entry]" = weakref.WeakKeyDictionary()
+        # A tensor's entry sits on the tensor (`Tensor._dev`). Parameters and other externals are listed here as well, so that a
+        # tensor two backends take turns with keeps its buffers in both.
+        self._uid = next(_uids)
+        self._externals: "weakref.WeakKeyDictionary[Tensor, _Entry]" = weakref.WeakKeyDictionary()
+        self._tape: List[Tensor] = []          # outputs recorded with a backward closure since the last sync
+        self._free: Dict[int, List[int]] = {}  # recycled blocks by size (a dictionary access instead of two library calls)
         self._touched: Dict[int, Tensor] = {}
         self._keptOnDevice: "weakref.WeakSet[Tensor]" = weakref.WeakSet()
         self._transients: List[tuple] = []     # (addr, size)
         self._regionFree: List[tuple] = []
+        self._outer: List[tuple] = []          # gradient buffers made inside a region for tensors that outlive it
+        self._outerMark = 0
+        self._regionStack: List[tuple] = []    # (serial of the region, tape length when it opened)
         self._regionsOpened = 0
         # Attention outputs kept across a recompute region (see regionToken / replayOf)
         self.keepAttentionAcrossRecompute = True
@@ -281,33 +321,67 @@ class CudaBackend:
     def kernelLaunches(self) -> int:
         return self.stats()["launches"]
 
+    @property
+    def _entries(self) -> _Entries:
+        return _Entries(self)
+
     # ------------------------------------------------------------------ memory
     def _alloc(self, nbytes: int) -> tuple:
+        size = (nbytes + 255) & ~255 if nbytes > 256 else 256
+        blocks = self._free.get(size)
+        if blocks:
+            return blocks.pop(), size
         out = C.c_uint64()
-        self._check(self.lib.gt_alloc(self.ctx, max(nbytes, 4), C.byref(out)))
-        size = max(256, (max(nbytes, 4) + 255) // 256 * 256)
-        return int(out.value), size
+        self._check(self.lib.gt_alloc(self.ctx, size, C.byref(out)))
+        return out.value, size
+
+    def _release(self, addr: int, size: int):
+        """Back to the pool. One stream: whoever gets the block next is queued behind its last reader."""
+        blocks = self._free.get(size)
+        if blocks is None:
+            self._free[size] = [addr]
+        else:
+            blocks.append(addr)
 
     def _acquirePersistent(self, nbytes: int) -> int:
         return self._alloc(nbytes)[0]
 
     def _acquireTransient(self, nbytes: int) -> int:
-        addr, size = self._alloc(nbytes)
-        self._transients.append((addr, size))
-        return addr
+        tr = self._alloc(nbytes)
+        self._transients.append(tr)
+        return tr[0]
 
     def _acquireRecycled(self, nbytes: int) -> int:
         """Best fit from the region free-list, else a fresh transient (webgpu.ts acquireRecycled)."""
-        want = max(256, (max(nbytes, 4) + 255) // 256 * 256)
-        best = -1
+        if not self._regionFree:
+            tr = self._alloc(nbytes)
+            self._transients.append(tr)
+            return tr[0]
+        want = (nbytes + 255) & ~255 if nbytes > 256 else 256
+        best, bestSize = -1, 0
         for i, (_a, size) in enumerate(self._regionFree):
-            if size >= want and (best < 0 or size < self._regionFree[best][1]):
+            if size == want:
                 best = i
+                break
+            if size > want and (best < 0 or size < bestSize):
+                best, bestSize = i, size
         if best < 0:
             return self._acquireTransient(nbytes)
         tr = self._regionFree.pop(best)
         self._transients.append(tr)
         return tr[0]
+
+    def _gradAddr(self, e: _Entry) -> int:
+        """The gradient buffer of an op's output, made when something is about to be written there: a forward that nothing
+        is trained on never has any. One made inside a recompute region for a tensor from outside it outlives the region."""
+        if e.grad == 0 and not e.external:
+            if e.region == (self._regionStack[-1][0] if self._regionStack else 0):
+                e.grad = self._acquireRecycled(e.bytes)
+            else:
+                tr = self._alloc(e.bytes)
+                self._outer.append(tr)
+                e.grad = tr[0]
+        return e.grad
 
     def _write(self, addr: int, arr: np.ndarray):
         arr = np.ascontiguousarray(arr)
@@ -342,21 +416,23 @@ class CudaBackend:
         self._write(addr, a)
         return addr
 
+    def _find(self, t: Tensor) -> Optional[_Entry]:
+        e = t._dev
+        if e is None or e.owner == self._uid:
+            return e
+        return self._externals.get(t)
+
+    def _newExternal(self, t: Tensor, data: int, grad: int) -> _Entry:
+        e = _Entry(self._uid, data, grad, t.size * 4, True, t.size)
+        self._externals[t] = e
+        t._dev = e
+        return e
+
     def _entryFor(self, t: Tensor) -> _Entry:
         """webgpu.ts:1539-1573: externals (params, test inputs) get persistent buffers on first use."""
-        e = self._entries.get(t)
-        if e is None and id(t) in self._pendingAct:
-            e = self._materializeAct(t)
-        if e is None and id(t) in self._pendingAdd:
-            e = self._materializeAdd(t)
-        if e is None:
-            nbytes = t.size * 4
-            if self._capturing:
-                raise _lib.GtError(4, "a tensor first reached the device inside a graph capture; upload it first")
-            e = _Entry(self._acquirePersistent(nbytes), self._acquirePersistent(nbytes) if t.requiresGrad else 0,
-                       nbytes, True, t.size)
-            self._entries[t] = e
-            self._write(e.data, t.data)
+        e = t._dev
+        if e is None or e.owner != self._uid:
+            e = self._firstUse(t)
         if e.pendingFwd:
             self._flushFwd()
         if e.lazy is not None:
@@ -365,9 +441,23 @@ class CudaBackend:
             self._touched[id(t)] = t
         return e
 
+    def _firstUse(self, t: Tensor) -> _Entry:
+        if id(t) in self._pendingAct:
+            return self._materializeAct(t)
+        if id(t) in self._pendingAdd:
+            return self._materializeAdd(t)
+        e = self._find(t)
+        if e is None:
+            if self._capturing:
+                raise _lib.GtError(4, "a tensor first reached the device inside a graph capture; upload it first")
+            nbytes = t.size * 4
+            e = self._newExternal(t, self._acquirePersistent(nbytes), self._acquirePersistent(nbytes) if t.requiresGrad else 0)
+            self._write(e.data, t.data)
+        return e
+
     def _entryOf(self, t: Tensor):
         """The device entry of a tensor some op produced (launching it first if it is a deferred activation), or None."""
-        e = self._entries.get(t)
+        e = self._find(t)
         if e is None and id(t) in self._pendingAct:
             e = self._materializeAct(t)
         if e is None and id(t) in self._pendingAdd:
@@ -378,13 +468,45 @@ class CudaBackend:
             self._materializeLazy(e)
         return e
 
-    def _makeOut(self, shape, prev) -> tuple:
-        t = Tensor.zeros(shape)
-        t._prev = list(prev)
+    @staticmethod
+    def _flows(t: Tensor, e: _Entry) -> bool:
+        """Does a gradient of `t` have anywhere to go (webgpu.ts:898-901: a frozen input is skipped)?"""
+        return e.needs and (t.requiresGrad or not e.external)
+
+    def _makeOut(self, shape: List[int], size: int, prev: List[Tensor], needs: bool) -> tuple:
+        t = Tensor.output(shape, size, prev)
+        return t, self._newEntry(t, needs)
+
+    def _newEntry(self, t: Tensor, needs: bool) -> _Entry:
         nbytes = t.size * 4
-        e = _Entry(self._acquireRecycled(nbytes), self._acquireRecycled(nbytes), nbytes, False, t.size)
-        self._entries[t] = e
-        return t, e
+        e = _Entry(self._uid, self._acquireRecycled(nbytes), 0, nbytes, False, t.size)
+        e.needs = t._needs = needs
+        if self._regionStack:
+            e.region = self._regionStack[-1][0]
+        t._dev = e
+        return e
+
+    def _record(self, t: Tensor, needs: bool, bw) -> Tensor:
+        """Put an op's backward closure on the tape, or nothing where no gradient can flow: such a tensor is freed with its
+        last reader instead of being kept (with everything it was computed from) until the graph goes."""
+        if needs:
+            t._backward = bw
+            self._tape.append(t)
+        else:
+            t._backward = self._ensureBackwardBegun
+            t._prev = []
+        return t
+
+    def _dropTape(self, mark: int = 0, keep: Sequence[Tensor] = ()):
+        """The buffers of these graphs have been recycled: a backward over them is refused or does nothing, and without their
+        closures the tensors are freed by reference count (a closure and its tensor refer to each other, and waiting for the
+        cycle collector costs a training loop more time than its launches)."""
+        for t in self._tape[mark:]:
+            if any(t is k for k in keep):
+                continue
+            t._backward = self._ensureBackwardBegun
+            t._prev = []
+        del self._tape[mark:]
 
     # The input gradient of `linear` is dX (+)= dY.W. An activation that feeds several projections (the normed input
     # of q, k and v; of gate and up) collects one such product per consumer, and the reference issues them one by one,
@@ -410,7 +532,7 @@ class CudaBackend:
     # gradients are handed to someone outside the ops (an optimizer, an exchange, a sync) only parameters matter, so the
     # copy into a transient's gradient is not made there (60 copies of [T, hidden] per step of a 30-layer model).
     def _materializeCopy(self, e: _Entry):
-        self._check(self.lib.gt_copy(self.ctx, e.grad, e.copyFrom, e.bytes))
+        self._check(self.lib.gt_copy(self.ctx, self._gradAddr(e), e.copyFrom, e.bytes))
         e.copyFrom = 0
         e.gradLive = True
         self._pendingCopy.pop(id(e), None)
@@ -433,13 +555,14 @@ class CudaBackend:
         self._pendingDx.pop(id(e), None)
         acc = 1 if e.gradLive else 0
         e.gradLive = True
+        self._gradAddr(e)
         n = len(parts)
         if n == 1:
             self._gemm("NN", acc, rows, cols, parts[0][2], parts[0][0], parts[0][1], e.grad)
             return
-        Ks = (C.c_int32 * n)(*[p[2] for p in parts])
-        As = (C.c_uint64 * n)(*[p[0] for p in parts])
-        Bs = (C.c_uint64 * n)(*[p[1] for p in parts])
+        Ks = _I32[n](*[p[2] for p in parts])
+        As = _U64[n](*[p[0] for p in parts])
+        Bs = _U64[n](*[p[1] for p in parts])
         self._check(self.lib.gt_gemm_multi(self.ctx, _KIND["NN"], acc, rows, cols, n, Ks, As, Bs, e.grad))
 
     # Projections of the same activation (q, k and v of the normed input; gate and up) are noted when recorded and
@@ -475,11 +598,11 @@ class CudaBackend:
             if n == 1:
                 self._check(self.lib.gt_gemm_scaled(self.ctx, _KIND["NT"], 0, T, r, inDim, p0["ex"].data, p0["ea"].data, p0["ts"], s))
             else:
-                Ms, Ns = (C.c_int32 * n)(*([T] * n)), (C.c_int32 * n)(*([r] * n))
-                As = (C.c_uint64 * n)(*([p0["ex"].data] * n))
-                Bs = (C.c_uint64 * n)(*[p["ea"].data for p in parts])
-                Cs = (C.c_uint64 * n)(*[p["ts"] for p in parts])
-                acc = (C.c_int32 * n)(*([0] * n))
+                Ms, Ns = _I32[n](*([T] * n)), _I32[n](*([r] * n))
+                As = _U64[n](*([p0["ex"].data] * n))
+                Bs = _U64[n](*[p["ea"].data for p in parts])
+                Cs = _U64[n](*[p["ts"] for p in parts])
+                acc = _I32[n](*([0] * n))
                 self._check(self.lib.gt_gemm_grouped_scaled(self.ctx, _KIND["NT"], n, Ms, Ns, inDim, As, Bs, Cs, acc, s))
             for p in parts:
                 self._gemm2("NT", 0, T, p["outDim"], inDim, p["ex"].data, p["ew"].data, r, p["ts"], p["eb"].data, p["eo"].data)
@@ -508,21 +631,21 @@ class CudaBackend:
             for p in roped:
                 p["rope"][0].pendingFwd = False
                 p["eo"].lazy = (lambda p=p: self._gemm("NT", 0, p["T"], p["outDim"], p["inDim"], p["ex"].data, p["ew"].data, p["eo"].data))
-            Ns = (C.c_int32 * n)(*[p["outDim"] for p in parts])
-            Ws = (C.c_uint64 * n)(*[p["ew"].data for p in parts])
-            Ys = (C.c_uint64 * n)(*[(p["rope"][0].data if "rope" in p else p["eo"].data) for p in parts])
-            Hs = (C.c_int32 * n)(*[(p["rope"][1] if "rope" in p else 0) for p in parts])
+            Ns = _I32[n](*[p["outDim"] for p in parts])
+            Ws = _U64[n](*[p["ew"].data for p in parts])
+            Ys = _U64[n](*[(p["rope"][0].data if "rope" in p else p["eo"].data) for p in parts])
+            Hs = _I32[n](*[(p["rope"][1] if "rope" in p else 0) for p in parts])
             self._check(self.lib.gt_linear_rope_grouped(self.ctx, n, T, inDim, parts[0]["ex"].data, Ns, Ws, Ys, Hs, hd, float(base), posOffset))
             return
         if n == 1:
             self._gemm("NT", 0, T, parts[0]["outDim"], inDim, parts[0]["ex"].data, parts[0]["ew"].data, parts[0]["eo"].data)
             return
-        Ms = (C.c_int32 * n)(*([T] * n))
-        Ns = (C.c_int32 * n)(*[p["outDim"] for p in parts])
-        As = (C.c_uint64 * n)(*[p["ex"].data for p in parts])
-        Bs = (C.c_uint64 * n)(*[p["ew"].data for p in parts])
-        Cs = (C.c_uint64 * n)(*[p["eo"].data for p in parts])
-        acc = (C.c_int32 * n)(*([0] * n))
+        Ms = _I32[n](*([T] * n))
+        Ns = _I32[n](*[p["outDim"] for p in parts])
+        As = _U64[n](*[p["ex"].data for p in parts])
+        Bs = _U64[n](*[p["ew"].data for p in parts])
+        Cs = _U64[n](*[p["eo"].data for p in parts])
+        acc = _I32[n](*([0] * n))
         self._check(self.lib.gt_gemm_grouped(self.ctx, _KIND["NT"], n, Ms, Ns, inDim, As, Bs, Cs, acc))
 
     def _materializeLazy(self, e: _Entry):
@@ -563,12 +686,12 @@ class CudaBackend:
             dy, x, gw, acc, outDim, inDim, _e = parts[0]
             self._gemm("TN", acc, outDim, inDim, rows, dy, x, gw)
             return
-        Ms = (C.c_int32 * n)(*[p[4] for p in parts])
-        Ns = (C.c_int32 * n)(*[p[5] for p in parts])
-        As = (C.c_uint64 * n)(*[p[0] for p in parts])
-        Bs = (C.c_uint64 * n)(*[p[1] for p in parts])
-        Cs = (C.c_uint64 * n)(*[p[2] for p in parts])
-        acc = (C.c_int32 * n)(*[p[3] for p in parts])
+        Ms = _I32[n](*[p[4] for p in parts])
+        Ns = _I32[n](*[p[5] for p in parts])
+        As = _U64[n](*[p[0] for p in parts])
+        Bs = _U64[n](*[p[1] for p in parts])
+        Cs = _U64[n](*[p[2] for p in parts])
+        acc = _I32[n](*[p[3] for p in parts])
         self._check(self.lib.gt_gemm_grouped(self.ctx, _KIND["TN"], n, Ms, Ns, rows, As, Bs, Cs, acc))
 
     def flushDeferred(self):
@@ -578,7 +701,7 @@ class CudaBackend:
 
     def _gradTarget(self, t: Tensor, e: _Entry):
         """(grad address or 0, accum flag) for a backward kernel about to write into t's gradient."""
-        if e.grad == 0 or (e.external and not t.requiresGrad):
+        if not self._flows(t, e):
             return 0, 0
         if e.pendingDw:
             self._flushDw()             # an earlier product into this gradient goes first
@@ -588,7 +711,7 @@ class CudaBackend:
             self._flushDx(e)
         acc = 1 if e.gradLive else 0
         e.gradLive = True
-        return e.grad, acc
+        return e.grad or self._gradAddr(e), acc
 
     def _gradSource(self, e: _Entry) -> int:
         """The upstream gradient of an op output. Never written means it is exactly zero."""
@@ -599,7 +722,7 @@ class CudaBackend:
         if e.copyFrom:
             return e.copyFrom          # still exactly the upstream buffer of an `add`: read it there, no copy
         if not e.gradLive:
-            self._check(self.lib.gt_zero(self.ctx, e.grad, e.bytes))
+            self._check(self.lib.gt_zero(self.ctx, self._gradAddr(e), e.bytes))
             self.gradClearsIssued += 1
             e.gradLive = True
         return e.grad
@@ -618,15 +741,13 @@ class CudaBackend:
         total = 0
         offs = []
         for t in tensors:
-            if t in self._entries:
+            if self._find(t) is not None:
                 raise _lib.GtError(4, "reserveGradArena must run before the tensors are first used")
             offs.append(total)
             total += (t.size + 63) // 64 * 64   # 256-byte aligned slices
         base = self.createStateBuffer(total * 4)
         for t, off in zip(tensors, offs):
-            nbytes = t.size * 4
-            e = _Entry(self._acquirePersistent(nbytes), base + off * 4, nbytes, True, t.size)
-            self._entries[t] = e
+            e = self._newExternal(t, self._acquirePersistent(t.size * 4), base + off * 4)
             self._write(e.data, t.data)
         return base, total, offs
 
@@ -645,14 +766,14 @@ class CudaBackend:
             if id(t) in seen:
                 continue
             seen.add(id(t))
-            e = self._entries.get(t)
+            e = self._find(t)
             if e is None:
                 continue
             if e.lazy is not None:
                 self._materializeLazy(e)
             self._read(e.data, t.dataForReading())
         for t in list(self._touched.values()):
-            e = self._entries.get(t)
+            e = self._find(t)
             if e is None:
                 continue
             if t.requiresGrad and e.grad:
@@ -665,12 +786,12 @@ class CudaBackend:
             e.gradLive = False   # the next graph's first writer overwrites (the deferred clear)
         self._check(self.lib.gt_sync(self.ctx))
         self.lastSyncReadbackBytes = self._readback
-        for addr, _size in self._transients:
-            self._check(self.lib.gt_free(self.ctx, addr))
-        self._transients = []
-        for addr, _size in self._regionFree:
-            self._check(self.lib.gt_free(self.ctx, addr))
-        self._regionFree = []
+        for blocks in (self._transients, self._regionFree, self._outer):
+            for addr, size in blocks:
+                self._release(addr, size)
+        self._transients, self._regionFree, self._outer = [], [], []
+        self._dropTape()
+        self._regionStack = []
         self._touched.clear()
         self._backwardBegun = False
         if self._graphOpen:                    # (a sync with no graph behind it, e.g. after building an optimizer, arms nothing)
@@ -682,10 +803,10 @@ class CudaBackend:
 
     def reclaimStepTransients(self, keep: Sequence[Tensor] = ()):
         """webgpu.ts:612-633: recycle this micro-batch's transients without the readback."""
-        self._flushAllDx()
+        self._flushAllDx("drop")
         keepBufs = set()
         for t in keep:
-            e = self._entries.get(t)
+            e = self._find(t)
             if e is not None:
                 keepBufs.add(e.data)
         retained = []
@@ -693,16 +814,19 @@ class CudaBackend:
             if tr[0] in keepBufs:
                 retained.append(tr)
             else:
-                self._check(self.lib.gt_free(self.ctx, tr[0]))
+                self._release(*tr)
         self._transients = retained
-        for addr, _size in self._regionFree:
-            self._check(self.lib.gt_free(self.ctx, addr))
-        self._regionFree = []
+        for blocks in (self._regionFree, self._outer):
+            for addr, size in blocks:
+                self._release(addr, size)
+        self._regionFree, self._outer = [], []
+        self._dropTape()
 
     # ------------------------------------------------------------------ regions (RegionBackend)
     def beginRegion(self) -> int:
         self._regionsOpened += 1
         self._regionDepth += 1
+        self._regionStack.append((self._regionsOpened, len(self._tape)))
         if self._regionDepth == 1 and self.keepAttentionAcrossRecompute:
             self._curRec = {"id": self._nextRegionId, "saved": [], "pos": 0, "replay": False}
             self._nextRegionId += 1
@@ -743,12 +867,17 @@ class CudaBackend:
                 f"a sync() or reclaim ran inside the region")
         self._flushAllDx()
         self._flushPendingActs(only=list(keep))
+        _serial, tapeMark = self._regionStack.pop() if self._regionStack else (0, len(self._tape))
+        outer = self._regionStack[-1][0] if self._regionStack else 0
+        self._dropTape(tapeMark, keep)
         keepBufs = set()
         for t in keep:
-            e = self._entries.get(t)
+            e = self._find(t)
             if e is not None:
                 keepBufs.add(e.data)
                 keepBufs.add(e.grad)
+                e.region = outer
+                self._tape.append(t)
         rec = self._curRec if self._regionDepth == 1 else None
         self._regionDepth = max(0, self._regionDepth - 1)
         release = set()
@@ -781,7 +910,7 @@ class CudaBackend:
             raise RuntimeError("seedGradFrom: tensor has no GPU buffers")
         if dst.size != src.size:
             raise RuntimeError(f"seedGradFrom: size mismatch {dst.size} vs {src.size}")
-        self._check(self.lib.gt_copy(self.ctx, ed.grad, self._gradSource(es), src.size * 4))
+        self._check(self.lib.gt_copy(self.ctx, self._gradAddr(ed), self._gradSource(es), src.size * 4))
         ed.gradLive = True
 
     def seedGradFromHost(self, t: Tensor):
@@ -790,7 +919,7 @@ class CudaBackend:
         e = self._entryOf(t)
         if e is None:
             raise RuntimeError("seedGradFromHost: tensor has no GPU buffers")
-        self._write(e.grad, t.grad)
+        self._write(self._gradAddr(e), t.grad)
         e.gradLive = True
 
     def _beginForwardOp(self, keepPending: bool = False):
@@ -869,14 +998,15 @@ class CudaBackend:
         if self._seedBuf == 0:
             self._seedBuf = self.createStateBuffer(4)
         self._write(self._seedBuf, np.array([seed], np.float32))
-        for t, e in list(self._entries.items()):
-            if e.external and e.grad:
+        for e in self._externals.values():
+            if e.grad:
                 e.gradLive = bool(accumulate)
         self._check(self.lib.gt_graph_begin(self.ctx))
         self._capturing = True
         self._captureInputs = []
         self._captureSegments = []
         self._captureMark = len(self._transients)
+        self._outerMark = len(self._outer)
 
     def cutCapture(self) -> int:
         """Close the graph recorded so far and start the next one: the place where the replayer will issue work from
@@ -895,10 +1025,12 @@ class CudaBackend:
         self._flushAllDx("drop")
         self._capturing = False
         self._check(self.lib.gt_graph_end(self.ctx, C.byref(h)))
-        owned = self._transients[self._captureMark:] + self._regionFree
+        owned = self._transients[self._captureMark:] + self._regionFree + self._outer[self._outerMark:]
         self._transients = self._transients[:self._captureMark]
+        self._outer = self._outer[:self._outerMark]
         self._regionFree = []
-        owned = owned + [(a, n * 4) for a, n, _r, _b in self._captureInputs]
+        self._dropTape()
+        owned = owned + [(a, max(256, (n * 4 + 255) & ~255)) for a, n, _r, _b in self._captureInputs]
         outs = {}
         for name, t in (outputs or {}).items():
             e = self._entries[t]
@@ -937,7 +1069,8 @@ class CudaBackend:
         T, inDim = x.shape
         outDim = w.shape[0]
         ex, ew = self._entryFor(x), self._entryFor(w)
-        out, eo = self._makeOut([T, outDim], [x, w])
+        needs = self._flows(x, ex) or self._flows(w, ew)
+        out, eo = self._makeOut([T, outDim], T * outDim, [x, w], needs)
         if self.groupForward:
             self._deferLinear(ex, ew, eo, T, inDim, outDim)
         else:
@@ -947,9 +1080,9 @@ class CudaBackend:
         def _bw():
             self._ensureBackwardBegun()
             go = self._gradSource(eo)
-            if ex.grad and not (ex.external and not x.requiresGrad):
+            if self._flows(x, ex):
                 self._deferDx(ex, T, inDim, go, ew.data, outDim)
-            if w.requiresGrad:
+            if self._flows(w, ew):
                 gw, aw = self._gradTarget(w, ew)
                 if gw:
                     # (a product with many output tiles, the readout's, fills the GPU alone and is launched as it comes)
@@ -958,8 +1091,7 @@ class CudaBackend:
                     else:
                         self._gemm("TN", aw, outDim, inDim, T, go, ex.data, gw)
 
-        out._backward = _bw
-        return out
+        return self._record(out, needs, _bw)
 
     def loraLinear(self, x: Tensor, w: Tensor, a: Tensor, b: Tensor, scale: float) -> Tensor:
         """The adapter-carrying projection of autograd.ts:311-319, y = x·Wᵀ + scale·((x·Aᵀ)·Bᵀ), as one op. Recorded as
@@ -973,7 +1105,8 @@ class CudaBackend:
         T, inDim = x.shape
         outDim, r = w.shape[0], a.shape[0]
         ex, ew, ea, eb = self._entryFor(x), self._entryFor(w), self._entryFor(a), self._entryFor(b)
-        out, eo = self._makeOut([T, outDim], [x, w, a, b])
+        needs = self._flows(x, ex) or self._flows(w, ew) or self._flows(a, ea) or self._flows(b, eb)
+        out, eo = self._makeOut([T, outDim], T * outDim, [x, w, a, b], needs)
         small = T * r * 4
         ts, dt = self._acquireRecycled(small), self._acquireRecycled(small)
         s = float(scale)
@@ -995,7 +1128,7 @@ class CudaBackend:
         def _bw():
             self._ensureBackwardBegun()
             go = self._gradSource(eo)
-            wantDx = bool(ex.grad) and not (ex.external and not x.requiresGrad)
+            wantDx = self._flows(x, ex)
             self._check(self.lib.gt_gemm_scaled(self.ctx, kNN, 0, T, r, outDim, go, eb.data, dt, s))   # dt = scale·(g·B)
             # dB = gᵀ·ts and dA = dtᵀ·x: thin outputs contracted over every row, bound by reading g and x; the fourteen of a
             # layer go out as two grouped launches (_deferDw) instead of one launch each
@@ -1021,14 +1154,14 @@ class CudaBackend:
                 if gw:
                     self._gemm("TN", aw, outDim, inDim, T, go, ex.data, gw)
 
-        out._backward = _bw
-        return out
+        return self._record(out, needs, _bw)
 
     def _elementwise(self, op: str, a: Tensor, b: Optional[Tensor], c: float) -> Tensor:
         self._beginForwardOp()
         ea = self._entryFor(a)
         eb = self._entryFor(b) if b is not None else None
-        out, eo = self._makeOut(a.shape, [a, b] if b is not None else [a])
+        needs = self._flows(a, ea) or (eb is not None and self._flows(b, eb))
+        out, eo = self._makeOut(list(a.shape), a.size, [a, b] if b is not None else [a], needs)
         n = a.size
         code = _EW[op]
         self._check(self.lib.gt_ew_fwd(self.ctx, code, n, ea.data, eb.data if eb else 0, c, eo.data))
@@ -1045,8 +1178,7 @@ class CudaBackend:
             gb, ab = self._gradTarget(b, eb) if eb is not None else (0, 0)
             self._check(self.lib.gt_ew_bwd(self.ctx, code, n, ea.data, eb.data if eb else 0, c, go, ga, aa, gb, ab))
 
-        out._backward = _bw
-        return out
+        return self._record(out, needs, _bw)
 
     def add(self, a, b):
         """webgpu.ts:905-960. Not launched when recorded: if the first use of the sum is a norm (every residual
@@ -1056,19 +1188,19 @@ class CudaBackend:
             return self._elementwise("add", a, b, 0.0)
         self._beginForwardOp(keepPending=True)
         ea, eb = self._entryFor(a), self._entryFor(b)
-        out = Tensor.zeros(a.shape)
-        out._prev = [a, b]
+        out = Tensor.output(list(a.shape), a.size, [a, b])
+        out._needs = self._flows(a, ea) or self._flows(b, eb)
         self._pendingAdd[id(out)] = (out, a, b)
         n = a.size
 
         def _bw():
-            eo = self._entries.get(out)
+            eo = self._find(out)
             if eo is None:
                 return          # never used by anything: no gradient reaches it
             self._ensureBackwardBegun()
             go = self._gradSource(eo)
             for t, e, first in ((a, ea, True), (b, eb, False)):
-                if e.grad == 0 or (e.external and not t.requiresGrad):
+                if not self._flows(t, e):
                     continue
                 if e.pendingDx is not None:
                     self._flushDx(e)
@@ -1080,20 +1212,13 @@ class CudaBackend:
                     e.copyFrom = go
                     self._pendingCopy[id(e)] = e
 
-        out._backward = _bw
-        return out
-
-    def _newEntry(self, t: Tensor) -> _Entry:
-        nbytes = t.size * 4
-        e = _Entry(self._acquireRecycled(nbytes), self._acquireRecycled(nbytes), nbytes, False, t.size)
-        self._entries[t] = e
-        return e
+        return self._record(out, out._needs, _bw)
 
     def _materializeAdd(self, t: Tensor) -> _Entry:
         _t, a, b = self._pendingAdd.pop(id(t))
-        ea, eb = self._entries[a], self._entries[b]
+        ea, eb = self._find(a), self._find(b)
         self._flushFwd()
-        e = self._newEntry(t)
+        e = self._newEntry(t, t._needs)
         self._check(self.lib.gt_ew_fwd(self.ctx, _EW["add"], t.size, ea.data, eb.data, 0.0, e.data))
         return e
 
@@ -1117,15 +1242,15 @@ class CudaBackend:
         if not self.fuseGatedUnits:
             return self._elementwise(op, x, None, 0.0)
         self._beginForwardOp(keepPending=True)
-        e0 = self._entries.get(x)
+        e0 = self._find(x)
         if e0 is None or not e0.pendingFwd:      # (a projection still waiting to be launched stays waiting: see _gatedUnit)
-            self._entryFor(x)
-        t = Tensor.zeros(x.shape)
-        t._prev = [x]
+            e0 = self._entryFor(x)
+        t = Tensor.output(list(x.shape), x.size, [x])
+        t._needs = self._flows(x, e0)
         self._pendingAct[id(t)] = (t, _EW[op], x)
 
         def _bw():
-            e = self._entries.get(t)
+            e = self._find(t)
             if e is None or not (e.gradLive or e.copyFrom or e.pendingDx is not None):
                 return          # consumed only by fused products, which sent their gradient straight to x
             self._ensureBackwardBegun()
@@ -1134,18 +1259,15 @@ class CudaBackend:
             gx, ax = self._gradTarget(x, ex)
             self._check(self.lib.gt_ew_bwd(self.ctx, _EW[op], x.size, ex.data, 0, 0.0, go, gx, ax, 0, 0))
 
-        t._backward = _bw
-        return t
+        return self._record(t, t._needs, _bw)
 
     def _materializeAct(self, t: Tensor) -> _Entry:
         _t, code, x = self._pendingAct.pop(id(t))
-        ex = self._entries[x]
+        ex = self._find(x)
         self._flushFwd()
         if ex.lazy is not None:
             self._materializeLazy(ex)
-        nbytes = t.size * 4
-        e = _Entry(self._acquireRecycled(nbytes), self._acquireRecycled(nbytes), nbytes, False, t.size)
-        self._entries[t] = e
+        e = self._newEntry(t, t._needs)
         self._check(self.lib.gt_ew_fwd(self.ctx, code, t.size, ex.data, 0, 0.0, e.data))
         return e
 
@@ -1162,7 +1284,7 @@ class CudaBackend:
     def _gatedUnit(self, act: Tensor, u: Tensor) -> Tensor:
         _t, code, x = self._pendingAct[id(act)]
         self._beginForwardOp(keepPending=True)
-        ex, eu = self._entries[x], self._entries.get(u)
+        ex, eu = self._find(x), self._find(u)
         pend = self._pendingFwd
         if (eu is not None and len(pend) == 2 and ex.pendingFwd and eu.pendingFwd and ex is not eu
                 and {id(pend[0]["eo"]), id(pend[1]["eo"])} == {id(ex), id(eu)} and pend[0]["outDim"] == pend[1]["outDim"]
@@ -1171,7 +1293,8 @@ class CudaBackend:
             pg, pu = (pend[0], pend[1]) if pend[0]["eo"] is ex else (pend[1], pend[0])
             self._pendingFwd = []
             ex.pendingFwd = eu.pendingFwd = False
-            out, eo = self._makeOut(act.shape, [act, u])
+            needs = self._flows(x, ex) or self._flows(u, eu)
+            out, eo = self._makeOut(list(act.shape), act.size, [act, u], needs)
             self._check(self.lib.gt_glu_linear_fwd(self.ctx, code, pg["T"], pg["outDim"], pg["inDim"], pg["ex"].data, pg["ew"].data,
                                                    pu["ew"].data, ex.data, eu.data, eo.data))
         else:
@@ -1179,7 +1302,8 @@ class CudaBackend:
             if ex.lazy is not None:
                 self._materializeLazy(ex)
             eu = self._entryFor(u)
-            out, eo = self._makeOut(act.shape, [act, u])
+            needs = self._flows(x, ex) or self._flows(u, eu)
+            out, eo = self._makeOut(list(act.shape), act.size, [act, u], needs)
             self._check(self.lib.gt_glu_fwd(self.ctx, code, act.size, ex.data, eu.data, eo.data))
         n = act.size
 
@@ -1194,8 +1318,7 @@ class CudaBackend:
             else:
                 self._check(self.lib.gt_glu_bwd(self.ctx, code, n, ex.data, eu.data, go, gx, ax, gu, au))
 
-        out._backward = _bw
-        return out
+        return self._record(out, needs, _bw)
 
     def scale(self, x, c):
         return self._elementwise("scale", x, None, float(c))
@@ -1204,17 +1327,19 @@ class CudaBackend:
         """webgpu.ts:1673-1701. `heads` = (T, H): a per-head norm that may wait for the rotary embedding after it."""
         self._beginForwardOp(keepPending=heads is not None)
         ew = self._entryFor(w)
-        if id(x) in self._pendingAdd and x not in self._entries:
+        if id(x) in self._pendingAdd and self._find(x) is None:
             # x = a + b has not been launched and this norm is its first use: one kernel writes both
             _t, a, b = self._pendingAdd.pop(id(x))
-            ea, eb = self._entries[a], self._entries[b]
-            ex = self._newEntry(x)
-            out, eo = self._makeOut(shape, [x, w])
+            ea, eb = self._find(a), self._find(b)
+            ex = self._newEntry(x, x._needs)
+            needs = self._flows(x, ex) or self._flows(w, ew)
+            out, eo = self._makeOut(shape, x.size, [x, w], needs)
             rinv = self._acquireRecycled(rows * 4)
             self._check(self.lib.gt_add_rmsnorm_fwd(self.ctx, rows, d, ea.data, eb.data, ew.data, eps, ex.data, eo.data, rinv))
         else:
             ex = self._entryFor(x)
-            out, eo = self._makeOut(shape, [x, w])
+            needs = self._flows(x, ex) or self._flows(w, ew)
+            out, eo = self._makeOut(shape, x.size, [x, w], needs)
             rinv = self._acquireRecycled(rows * 4)
             if heads is not None:
                 self._deferHeadNorm(ex, ew, eo, rinv, heads[0], heads[1], d, eps)
@@ -1224,30 +1349,29 @@ class CudaBackend:
         def _bw():
             self._ensureBackwardBegun()
             go = self._gradSource(eo)
-            wantX = bool(ex.grad) and not (ex.external and not x.requiresGrad)
+            wantX = self._flows(x, ex)
             if wantX and ex.pendingDx is not None:
                 self._flushDx(ex)
-            gw, aw = self._gradTarget(w, ew) if w.requiresGrad else (0, 0)
+            gw, aw = self._gradTarget(w, ew)
             if wantX and ex.copyFrom and not ex.gradLive:
                 # the gradient so far is an `add`'s upstream buffer: dx = that buffer + this term, written in one pass
                 gadd = ex.copyFrom
                 ex.copyFrom = 0
                 self._pendingCopy.pop(id(ex), None)
                 ex.gradLive = True
-                self._check(self.lib.gt_rmsnorm_bwd_add(self.ctx, rows, d, ex.data, ew.data, rinv, go, gadd, ex.grad, gw, aw))
+                self._check(self.lib.gt_rmsnorm_bwd_add(self.ctx, rows, d, ex.data, ew.data, rinv, go, gadd, self._gradAddr(ex), gw, aw))
                 return
             gx, ax = self._gradTarget(x, ex)
             self._check(self.lib.gt_rmsnorm_bwd(self.ctx, rows, d, ex.data, ew.data, rinv, go, gx, ax, gw, aw))
 
-        out._backward = _bw
-        return out
+        return self._record(out, needs, _bw)
 
     def rmsNorm(self, x, weight, eps):
         T, d = x.shape
         return self._rmsNormRows(x, weight, T, d, eps, [T, d])
 
     def rmsNormHeads(self, x, weight, T, H, hd, eps):
-        wait = self.fuseRope and hd in (64, 128, 256) and not (id(x) in self._pendingAdd and x not in self._entries)
+        wait = self.fuseRope and hd in (64, 128, 256) and not (id(x) in self._pendingAdd and self._find(x) is None)
         return self._rmsNormRows(x, weight, T * H, hd, eps, [T, H * hd], heads=(T, H) if wait else None)
 
     def embedding(self, weight: Tensor, ids) -> Tensor:
@@ -1257,7 +1381,8 @@ class CudaBackend:
         T = len(ids)
         ew = self._entryFor(weight)
         idBuf = self._uploadU32(ids, "ids", weight.shape[0])
-        out, eo = self._makeOut([T, d], [weight])
+        needs = self._flows(weight, ew)
+        out, eo = self._makeOut([T, d], T * d, [weight], needs)
         self._check(self.lib.gt_embedding_fwd(self.ctx, T, d, ew.data, idBuf, eo.data))
 
         def _bw():
@@ -1277,8 +1402,7 @@ class CudaBackend:
                 ew.gradLive = True
             self._check(self.lib.gt_embedding_bwd(self.ctx, T, d, go, idBuf, ew.grad))
 
-        out._backward = _bw
-        return out
+        return self._record(out, needs, _bw)
 
     def _checkT(self, T: int, rows: int, where: str):
         b, sl = self._batch
@@ -1294,7 +1418,7 @@ class CudaBackend:
         Gemma 3 blocks), by the norm's pass (gt_rmsnorm_heads_rope_fwd). No pass of its own runs in either case; the
         gradient side is in `attention`."""
         self._checkT(T, x.shape[0], "rope")
-        e0 = self._entries.get(x)
+        e0 = self._find(x)
         part = None
         if self.fuseRope and e0 is not None and e0.pendingFwd:
             part = next((p for p in self._pendingFwd if p["eo"] is e0), None)
@@ -1311,15 +1435,18 @@ class CudaBackend:
         if part is not None:
             self._beginForwardOp(keepPending=True)
             ex = e0
-            out, eo = self._makeOut([T, H * hd], [x])
+            needs = self._flows(x, ex)
+            out, eo = self._makeOut([T, H * hd], T * H * hd, [x], needs)
             part["rope"] = (eo, H, hd, base, posOffset)
             eo.pendingFwd = True
         else:
             self._beginForwardOp()
             ex = self._entryFor(x)
-            out, eo = self._makeOut([T, H * hd], [x])
+            needs = self._flows(x, ex)
+            out, eo = self._makeOut([T, H * hd], T * H * hd, [x], needs)
             self._check(self.lib.gt_rope_fwd(self.ctx, T, H, hd, float(base), posOffset, ex.data, eo.data))
-        eo.ropeOf = (x, ex, H, hd, base, posOffset)
+        if needs:
+            eo.ropeOf = (x, ex, H, hd, base, posOffset)
 
         def _bw():
             self._ensureBackwardBegun()
@@ -1329,26 +1456,26 @@ class CudaBackend:
             gx, ax = self._gradTarget(x, ex)
             self._check(self.lib.gt_rope_bwd(self.ctx, T, H, hd, float(base), posOffset, go, gx, ax))
 
-        out._backward = _bw
-        return out
+        return self._record(out, needs, _bw)
 
     def attention(self, q: Tensor, k: Tensor, v: Tensor, T: int, Hq: int, Hkv: int, hd: int, window: int) -> Tensor:
         """webgpu.ts:1125-1192."""
         self._beginForwardOp()
         self._checkT(T, q.shape[0], "attention")
         eq, ek, ev = self._entryFor(q), self._entryFor(k), self._entryFor(v)
+        needs = self._flows(q, eq) or self._flows(k, ek) or self._flows(v, ev)
         rec = self._curRec
         nbytes = T * Hq * hd * 4
         if rec is not None and rec["replay"] and rec["pos"] < len(rec["saved"]) and rec["saved"][rec["pos"]][2] == nbytes:
             # replay of a recompute region: the first run's output and row statistics, no launch
             data, lse, _n = rec["saved"][rec["pos"]]
             rec["pos"] += 1
-            out = Tensor.zeros([T, Hq * hd])
-            out._prev = [q, k, v]
-            eo = _Entry(data, self._acquireRecycled(nbytes), nbytes, False, out.size)
-            self._entries[out] = eo
+            out = Tensor.output([T, Hq * hd], T * Hq * hd, [q, k, v])
+            eo = _Entry(self._uid, data, 0, nbytes, False, out.size)
+            eo.needs, eo.region = needs, self._regionStack[-1][0]
+            out._needs, out._dev = needs, eo
         else:
-            out, eo = self._makeOut([T, Hq * hd], [q, k, v])
+            out, eo = self._makeOut([T, Hq * hd], T * Hq * hd, [q, k, v], needs)
             lse = self._acquireRecycled(Hq * T * 4)
             self._check(self.lib.gt_attention_fwd(self.ctx, T, Hq, Hkv, hd, window, eq.data, ek.data, ev.data, eo.data, lse))
             if rec is not None and not rec["replay"]:
@@ -1377,19 +1504,19 @@ class CudaBackend:
             self._check(self.lib.gt_attention_bwd(self.ctx, T, Hq, Hkv, hd, window, eq.data, ek.data, ev.data, eo.data,
                                                   lse, go, gq, aq, gk, ak, gv, av))
 
-        out._backward = _bw
-        return out
+        return self._record(out, needs, _bw)
 
     def _nseq(self) -> int:
         return self._batch[0] if self._batch[0] else 1
 
-    def _lossOut(self, prev):
+    def _lossOut(self, prev, needs: bool):
         """The scalar loss tensor plus its device-side companions: [1+nseq] losses and [nseq] 1/kept."""
         nseq = self._nseq()
-        loss = Tensor.zeros([1])
-        loss._prev = list(prev)
-        e = _Entry(self._acquireRecycled((1 + nseq) * 4), self._acquireRecycled(4), 4, False, 1)
-        self._entries[loss] = e
+        loss = Tensor.output([1], 1, list(prev))
+        e = _Entry(self._uid, self._acquireRecycled((1 + nseq) * 4), 0, 4, False, 1)
+        e.needs = loss._needs = needs
+        e.region = self._regionStack[-1][0] if self._regionStack else 0
+        loss._dev = e
         invKept = self._acquireRecycled(nseq * 4)
         return loss, e, invKept
 
@@ -1400,7 +1527,7 @@ class CudaBackend:
         if self._capturing:
             return self._seedBuf
         if not e.gradLive:
-            self._write(e.grad, loss.grad[:1])
+            self._write(self._gradAddr(e), loss.grad[:1])
             e.gradLive = True
         return e.grad
 
@@ -1412,7 +1539,8 @@ class CudaBackend:
         el = self._entryFor(logits)
         tgt = self._uploadU32(targets, "targets", V)
         stats = self._acquireRecycled(T * 16)
-        loss, eo, invKept = self._lossOut([logits])
+        needs = self._flows(logits, el)
+        loss, eo, invKept = self._lossOut([logits], needs)
         self._check(self.lib.gt_ce_fwd(self.ctx, T, V, el.data, tgt, stats, eo.data, invKept))
 
         def _bw():
@@ -1421,8 +1549,7 @@ class CudaBackend:
             gl, al = self._gradTarget(logits, el)
             self._check(self.lib.gt_ce_bwd(self.ctx, T, V, el.data, tgt, stats, invKept, seed, gl, al))
 
-        loss._backward = _bw
-        return loss
+        return self._record(loss, needs, _bw)
 
     def fusedCrossEntropy(self, hidden: Tensor, w: Tensor, targets, chunk: int, kept: int) -> Tensor:
         """webgpu.ts:1214-1278: per vocab span, logits = hidden·W[span]ᵀ then online (max, sum, target
@@ -1435,7 +1562,8 @@ class CudaBackend:
         run = self._acquireRecycled(T * 12)
         width = min(chunk, V)
         ch = self._acquireRecycled(T * width * 4)
-        loss, eo, invKept = self._lossOut([hidden, w])
+        needs = self._flows(hidden, eh) or self._flows(w, ew)
+        loss, eo, invKept = self._lossOut([hidden, w], needs)
         for v0 in range(0, V, chunk):
             n = min(chunk, V - v0)
             self._gemm("NT", 0, T, n, H, eh.data, ew.data + v0 * H * 4, ch)
@@ -1446,7 +1574,7 @@ class CudaBackend:
             self._ensureBackwardBegun()
             seed = self._lossGrad(loss, eo)
             gh, ah = self._gradTarget(hidden, eh)
-            gw, aw = self._gradTarget(w, ew) if w.requiresGrad else (0, 0)
+            gw, aw = self._gradTarget(w, ew)
             for v0 in range(0, V, chunk):
                 n = min(chunk, V - v0)
                 self._gemm("NT", 0, T, n, H, eh.data, ew.data + v0 * H * 4, ch)
@@ -1458,8 +1586,7 @@ class CudaBackend:
                     # rows [v0, v0+n) of dW; each span is written by exactly one product
                     self._gemm("TN", aw, n, H, T, ch, eh.data, gw + v0 * H * 4)
 
-        loss._backward = _bw
-        return loss
+        return self._record(loss, needs, _bw)
 
     def softCrossEntropy(self, logits: Tensor, teacherIds, teacherProbs, k: int, kept: int) -> Tensor:
         """webgpu.ts:1331-1378."""
@@ -1469,7 +1596,8 @@ class CudaBackend:
         ids = self._uploadU32(teacherIds, "teacher", V)
         probs = self._uploadF32(teacherProbs)
         stats = self._acquireRecycled(T * 16)
-        loss, eo, invKept = self._lossOut([logits])
+        needs = self._flows(logits, el)
+        loss, eo, invKept = self._lossOut([logits], needs)
         self._check(self.lib.gt_soft_ce_fwd(self.ctx, T, V, k, el.data, ids, probs, stats, eo.data, invKept))
 
         def _bw():
@@ -1478,8 +1606,7 @@ class CudaBackend:
             gl, al = self._gradTarget(logits, el)
             self._check(self.lib.gt_soft_ce_bwd(self.ctx, T, V, k, el.data, ids, probs, stats, invKept, seed, gl, al))
 
-        loss._backward = _bw
-        return loss
+        return self._record(loss, needs, _bw)
 
     # ------------------------------------------------------------------ per-sequence losses of a batched call
     def sequenceLosses(self, loss: Tensor) -> np.ndarray:

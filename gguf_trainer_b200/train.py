@@ -7,6 +7,7 @@ draws the same windows in both loops.
 """
 from __future__ import annotations
 
+import gc
 import math
 import time
 from typing import Callable, Dict, List, Optional, Sequence
@@ -61,8 +62,16 @@ def trainLMGpuResident(model, gpu: CudaBackend, tokens: np.ndarray, seqLen: int,
         for L in (qk["pairs"] if qk else []):
             normTensors.extend([L["qNorm"], L["kNorm"]])
     gpu.install()
+    # The tape of a micro-batch is thousands of objects that all die by reference count when the backend drops it, but while
+    # they live they trip the cycle collector into full passes over everything the process has loaded (150 ms each beside a
+    # deep-learning library, every third call of a 30-layer model). So it runs between steps here: the young generations
+    # after every step, everything after every hundredth.
+    collect = gc.isenabled()
+    gc.disable()
     try:
         for step in range(steps):
+            if collect and step:
+                gc.collect(2 if step % 100 == 0 else 1)
             t0 = time.perf_counter()
             if schedule:
                 optimizer.setLrScale(schedule(step))
@@ -102,6 +111,8 @@ def trainLMGpuResident(model, gpu: CudaBackend, tokens: np.ndarray, seqLen: int,
                 lastCheckpointAt = time.perf_counter()
     finally:
         gpu.uninstall()
+        if collect:
+            gc.enable()
     optimizer.syncWeightsToHost()
     return history
 
