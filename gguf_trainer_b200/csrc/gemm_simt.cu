@@ -1,132 +1,337 @@
 // Strict-f32 matrix product: f32 loads, FFMA, f32 accumulate. This is the precision mode whose results
 // must stay within 1e-5 relative L2 of the reference's f64-accumulating loops (src/model/autograd.ts:348-377);
 // the tensor-core path lives in gemm_tc.cu. Covers the three operand layouts of WebGPUBackend.gemm
-// (src/backend/webgpu.ts:1654-1671) with ragged edges in every dimension.
+// (src/backend/webgpu.ts:1654-1671) with ragged edges in every dimension, sums of products written once and groups of
+// independent products in one launch.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 16, TM = 8, TN = 8, PAD = 4;
+// Tile of a CTA: BM x BN outputs, BK deep per stage, TM x TN outputs per thread (as 4-row and 4-column strips, so that a
+// warp's shared-memory reads are 16-byte, conflict-free or broadcast).
+// What bounds it is the FMA pipe (128 per clock and SM) and, below a few hundred tiles, the number of SMs at work.
+//  * 128 x 128: 64 FMAs per four 16-byte shared-memory reads and thread; for products whose tiles fill the SMs.
+//  * 64 x 64: a quarter of the tile, for everything else; the contraction is cut over a cluster of up to 8 CTAs, which add
+//    their tiles through distributed shared memory in rank order (no atomics, no scratch, the same bits on every run).
+// Both keep one stage in registers on its way from global memory while the stage before it is multiplied, and write
+// shared memory double-buffered: one barrier per stage. Two FMAs issue as one packed instruction (fma.rn.f32x2): the same
+// IEEE operations at half the issue slots.
+template <int BM_, int BN_, int BK_, int TM_, int TN_>
+struct Tile {
+  static constexpr int BM = BM_, BN = BN_, BK = BK_, TM = TM_, TN = TN_;
+  static constexpr int THREADS = (BM / TM) * (BN / TN);
+  static constexpr int STAGE = BK * (BM + BN);
+  static constexpr int SMEM = (2 * STAGE > BM * BN ? 2 * STAGE : BM * BN) * 4;   // (the reduction reuses it for a whole tile)
+  static constexpr int QA = BM * BK / 4 / THREADS, QB = BN * BK / 4 / THREADS;   // 16-byte loads per thread and stage
+};
+using Big = Tile<128, 128, 16, 8, 8>;
+using Small = Tile<64, 64, 32, 8, 4>;
 
-// Element (m,k) of A is a[m*sam + k*sak]; element (n,k) of B is b[n*sbn + k*sbk].
-template <bool A_KCONTIG, bool B_KCONTIG>
-__global__ void __launch_bounds__(256) gemm_f32_kernel(int M, int N, int K, const float* __restrict__ a, long sam, long sak,
-                                                       const float* __restrict__ b, long sbn, long sbk,
-                                                       float* __restrict__ c, int accum, int ksplit, float alpha,
-                                                       float* __restrict__ part) {
-  __shared__ __align__(16) float As[BK][BM + PAD];
-  __shared__ __align__(16) float Bs[BK][BN + PAD];
-  const int tid = threadIdx.x;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int tx = tid % 16, ty = tid / 16;
-  // split-K: slice z covers k in [kb, ke)
-  const int kper = ((K + ksplit - 1) / ksplit + BK - 1) / BK * BK;
-  const int kb = blockIdx.z * kper;
-  const int ke = min(K, kb + kper);
+// Stages are [BK][R] with column r of row k at r ^ swz(k): an operand that is contiguous along K is transposed on its way
+// into shared memory, and with this the 32 lanes of a warp, which hold four rows' worth of k for 128 / BK columns,
+// store to 32 different banks; quads of columns stay together, so reads are 16-byte loads as before.
+template <int BK>
+__device__ __forceinline__ constexpr int swz(int k) { return ((k / 4) % (BK / 4)) * (128 / BK); }
 
-  float acc[TM][TN];
+constexpr int MAX_PARTS = 8;
+struct F32Args {
+  const float* a[MAX_PARTS];
+  const float* b[MAX_PARTS];
+  float* c[MAX_PARTS];
+  int K[MAX_PARTS];
+  int M[MAX_PARTS], N[MAX_PARTS], accum[MAX_PARTS];
+  int tile_end[MAX_PARTS];   // grouped: group g owns tiles [tile_end[g-1], tile_end[g])
+  int nparts, ngroups;       // one of the two is 1: products summed into c[0], or independent products of one K
+  float alpha;
+};
+
+// a quad of four consecutive floats along the contiguous axis, zero outside [0, n) x [0, m)
+template <bool VEC>
+__device__ __forceinline__ float4 quad(const float* __restrict__ p, long row, int ld, int i, int n, bool row_ok) {
+  if (!row_ok || i >= n) return make_float4(0.f, 0.f, 0.f, 0.f);
+  const float* s = p + row * ld + i;
+  if (VEC) return __ldg(reinterpret_cast<const float4*>(s));   // (n is a multiple of 4: the whole quad is inside)
+  float4 v = make_float4(__ldg(s), 0.f, 0.f, 0.f);
+  if (i + 1 < n) v.y = __ldg(s + 1);
+  if (i + 2 < n) v.z = __ldg(s + 2);
+  if (i + 3 < n) v.w = __ldg(s + 3);
+  return v;
+}
+
+// One operand's stage in registers: R rows (the M or N extent) x BK. KC: the operand is [R, K] with K contiguous, else [K, R].
+template <int R, int BK, int Q, int THREADS, bool KC, bool VEC>
+struct Operand {
+  float4 v[Q];
+  __device__ __forceinline__ void load(const float* __restrict__ p, int rows, int K, int r0, int k0) {
+#pragma unroll
+    for (int i = 0; i < Q; i++) {
+      const int idx = threadIdx.x + i * THREADS;
+      if (KC) {
+        const int kq = idx % (BK / 4), r = idx / (BK / 4);
+        v[i] = quad<VEC>(p, r0 + r, K, k0 + kq * 4, K, r0 + r < rows);
+      } else {
+        const int rq = idx % (R / 4), k = idx / (R / 4);
+        v[i] = quad<VEC>(p, k0 + k, rows, r0 + rq * 4, rows, k0 + k < K);
+      }
+    }
+  }
+  __device__ __forceinline__ void store(float* s) const {
+#pragma unroll
+    for (int i = 0; i < Q; i++) {
+      const int idx = threadIdx.x + i * THREADS;
+      if (KC) {
+        const int kq = idx % (BK / 4), r = idx / (BK / 4);
+        float* d = s + kq * 4 * R + (r ^ swz<BK>(kq * 4));
+        d[0] = v[i].x; d[R] = v[i].y; d[2 * R] = v[i].z; d[3 * R] = v[i].w;
+      } else {
+        const int rq = idx % (R / 4), k = idx / (R / 4);
+        *reinterpret_cast<float4*>(s + k * R + ((rq * 4) ^ swz<BK>(k))) = v[i];
+      }
+    }
+  }
+};
+
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+// gridDim.x = tiles x ksplit, the ksplit CTAs of a tile adjacent and, when there are several, one cluster.
+template <class T, bool A_K, bool B_K, bool VEC>
+__global__ void __launch_bounds__(T::THREADS) gemm_f32_kernel(const __grid_constant__ F32Args p, int ksplit) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int BM = T::BM, BN = T::BN, BK = T::BK, TM = T::TM, TN = T::TN;
+  constexpr int TX = BN / TN, TY = BM / TM;
+  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+  const int z = blockIdx.x % ksplit;
+  int t = blockIdx.x / ksplit, g = 0;
+  if (p.ngroups > 1) {
+    while (t >= p.tile_end[g]) g++;
+    if (g) t -= p.tile_end[g - 1];
+  }
+  const int M = p.M[g], N = p.N[g];
+  const int tn = (N + BN - 1) / BN, n0 = (t % tn) * BN, m0 = (t / tn) * BM;
+  int kblocks = 0;
+  for (int i = 0; i < p.nparts; i++) kblocks += (p.K[g + i] + BK - 1) / BK;
+  const int per = (kblocks + ksplit - 1) / ksplit;
+  const int kb0 = min(kblocks, z * per), kb1 = min(kblocks, kb0 + per);
+
+  unsigned long long acc[TM][TN / 2];
 #pragma unroll
   for (int i = 0; i < TM; i++)
 #pragma unroll
-    for (int j = 0; j < TN; j++) acc[i][j] = 0.f;
+    for (int j = 0; j < TN / 2; j++) acc[i][j] = 0ull;
 
-  for (int k0 = kb; k0 < ke; k0 += BK) {
-#pragma unroll
-    for (int i = 0; i < (BM * BK) / 256; i++) {
-      int idx = tid + i * 256;
-      int mm, kk;
-      if (A_KCONTIG) { kk = idx % BK; mm = idx / BK; } else { mm = idx % BM; kk = idx / BM; }
-      int gm = m0 + mm, gk = k0 + kk;
-      As[kk][mm] = (gm < M && gk < ke) ? a[(long)gm * sam + (long)gk * sak] : 0.f;
-    }
-#pragma unroll
-    for (int i = 0; i < (BN * BK) / 256; i++) {
-      int idx = tid + i * 256;
-      int nn, kk;
-      if (B_KCONTIG) { kk = idx % BK; nn = idx / BK; } else { nn = idx % BN; kk = idx / BN; }
-      int gn = n0 + nn, gk = k0 + kk;
-      Bs[kk][nn] = (gn < N && gk < ke) ? b[(long)gn * sbn + (long)gk * sbk] : 0.f;
-    }
-    __syncthreads();
+  Operand<BM, BK, T::QA, T::THREADS, A_K, VEC> oa;
+  Operand<BN, BK, T::QB, T::THREADS, B_K, VEC> ob;
+  // K block kb lies in product `part`, from its row k0 on
+  int part = g, k0 = kb0 * BK;
+  while (part < g + p.nparts - 1 && k0 >= (p.K[part] + BK - 1) / BK * BK) { k0 -= (p.K[part] + BK - 1) / BK * BK; part++; }
+  auto fetch = [&] {
+    oa.load(p.a[part], M, p.K[part], m0, k0);
+    ob.load(p.b[part], N, p.K[part], n0, k0);
+    k0 += BK;
+    if (k0 >= p.K[part] && part < g + p.nparts - 1) { k0 = 0; part++; }
+  };
+  if (kb0 < kb1) {
+    fetch();
+    oa.store(sm); ob.store(sm + BK * BM);
+  }
+  __syncthreads();
+  for (int kb = kb0; kb < kb1; kb++) {
+    const float* As = sm + ((kb - kb0) & 1) * T::STAGE;
+    const float* Bs = As + BK * BM;
+    if (kb + 1 < kb1) fetch();
 #pragma unroll
     for (int kk = 0; kk < BK; kk++) {
-      float av[TM], bv[TN];
-      // two float4 per operand: rows ty*4..+3 and 64+ty*4..+3 (same for columns)
-      *(float4*)&av[0] = *(const float4*)&As[kk][ty * 4];
-      *(float4*)&av[4] = *(const float4*)&As[kk][64 + ty * 4];
-      *(float4*)&bv[0] = *(const float4*)&Bs[kk][tx * 4];
-      *(float4*)&bv[4] = *(const float4*)&Bs[kk][64 + tx * 4];
+      float av[TM];
+      unsigned long long bv[TN / 2];
 #pragma unroll
-      for (int i = 0; i < TM; i++)
+      for (int i = 0; i < TM / 4; i++) *reinterpret_cast<float4*>(&av[4 * i]) = *reinterpret_cast<const float4*>(As + kk * BM + ((i * (4 * TY) + ty * 4) ^ swz<BK>(kk)));
 #pragma unroll
-        for (int j = 0; j < TN; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+      for (int j = 0; j < TN / 4; j++) {
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(Bs + kk * BN + ((j * (4 * TX) + tx * 4) ^ swz<BK>(kk)));
+        bv[2 * j] = w.x; bv[2 * j + 1] = w.y;
+      }
+#pragma unroll
+      for (int i = 0; i < TM; i++) {
+        const unsigned long long aa = pack2(av[i], av[i]);
+#pragma unroll
+        for (int j = 0; j < TN / 2; j++) fma2(acc[i][j], aa, bv[j]);
+      }
+    }
+    if (kb + 1 < kb1) {
+      float* d = sm + ((kb + 1 - kb0) & 1) * T::STAGE;
+      oa.store(d); ob.store(d + BK * BM);
     }
     __syncthreads();
   }
 
-#pragma unroll
-  for (int i = 0; i < TM; i++) {
-    int gm = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < TN; j++) {
-      int gn = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4);
-      if (gn >= N) continue;
-      float* dst = c + (long)gm * N + gn;
-      const float v = acc[i][j] * alpha;
-      if (ksplit > 1) part[((size_t)blockIdx.z * M + gm) * N + gn] = v;   // summed in slice order by splitk_sum_kernel
-      else *dst = accum ? *dst + v : v;
+  float* C = p.c[g];
+  const int accum = p.accum[g];
+  const bool vecC = (N & 3) == 0 && (((uintptr_t)C) & 15) == 0;
+  auto put = [&](int m, int n, float4 v) {     // four outputs of a row
+    if (m >= M || n >= N) return;
+    float* d = C + (long)m * N + n;
+    v.x *= p.alpha; v.y *= p.alpha; v.z *= p.alpha; v.w *= p.alpha;
+    if (vecC) {
+      if (accum) { const float4 o = *reinterpret_cast<const float4*>(d); v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w; }
+      *reinterpret_cast<float4*>(d) = v;
+      return;
     }
+    d[0] = accum ? d[0] + v.x : v.x;
+    if (n + 1 < N) d[1] = accum ? d[1] + v.y : v.y;
+    if (n + 2 < N) d[2] = accum ? d[2] + v.z : v.z;
+    if (n + 3 < N) d[3] = accum ? d[3] + v.w : v.w;
+  };
+  if (ksplit == 1) {
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+      for (int j = 0; j < TN / 4; j++) {
+        const float2 u = unpack2(acc[i][2 * j]), w = unpack2(acc[i][2 * j + 1]);
+        put(m0 + (i / 4) * (4 * TY) + ty * 4 + i % 4, n0 + j * (4 * TX) + tx * 4, make_float4(u.x, u.y, w.x, w.y));
+      }
+    return;
   }
+  // the cluster's slices: every CTA leaves its tile in shared memory and adds up its share of the rows over all of them
+#pragma unroll
+  for (int i = 0; i < TM; i++)
+#pragma unroll
+    for (int j = 0; j < TN / 4; j++) {
+      const float2 u = unpack2(acc[i][2 * j]), w = unpack2(acc[i][2 * j + 1]);
+      *reinterpret_cast<float4*>(sm + ((i / 4) * (4 * TY) + ty * 4 + i % 4) * BN + j * (4 * TX) + tx * 4) = make_float4(u.x, u.y, w.x, w.y);
+    }
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  for (int q = z * T::THREADS + tid; q < BM * BN / 4; q += ksplit * T::THREADS) {
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r = 0; r < ksplit; r++) {
+      const float4 v = *(reinterpret_cast<const float4*>(cluster.map_shared_rank(sm, r)) + q);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    put(m0 + q / (BN / 4), n0 + (q % (BN / 4)) * 4, s);
+  }
+  cluster.sync();      // (nobody leaves while its tile may still be read)
 }
 
-// c (+)= part[0] + part[1] + ... in slice order: split-K without atomics, the same bits on every run
-__global__ void splitk_sum_kernel(long n, int ksplit, const float* __restrict__ part, float* __restrict__ c, int accum) {
-  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    float acc = accum ? c[i] : 0.f;
-    for (int z = 0; z < ksplit; z++) acc += part[(size_t)z * n + i];
-    c[i] = acc;
+template <class T, bool A_K, bool B_K, bool VEC>
+gt_status launch(gt_ctx* ctx, const F32Args& p, long tiles, int ksplit) {
+  auto kern = gemm_f32_kernel<T, A_K, B_K, VEC>;
+  static bool attr_set[64] = {};
+  if (ctx->device >= 0 && ctx->device < 64 && !attr_set[ctx->device]) {
+    GT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM));
+    attr_set[ctx->device] = true;
   }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * ksplit), 1, 1);
+  cfg.blockDim = dim3(T::THREADS, 1, 1);
+  cfg.dynamicSmemBytes = T::SMEM;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ksplit;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = ksplit > 1 ? 1 : 0;
+  GT_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, p, ksplit));
+  GT_LAUNCHED(ctx, "gemm_f32_kernel");
+  return GT_OK;
 }
+
+template <class T, bool VEC>
+gt_status launch_kind(gt_ctx* ctx, int kind, const F32Args& p, long tiles, int ksplit) {
+  if (kind == GT_GEMM_NT) return launch<T, true, true, VEC>(ctx, p, tiles, ksplit);
+  if (kind == GT_GEMM_NN) return launch<T, true, false, VEC>(ctx, p, tiles, ksplit);
+  return launch<T, false, false, VEC>(ctx, p, tiles, ksplit);
+}
+
+template <class T>
+long tiles_of(F32Args& p) {
+  long n = 0;
+  for (int g = 0; g < p.ngroups; g++) {
+    n += (long)gt_cdiv(p.M[g], T::BM) * gt_cdiv(p.N[g], T::BN);
+    p.tile_end[g] = (int)n;
+  }
+  return n;
+}
+
+// Tile and slices by predicted cycles of the SM with the most work: CTAs there x K rows each x cycles per K row, plus what
+// a CTA costs whatever its depth. A K row of a tile is BM x BN / 128 cycles of the FMA pipe, of which resident CTAs
+// together reach about 0.8, and a 64 x 64 CTA that has an SM to itself (four warps) about half.
+template <class T>
+double cost_of(gt_ctx* ctx, const F32Args& p, long tiles, int ksplit) {
+  double rows = 0;
+  for (int i = 0; i < p.nparts; i++) rows += gt_cdiv(p.K[i], T::BK) * T::BK;
+  const double per = gt_cdiv((long)rows / T::BK, ksplit) * T::BK;
+  const double ctas = gt_cdiv(tiles * ksplit, ctx->sm_count);
+  const double row = T::BM * T::BN / 128.0;
+  const double busy = ctas * row / 0.8, alone = row / (T::THREADS >= 256 ? 0.7 : 0.5);
+  return per * (busy > alone ? busy : alone) + 2200.0 + (ksplit > 1 ? 1200.0 + 250.0 * ksplit : 0.0) + 400.0 * (ctas - 1);
+}
+
+gt_status run(gt_ctx* ctx, int kind, F32Args& p) {
+  bool vec = true;
+  for (int i = 0; i < p.nparts + p.ngroups - 1; i++) {
+    const int m = p.M[p.ngroups > 1 ? i : 0], n = p.N[p.ngroups > 1 ? i : 0];
+    const int ia = kind == GT_GEMM_TN ? m : p.K[i], ib = kind == GT_GEMM_NT ? p.K[i] : n;
+    vec = vec && ((ia | ib) & 3) == 0 && ((((uintptr_t)p.a[i]) | ((uintptr_t)p.b[i])) & 15) == 0;
+  }
+  const long big = tiles_of<Big>(p);
+  double best = cost_of<Big>(ctx, p, big, 1);
+  int ksplit = 0;            // 0: the big tile
+  const long small = tiles_of<Small>(p);
+  for (int ks = 1; ks <= 8; ks *= 2) {
+    const double c = cost_of<Small>(ctx, p, small, ks);
+    if (c < best) { best = c; ksplit = ks; }
+  }
+  if (ksplit) return vec ? launch_kind<Small, true>(ctx, kind, p, small, ksplit) : launch_kind<Small, false>(ctx, kind, p, small, ksplit);
+  tiles_of<Big>(p);
+  return vec ? launch_kind<Big, true>(ctx, kind, p, big, 1) : launch_kind<Big, false>(ctx, kind, p, big, 1);
+}
+
+bool kind_ok(int kind) { return kind == GT_GEMM_NT || kind == GT_GEMM_NN || kind == GT_GEMM_TN; }
 
 }  // namespace
 
+// c (+)= alpha * sum_p op(a_p).op(b_p)
+static gt_status f32_multi(gt_ctx* ctx, int kind, int accum, int M, int N, int nparts, const int* Ks, const float* const* as,
+                           const float* const* bs, float* c, float alpha) {
+  if (!kind_ok(kind)) return gt_fail(ctx, GT_ERR_ARG, "gt_gemm: unknown kind %d", kind);
+  F32Args p = {};
+  p.nparts = nparts; p.ngroups = 1; p.alpha = alpha;
+  p.M[0] = M; p.N[0] = N; p.accum[0] = accum; p.c[0] = c;
+  for (int i = 0; i < nparts; i++) { p.a[i] = as[i]; p.b[i] = bs[i]; p.K[i] = Ks[i]; }
+  return run(ctx, kind, p);
+}
+
+static gt_status f32_grouped(gt_ctx* ctx, int kind, int ngroups, const int* Ms, const int* Ns, int K, const float* const* as,
+                             const float* const* bs, float* const* cs, const int* accums, float alpha) {
+  if (!kind_ok(kind)) return gt_fail(ctx, GT_ERR_ARG, "gt_gemm: unknown kind %d", kind);
+  F32Args p = {};
+  p.nparts = 1; p.ngroups = ngroups; p.alpha = alpha;
+  for (int g = 0; g < ngroups; g++) {
+    p.a[g] = as[g]; p.b[g] = bs[g]; p.c[g] = cs[g]; p.K[g] = K;
+    p.M[g] = Ms[g]; p.N[g] = Ns[g]; p.accum[g] = accums[g];
+  }
+  return run(ctx, kind, p);
+}
+
 gt_status gt_gemm_simt(gt_ctx* ctx, int kind, int accum, int M, int N, int K, const float* a, const float* b, float* c, float alpha) {
-  dim3 grid(gt_cdiv(N, BN), gt_cdiv(M, BM), 1);
-  // Few output tiles and a deep K (the dW product, K = rows): split K across CTAs; the slices' partial products go
-  // to scratch and are added in slice order by a second kernel, so the result does not depend on scheduling.
-  int ksplit = 1;
-  long tiles = (long)grid.x * grid.y;
-  if (tiles < ctx->sm_count && K >= 1024) {
-    ksplit = (int)min((long)(2 * ctx->sm_count / tiles), (long)(K / 256));
-    if (ksplit < 1) ksplit = 1;
-  }
-  float* part = nullptr;
-  if (ksplit > 1) {
-    gt_status s = gt_scratch(ctx, sizeof(float) * (size_t)ksplit * M * N, &part);
-    if (s) return s;
-  }
-  grid.z = ksplit;
-  switch (kind) {
-    case GT_GEMM_NT:
-      gemm_f32_kernel<true, true><<<grid, 256, 0, ctx->stream>>>(M, N, K, a, K, 1, b, K, 1, c, accum, ksplit, alpha, part);
-      break;
-    case GT_GEMM_NN:
-      gemm_f32_kernel<true, false><<<grid, 256, 0, ctx->stream>>>(M, N, K, a, K, 1, b, 1, N, c, accum, ksplit, alpha, part);
-      break;
-    case GT_GEMM_TN:
-      gemm_f32_kernel<false, false><<<grid, 256, 0, ctx->stream>>>(M, N, K, a, 1, M, b, 1, N, c, accum, ksplit, alpha, part);
-      break;
-    default:
-      return gt_fail(ctx, GT_ERR_ARG, "gt_gemm: unknown kind %d", kind);
-  }
-  GT_LAUNCHED(ctx, "gemm_f32_kernel");
-  if (ksplit > 1) {
-    const long n = (long)M * N;
-    splitk_sum_kernel<<<(int)min((long)ctx->sm_count * 8, (n + 255) / 256), 256, 0, ctx->stream>>>(n, ksplit, part, c, accum);
-    GT_LAUNCHED(ctx, "splitk_sum_kernel");
-  }
-  return GT_OK;
+  return f32_multi(ctx, kind, accum, M, N, 1, &K, &a, &b, c, alpha);
 }
 
 gt_status gt_gemm_batched(gt_ctx* ctx, int kind, int accum, int M, int N, int K, const float* a, const float* b, float* c, int batch) {
@@ -135,8 +340,17 @@ gt_status gt_gemm_batched(gt_ctx* ctx, int kind, int accum, int M, int N, int K,
     gt_status s = gt_gemm_tc_batched(ctx, kind, accum, M, N, K, a, b, c, batch, &handled);
     if (s != GT_OK || handled) return s;
   }
-  for (int i = 0; i < batch; i++) {
-    gt_status s = gt_gemm_simt(ctx, kind, accum, M, N, K, a + (size_t)i * M * K, b + (size_t)i * N * K, c + (size_t)i * M * N, 1.f);
+  for (int i0 = 0; i0 < batch; i0 += MAX_PARTS) {     // eight matrices to a launch
+    const int n = min(MAX_PARTS, batch - i0);
+    const float* pa[MAX_PARTS];
+    const float* pb[MAX_PARTS];
+    float* pc[MAX_PARTS];
+    int m[MAX_PARTS], nn[MAX_PARTS], acc[MAX_PARTS];
+    for (int i = 0; i < n; i++) {
+      pa[i] = a + (size_t)(i0 + i) * M * K; pb[i] = b + (size_t)(i0 + i) * N * K; pc[i] = c + (size_t)(i0 + i) * M * N;
+      m[i] = M; nn[i] = N; acc[i] = accum;
+    }
+    gt_status s = f32_grouped(ctx, kind, n, m, nn, K, pa, pb, pc, acc, 1.f);
     if (s) return s;
   }
   return GT_OK;
@@ -176,6 +390,7 @@ extern "C" gt_status gt_gemm_multi(gt_ctx* ctx, int32_t kind, int32_t accum, int
     gt_status s = gt_gemm_tc_multi(ctx, kind, accum, M, N, nparts, k, pa, pb, gt_ptr<float>(c), &handled);
     if (s != GT_OK || handled) return s;
   }
+  if (ctx->precision == GT_PREC_FP32) return f32_multi(ctx, kind, accum, M, N, nparts, k, pa, pb, gt_ptr<float>(c), 1.f);
   for (int p = 0; p < nparts; p++) {
     gt_status s = gt_gemm(ctx, kind, p ? 1 : accum, M, N, k[p], as[p], bs[p], c);
     if (s) return s;
@@ -202,6 +417,7 @@ extern "C" gt_status gt_gemm_grouped_scaled(gt_ctx* ctx, int32_t kind, int32_t n
     gt_status s = gt_gemm_tc_grouped(ctx, kind, ngroups, m, n, K, pa, pb, pc, acc, nullptr, nullptr, 0, alpha, &handled);
     if (s != GT_OK || handled) return s;
   }
+  if (ctx->precision == GT_PREC_FP32) return f32_grouped(ctx, kind, ngroups, m, n, K, pa, pb, pc, acc, alpha);
   for (int g = 0; g < ngroups; g++) {
     gt_status s = gt_gemm_scaled(ctx, kind, acc[g], m[g], n[g], K, as[g], bs[g], cs[g], alpha);
     if (s) return s;
@@ -244,6 +460,12 @@ extern "C" gt_status gt_linear_rope_grouped(gt_ctx* ctx, int32_t ngroups, int32_
     bool handled = false;
     gt_status s = gt_gemm_tc_grouped(ctx, GT_GEMM_NT, ngroups, m, n, K, pa, pb, pc, acc, rp, tab, period, 1.f, &handled);
     if (s != GT_OK || handled) return s;
+  }
+  if (ctx->precision == GT_PREC_FP32) {
+    gt_status s = f32_grouped(ctx, GT_GEMM_NT, ngroups, m, n, K, pa, pb, pc, acc, 1.f);
+    for (int g = 0; g < ngroups && !s; g++)
+      if (rp[g]) s = gt_rope_apply(ctx, false, rows, heads[g], hd, base, pos_offset, pc[g], pc[g], 0);
+    return s;
   }
   for (int g = 0; g < ngroups; g++) {
     gt_status s = gt_gemm(ctx, GT_GEMM_NT, 0, rows, n[g], K, x, ws[g], ys[g]);
