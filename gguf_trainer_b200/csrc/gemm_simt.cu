@@ -4,6 +4,7 @@
 // (src/backend/webgpu.ts:1654-1671) with ragged edges in every dimension, sums of products written once and groups of
 // independent products in one launch.
 #include <cooperative_groups.h>
+#include <math.h>
 
 #include "common.cuh"
 
@@ -129,11 +130,11 @@ __global__ void __launch_bounds__(T::THREADS) gemm_f32_kernel(const __grid_const
   const int per = (kblocks + ksplit - 1) / ksplit;
   const int kb0 = min(kblocks, z * per), kb1 = min(kblocks, kb0 + per);
 
-  unsigned long long acc[TM][TN / 2];
+  unsigned long long acc[TM / 2][TN];      // pairs of rows: only the TN values of B need duplicating per K row
 #pragma unroll
-  for (int i = 0; i < TM; i++)
+  for (int i = 0; i < TM / 2; i++)
 #pragma unroll
-    for (int j = 0; j < TN / 2; j++) acc[i][j] = 0ull;
+    for (int j = 0; j < TN; j++) acc[i][j] = 0ull;
 
   Operand<BM, BK, T::QA, T::THREADS, A_K, VEC> oa;
   Operand<BN, BK, T::QB, T::THREADS, B_K, VEC> ob;
@@ -157,20 +158,21 @@ __global__ void __launch_bounds__(T::THREADS) gemm_f32_kernel(const __grid_const
     if (kb + 1 < kb1) fetch();
 #pragma unroll
     for (int kk = 0; kk < BK; kk++) {
-      float av[TM];
-      unsigned long long bv[TN / 2];
+      unsigned long long av[TM / 2];
+      float bv[TN];
 #pragma unroll
-      for (int i = 0; i < TM / 4; i++) *reinterpret_cast<float4*>(&av[4 * i]) = *reinterpret_cast<const float4*>(As + kk * BM + ((i * (4 * TY) + ty * 4) ^ swz<BK>(kk)));
-#pragma unroll
-      for (int j = 0; j < TN / 4; j++) {
-        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(Bs + kk * BN + ((j * (4 * TX) + tx * 4) ^ swz<BK>(kk)));
-        bv[2 * j] = w.x; bv[2 * j + 1] = w.y;
+      for (int i = 0; i < TM / 4; i++) {
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(As + kk * BM + ((i * (4 * TY) + ty * 4) ^ swz<BK>(kk)));
+        av[2 * i] = w.x; av[2 * i + 1] = w.y;
       }
 #pragma unroll
-      for (int i = 0; i < TM; i++) {
-        const unsigned long long aa = pack2(av[i], av[i]);
+      for (int j = 0; j < TN / 4; j++)
+        *reinterpret_cast<float4*>(&bv[4 * j]) = *reinterpret_cast<const float4*>(Bs + kk * BN + ((j * (4 * TX) + tx * 4) ^ swz<BK>(kk)));
 #pragma unroll
-        for (int j = 0; j < TN / 2; j++) fma2(acc[i][j], aa, bv[j]);
+      for (int j = 0; j < TN; j++) {
+        const unsigned long long bb = pack2(bv[j], bv[j]);
+#pragma unroll
+        for (int i = 0; i < TM / 2; i++) fma2(acc[i][j], av[i], bb);
       }
     }
     if (kb + 1 < kb1) {
@@ -180,6 +182,15 @@ __global__ void __launch_bounds__(T::THREADS) gemm_f32_kernel(const __grid_const
     __syncthreads();
   }
 
+  auto quad_of = [&](int i, int j) {           // row i, columns 4 j .. 4 j + 3 of this thread's outputs
+    float v[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const float2 u = unpack2(acc[i / 2][4 * j + e]);
+      v[e] = (i & 1) ? u.y : u.x;
+    }
+    return make_float4(v[0], v[1], v[2], v[3]);
+  };
   float* C = p.c[g];
   const int accum = p.accum[g];
   const bool vecC = (N & 3) == 0 && (((uintptr_t)C) & 15) == 0;
@@ -201,20 +212,15 @@ __global__ void __launch_bounds__(T::THREADS) gemm_f32_kernel(const __grid_const
 #pragma unroll
     for (int i = 0; i < TM; i++)
 #pragma unroll
-      for (int j = 0; j < TN / 4; j++) {
-        const float2 u = unpack2(acc[i][2 * j]), w = unpack2(acc[i][2 * j + 1]);
-        put(m0 + (i / 4) * (4 * TY) + ty * 4 + i % 4, n0 + j * (4 * TX) + tx * 4, make_float4(u.x, u.y, w.x, w.y));
-      }
+      for (int j = 0; j < TN / 4; j++) put(m0 + (i / 4) * (4 * TY) + ty * 4 + i % 4, n0 + j * (4 * TX) + tx * 4, quad_of(i, j));
     return;
   }
   // the cluster's slices: every CTA leaves its tile in shared memory and adds up its share of the rows over all of them
 #pragma unroll
   for (int i = 0; i < TM; i++)
 #pragma unroll
-    for (int j = 0; j < TN / 4; j++) {
-      const float2 u = unpack2(acc[i][2 * j]), w = unpack2(acc[i][2 * j + 1]);
-      *reinterpret_cast<float4*>(sm + ((i / 4) * (4 * TY) + ty * 4 + i % 4) * BN + j * (4 * TX) + tx * 4) = make_float4(u.x, u.y, w.x, w.y);
-    }
+    for (int j = 0; j < TN / 4; j++)
+      *reinterpret_cast<float4*>(sm + ((i / 4) * (4 * TY) + ty * 4 + i % 4) * BN + j * (4 * TX) + tx * 4) = quad_of(i, j);
   cg::cluster_group cluster = cg::this_cluster();
   cluster.sync();
   for (int q = z * T::THREADS + tid; q < BM * BN / 4; q += ksplit * T::THREADS) {
@@ -270,17 +276,20 @@ long tiles_of(F32Args& p) {
 }
 
 // Tile and slices by predicted cycles of the SM with the most work: CTAs there x K rows each x cycles per K row, plus what
-// a CTA costs whatever its depth. A K row of a tile is BM x BN / 128 cycles of the FMA pipe, of which resident CTAs
-// together reach about 0.8, and a 64 x 64 CTA that has an SM to itself (four warps) about half.
+// a CTA costs whatever its depth. A K row of a tile is BM x BN / 128 cycles of the FMA pipe; `eff` is the part of that rate
+// that the resident CTAs reach together (one 64 x 64 CTA, four warps, 0.44; four of them 0.68; 128 x 128, eight warps,
+// 0.62 and 0.74). Clusters of four and more land unevenly on the SMs when there are few. Fitted on eleven shapes from
+// 512 x 128 x 128 to 8192 x 8192 x 1024, where it picks the fastest choice or one within 15 %: 53 TFLOP/s at the largest
+// (128 x 128), 57 us for 512 x 576 x 1536 in one slice against 31 in eight.
 template <class T>
 double cost_of(gt_ctx* ctx, const F32Args& p, long tiles, int ksplit) {
   double rows = 0;
   for (int i = 0; i < p.nparts; i++) rows += gt_cdiv(p.K[i], T::BK) * T::BK;
   const double per = gt_cdiv((long)rows / T::BK, ksplit) * T::BK;
-  const double ctas = gt_cdiv(tiles * ksplit, ctx->sm_count);
-  const double row = T::BM * T::BN / 128.0;
-  const double busy = ctas * row / 0.8, alone = row / (T::THREADS >= 256 ? 0.7 : 0.5);
-  return per * (busy > alone ? busy : alone) + 2200.0 + (ksplit > 1 ? 1200.0 + 250.0 * ksplit : 0.0) + 400.0 * (ctas - 1);
+  const double share = (double)tiles * ksplit / ctx->sm_count;
+  const double ctas = share <= 0.5 ? 1.0 : ceil(share * (ksplit >= 4 && share < 4.0 ? 1.25 : 1.0));
+  const double eff = T::THREADS >= 256 ? (ctas < 2 ? 0.62 : 0.74) : (ctas < 2 ? 0.44 : ctas < 3 ? 0.54 : ctas < 4 ? 0.60 : 0.68);
+  return per * ctas * (T::BM * T::BN / 128.0) / eff + 3500.0 + (ksplit > 1 ? 1000.0 + 500.0 * ksplit : 0.0) + 600.0 * (ctas - 1);
 }
 
 gt_status run(gt_ctx* ctx, int kind, F32Args& p) {
@@ -289,6 +298,17 @@ gt_status run(gt_ctx* ctx, int kind, F32Args& p) {
     const int m = p.M[p.ngroups > 1 ? i : 0], n = p.N[p.ngroups > 1 ? i : 0];
     const int ia = kind == GT_GEMM_TN ? m : p.K[i], ib = kind == GT_GEMM_NT ? p.K[i] : n;
     vec = vec && ((ia | ib) & 3) == 0 && ((((uintptr_t)p.a[i]) | ((uintptr_t)p.b[i])) & 15) == 0;
+  }
+  // Weight gradients of a model's projections are launched in whatever groups the backward pass gives (they differ with and
+  // without recompute), and a strict-f32 result may not depend on that: their slices follow from the depth alone.
+  if (kind == GT_GEMM_TN && p.nparts == 1) {
+    bool projection = true;
+    for (int g = 0; g < p.ngroups; g++) projection = projection && (long)gt_cdiv(p.M[g], Small::BM) * gt_cdiv(p.N[g], Small::BN) <= 1024;
+    if (projection) {
+      const int ks = p.K[0] >= 2048 ? 8 : p.K[0] >= 512 ? 4 : p.K[0] >= 256 ? 2 : 1;
+      const long n = tiles_of<Small>(p);
+      return vec ? launch_kind<Small, true>(ctx, kind, p, n, ks) : launch_kind<Small, false>(ctx, kind, p, n, ks);
+    }
   }
   const long big = tiles_of<Big>(p);
   double best = cost_of<Big>(ctx, p, big, 1);
