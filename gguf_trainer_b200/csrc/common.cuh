@@ -13,6 +13,7 @@
 struct GtAdamW;
 struct GtMuon;
 struct GtDp;
+struct GtHostCopy;   // staging ring and copy threads of gt_read (ctx.cu)
 
 struct gt_ctx {
   int device = 0;
@@ -50,6 +51,8 @@ struct gt_ctx {
   // staging
   void* pinned = nullptr;
   uint64_t pinned_bytes = 0, pinned_cursor = 0;
+  GtHostCopy* host_copy = nullptr;
+  int* flag_words = nullptr;   // pinned: the latched device words as gt_sync last saw them
   bool capturing = false;
   std::vector<GtAdamW*> adamws;
   std::vector<GtMuon*> muons;
@@ -115,7 +118,9 @@ gt_status gt_rope_table(gt_ctx* ctx, int rows, int hd, double base, int pos_offs
 gt_status gt_rope_apply(gt_ctx* ctx, bool bwd, int rows, int H, int hd, double base, int pos_offset, const float* in, float* out, int accum);
 gt_status gt_glu_linear_tc(gt_ctx* ctx, int op, int rows, int ffn, int in, const float* x, const float* wg, const float* wu, float* gate,
                            float* up, float* out, bool* handled);
-gt_status gt_gemm_tc_check(gt_ctx* ctx);
+// the tensor-core kernels' latched word (null before their first launch), and the answer to a code read from it
+int* gt_gemm_tc_word(gt_ctx* ctx);
+gt_status gt_gemm_tc_answer(gt_ctx* ctx, int code);
 void gt_optim_destroy(gt_ctx* ctx);
 void gt_dp_teardown(gt_ctx* ctx);
 // rank and world of the context's communicator (an error when gt_dp_init has not run)

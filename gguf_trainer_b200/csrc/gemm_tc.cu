@@ -740,18 +740,12 @@ extern "C" gt_status gt_selftest_bounded_wait(gt_ctx* ctx, int32_t limit_us) {
   return GT_OK;
 }
 
-// Reads and clears the device flag the kernels raise when a bounded wait expires.
-gt_status gt_gemm_tc_check(gt_ctx* ctx) {
-  int* f = g_flag[ctx->device];
-  if (!f) return GT_OK;
-  int h = 0;
-  GT_CUDA(ctx, cudaMemcpyAsync(&h, f, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  GT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (h != 0) {
-    cudaMemsetAsync(f, 0, sizeof(int), ctx->stream);
-    return gt_fail(ctx, GT_ERR_CUDA, "tensor-core kernel: a pipeline wait expired (code %d); results of that launch are invalid", h);
-  }
-  return GT_OK;
+// The device flag the kernels raise when a bounded wait expires: gt_sync reads it with its other latched words.
+int* gt_gemm_tc_word(gt_ctx* ctx) { return g_flag[ctx->device]; }
+gt_status gt_gemm_tc_answer(gt_ctx* ctx, int code) {
+  if (code == 0) return GT_OK;
+  cudaMemsetAsync(g_flag[ctx->device], 0, sizeof(int), ctx->stream);
+  return gt_fail(ctx, GT_ERR_CUDA, "tensor-core kernel: a pipeline wait expired (code %d); results of that launch are invalid", code);
 }
 
 // `batch` independent products of the same shape, matrix i of each operand `M*K`, `N*K`, `M*N` elements after matrix i-1.
