@@ -29,7 +29,6 @@ struct GtHostCopy {
   static constexpr int SLOTS = 8, THREADS = 4;
   static constexpr uint64_t BLOCK = 1 << 20;
   struct Job { void* dst; int slot; uint64_t bytes; };
-  int device = 0;
   char* ring = nullptr;
   cudaEvent_t landed[SLOTS] = {};
   std::atomic<int> busy[SLOTS];          // 1 from the copy's launch until a thread has emptied the block
@@ -38,7 +37,6 @@ struct GtHostCopy {
   std::deque<Job> jobs;
   std::atomic<int> queued{0}, asleep{0};
   std::atomic<bool> stop{false};
-  std::atomic<int> failed{0};
   std::vector<std::thread> threads;
 
   bool take(Job& j) {
@@ -51,8 +49,7 @@ struct GtHostCopy {
     return true;
   }
   void empty(const Job& j) {
-    if (cudaEventSynchronize(landed[j.slot]) == cudaSuccess) memcpy(j.dst, ring + (uint64_t)j.slot * BLOCK, j.bytes);
-    else failed = 1;
+    memcpy(j.dst, ring + (uint64_t)j.slot * BLOCK, j.bytes);
     busy[j.slot].store(0, std::memory_order_release);
   }
   void put(const Job& j) {
@@ -64,7 +61,6 @@ struct GtHostCopy {
     if (asleep.load()) cv.notify_one();
   }
   void work() {
-    cudaSetDevice(device);
     Job j;
     while (!stop) {
       if (take(j)) { empty(j); continue; }
@@ -78,8 +74,7 @@ struct GtHostCopy {
       asleep.fetch_sub(1);
     }
   }
-  cudaError_t start(int dev) {
-    device = dev;
+  cudaError_t start() {
     cudaError_t e = cudaMallocHost(&ring, SLOTS * BLOCK);
     for (int i = 0; i < SLOTS && e == cudaSuccess; i++) {
       busy[i] = 0;
@@ -329,7 +324,7 @@ gt_status gt_read(gt_ctx* ctx, gt_buf src, void* host, uint64_t bytes) {
   if (ctx->capturing) return gt_fail(ctx, GT_ERR_STATE, "gt_read inside a graph capture");
   if (!ctx->host_copy) {
     GtHostCopy* hc = new GtHostCopy();
-    cudaError_t e = hc->start(ctx->device);
+    cudaError_t e = hc->start();
     if (e != cudaSuccess) { delete hc; return gt_check_cuda(ctx, e, "gt_read: staging"); }
     ctx->host_copy = hc;
   }
@@ -341,25 +336,35 @@ gt_status gt_read(gt_ctx* ctx, gt_buf src, void* host, uint64_t bytes) {
     ctx->readback_bytes += bytes;
     return GT_OK;
   }
-  // blocks of a quarter megabyte up to one, so that a read of a few megabytes keeps every thread busy too
-  uint64_t block = (bytes / 16 + 4095) / 4096 * 4096;
-  block = block < (256u << 10) ? (256u << 10) : block > GtHostCopy::BLOCK ? GtHostCopy::BLOCK : block;
+  // Blocks of an eighth of the read between 128 KB and 1 MB, so that a read of a few megabytes keeps every thread busy too.
+  // This thread alone talks to the driver (waits in several threads would queue up behind its launches): it keeps LAG
+  // copies ahead of the block it waits for and hands over what has landed.
+  constexpr uint64_t LAG = 5;
+  uint64_t block = (bytes / 8 + 4095) / 4096 * 4096;
+  block = block < (128u << 10) ? (128u << 10) : block > GtHostCopy::BLOCK ? GtHostCopy::BLOCK : block;
+  const uint64_t n = (bytes + block - 1) / block;
   cudaError_t err = cudaSuccess;
-  int slot = 0;
-  for (uint64_t off = 0; off < bytes && err == cudaSuccess; off += block, slot = (slot + 1) % GtHostCopy::SLOTS) {
-    const uint64_t n = bytes - off < block ? bytes - off : block;
-    while (hc.busy[slot].load(std::memory_order_acquire)) cpu_pause();
-    err = cudaMemcpyAsync(hc.ring + (uint64_t)slot * GtHostCopy::BLOCK, (char*)gt_ptr<void>(src) + off, n, cudaMemcpyDeviceToHost, ctx->stream);
-    if (err == cudaSuccess) err = cudaEventRecord(hc.landed[slot], ctx->stream);
-    if (err != cudaSuccess) break;
-    hc.busy[slot].store(1, std::memory_order_relaxed);
-    hc.put({(char*)host + off, slot, n});
+  auto len = [&](uint64_t i) { return i + 1 < n ? block : bytes - i * block; };
+  for (uint64_t i = 0; i < n + LAG && err == cudaSuccess; i++) {
+    if (i < n) {
+      const int slot = (int)(i % GtHostCopy::SLOTS);
+      while (hc.busy[slot].load(std::memory_order_acquire)) cpu_pause();
+      err = cudaMemcpyAsync(hc.ring + (uint64_t)slot * GtHostCopy::BLOCK, (char*)gt_ptr<void>(src) + i * block, len(i), cudaMemcpyDeviceToHost, ctx->stream);
+      if (err == cudaSuccess) err = cudaEventRecord(hc.landed[slot], ctx->stream);
+      if (err == cudaSuccess) hc.busy[slot].store(1, std::memory_order_relaxed);
+    }
+    if (i >= LAG && i - LAG < n && err == cudaSuccess) {
+      const int slot = (int)((i - LAG) % GtHostCopy::SLOTS);
+      err = cudaEventSynchronize(hc.landed[slot]);
+      if (err == cudaSuccess) hc.put({(char*)host + (i - LAG) * block, slot, len(i - LAG)});
+    }
   }
   for (GtHostCopy::Job j; hc.take(j);) hc.empty(j);
-  for (int i = 0; i < GtHostCopy::SLOTS; i++)
-    while (hc.busy[i].load(std::memory_order_acquire)) cpu_pause();
+  for (auto& b : hc.busy) {
+    if (err != cudaSuccess) b = 0;           // (blocks that were never handed over)
+    while (b.load(std::memory_order_acquire)) cpu_pause();
+  }
   if (err != cudaSuccess) return gt_check_cuda(ctx, err, "gt_read");
-  if (hc.failed.exchange(0)) { GT_CUDA(ctx, cudaStreamSynchronize(ctx->stream)); return gt_fail(ctx, GT_ERR_CUDA, "gt_read: a staged copy failed"); }
   ctx->readback_bytes += bytes;
   return GT_OK;
 }
