@@ -64,6 +64,7 @@ struct PartMaps {
   int gM[MAX_PARTS], gN[MAX_PARTS], g_accum[MAX_PARTS], unit_end[MAX_PARTS];
   // Rotary form (EPI_ROPE): the outputs of the groups with g_rope[g] set are rotated as they are written (see the kernel).
   int g_rope[MAX_PARTS];
+  float* cp[MAX_PARTS];     // the outputs themselves (gemm_tf32_small_kernel stores without a tensor map)
   const float2* rope_tab;   // [rope_period][32] (cos, sin) of the 32 pairs of a 64-wide head
   int rope_period;          // positions per sequence: row r is position r % rope_period
 };
@@ -568,9 +569,317 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
 }
 
 // ---------------------------------------------------------------------------------------------
+// The same products when their tiles do not fill the SMs: decoding and short sequences (M of a few dozen to a few hundred
+// rows), weight gradients of short batches, the thin products of adapters. One tile of 128 x BN per CTA, BN 32, 64 or
+// 128, the contraction cut over a cluster of up to 8 CTAs. Each leaves its partial tile in shared memory and finishes its
+// share of the rows over all of them, in rank order, so that C is written once: no clear before the launch, no reduce-adds in
+// L2, and the result does not depend on which slice came first. What bounds these launches is latency (start-up, first
+// copies, the last products, the hand-over), so nothing is persistent and all four warps drain the accumulator.
+// At 512 rows, K 576: 5 us a launch where the persistent kernel with its clear took 8 + 1.5 us; gate, up and the gated unit
+// of a decode step (40 rows, 7 MB of weights) 28.6 -> 6 us.
+// ---------------------------------------------------------------------------------------------
+template <int BN>
+struct SmallSmem {
+  static constexpr int A_BYTES = BM1 * BK * 4, B_BYTES = BN * BK * 4, STAGE = A_BYTES + B_BYTES;
+  static constexpr int STAGES = 4;                    // two CTAs per SM at BN 32 and 64
+  static constexpr int PITCH = BN + 4;                // of the partial tile (reuses the stages)
+  static constexpr int TOTAL = STAGES * STAGE + 1024 + 128;
+  static constexpr uint32_t TMEM_COLS = BN;
+  static constexpr int THREADS = 256;
+  static_assert(BM1 * PITCH * 4 <= STAGES * STAGE && TOTAL <= 232448, "shared memory");
+};
+
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));   // (ordered after the cluster barrier, which is volatile too)
+  return v;
+}
+
+// EPI: 0, GT_EW_SILU, GT_EW_GELU (gate, up and the gated unit) or EPI_ROPE, as in gemm_tf32_kernel. gridDim.x = tiles x ksplit,
+// the slices of a tile adjacent and one cluster.
+template <bool A_K, bool B_K, int BN, int EPI>
+__global__ void __launch_bounds__(SmallSmem<BN>::THREADS)
+gemm_tf32_small_kernel(const __grid_constant__ PartMaps maps, int M_, int N_, int accum_, int ksplit, float out_scale, int* __restrict__ flag) {
+  extern __shared__ uint8_t smem_raw[];
+  using S = SmallSmem<BN>;
+  constexpr int STAGES = S::STAGES;
+  constexpr bool IS_GLU = EPI == GT_EW_SILU || EPI == GT_EW_GELU;
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t bars = base + STAGES * S::STAGE;     // full[STAGES], empty[STAGES], acc_full, tmem slot
+  auto full_bar = [&](int s) { return bars + 8u * s; };
+  auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };
+  const uint32_t acc_full = bars + 8u * (2 * STAGES), tmem_slot = acc_full + 8;
+  volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int z = (int)blockIdx.x % ksplit;
+  int t = (int)blockIdx.x / ksplit, g = 0, bi = 0;
+  if (maps.ngroups > 1) {
+    while (t >= maps.unit_end[g]) g++;
+    if (g) t -= maps.unit_end[g - 1];
+  }
+  const int M = maps.ngroups > 1 ? maps.gM[g] : M_, N = maps.ngroups > 1 ? maps.gN[g] : N_;
+  const int accum = maps.ngroups > 1 ? maps.g_accum[g] : accum_;
+  const int tn = (N + BN - 1) / BN, tmn = tn * ((M + BM1 - 1) / BM1);
+  bi = t / tmn;                                       // matrix of a batch
+  t -= bi * tmn;
+  const int n0 = (t % tn) * BN, m0 = (t / tn) * BM1;
+  const int kblocks = maps.kb_end[maps.nparts - 1];
+  const int per = (kblocks + ksplit - 1) / ksplit;
+  const int kb0 = min(kblocks, z * per), kb1 = min(kblocks, kb0 + per);
+
+  bool dead = false;
+  auto wait = [&](uint32_t bar, uint32_t parity, int code) {
+    if (dead) return;
+    if (!mbar_wait(bar, parity)) { dead = true; atomicExch(flag, code); }
+  };
+  int part = maps.ngroups > 1 ? g : 0;
+  auto load = [&](int kb) {                           // K block kb of this slice (called in order, by thread 0)
+    const int s = (kb - kb0) % STAGES;
+    const uint32_t a_dst = base + s * S::STAGE, b_dst = a_dst + S::A_BYTES;
+    if (maps.ngroups == 1) while (kb >= maps.kb_end[part]) part++;
+    const CUtensorMap* pa = &maps.a[part];
+    const CUtensorMap* pb = &maps.b[part];
+    const int k0 = (maps.ngroups == 1 ? kb - (part ? maps.kb_end[part - 1] : 0) : kb) * BK;
+    mbar_expect_tx(full_bar(s), S::STAGE);
+    if (A_K) tma_load_3d(a_dst, pa, k0, m0, bi, full_bar(s));
+    else
+      for (int c = 0; c < BM1 / 32; c++) tma_load_3d(a_dst + c * 4096, pa, m0 + 32 * c, k0, bi, full_bar(s));
+    if (IS_GLU) {
+      tma_load_3d(b_dst, &maps.b[0], k0, n0 >> 1, bi, full_bar(s));
+      tma_load_3d(b_dst + (BN / 2) * 128, &maps.b[1], k0, n0 >> 1, bi, full_bar(s));
+    } else if (B_K) tma_load_3d(b_dst, pb, k0, n0, bi, full_bar(s));
+    else
+      for (int c = 0; c < BN / 32; c++) tma_load_3d(b_dst + c * 4096, pb, n0 + 32 * c, k0, bi, full_bar(s));
+  };
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; s++) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+    mbar_init(acc_full, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_async_smem();
+    for (int kb = kb0; kb < min(kb1, kb0 + STAGES); kb++) load(kb);   // the first copies start before anything else is set up
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, S::TMEM_COLS);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot_ptr;
+
+  if (warp == 0) {
+    if (lane == 0)
+      for (int kb = kb0 + STAGES; kb < kb1; kb++) {
+        wait(empty_bar((kb - kb0) % STAGES), (((kb - kb0) / STAGES) & 1) ^ 1, 5);
+        load(kb);
+      }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = idesc_tf32(!A_K, !B_K, BM1, BN);
+      const uint64_t a_desc0 = A_K ? desc_kmajor(base) : desc_mnmajor(base);
+      const uint64_t b_desc0 = B_K ? desc_kmajor(base + S::A_BYTES) : desc_mnmajor(base + S::A_BYTES);
+      constexpr uint32_t A_STEP = A_K ? 32 : 1024, B_STEP = B_K ? 32 : 1024;
+      for (int kb = kb0, it = 0; kb < kb1; kb++, it++) {
+        const int s = it % STAGES;
+        wait(full_bar(s), (it / STAGES) & 1, 6);
+        tc_fence_after();
+        const uint32_t soff = (uint32_t)(s * S::STAGE) >> 4;
+#pragma unroll
+        for (int j = 0; j < BK / UMMA_K; j++)
+          umma_tf32(tmem, a_desc0 + soff + ((j * A_STEP) >> 4), b_desc0 + soff + ((j * B_STEP) >> 4), idesc, (kb > kb0 || j > 0) ? 1u : 0u);
+        umma_commit(empty_bar(s));
+      }
+      if (kb1 > kb0) umma_commit(acc_full);
+    }
+  }
+  __syncwarp();
+  const bool have = kb1 > kb0;
+  if (have) wait(acc_full, 0, 7);      // every product has completed: the stages are free, the accumulator is whole
+  dead = __any_sync(0xffffffffu, dead);
+  tc_fence_after();
+  // the partial tile, row by row: warps w and w + 4 take accumulator rows 32 (w mod 4) .. + 31, every other 32 columns each
+  {
+    const int qd = warp & 3;
+    float* tile = reinterpret_cast<float*>(smem_raw + (base - smem_u32(smem_raw))) + (qd * 32 + lane) * S::PITCH;
+#pragma unroll 1
+    for (int c = warp >> 2; c < BN / 32; c += 2) {
+      float v[32];
+      if (have) tmem_ld32(tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(c * 32), v);
+#pragma unroll
+      for (int j = 0; j < 32; j += 4)
+        *reinterpret_cast<float4*>(tile + c * 32 + j) = have ? make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  tc_fence_before();
+  if (ksplit > 1) cluster_sync_all(); else __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, S::TMEM_COLS);
+  }
+  const int mrows = min(BM1, M - m0);
+  // four columns of a row over the slices, scaled; every slice's load is issued before the first is used
+  auto sum = [&](int r, int col) {
+    const uint32_t at = base + (uint32_t)(r * S::PITCH + col) * 4u;
+    float4 v[8];
+    if (ksplit == 1) v[0] = *reinterpret_cast<const float4*>(smem_raw + (at - smem_u32(smem_raw)));
+    else {
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (k < ksplit) v[k] = ld_cluster_f32x4(cluster_addr_of(at, k));
+    }
+    float4 s = v[0];
+#pragma unroll
+    for (int k = 1; k < 8; k++)
+      if (k < ksplit) { s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
+    s.x *= out_scale; s.y *= out_scale; s.z *= out_scale; s.w *= out_scale;
+    return s;
+  };
+  auto put = [&](float* C, int pitch, int row, int col, int ncols, float4 v, int acc) {
+    if (col >= ncols || dead) return;
+    float* d = C + (size_t)row * pitch + col;
+    if ((pitch & 3) == 0 && col + 4 <= ncols && (((uintptr_t)C) & 15) == 0) {
+      if (acc) { const float4 o = *reinterpret_cast<const float4*>(d); v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w; }
+      *reinterpret_cast<float4*>(d) = v;
+      return;
+    }
+    d[0] = acc ? d[0] + v.x : v.x;
+    if (col + 1 < ncols) d[1] = acc ? d[1] + v.y : v.y;
+    if (col + 2 < ncols) d[2] = acc ? d[2] + v.z : v.z;
+    if (col + 3 < ncols) d[3] = acc ? d[3] + v.w : v.w;
+  };
+  float* C = maps.cp[IS_GLU ? 0 : g] + (size_t)bi * M * N;
+  if constexpr (IS_GLU) {
+    const int ffn = maps.gN[0];
+    for (int q = z * S::THREADS + threadIdx.x; q < mrows * (BN / 8); q += ksplit * S::THREADS) {
+      const int r = q / (BN / 8), c = (q % (BN / 8)) * 4, col = (n0 >> 1) + c;
+      if (col >= ffn) continue;
+      const float4 a = sum(r, c), u = sum(r, c + BN / 2);
+      auto act = [](float x) {
+        if (EPI == GT_EW_SILU) return x / (1.f + __expf(-x));
+        return 0.5f * x * (1.f + tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x)));
+      };
+      put(maps.cp[0], ffn, m0 + r, col, ffn, a, 0);
+      put(maps.cp[1], ffn, m0 + r, col, ffn, u, 0);
+      put(maps.cp[2], ffn, m0 + r, col, ffn, make_float4(act(a.x) * u.x, act(a.y) * u.y, act(a.z) * u.z, act(a.w) * u.w), 0);
+    }
+  } else if (EPI == EPI_ROPE && maps.g_rope[g]) {
+    // heads of 64 columns, BN a multiple of 64: quads j and j + 32 of a head are rotated together
+    for (int q = z * S::THREADS + threadIdx.x; q < mrows * (BN / 8); q += ksplit * S::THREADS) {
+      const int r = q / (BN / 8), e = q % (BN / 8), c = (e / 8) * 64 + (e % 8) * 4;
+      if (n0 + c >= N) continue;
+      const float4* tab = reinterpret_cast<const float4*>(maps.rope_tab + (size_t)((m0 + r) % maps.rope_period) * 32 + (e % 8) * 4);
+      const float4 a = sum(r, c), b = sum(r, c + 32), t0 = __ldg(tab), t1 = __ldg(tab + 1);   // (cos, sin) of four pairs
+      put(C, N, m0 + r, n0 + c, N, make_float4(a.x * t0.x - b.x * t0.y, a.y * t0.z - b.y * t0.w, a.z * t1.x - b.z * t1.y, a.w * t1.z - b.w * t1.w), accum);
+      put(C, N, m0 + r, n0 + c + 32, N, make_float4(a.x * t0.y + b.x * t0.x, a.y * t0.w + b.y * t0.z, a.z * t1.y + b.z * t1.x, a.w * t1.w + b.w * t1.z), accum);
+    }
+  } else {
+    const int end = mrows * (BN / 4), step = ksplit * S::THREADS;
+    for (int q = z * S::THREADS + threadIdx.x; q < end; q += 2 * step) {     // two quads at a time, their loads together
+      const int q1 = q + step < end ? q + step : q;
+      const int r = q / (BN / 4), c = (q % (BN / 4)) * 4, r1 = q1 / (BN / 4), c1 = (q1 % (BN / 4)) * 4;
+      const float4 v = sum(r, c), v1 = sum(r1, c1);
+      if (n0 + c < N) put(C, N, m0 + r, n0 + c, N, v, accum);
+      if (q1 != q && n0 + c1 < N) put(C, N, m0 + r1, n0 + c1, N, v1, accum);
+    }
+  }
+  __syncwarp();
+  if (ksplit > 1) cluster_sync_all();                 // nobody leaves while its tile may still be read
+}
+
+// ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
 int* g_flag[64] = {};
+
+template <bool A_K, bool B_K, int BN, int EPI>
+gt_status launch_small(gt_ctx* ctx, const PartMaps& maps, long tiles, int M, int N, int accum, int ksplit, float out_scale) {
+  auto kern = gemm_tf32_small_kernel<A_K, B_K, BN, EPI>;
+  using S = SmallSmem<BN>;
+  static bool attr_set[64] = {};
+  if (!attr_set[ctx->device]) {
+    GT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL));
+    attr_set[ctx->device] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * ksplit), 1, 1);
+  cfg.blockDim = dim3(S::THREADS, 1, 1);
+  cfg.dynamicSmemBytes = S::TOTAL;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ksplit;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = ksplit > 1 ? 1 : 0;
+  GT_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, maps, M, N, accum, ksplit, out_scale, g_flag[ctx->device]));
+  GT_LAUNCHED(ctx, "gemm_tf32_small_kernel");
+  return GT_OK;
+}
+
+template <int BN, int EPI = 0>
+gt_status launch_small_kind(gt_ctx* ctx, int kind, const PartMaps& maps, long tiles, int M, int N, int accum, int ksplit, float out_scale) {
+  if (kind == GT_GEMM_NT) return launch_small<true, true, BN, EPI>(ctx, maps, tiles, M, N, accum, ksplit, out_scale);
+  if constexpr (EPI == 0) {
+    if (kind == GT_GEMM_NN) return launch_small<true, false, BN, EPI>(ctx, maps, tiles, M, N, accum, ksplit, out_scale);
+    return launch_small<false, false, BN, EPI>(ctx, maps, tiles, M, N, accum, ksplit, out_scale);
+  }
+  return GT_ERR_ARG;
+}
+
+// CTAs that can be resident at once, one per SM, when they come in clusters of `c` (clusters lie inside a group of SMs, and the
+// groups are not all of one size).
+int cluster_room(gt_ctx* ctx, int c) {
+  static int room[64][9] = {};
+  int& r = room[ctx->device][c];
+  if (r == 0) {
+    auto kern = gemm_tf32_small_kernel<true, true, 128, 0>;
+    int n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(ctx->sm_count / c * c), 1, 1);
+    cfg.blockDim = dim3(SmallSmem<128>::THREADS, 1, 1);
+    cfg.dynamicSmemBytes = SmallSmem<128>::TOTAL;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = c;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SmallSmem<128>::TOTAL) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    r = n > 0 ? n * c : c;
+    if (getenv("GT_GEMM_TILE")) fprintf(stderr, "[gguftrain] resident CTAs in clusters of %d: %d\n", c, r);
+  }
+  return r;
+}
+
+// The best shape of the one-tile-per-CTA kernel for `tiles(bn)` tiles of 128 x bn and its predicted cycles, on the scale of
+// the persistent kernel's cost model. A K block costs its shared-memory traffic (the stage written and read once at
+// 128 B/clk); resident CTAs of an SM share that.
+constexpr double SMALL_FIXED = 10500.0, SMALL_WAVE = 8500.0;
+struct SmallPick { int bn = 0, ks = 1; double cost = 1e30; };
+template <typename F>
+SmallPick pick_small(gt_ctx* ctx, int kblocks, F tiles, int min_bn) {
+  const long workers = ctx->sm_count - ctx->sm_reserved;
+  SmallPick p;
+  for (int bn = min_bn; bn <= 128; bn *= 2) {
+    const long n = tiles(bn);
+    if (n > 4 * workers) continue;
+    const double per_kb = 2.0 * (BM1 + bn) * BK * 4 / 128.0;
+    for (int ks = 1; ks <= 8 && ks <= kblocks; ks++) {
+      const int per = gt_cdiv(kblocks, ks);
+      if ((long)(ks - 1) * per >= kblocks) continue;   // (an empty slice)
+      const long room = ks == 1 ? workers : max((long)ks, (long)cluster_room(ctx, ks) - ctx->sm_reserved);   // two CTAs of up to 64 columns share an SM
+      const double share = n * ks > room && bn <= 64 ? 2.0 : 1.0;
+      const double waves = ceil((double)(n * ks) / (room * share));
+      const double cost = waves * (per * per_kb * share + SMALL_WAVE) + (SMALL_FIXED - SMALL_WAVE) + (share > 1.0 ? 5000.0 : 0.0) + 6.0 * bn;
+      if (cost < p.cost) { p.cost = cost; p.bn = bn; p.ks = ks; }
+    }
+  }
+  return p;
+}
+// what a launch of the persistent kernel costs beside its tiles, and the clear before one whose slices meet in L2
+constexpr double PERSISTENT_FIXED = 9500.0, CLEAR_FIXED = 2800.0;
 
 template <bool A_K, bool B_K, int BN, int MT, int GLU = 0>
 gt_status launch(gt_ctx* ctx, const PartMaps& maps, long ntiles, int tma_store, float* c, int M, int N, int accum, int ksplit,
@@ -770,7 +1079,7 @@ static gt_status gemm_tc_dispatch(gt_ctx* ctx, int kind, int accum, int M, int N
   // the most work: waves x (K blocks x cycles per K block + epilogue)), calibrated on in-kernel cycle counts.
   struct Cfg { int mt, bn; };   // mt 1, 2: 128 / 256 rows on one CTA; mt 3: 256 rows on a CTA pair
   static const Cfg cfgs[6] = {{1, 192}, {1, 128}, {2, 256}, {2, 192}, {3, 192}, {3, 256}};
-  const char* force = getenv("GT_GEMM_TILE");   // "mt,bn": forces one tile shape (read per call so tests can switch it)
+  const char* force = getenv("GT_GEMM_TILE");   // "mt,bn": forces one tile shape (read per call so tests can switch it); mt 0: one tile per CTA
   const char* ds = getenv("GT_GEMM_DEEP_SPLIT");   // "0": never cut a product that already fills the SMs along K (for comparison)
   const bool deep_split = !(ds && ds[0] == '0');
   const int npairs = max(0, pair_capacity(ctx) - (ctx->sm_reserved + 1) / 2);
@@ -804,7 +1113,7 @@ static gt_status gemm_tc_dispatch(gt_ctx* ctx, int kind, int accum, int M, int N
                                 : 0.92 * ((bm * 128.0 + bn * 128.0) + mt * (BM1 * 128.0 + bn * 128.0)) / 128.0;
     const double per_kb = tensor > smem ? tensor : smem;
     const double epilogue = mt == 2 ? 14.0 * bn + 900.0 : 1500.0;
-    const double cost = gt_cdiv(tiles * ks, workers) * ((double)gt_cdiv(kblocks, ks) * per_kb + epilogue);
+    const double cost = gt_cdiv(tiles * ks, workers) * ((double)gt_cdiv(kblocks, ks) * per_kb + epilogue) + PERSISTENT_FIXED + (ks > 1 && !accum ? CLEAR_FIXED : 0.0);
     if (cost < best_cost) { best_cost = cost; best = i; ksplit = ks; }
     // A deep product whose tiles fill the SMs unevenly (the readout's dX: 384 tiles of 128 x 192 on 148 SMs are 2.6
     // waves, run as 3) may be cut along K as well when that evens the waves out: as 192 tiles of 256 x 192 in three
@@ -820,14 +1129,21 @@ static gt_status gemm_tc_dispatch(gt_ctx* ctx, int kind, int accum, int M, int N
         if (w2 < best_w - 0.05) { best_w = w2; k2best = k2; }
       }
       if (k2best > 1) {
-        const double c2 = gt_cdiv(tiles * k2best, workers) * ((double)gt_cdiv(kblocks, k2best) * per_kb + epilogue + 600.0) + 8000.0;
+        const double c2 = gt_cdiv(tiles * k2best, workers) * ((double)gt_cdiv(kblocks, k2best) * per_kb + epilogue + 600.0) + 8000.0 + PERSISTENT_FIXED;
         if (c2 < cost_deep) { cost_deep = c2; best_deep = i; ks_deep = k2best; }
       }
     }
   }
   if (cost_deep < 0.92 * best_cost) { best_cost = cost_deep; best = best_deep; ksplit = ks_deep; }
-  if (best_cost >= 1e30) return GT_OK;
-  const int mt = cfgs[best].mt, bn = cfgs[best].bn;
+  int fm = -1, fb = 0;
+  if (force && sscanf(force, "%d,%d", &fm, &fb) < 1) fm = -1;
+  SmallPick small;
+  if (fm <= 0)
+    small = pick_small(ctx, kblocks, [&](int b) { return (fm == 0 && fb && b != fb) ? 1l << 40 : (long)gt_cdiv(N, b) * gt_cdiv(M, BM1) * batch; }, 32);
+  const bool use_small = small.bn && small.cost < best_cost;
+  if (best_cost >= 1e30 && !use_small) return GT_OK;
+  if (use_small) ksplit = small.ks;
+  const int mt = use_small ? 1 : cfgs[best].mt, bn = use_small ? small.bn : cfgs[best].bn;
   const int a_box = mt == 2 ? 2 * BM1 : BM1, b_box = mt == 3 ? bn / 2 : bn;   // rows one TMA copy brings
   PartMaps maps;
   maps.nparts = nparts;
@@ -845,6 +1161,16 @@ static gt_status gemm_tc_dispatch(gt_ctx* ctx, int kind, int accum, int M, int N
   // the output goes through TMA (32x32 blocks of whole 128-byte rows) whenever its row pitch allows a tensor map
   const uint64_t sc = (uint64_t)M * N;
   maps.ngroups = 1;
+  if (use_small) {
+    maps.cp[0] = c;
+    const long tiles = (long)gt_cdiv(N, bn) * gt_cdiv(M, BM1) * batch;
+    gt_status s = bn == 32 ? launch_small_kind<32>(ctx, kind, maps, tiles, M, N, accum, ksplit, alpha * TRUNC_COMP)
+                : bn == 64 ? launch_small_kind<64>(ctx, kind, maps, tiles, M, N, accum, ksplit, alpha * TRUNC_COMP)
+                           : launch_small_kind<128>(ctx, kind, maps, tiles, M, N, accum, ksplit, alpha * TRUNC_COMP);
+    if (s) return s;
+    *handled = true;
+    return GT_OK;
+  }
   maps.c[0] = maps.a[0];
   const int tma_store = ((N & 3) == 0 && make_map_3d(&maps.c[0], c, N, M, batch, N, sc, 32, true)) ? 1 : 0;
   for (int p = 1; p < MAX_PARTS; p++) maps.c[p] = maps.c[0];
@@ -888,6 +1214,8 @@ static gt_status gemm_tc_grouped(gt_ctx* ctx, int kind, int ngroups, const int* 
   if (ctx->device < 0 || ctx->device >= 64 || !device_flag(ctx)) return GT_OK;
   const int kblocks = gt_cdiv(K, BK);
   const long workers = ctx->sm_count - ctx->sm_reserved;
+  int clears = 0;      // (one clear per product that does not accumulate)
+  for (int g = 0; g < ngroups; g++) clears += !accums[g];
   // 256 x 192 or 128 x 192 tiles; the split-K factor (one for the whole launch) that wastes least of the last wave,
   // among those that leave a slice at least 8 K blocks and add at most 8 partial sums per output element
   int best_mt = 1, best_ks = 1;
@@ -901,12 +1229,27 @@ static gt_status gemm_tc_grouped(gt_ctx* ctx, int kind, int ngroups, const int* 
     const double epilogue = mt == 2 ? 14.0 * 192 + 900.0 : 1500.0;
     for (int ks = 1; ks <= 8 && (ks == 1 || kblocks / ks >= 8); ks++) {
       const long waves = gt_cdiv(tiles * ks, workers);
-      const double cost = waves * (gt_cdiv(kblocks, ks) * per_kb + epilogue + (ks > 1 ? 600.0 : 0.0));
+      const double cost = waves * (gt_cdiv(kblocks, ks) * per_kb + epilogue + (ks > 1 ? 600.0 : 0.0)) + PERSISTENT_FIXED + (ks > 1 ? clears * CLEAR_FIXED : 0.0);
       if (cost < best_cost) { best_cost = cost; best_mt = mt; best_ks = ks; }
     }
   }
-  if (best_cost >= 1e30) return GT_OK;
-  const int mt = best_mt, ksplit = best_ks, bm = mt * BM1;
+  int fm = -1, fb = 0;
+  if (force && sscanf(force, "%d,%d", &fm, &fb) < 1) fm = -1;
+  // (outputs that could be whole heads take the tiles a rotation needs whether it is applied or not: its values then do not
+  // depend on where it runs)
+  bool heads64 = kind == GT_GEMM_NT;
+  for (int g = 0; g < ngroups; g++) heads64 = heads64 && (Ns[g] & 63) == 0;
+  SmallPick small;
+  if (fm <= 0)
+    small = pick_small(ctx, kblocks, [&](int b) {
+      if (fm == 0 && fb && b != fb) return 1l << 40;
+      long n = 0;
+      for (int g = 0; g < ngroups; g++) n += (long)gt_cdiv(Ns[g], b) * gt_cdiv(Ms[g], BM1);
+      return n;
+    }, any_rope || heads64 ? 64 : 32);
+  const bool use_small = small.bn && small.cost < best_cost;
+  if (best_cost >= 1e30 && !use_small) return GT_OK;
+  const int mt = use_small ? 1 : best_mt, ksplit = use_small ? small.ks : best_ks, bm = mt * BM1, bn = use_small ? small.bn : 192;
   PartMaps maps;
   maps.nparts = 1;
   maps.ngroups = ngroups;
@@ -914,10 +1257,11 @@ static gt_status gemm_tc_grouped(gt_ctx* ctx, int kind, int ngroups, const int* 
   for (int g = 0; g < ngroups; g++) {
     const int M = Ms[g], N = Ns[g];
     const bool oka = a_k ? make_map_3d(&maps.a[g], as[g], K, M, 1, K, (uint64_t)M * K, bm, true) : make_map_3d(&maps.a[g], as[g], M, K, 1, M, (uint64_t)M * K, BK, false);
-    const bool okb = b_k ? make_map_3d(&maps.b[g], bs[g], K, N, 1, K, (uint64_t)N * K, 192, true) : make_map_3d(&maps.b[g], bs[g], N, K, 1, N, (uint64_t)N * K, BK, false);
-    const bool okc = make_map_3d(&maps.c[g], cs[g], N, M, 1, N, (uint64_t)M * N, 32, true);
+    const bool okb = b_k ? make_map_3d(&maps.b[g], bs[g], K, N, 1, K, (uint64_t)N * K, bn, true) : make_map_3d(&maps.b[g], bs[g], N, K, 1, N, (uint64_t)N * K, BK, false);
+    const bool okc = use_small || make_map_3d(&maps.c[g], cs[g], N, M, 1, N, (uint64_t)M * N, 32, true);
     if (!oka || !okb || !okc) return GT_OK;
-    units += gt_cdiv(N, 192) * gt_cdiv(M, bm) * ksplit;
+    maps.cp[g] = cs[g];
+    units += gt_cdiv(N, bn) * gt_cdiv(M, bm) * (use_small ? 1 : ksplit);
     maps.unit_end[g] = units;
     maps.gM[g] = M; maps.gN[g] = N; maps.g_accum[g] = accums[g];
     maps.g_rope[g] = any_rope ? ropes[g] : 0;
@@ -925,6 +1269,17 @@ static gt_status gemm_tc_grouped(gt_ctx* ctx, int kind, int ngroups, const int* 
   }
   maps.rope_tab = rope_tab;
   maps.rope_period = rope_period;
+  if (use_small) {
+    const float scale = alpha * TRUNC_COMP;
+    gt_status s = any_rope ? (bn == 64 ? launch_small_kind<64, EPI_ROPE>(ctx, kind, maps, units, 0, 0, 0, ksplit, scale)
+                                       : launch_small_kind<128, EPI_ROPE>(ctx, kind, maps, units, 0, 0, 0, ksplit, scale))
+                : bn == 32 ? launch_small_kind<32>(ctx, kind, maps, units, 0, 0, 0, ksplit, scale)
+                : bn == 64 ? launch_small_kind<64>(ctx, kind, maps, units, 0, 0, 0, ksplit, scale)
+                           : launch_small_kind<128>(ctx, kind, maps, units, 0, 0, 0, ksplit, scale);
+    if (s) return s;
+    *handled = true;
+    return GT_OK;
+  }
   for (int g = ngroups; g < MAX_PARTS; g++) {
     maps.a[g] = maps.a[0]; maps.b[g] = maps.b[0]; maps.c[g] = maps.c[0];
     maps.unit_end[g] = units; maps.gM[g] = Ms[0]; maps.gN[g] = Ns[0]; maps.g_accum[g] = accums[0]; maps.kb_end[g] = kblocks;
@@ -957,6 +1312,32 @@ gt_status gt_glu_linear_tc(gt_ctx* ctx, int op, int rows, int ffn, int in, const
   maps.nparts = 1;
   maps.ngroups = 1;
   const int kblocks = gt_cdiv(in, BK);
+  const long workers = ctx->sm_count - ctx->sm_reserved;
+  const double cost = (double)gt_cdiv((long)gt_cdiv(ffn, BN / 2) * gt_cdiv(rows, BM1), workers) * (kblocks * 0.92 * 2.0 * (BM1 + BN) + 1500.0) + PERSISTENT_FIXED;
+  const SmallPick small = pick_small(ctx, kblocks, [&](int b) { return (long)gt_cdiv(ffn, b / 2) * gt_cdiv(rows, BM1); }, 32);
+  const char* force = getenv("GT_GEMM_TILE");
+  if (small.bn && small.cost < cost && (!force || force[0] == '0')) {
+    const int bn = small.bn;
+    if (!make_map_3d(&maps.a[0], x, in, rows, 1, in, (uint64_t)rows * in, BM1, true) ||
+        !make_map_3d(&maps.b[0], wg, in, ffn, 1, in, (uint64_t)ffn * in, bn / 2, true) ||
+        !make_map_3d(&maps.b[1], wu, in, ffn, 1, in, (uint64_t)ffn * in, bn / 2, true))
+      return GT_OK;
+    maps.kb_end[0] = kblocks;
+    maps.gN[0] = ffn;
+    maps.cp[0] = gate; maps.cp[1] = up; maps.cp[2] = out;
+    const long tiles = (long)gt_cdiv(ffn, bn / 2) * gt_cdiv(rows, BM1);
+    const int n2 = 2 * gt_cdiv(ffn, bn / 2) * (bn / 2);
+    gt_status s = GT_OK;
+#define GT_SMALL_GLU(B) s = op == GT_EW_SILU ? launch_small<true, true, B, GT_EW_SILU>(ctx, maps, tiles, rows, n2, 0, small.ks, TRUNC_COMP) \
+                                             : launch_small<true, true, B, GT_EW_GELU>(ctx, maps, tiles, rows, n2, 0, small.ks, TRUNC_COMP)
+    if (bn == 32) GT_SMALL_GLU(32);
+    else if (bn == 64) GT_SMALL_GLU(64);
+    else GT_SMALL_GLU(128);
+#undef GT_SMALL_GLU
+    if (s) return s;
+    *handled = true;
+    return GT_OK;
+  }
   bool ok = make_map_3d(&maps.a[0], x, in, rows, 1, in, (uint64_t)rows * in, BM1, true);
   ok = ok && make_map_3d(&maps.b[0], wg, in, ffn, 1, in, (uint64_t)ffn * in, BN / 2, true);
   ok = ok && make_map_3d(&maps.b[1], wu, in, ffn, 1, in, (uint64_t)ffn * in, BN / 2, true);
