@@ -30,15 +30,18 @@ constexpr int UMMA_K = 8;        // tf32: 32 bytes of K per instruction
 // bandwidth, not by the tensor pipe: every stage is written once by TMA and read by the MMAs once per 128-row
 // half, at 128 B/clk. A 256-row tile moves fewer bytes per flop (the B tile is fetched once for both halves), which
 // pays when the tile count still fills the SMs evenly; the host picks per product.
-template <int BN, int MT>
+// SUB epilogue warps share the rows of a TMEM lane quadrant and take turns at its column blocks: one for plain outputs, whose
+// epilogue hides under the next tile's main loop; three where the epilogue computes (the gated unit, the rotation): with one
+// it took 10 us a tile against 6 us of main loop at K 576 and set the pace (gate, up and the unit at 16384 rows: 137 us).
+template <int BN, int MT, int SUB = 1>
 struct Smem {
   static constexpr int BM = BM1 * MT;
   static constexpr int A_BYTES = BM * BK * 4;   // 16 / 32 KB
   static constexpr int B_BYTES = BN * BK * 4;
   static constexpr int STAGE = A_BYTES + B_BYTES;
   static constexpr int STAGES = MT == 2 ? 3 : (BN <= 128 ? 5 : 4);
-  static constexpr int EPI_WARPS = 4 * MT;
-  static constexpr int EPI_TILES = MT == 2 ? 1 : 2;   // 32x32 f32 staging tiles per epilogue warp for the TMA store
+  static constexpr int EPI_WARPS = 4 * MT * SUB;
+  static constexpr int EPI_TILES = MT == 2 || SUB > 1 ? 1 : 2;   // 32x32 f32 staging tiles per epilogue warp for the TMA store
   static constexpr int EPI_BYTES = EPI_WARPS * EPI_TILES * 4096;
   static constexpr int TOTAL = STAGES * STAGE + EPI_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
   static constexpr uint32_t TMEM_COLS = 2 * BN <= 256 ? 256 : 512;   // two accumulators (MT = 1) or two halves (MT = 2)
@@ -80,12 +83,15 @@ constexpr int EPI_ROPE = 8;   // a value of the kernel's GLU argument that is ne
 // 192-column tile is three whole heads; the thread that owns a row loads the two 32-column halves of a head, rotates
 // pair (j, j + 32) by the angle of (row's position, j) from the table, and both halves go out as they would have.
 // The unrotated projection is never written.
+template <int MT, int GLU>
+struct EpiSub { static constexpr int N = MT == 1 && GLU != 0 ? 3 : 1; };
 template <bool A_K, bool B_K, int BN, int MT, int GLU = 0>
-__global__ void __launch_bounds__(Smem<BN, MT>::THREADS, 1)
+__global__ void __launch_bounds__(Smem<BN, MT, EpiSub<MT, GLU>::N>::THREADS, 1)
 gemm_tf32_kernel(const __grid_constant__ PartMaps maps, float* __restrict__ C, int M_, int N_,
                  int accum_, int ksplit, int use_tma_store, int batch, float out_scale, int* __restrict__ flag) {
   extern __shared__ uint8_t smem_raw[];
-  using S = Smem<BN, MT>;
+  constexpr int SUB = EpiSub<MT, GLU>::N;
+  using S = Smem<BN, MT, SUB>;
   const int M = M_, N = N_;   // (of the single product; a grouped launch takes each group's from `maps`)
   constexpr int STAGES = S::STAGES, BM = S::BM;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -136,7 +142,7 @@ gemm_tf32_kernel(const __grid_constant__ PartMaps maps, float* __restrict__ C, i
     if (use_tma_store)
       for (int g = 0; g < ngroups; g++) tma_prefetch_map(&maps.c[g]);
     for (int s = 0; s < STAGES; s++) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 128); }
+    for (int b = 0; b < 2; b++) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 128 * SUB); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(tmem_slot, S::TMEM_COLS);
@@ -219,7 +225,7 @@ gemm_tf32_kernel(const __grid_constant__ PartMaps maps, float* __restrict__ C, i
     }
   } else {
     // ---- epilogue: warp w may touch TMEM lanes [32*(w%4), 32*(w%4)+32) ----
-    const int q = warp & 3, ew = warp - 2, half = ew >> 2;
+    const int q = warp & 3, ew = warp - 2, half = MT == 2 ? ew >> 2 : 0, sub = MT == 2 ? 0 : ew >> 2;
     const bool vec = (N & 3) == 0;
     uint32_t tl = 0, nst = 0;   // nst: TMA stores issued by this warp
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, tl++) {
@@ -251,7 +257,7 @@ gemm_tf32_kernel(const __grid_constant__ PartMaps maps, float* __restrict__ C, i
           nst++;
         };
 #pragma unroll 1
-        for (int c = 0; c < BN / 64; c++) {
+        for (int c = sub; c < BN / 64; c += SUB) {
           const int col0 = (n0 >> 1) + c * 32;
           if (col0 >= (N >> 1)) break;   // uniform across the warp
           float vg[32], vu[32];
@@ -294,7 +300,7 @@ gemm_tf32_kernel(const __grid_constant__ PartMaps maps, float* __restrict__ C, i
         // (cos, sin) of this row's position, pairs 0..31; rows past M are clipped by the store and read row M - 1's
         const float4* tab4 = reinterpret_cast<const float4*>(maps.rope_tab + (size_t)((row < M ? row : M - 1) % maps.rope_period) * 32);
 #pragma unroll 1
-        for (int c = 0; c < BN / 64; c++) {
+        for (int c = sub; c < BN / 64; c += SUB) {
           const int col0 = n0 + c * 64;
           if (col0 >= N) break;   // uniform across the warp
           float v0[32], v1[32];
@@ -316,7 +322,7 @@ gemm_tf32_kernel(const __grid_constant__ PartMaps maps, float* __restrict__ C, i
         }
       } else if (have) {
 #pragma unroll 1
-        for (int c = 0; c < BN / 32; c++) {
+        for (int c = sub; c < BN / 32; c += SUB) {
           const int col0 = n0 + c * 32;
           if (col0 >= N) break;   // uniform across the warp
           float v[32];
@@ -885,7 +891,7 @@ template <bool A_K, bool B_K, int BN, int MT, int GLU = 0>
 gt_status launch(gt_ctx* ctx, const PartMaps& maps, long ntiles, int tma_store, float* c, int M, int N, int accum, int ksplit,
                  int batch, float out_scale) {
   auto kern = gemm_tf32_kernel<A_K, B_K, BN, MT, GLU>;
-  using S = Smem<BN, MT>;
+  using S = Smem<BN, MT, EpiSub<MT, GLU>::N>;
   static bool attr_set[64] = {};
   if (!attr_set[ctx->device]) {
     GT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL));
