@@ -450,7 +450,10 @@ __global__ void attn_bwd_d_tc_kernel(long nitems, float scale, const float* __re
 // ---- dK, dV: CTA = 128 keys of one kv head; loop over the group's query heads and over blocks of NQ queries ----
 // Transposed products so that keys are the rows: S^T = K.Q^T and dP^T = V.dO^T (M=128 keys, N=NQ queries); then
 // dV += P^T.dO and dK += dS^T.Q with P^T, dS^T written to shared memory as K-major A operands (K = queries) and
-// dO, Q read a second time as [queries, hd] operands (hd contiguous). KBUF = 2 keeps two blocks of the K-major
+// dO, Q read a second time as [queries, hd] operands (hd contiguous). With `hs` > 1 the query heads of the group are dealt
+// out to a cluster of hs CTAs (pairs of CTAs at head size 256), which add their dK and dV through distributed shared
+// memory at the end: three sequences of 777 tokens with 3 kv heads are 63 tiles, and with one CTA each 85 SMs had
+// nothing to do (80 us; as 189 CTAs 41 us). KBUF = 2 keeps two blocks of the K-major
 // Q / dO copies in flight (their fetch is the longest latency of the loop) where shared memory has the room.
 template <int HD, int NQ, int KBUF, int MBUF, int SPLIT>
 struct DkvSmem {
@@ -472,7 +475,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_co
                        const __grid_constant__ CUtensorMap mapGk, const __grid_constant__ CUtensorMap mapGm,
                        const float* __restrict__ lse, const float* __restrict__ Ds, float* gk, int accum_k, float* gv, int accum_v,
                        int rows, int T, int Hq, int Hkv, int window, float scale2, float dp_scale, const float2* __restrict__ rope,
-                       const int* __restrict__ order, int* __restrict__ flag) {
+                       const int* __restrict__ order, int hs, int* __restrict__ flag) {
   extern __shared__ uint8_t smem_raw[];
   using S = DkvSmem<HD, NQ, KBUF, MBUF, SPLIT>;
   constexpr int ATOMS = HD / 32, NH = NQ / 2, HH = HD / 2, HDF = HD * SPLIT;
@@ -498,9 +501,10 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_co
     tile_x = lin % (int)gridDim.x;
   }
   const int k0 = tile_y * ROWS;
-  const int crank = SPLIT == 2 ? (int)(tile_x & 1) : 0, bx = tile_x / SPLIT;   // which half of the head; tile
+  const int crank = SPLIT == 2 ? (int)(tile_x & 1) : 0;    // which half of the head
+  const int hsub = tile_x / SPLIT % hs, bx = tile_x / SPLIT / hs;   // which share of the group's heads; tile
   const int kvh = bx % Hkv, seq = bx / Hkv;
-  const int group = Hq / Hkv;
+  const int group = Hq / Hkv / hs, h_first = kvh * (Hq / Hkv) + hsub * group;
   const int row0 = seq * T;
   const int k_last = min(k0 + ROWS - 1, T - 1);
   const int q_max = (window > 0) ? min(T - 1, k_last + window - 1) : T - 1;
@@ -528,7 +532,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_co
   const uint32_t tm_dv = tmem + 4 * NQ, tm_dk = tmem + 4 * NQ + HD;
   Waiter w{false, flag};
   PairSum xs;
-  if (SPLIT == 2 && warp < MATH_WARPS) xs.init(base + S::XC_OFF, base_ptr + S::XC_OFF, x_full + 8 * warp, x_free + 8 * warp, (uint32_t)(crank ^ 1));
+  if (SPLIT == 2 && warp < MATH_WARPS) xs.init(base + S::XC_OFF, base_ptr + S::XC_OFF, x_full + 8 * warp, x_free + 8 * warp, cluster_ctarank() ^ 1u);
   // barrier and parity of the K-major copies of block `it`, and of its score products
   auto qk_bar = [&](int it) { return (KBUF == 2 && (it & 1)) ? qk_full1 : qk_full0; };
   auto qk_par = [&](int it) { return (uint32_t)((KBUF == 2 ? it >> 1 : it) & 1); };
@@ -546,7 +550,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_co
     if (lane == 0) {
       // Both copies are requested block after block, so (head, query block) of the next request is kept by counting:
       // a division by the run-time block count costs this single thread more than the copy instructions themselves.
-      int k_h = kvh * group, k_qb = 0, m_h = kvh * group, m_qb = 0;
+      int k_h = h_first, k_qb = 0, m_h = h_first, m_qb = 0;
       auto load_k = [&](int it) {   // K-major copies of Q and dO, block `it` (called with it = 0, 1, 2, ...)
         const int qr = row0 + (qb_lo + k_qb) * NQ;
         const uint32_t bar = qk_bar(it), off = (KBUF == 2 && (it & 1)) ? S::QT_BYTES : 0;
@@ -638,7 +642,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_co
     const int qd = warp & 3, half = warp >> 2;
     const int kg = k0 + qd * 32 + lane;      // key position in the sequence: one row of the tile per thread
     const uint32_t lane_base = (uint32_t)(qd * 32) << 16;
-    int c_h = kvh * group, c_qb = 0;         // (head, query block) of block i, kept by counting
+    int c_h = h_first, c_qb = 0;         // (head, query block) of block i, kept by counting
     for (int i = 0; i < iters; i++) {
       const int h = c_h;
       const int qpos0 = (qb_lo + c_qb) * NQ + half * NH;         // first query of this thread's columns
@@ -699,11 +703,22 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_co
       mbar_arrive(p_bar(i));
     }
     RopeRow<HD >= 64 ? HH : 32> rr;   // (unused below head size 64: the host then launches the rotation's backward itself)
-    const bool roped = SPLIT == 1 && HD >= 64 && rope != nullptr && gk != nullptr;
+    const bool roped = SPLIT == 1 && HD >= 64 && rope != nullptr && gk != nullptr && hs == 1;
     if (roped) rr.fetch(rope + (size_t)(kg < T ? kg : 0) * HH, half);
     w.wait(all_done, 0, 28);
     tc_fence_after();
-    {   // warp-uniform: the TMEM loads are warp-wide instructions, only the stores are per-row
+    if (hs > 1) {   // this CTA's heads into shared memory (every operand tile has been read for the last time)
+      const int r = qd * 32 + lane;
+      float* part = reinterpret_cast<float*>(base_ptr);
+#pragma unroll
+      for (int m = 0; m < 2; m++) {
+        float t[HH];
+        tmem_ld<HH>((m ? tm_dk : tm_dv) + half * HH + lane_base, t);
+        float* dst = part + (m * ROWS + r) * (HD + 4) + half * HH;
+#pragma unroll
+        for (int d = 0; d < HH; d += 4) *reinterpret_cast<float4*>(dst + d) = make_float4(t[d], t[d + 1], t[d + 2], t[d + 3]);
+      }
+    } else {   // warp-uniform: the TMEM loads are warp-wide instructions, only the stores are per-row
       const bool st = !w.dead && kg < T;
       const size_t off = (size_t)(row0 + (kg < T ? kg : 0)) * Hkv * HDF + (size_t)kvh * HDF + crank * HD + half * HH;
       float t[HH];
@@ -736,7 +751,46 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_co
     }
   }
   tc_fence_before();
-  if (SPLIT == 2) cluster_sync_all(); else __syncthreads();   // neither CTA of a pair leaves while the other may still write to it
+  if (hs > 1) {
+    static_assert(2 * ROWS * (HD + 4) * 4 <= S::XC_OFF, "partial dK and dV");
+    __syncwarp();
+    cluster_sync_all();            // every share is in place
+    const bool dead = __any_sync(0xffffffffu, w.dead);
+    // rows x 16-byte columns of dV, then of dK, dealt out to the CTAs of the cluster
+    auto sum = [&](int m, int r, int col) {
+      float4 v[8];
+#pragma unroll
+      for (int c = 0; c < 8; c++)
+        if (c < hs) v[c] = ld_cluster_f32x4(cluster_addr_of(base + (uint32_t)((m * ROWS + r) * (HD + 4) + col) * 4u, (uint32_t)(c * SPLIT + crank)));
+      float4 t = v[0];
+#pragma unroll
+      for (int c = 1; c < 8; c++)
+        if (c < hs) { t.x += v[c].x; t.y += v[c].y; t.z += v[c].z; t.w += v[c].w; }
+      return make_float4(t.x * TRUNC_COMP, t.y * TRUNC_COMP, t.z * TRUNC_COMP, t.w * TRUNC_COMP);
+    };
+    auto put = [&](float* g, int accum, int r, int col, float4 v) {
+      float* dst = g + (size_t)(row0 + k0 + r) * Hkv * HDF + (size_t)kvh * HDF + crank * HD + col;
+      if (accum) { const float4 o = *reinterpret_cast<const float4*>(dst); v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w; }
+      *reinterpret_cast<float4*>(dst) = v;
+    };
+    const int nrows = dead ? 0 : min(ROWS, T - k0), step = hs * THREADS, first = hsub * THREADS + (int)threadIdx.x;
+    if (gv)
+      for (int e = first; e < nrows * (HD / 4); e += step) put(gv, accum_v, e / (HD / 4), e % (HD / 4) * 4, sum(0, e / (HD / 4), e % (HD / 4) * 4));
+    if (gk && rope != nullptr) {   // pairs (j, j + HD / 2) rotated back together
+      for (int e = first; e < nrows * (HD / 8); e += step) {
+        const int r = e / (HD / 8), col = e % (HD / 8) * 4;
+        const float4 a = sum(1, r, col), b = sum(1, r, col + HH);
+        const float4* cs = reinterpret_cast<const float4*>(rope + (size_t)(k0 + r) * HH + col);
+        const float4 u = __ldg(cs), q = __ldg(cs + 1);
+        put(gk, accum_k, r, col, make_float4(u.x * a.x + u.y * b.x, u.z * a.y + u.w * b.y, q.x * a.z + q.y * b.z, q.z * a.w + q.w * b.w));
+        put(gk, accum_k, r, col + HH, make_float4(u.x * b.x - u.y * a.x, u.z * b.y - u.w * a.y, q.x * b.z - q.y * a.z, q.z * b.w - q.w * a.w));
+      }
+    } else if (gk) {
+      for (int e = first; e < nrows * (HD / 4); e += step) put(gk, accum_k, e / (HD / 4), e % (HD / 4) * 4, sum(1, e / (HD / 4), e % (HD / 4) * 4));
+    }
+    __syncwarp();
+  }
+  if (SPLIT == 2 || hs > 1) cluster_sync_all(); else __syncthreads();   // no CTA of a cluster leaves while another may still read or write its memory
   if (warp == MMA_WARP) {
     tc_fence_after();
     tmem_dealloc(tmem, S::TMEM_COLS);
@@ -1084,6 +1138,39 @@ gt_status attn_dkv_order(gt_ctx* ctx, int nkb, int ntx, int group, int T, int NQ
   return GT_OK;
 }
 
+// How many CTAs (pairs at head size 256) share the query heads of a dK/dV tile. In iterations of a tile's loop: the launch
+// ends at the mean load of an SM or with the longest tile, plus 15 % of the latter where tiles are handed out heaviest first
+// (5 % where they are packed, see attn_dkv_order). A share costs its own start and end (3 iterations) and the sum over
+// the cluster (2 more on the critical path, 7 of an SM's time). More than one is taken when predicted 15 % ahead: 1 x 256
+// tokens of 9/3 heads of 64 27.6 -> 14.3 us, 2 x 500 of 16/8 of 128 58 -> 35, 3 x 400 of 4/1 of 256 148 -> 45; at 8 x 2048
+// of 4/1 of 256 one CTA per tile stays ahead, 709 against 906.
+int dkv_head_split(gt_ctx* ctx, int Hkv, int group, int nseq, int T, int NQ, int window, int split) {
+  const char* force = getenv("GT_ATTN_HEAD_SPLIT");
+  double total = 0.0, longest = 0.0;
+  const int nkb = gt_cdiv(T, ROWS), tiles = nkb * Hkv * nseq;
+  for (int kb = 0; kb < nkb; kb++) {
+    const int k0 = kb * ROWS, k_last = min(k0 + ROWS - 1, T - 1);
+    const int q_max = window > 0 ? min(T - 1, k_last + window - 1) : T - 1;
+    const double n = (double)(q_max / NQ - k0 / NQ + 1) * group;
+    total += n * Hkv * nseq;
+    longest = n > longest ? n : longest;
+  }
+  const double slots = (double)(ctx->sm_count / split);
+  int best = 1;
+  double best_cost = 1e30;
+  for (int hs = 1; hs <= group && hs * split <= 8; hs++) {
+    if (group % hs) continue;
+    if (force && atoi(force) == hs) return hs;
+    const double tile = longest / hs + (hs > 1 ? 5.0 : 3.0);
+    const double mean = (total + (hs > 1 ? 10.0 : 3.0) * tiles * hs) / slots;
+    const double tail = hs == 1 && split == 1 && tiles > ctx->sm_count ? 0.05 : 0.15;
+    double cost = (mean > tile ? mean : tile) + tail * tile;
+    if (hs > 1) cost /= 0.85;
+    if (cost < best_cost) { best_cost = cost; best = hs; }
+  }
+  return best;
+}
+
 template <int HD, int NQ, int NK, int DKV_KBUF, int DKV_MBUF, int DQ_KBUF, bool DQ_SB, int SPLIT>
 gt_status launch_bwd(gt_ctx* ctx, int rows, int T, int Hq, int Hkv, int window, const float* q, const float* k, const float* v,
                      const float* out, const float* lse, const float* go, float* gq, int accum_q, float* gk, int accum_k, float* gv,
@@ -1112,18 +1199,15 @@ gt_status launch_bwd(gt_ctx* ctx, int rows, int T, int Hq, int Hkv, int window, 
     static bool done[64] = {};
     st = set_smem(ctx, kern, SM::TOTAL, done);
     if (st) return st;
-    dim3 grid(Hkv * nseq * SPLIT, gt_cdiv(T, ROWS), 1);
+    const int hs = dkv_head_split(ctx, Hkv, Hq / Hkv, nseq, T, NQ, window, SPLIT);
+    dim3 grid(Hkv * nseq * SPLIT * hs, gt_cdiv(T, ROWS), 1);
     const int* order = nullptr;
-    if (SPLIT == 1 && (int)(grid.x * grid.y) > ctx->sm_count && !getenv("GT_ATTN_INDEX_ORDER")) {   // (the variable keeps index order, for comparison)
+    if (SPLIT == 1 && hs == 1 && (int)(grid.x * grid.y) > ctx->sm_count && !getenv("GT_ATTN_INDEX_ORDER")) {   // (the variable keeps index order, for comparison)
       st = attn_dkv_order(ctx, (int)grid.y, (int)grid.x, Hq / Hkv, T, NQ, window, &order);
       if (st) return st;
     }
-    if (SPLIT == 1)
-      kern<<<grid, THREADS, SM::TOTAL, ctx->stream>>>(mK, mV, mQk, mQm, mGk, mGm, lse, D, gk, accum_k, gv, accum_v, rows, T, Hq, Hkv, window, scale2,
-                                                      dp_scale, rope, order, flag);
-    else
-      GT_CUDA(ctx, launch_split(kern, grid, THREADS, SM::TOTAL, ctx->stream, SPLIT, mK, mV, mQk, mQm, mGk, mGm, lse, D, gk, accum_k, gv, accum_v,
-                                rows, T, Hq, Hkv, window, scale2, dp_scale, rope, order, flag));
+    GT_CUDA(ctx, launch_split(kern, grid, THREADS, SM::TOTAL, ctx->stream, SPLIT * hs, mK, mV, mQk, mQm, mGk, mGm, lse, D, gk, accum_k, gv, accum_v,
+                              rows, T, Hq, Hkv, window, scale2, dp_scale, rope, order, hs, flag));
     GT_LAUNCHED(ctx, "attn_bwd_dkv_tc_kernel");
   }
   if (gq) {

@@ -595,12 +595,6 @@ struct SmallSmem {
   static_assert(BM1 * PITCH * 4 <= STAGES * STAGE && TOTAL <= 232448, "shared memory");
 };
 
-__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));   // (ordered after the cluster barrier, which is volatile too)
-  return v;
-}
-
 // EPI: 0, GT_EW_SILU, GT_EW_GELU (gate, up and the gated unit) or EPI_ROPE, as in gemm_tf32_kernel. gridDim.x = tiles x ksplit,
 // the slices of a tile adjacent and one cluster.
 template <bool A_K, bool B_K, int BN, int EPI>

@@ -14,25 +14,35 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Column sums for dw, two ways. Atomic: warps add into the CTA's shared array and CTAs into gw with f32 atomics, in
-// whatever order they arrive (the tensor-core modes, whose split-K products are order-dependent anyway). Ordered
-// (`part` given; strict-f32 mode): warps add one after the other, each CTA stores its sums to part[cta][d], and the
-// CTA that arrives last (a counter it leaves at zero again) adds the CTAs' rows in index order on top of gw or of
-// zero: the same bits on every run, which is what lets a recompute step equal a plain one bit for bit.
-template <typename AddOwn>
-__device__ __forceinline__ void dw_finish(float* sdw, int d, float* gw, int accum_w, float* part, int* counter, AddOwn add_own) {
-  if (part == nullptr) {
-    add_own(true);
-    __syncthreads();
-    for (int j = threadIdx.x; j < d; j += blockDim.x) atomicAdd(&gw[j], sdw[j]);
-    return;
-  }
+// Column sums for dw. Every warp leaves its sums in a row of its own in shared memory and the CTA's threads add the rows in
+// warp order (adding them in place with shared-memory atomics made 16 warps queue up for the same words: 7 us of a
+// backward pass over 256 rows of 576); where the rows do not fit, the warps add one after the other. The CTAs' sums meet
+// in one of two ways. Atomic: f32 atomics on gw in whatever order they arrive (many CTAs in the tensor-core modes, whose
+// split-K products are order-dependent anyway). Ordered (`part` given; strict-f32 mode, and any launch of few CTAs, which
+// then needs no clear before it): each CTA stores its sums to part[cta][d], and the CTA that arrives last (a counter it
+// leaves at zero again) adds the CTAs' rows in index order on top of gw or of zero: the same bits on every run, which is
+// what lets a recompute step equal a plain one bit for bit.
+// `put(dst, add)`: this lane's sums into dst[column], overwriting or adding.
+template <typename Put>
+__device__ __forceinline__ void dw_finish(float* sdw, int d, int warp_rows, float* gw, int accum_w, float* part, int* counter, Put put) {
   const int wcta = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int wi = 0; wi < nw; wi++) {
-    if (wcta == wi) add_own(false);
+  if (warp_rows) {
+    put(sdw + wcta * d, false);
     __syncthreads();
+  } else {
+    for (int wi = 0; wi < nw; wi++) {
+      if (wcta == wi) put(sdw, wi > 0);
+      __syncthreads();
+    }
   }
-  for (int j = threadIdx.x; j < d; j += blockDim.x) part[(size_t)blockIdx.x * d + j] = sdw[j];
+  const int n = warp_rows ? nw : 1;
+  for (int j = threadIdx.x; j < d; j += blockDim.x) {
+    float acc = sdw[j];
+    for (int wi = 1; wi < n; wi++) acc += sdw[wi * d + j];
+    if (part) part[(size_t)blockIdx.x * d + j] = acc;
+    else atomicAdd(&gw[j], acc);
+  }
+  if (!part) return;
   __threadfence();
   __shared__ int s_last;
   __syncthreads();
@@ -42,6 +52,7 @@ __device__ __forceinline__ void dw_finish(float* sdw, int d, float* gw, int accu
   __threadfence();
   for (int j = threadIdx.x; j < d; j += blockDim.x) {
     float acc = accum_w ? gw[j] : 0.f;
+#pragma unroll 8
     for (unsigned b = 0; b < gridDim.x; b++) acc += __ldcg(&part[(size_t)b * d + j]);
     gw[j] = acc;
   }
@@ -186,15 +197,11 @@ template <int NPL>
 __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(int rows, int d, const float* __restrict__ x,
                                                           const float* __restrict__ w, const float* __restrict__ rinv,
                                                           const float* __restrict__ g, const float* gadd, float* gx, int accum_x,
-                                                          float* gw, int accum_w, float* part, int* counter) {
-  extern __shared__ float sdw[];  // [d] block-level column partials
+                                                          float* gw, int accum_w, int warp_rows, float* part, int* counter) {
+  extern __shared__ float sdw[];  // column sums: [warps][d], or [d]
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  if (gw) {
-    for (int j = threadIdx.x; j < d; j += blockDim.x) sdw[j] = 0.f;
-    __syncthreads();
-  }
   float wv[NPL], dwv[NPL];
 #pragma unroll
   for (int i = 0; i < NPL; i++) { int j = lane + 32 * i; wv[i] = j < d ? w[j] : 0.f; dwv[i] = 0.f; }
@@ -230,11 +237,11 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(int rows, int d, const
     for (int i = 0; i < NPL; i++) dwv[i] = fmaf(gv[i] * xv[i], r, dwv[i]);
   }
   if (gw) {
-    dw_finish(sdw, d, gw, accum_w, part, counter, [&](bool atomic) {
+    dw_finish(sdw, d, warp_rows, gw, accum_w, part, counter, [&](float* dst, bool add) {
 #pragma unroll
       for (int i = 0; i < NPL; i++) {
         int j = lane + 32 * i;
-        if (j < d) { if (atomic) atomicAdd(&sdw[j], dwv[i]); else sdw[j] += dwv[i]; }
+        if (j < d) dst[j] = add ? dst[j] + dwv[i] : dwv[i];
       }
     });
   }
@@ -246,16 +253,12 @@ template <int V4, int TH>
 __global__ void __launch_bounds__(TH) rmsnorm_bwd_vec_kernel(int rows, int d, const float* __restrict__ x, const float* __restrict__ w,
                                                               const float* __restrict__ rinv, const float* __restrict__ g,
                                                               const float* gadd, float* gx, int accum_x, float* gw, int accum_w,
-                                                              float* part, int* counter) {
-  extern __shared__ float sdw[];
+                                                              int warp_rows, float* part, int* counter) {
+  extern __shared__ __align__(16) float sdw[];
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int d4 = d >> 2;
-  if (gw) {
-    for (int j = threadIdx.x; j < d; j += blockDim.x) sdw[j] = 0.f;
-    __syncthreads();
-  }
   float4 wv[V4], dwv[V4];
 #pragma unroll
   for (int i = 0; i < V4; i++) {
@@ -309,27 +312,28 @@ __global__ void __launch_bounds__(TH) rmsnorm_bwd_vec_kernel(int rows, int d, co
     }
   }
   if (gw) {
-    dw_finish(sdw, d, gw, accum_w, part, counter, [&](bool atomic) {
+    dw_finish(sdw, d, warp_rows, gw, accum_w, part, counter, [&](float* dst, bool add) {
 #pragma unroll
       for (int i = 0; i < V4; i++) {
         const int j = lane + 32 * i;
         if (j < d4) {
-          if (atomic) {
-            atomicAdd(&sdw[4 * j + 0], dwv[i].x); atomicAdd(&sdw[4 * j + 1], dwv[i].y);
-            atomicAdd(&sdw[4 * j + 2], dwv[i].z); atomicAdd(&sdw[4 * j + 3], dwv[i].w);
-          } else {
-            sdw[4 * j + 0] += dwv[i].x; sdw[4 * j + 1] += dwv[i].y; sdw[4 * j + 2] += dwv[i].z; sdw[4 * j + 3] += dwv[i].w;
-          }
+          float4* o = reinterpret_cast<float4*>(dst) + j;
+          const float4 v = dwv[i];
+          if (add) { const float4 p = *o; *o = make_float4(p.x + v.x, p.y + v.y, p.z + v.z, p.w + v.w); }
+          else *o = v;
         }
       }
     });
   }
 }
 
+constexpr int FEW_CTAS = 32;
+int warp_rows_fit(int threads, int d) { return (size_t)(threads / 32) * d * sizeof(float) <= 48 * 1024 ? threads / 32 : 0; }
+
 // Prepares dw's accumulation: ordered mode gets the per-CTA partial rows (context scratch) and the arrival counter;
 // atomic mode clears gw first unless it accumulates.
 gt_status dw_mode(gt_ctx* ctx, int blocks, int d, float* gw, int accum_w, bool ordered, float** part, int** counter) {
-  if (ordered) {
+  if (ordered || blocks <= FEW_CTAS) {
     int* flags = gt_flags(ctx);
     if (!flags) return gt_fail(ctx, GT_ERR_STATE, "gt_rmsnorm_bwd: first use inside a graph capture; run the step once eagerly first");
     gt_status s = gt_scratch(ctx, sizeof(float) * (size_t)blocks * d, part);
@@ -354,7 +358,8 @@ gt_status launch_bwd_vec(gt_ctx* ctx, int rows, int d, const float* x, const flo
     gt_status s = dw_mode(ctx, blocks, d, gw, accum_w, ordered, &part, &counter);
     if (s) return s;
   }
-  rmsnorm_bwd_vec_kernel<V4, TH><<<blocks, TH, sizeof(float) * d, ctx->stream>>>(rows, d, x, w, rinv, g, gadd, gx, accum_x, gw, accum_w, part, counter);
+  const int wr = warp_rows_fit(TH, d);
+  rmsnorm_bwd_vec_kernel<V4, TH><<<blocks, TH, sizeof(float) * d * max(wr, 1), ctx->stream>>>(rows, d, x, w, rinv, g, gadd, gx, accum_x, gw, accum_w, wr, part, counter);
   GT_LAUNCHED(ctx, "rmsnorm_bwd_vec_kernel");
   return GT_OK;
 }
@@ -386,7 +391,8 @@ gt_status launch_bwd(gt_ctx* ctx, int rows, int d, const float* x, const float* 
     gt_status s = dw_mode(ctx, blocks, d, gw, accum_w, ordered, &part, &counter);
     if (s) return s;
   }
-  rmsnorm_bwd_kernel<NPL><<<blocks, 256, sizeof(float) * d, ctx->stream>>>(rows, d, x, w, rinv, g, gadd, gx, accum_x, gw, accum_w, part, counter);
+  const int wr = warp_rows_fit(256, d);
+  rmsnorm_bwd_kernel<NPL><<<blocks, 256, sizeof(float) * d * max(wr, 1), ctx->stream>>>(rows, d, x, w, rinv, g, gadd, gx, accum_x, gw, accum_w, wr, part, counter);
   GT_LAUNCHED(ctx, "rmsnorm_bwd_kernel");
   return GT_OK;
 }
