@@ -8,11 +8,18 @@ implementations here: with no backend installed every op raises. The device work
 """
 from __future__ import annotations
 
+import itertools
+import operator
 from typing import Callable, Dict, List, Optional, Sequence
 
 import numpy as np
 
-_tensors_created = 0
+_tensors_created = itertools.count()
+_new = object.__new__
+
+
+def _noop():
+    return None
 
 
 class Tensor:
@@ -26,7 +33,6 @@ class Tensor:
     __slots__ = ("_data", "_grad", "size", "shape", "requiresGrad", "_backward", "_prev", "seq", "_dev", "_needs", "__weakref__")
 
     def __init__(self, data: Optional[np.ndarray], shape: Sequence[int], requiresGrad: bool = False):
-        global _tensors_created
         n = 1
         for s in shape:
             n *= int(s)
@@ -35,30 +41,26 @@ class Tensor:
             if data.size != n:
                 raise ValueError(f"data length {data.size} != shape {list(shape)}")
         self._data = data
-        self._grad = None
+        self._grad = self._dev = None
+        self._needs = False
         self.size = n
         self.shape = [int(s) for s in shape]
         self.requiresGrad = requiresGrad
         self._backward: Callable[[], None] = _noop
         self._prev: List["Tensor"] = []
-        self._dev = None
-        self._needs = False
-        self.seq = _tensors_created
-        _tensors_created += 1
+        self.seq = next(_tensors_created)
 
     @staticmethod
     def output(shape: List[int], size: int, prev: List["Tensor"]) -> "Tensor":
         """The output of a backend's op: `zeros(shape)` recorded on `prev`, for a backend that has the element count."""
-        global _tensors_created
-        t = Tensor.__new__(Tensor)
+        t = _new(Tensor)
         t._data = t._grad = t._dev = None
-        t.size = size
-        t.shape = shape
         t.requiresGrad = t._needs = False
         t._backward = _noop
+        t.size = size
+        t.shape = shape
         t._prev = prev
-        t.seq = _tensors_created
-        _tensors_created += 1
+        t.seq = next(_tensors_created)
         return t
 
     @staticmethod
@@ -101,28 +103,29 @@ class Tensor:
             self._grad.fill(0)
 
 
-def _noop():
-    return None
+_by_seq = operator.attrgetter("seq")
+
+
+def _latest_first(root: Tensor, done: set) -> List[Tensor]:
+    """Everything `root` was computed from except what `done` (ids) already has, latest first. A tensor is created after its
+    inputs, so this is a reverse topological order."""
+    found: List[Tensor] = []
+    stack = [root] if id(root) not in done else []
+    while stack:
+        t = stack.pop()
+        if id(t) not in done:
+            done.add(id(t))
+            found.append(t)
+            stack.extend(t._prev)
+    found.sort(key=_by_seq, reverse=True)
+    return found
 
 
 def backward(loss: Tensor, seed: float = 1.0):
     """src/model/autograd.ts:81-93: reverse topological walk seeded with loss.grad[0] = seed."""
-    topo: List[Tensor] = []
-    seen = set()
-    stack = [(loss, 0)]
-    seen.add(id(loss))
-    while stack:
-        t, i = stack.pop()
-        if i < len(t._prev):
-            stack.append((t, i + 1))
-            p = t._prev[i]
-            if id(p) not in seen:
-                seen.add(id(p))
-                stack.append((p, 0))
-        else:
-            topo.append(t)
+    order = _latest_first(loss, set())
     loss.grad[0] = seed
-    for t in reversed(topo):
+    for t in order:
         t._backward()
 
 
@@ -179,7 +182,7 @@ def checkpoint(inputs: List[Tensor], fn: Callable[[], Tensor]) -> Tensor:
     if not _checkpointing:
         return fn()
     rb = _ops_backend if (_ops_backend is not None and hasattr(_ops_backend, "beginRegion")) else None
-    born = _tensors_created
+    born = next(_tensors_created)
     mark = rb.beginRegion() if rb else 0
     tok = rb.regionToken() if (rb is not None and hasattr(rb, "regionToken")) else None   # optional backend extension
     out = fn()
@@ -197,23 +200,7 @@ def checkpoint(inputs: List[Tensor], fn: Callable[[], Tensor]) -> Tensor:
             rb.seedGradFrom(replay, out)
         else:
             replay.grad[:] = out.grad
-        topo: List[Tensor] = []
-        seen = {id(t) for t in inputs}
-        stack = []
-        if id(replay) not in seen:
-            seen.add(id(replay))
-            stack.append((replay, 0))
-        while stack:
-            t, i = stack.pop()
-            if i < len(t._prev):
-                stack.append((t, i + 1))
-                p = t._prev[i]
-                if id(p) not in seen:
-                    seen.add(id(p))
-                    stack.append((p, 0))
-            else:
-                topo.append(t)
-        for t in reversed(topo):
+        for t in _latest_first(replay, {id(t) for t in inputs}):
             t._backward()
         if rb:
             rb.endRegion(mark2, [])

@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import ctypes as C
 import itertools
+from functools import partial
 import weakref
 from typing import Dict, List, Optional, Sequence
 
@@ -38,16 +39,16 @@ _U64 = [None] + [C.c_uint64 * n for n in range(1, 9)]
 
 class _Entry:
     __slots__ = ("owner", "needs", "region", "data", "grad", "bytes", "external", "gradLive", "size", "pendingDx", "copyFrom", "pendingDw", "pendingFwd",
-                 "lazy", "ropeOf", "ropeFused")
+                 "lazy", "ropeOf", "ropeFused", "touched")
 
-    def __init__(self, owner: int, data: int, grad: int, nbytes: int, external: bool, size: int):
+    def __init__(self, owner: int, data: int, nbytes: int, size: int):
         self.owner = owner        # `_uid` of the backend
         self.data = data
-        self.grad = grad          # 0 for a frozen external (webgpu.ts frozenGradStub), and for an op's output until written
-        self.needs = grad != 0    # an op's output: does a gradient flow through it? (an external: does it have a buffer)
+        self.grad = 0             # 0 for a frozen external (webgpu.ts frozenGradStub), and for an op's output until written
+        self.needs = False        # an op's output: does a gradient flow through it? (an external: does it have a buffer)
         self.region = 0           # the recompute region it was made in (0: none): how long a gradient buffer must live
         self.bytes = nbytes
-        self.external = external
+        self.external = self.touched = False   # touched: an external listed in _touched
         self.gradLive = False     # has anything been written to grad in the current graph?
         self.size = size
         self.pendingDx = None     # (rows, cols, [(dY address, W address, K)]): input-gradient products not launched yet
@@ -218,7 +219,7 @@ class CudaBackend:
         self._externals: "weakref.WeakKeyDictionary[Tensor, _Entry]" = weakref.WeakKeyDictionary()
         self._tape: List[Tensor] = []          # outputs recorded with a backward closure since the last sync
         self._free: Dict[int, List[int]] = {}  # recycled blocks by size (a dictionary access instead of two library calls)
-        self._touched: Dict[int, Tensor] = {}
+        self._touched: List[Tensor] = []       # externals used since the last sync
         self._keptOnDevice: "weakref.WeakSet[Tensor]" = weakref.WeakSet()
         self._transients: List[tuple] = []     # (addr, size)
         self._regionFree: List[tuple] = []
@@ -423,7 +424,8 @@ class CudaBackend:
         return self._externals.get(t)
 
     def _newExternal(self, t: Tensor, data: int, grad: int) -> _Entry:
-        e = _Entry(self._uid, data, grad, t.size * 4, True, t.size)
+        e = _Entry(self._uid, data, t.size * 4, t.size)
+        e.grad, e.needs, e.external = grad, grad != 0, True
         self._externals[t] = e
         t._dev = e
         return e
@@ -437,8 +439,9 @@ class CudaBackend:
             self._flushFwd()
         if e.lazy is not None:
             self._materializeLazy(e)
-        if e.external and id(t) not in self._touched:
-            self._touched[id(t)] = t
+        if e.external and not e.touched:
+            e.touched = True
+            self._touched.append(t)
         return e
 
     def _firstUse(self, t: Tensor) -> _Entry:
@@ -479,18 +482,25 @@ class CudaBackend:
 
     def _newEntry(self, t: Tensor, needs: bool) -> _Entry:
         nbytes = t.size * 4
-        e = _Entry(self._uid, self._acquireRecycled(nbytes), 0, nbytes, False, t.size)
-        e.needs = t._needs = needs
+        # (_acquireRecycled written out: this runs once per op)
+        blocks = self._free.get((nbytes + 255) & ~255 if nbytes > 256 else 256) if not self._regionFree else None
+        if blocks:
+            addr = blocks.pop()
+            self._transients.append((addr, (nbytes + 255) & ~255 if nbytes > 256 else 256))
+        else:
+            addr = self._acquireRecycled(nbytes)
+        t._dev = e = _Entry(self._uid, addr, nbytes, t.size)
+        if needs:
+            e.needs = t._needs = True
         if self._regionStack:
             e.region = self._regionStack[-1][0]
-        t._dev = e
         return e
 
-    def _record(self, t: Tensor, needs: bool, bw) -> Tensor:
-        """Put an op's backward closure on the tape, or nothing where no gradient can flow: such a tensor is freed with its
-        last reader instead of being kept (with everything it was computed from) until the graph goes."""
+    def _record(self, t: Tensor, needs: bool, bw, *args) -> Tensor:
+        """Put an op's backward on the tape, or nothing where no gradient can flow: such a tensor is freed with its last reader
+        instead of being kept (with everything it was computed from) until the graph goes."""
         if needs:
-            t._backward = bw
+            t._backward = partial(bw, *args) if args else bw
             self._tape.append(t)
         else:
             t._backward = self._ensureBackwardBegun
@@ -572,7 +582,7 @@ class CudaBackend:
         first = self._pendingFwd[0] if self._pendingFwd else None
         if first is not None and ("norm" in first or "lora" in first or first["ex"] is not ex or len(self._pendingFwd) == 8):
             self._flushFwd()
-        self._pendingFwd.append(dict(ex=ex, ew=ew, eo=eo, T=T, inDim=inDim, outDim=outDim))
+        self._pendingFwd.append({"ex": ex, "ew": ew, "eo": eo, "T": T, "inDim": inDim, "outDim": outDim})
         eo.pendingFwd = True
 
     # A per-head norm (q and k of the Qwen3 and Gemma 3 blocks) waits the same way for the rotary embedding that follows
@@ -772,10 +782,11 @@ class CudaBackend:
             if e.lazy is not None:
                 self._materializeLazy(e)
             self._read(e.data, t.dataForReading())
-        for t in list(self._touched.values()):
+        for t in self._touched:
             e = self._find(t)
             if e is None:
                 continue
+            e.touched = False
             if t.requiresGrad and e.grad:
                 if not e.gradLive:
                     # touched by a forward, never written by a backward: the reference's cleared buffer
@@ -783,7 +794,8 @@ class CudaBackend:
                     self.gradClearsIssued += 1
                 if t not in self._keptOnDevice:
                     self._read(e.grad, t.gradForReading())
-            e.gradLive = False   # the next graph's first writer overwrites (the deferred clear)
+            if e.gradLive:
+                e.gradLive = False   # the next graph's first writer overwrites (the deferred clear)
         self._check(self.lib.gt_sync(self.ctx))
         self.lastSyncReadbackBytes = self._readback
         for blocks in (self._transients, self._regionFree, self._outer):
@@ -792,7 +804,7 @@ class CudaBackend:
         self._transients, self._regionFree, self._outer = [], [], []
         self._dropTape()
         self._regionStack = []
-        self._touched.clear()
+        self._touched = []
         self._backwardBegun = False
         if self._graphOpen:                    # (a sync with no graph behind it, e.g. after building an optimizer, arms nothing)
             self._graphSynced = True
@@ -1076,22 +1088,20 @@ class CudaBackend:
         else:
             self._flushFwd()
             self._gemm("NT", 0, T, outDim, inDim, ex.data, ew.data, eo.data)
+        return self._record(out, needs, self._linearBackward, x, ex, w, ew, eo, T, inDim, outDim)
 
-        def _bw():
-            self._ensureBackwardBegun()
-            go = self._gradSource(eo)
-            if self._flows(x, ex):
-                self._deferDx(ex, T, inDim, go, ew.data, outDim)
-            if self._flows(w, ew):
-                gw, aw = self._gradTarget(w, ew)
-                if gw:
-                    # (a product with many output tiles, the readout's, fills the GPU alone and is launched as it comes)
-                    if self.groupWeightGradients and ((outDim + 255) // 256) * ((inDim + 191) // 192) <= 64:
-                        self._deferDw(ew, gw, aw, T, outDim, inDim, go, ex.data)
-                    else:
-                        self._gemm("TN", aw, outDim, inDim, T, go, ex.data, gw)
-
-        return self._record(out, needs, _bw)
+    def _linearBackward(self, x, ex, w, ew, eo, T, inDim, outDim):
+        self._ensureBackwardBegun()
+        go = self._gradSource(eo)
+        if self._flows(x, ex):
+            self._deferDx(ex, T, inDim, go, ew.data, outDim)
+        if self._flows(w, ew):
+            gw, aw = self._gradTarget(w, ew)
+            # (a product with many output tiles, the readout's, fills the GPU alone and is launched as it comes)
+            if self.groupWeightGradients and ((outDim + 255) // 256) * ((inDim + 191) // 192) <= 64:
+                self._deferDw(ew, gw, aw, T, outDim, inDim, go, ex.data)
+            else:
+                self._gemm("TN", aw, outDim, inDim, T, go, ex.data, gw)
 
     def loraLinear(self, x: Tensor, w: Tensor, a: Tensor, b: Tensor, scale: float) -> Tensor:
         """The adapter-carrying projection of autograd.ts:311-319, y = x·Wᵀ + scale·((x·Aᵀ)·Bᵀ), as one op. Recorded as
@@ -1191,28 +1201,26 @@ class CudaBackend:
         out = Tensor.output(list(a.shape), a.size, [a, b])
         out._needs = self._flows(a, ea) or self._flows(b, eb)
         self._pendingAdd[id(out)] = (out, a, b)
-        n = a.size
+        return self._record(out, out._needs, self._addBackward, out, a, ea, b, eb)
 
-        def _bw():
-            eo = self._find(out)
-            if eo is None:
-                return          # never used by anything: no gradient reaches it
-            self._ensureBackwardBegun()
-            go = self._gradSource(eo)
-            for t, e, first in ((a, ea, True), (b, eb, False)):
-                if not self._flows(t, e):
-                    continue
-                if e.pendingDx is not None:
-                    self._flushDx(e)
-                if e.gradLive or e.copyFrom:
-                    g, acc = self._gradTarget(t, e)
-                    self._check(self.lib.gt_ew_bwd(self.ctx, _EW["add"], n, ea.data, eb.data, 0.0, go,
-                                                   g if first else 0, acc, 0 if first else g, acc))
-                else:
-                    e.copyFrom = go
-                    self._pendingCopy[id(e)] = e
-
-        return self._record(out, out._needs, _bw)
+    def _addBackward(self, out, a, ea, b, eb):
+        eo = self._find(out)
+        if eo is None:
+            return          # never used by anything: no gradient reaches it
+        self._ensureBackwardBegun()
+        go = self._gradSource(eo)
+        for t, e, first in ((a, ea, True), (b, eb, False)):
+            if not self._flows(t, e):
+                continue
+            if e.pendingDx is not None:
+                self._flushDx(e)
+            if e.gradLive or e.copyFrom:
+                g, acc = self._gradTarget(t, e)
+                self._check(self.lib.gt_ew_bwd(self.ctx, _EW["add"], a.size, ea.data, eb.data, 0.0, go,
+                                               g if first else 0, acc, 0 if first else g, acc))
+            else:
+                e.copyFrom = go
+                self._pendingCopy[id(e)] = e
 
     def _materializeAdd(self, t: Tensor) -> _Entry:
         _t, a, b = self._pendingAdd.pop(id(t))
@@ -1248,18 +1256,17 @@ class CudaBackend:
         t = Tensor.output(list(x.shape), x.size, [x])
         t._needs = self._flows(x, e0)
         self._pendingAct[id(t)] = (t, _EW[op], x)
+        return self._record(t, t._needs, self._activationBackward, t, op, x)
 
-        def _bw():
-            e = self._find(t)
-            if e is None or not (e.gradLive or e.copyFrom or e.pendingDx is not None):
-                return          # consumed only by fused products, which sent their gradient straight to x
-            self._ensureBackwardBegun()
-            ex = self._entryOf(x)
-            go = self._gradSource(e)
-            gx, ax = self._gradTarget(x, ex)
-            self._check(self.lib.gt_ew_bwd(self.ctx, _EW[op], x.size, ex.data, 0, 0.0, go, gx, ax, 0, 0))
-
-        return self._record(t, t._needs, _bw)
+    def _activationBackward(self, t, op, x):
+        e = self._find(t)
+        if e is None or not (e.gradLive or e.copyFrom or e.pendingDx is not None):
+            return          # consumed only by fused products, which sent their gradient straight to x
+        self._ensureBackwardBegun()
+        ex = self._entryOf(x)
+        go = self._gradSource(e)
+        gx, ax = self._gradTarget(x, ex)
+        self._check(self.lib.gt_ew_bwd(self.ctx, _EW[op], x.size, ex.data, 0, 0.0, go, gx, ax, 0, 0))
 
     def _materializeAct(self, t: Tensor) -> _Entry:
         _t, code, x = self._pendingAct.pop(id(t))
@@ -1305,20 +1312,18 @@ class CudaBackend:
             needs = self._flows(x, ex) or self._flows(u, eu)
             out, eo = self._makeOut(list(act.shape), act.size, [act, u], needs)
             self._check(self.lib.gt_glu_fwd(self.ctx, code, act.size, ex.data, eu.data, eo.data))
-        n = act.size
+        return self._record(out, needs, self._gatedUnitBackward, code, act.size, x, ex, u, eu, eo)
 
-        def _bw():
-            self._ensureBackwardBegun()
-            go = self._gradSource(eo)
-            gx, ax = self._gradTarget(x, ex)
-            gu, au = self._gradTarget(u, eu)
-            if gx and gx == gu:      # act(x) * x: one buffer takes both terms, in two passes
-                self._check(self.lib.gt_glu_bwd(self.ctx, code, n, ex.data, eu.data, go, gx, ax, 0, 0))
-                self._check(self.lib.gt_glu_bwd(self.ctx, code, n, ex.data, eu.data, go, 0, 0, gu, 1))
-            else:
-                self._check(self.lib.gt_glu_bwd(self.ctx, code, n, ex.data, eu.data, go, gx, ax, gu, au))
-
-        return self._record(out, needs, _bw)
+    def _gatedUnitBackward(self, code, n, x, ex, u, eu, eo):
+        self._ensureBackwardBegun()
+        go = self._gradSource(eo)
+        gx, ax = self._gradTarget(x, ex)
+        gu, au = self._gradTarget(u, eu)
+        if gx and gx == gu:      # act(x) * x: one buffer takes both terms, in two passes
+            self._check(self.lib.gt_glu_bwd(self.ctx, code, n, ex.data, eu.data, go, gx, ax, 0, 0))
+            self._check(self.lib.gt_glu_bwd(self.ctx, code, n, ex.data, eu.data, go, 0, 0, gu, 1))
+        else:
+            self._check(self.lib.gt_glu_bwd(self.ctx, code, n, ex.data, eu.data, go, gx, ax, gu, au))
 
     def scale(self, x, c):
         return self._elementwise("scale", x, None, float(c))
@@ -1346,25 +1351,25 @@ class CudaBackend:
             else:
                 self._check(self.lib.gt_rmsnorm_fwd(self.ctx, rows, d, ex.data, ew.data, eps, eo.data, rinv))
 
-        def _bw():
-            self._ensureBackwardBegun()
-            go = self._gradSource(eo)
-            wantX = self._flows(x, ex)
-            if wantX and ex.pendingDx is not None:
-                self._flushDx(ex)
-            gw, aw = self._gradTarget(w, ew)
-            if wantX and ex.copyFrom and not ex.gradLive:
-                # the gradient so far is an `add`'s upstream buffer: dx = that buffer + this term, written in one pass
-                gadd = ex.copyFrom
-                ex.copyFrom = 0
-                self._pendingCopy.pop(id(ex), None)
-                ex.gradLive = True
-                self._check(self.lib.gt_rmsnorm_bwd_add(self.ctx, rows, d, ex.data, ew.data, rinv, go, gadd, self._gradAddr(ex), gw, aw))
-                return
-            gx, ax = self._gradTarget(x, ex)
-            self._check(self.lib.gt_rmsnorm_bwd(self.ctx, rows, d, ex.data, ew.data, rinv, go, gx, ax, gw, aw))
+        return self._record(out, needs, self._rmsNormBackward, x, ex, w, ew, eo, rinv, rows, d)
 
-        return self._record(out, needs, _bw)
+    def _rmsNormBackward(self, x, ex, w, ew, eo, rinv, rows, d):
+        self._ensureBackwardBegun()
+        go = self._gradSource(eo)
+        wantX = self._flows(x, ex)
+        if wantX and ex.pendingDx is not None:
+            self._flushDx(ex)
+        gw, aw = self._gradTarget(w, ew)
+        if wantX and ex.copyFrom and not ex.gradLive:
+            # the gradient so far is an `add`'s upstream buffer: dx = that buffer + this term, written in one pass
+            gadd = ex.copyFrom
+            ex.copyFrom = 0
+            self._pendingCopy.pop(id(ex), None)
+            ex.gradLive = True
+            self._check(self.lib.gt_rmsnorm_bwd_add(self.ctx, rows, d, ex.data, ew.data, rinv, go, gadd, self._gradAddr(ex), gw, aw))
+            return
+        gx, ax = self._gradTarget(x, ex)
+        self._check(self.lib.gt_rmsnorm_bwd(self.ctx, rows, d, ex.data, ew.data, rinv, go, gx, ax, gw, aw))
 
     def rmsNorm(self, x, weight, eps):
         T, d = x.shape
@@ -1448,15 +1453,15 @@ class CudaBackend:
         if needs:
             eo.ropeOf = (x, ex, H, hd, base, posOffset)
 
-        def _bw():
-            self._ensureBackwardBegun()
-            if eo.ropeFused and not (eo.gradLive or eo.copyFrom or eo.pendingDx is not None):
-                return                       # attention's backward already delivered this gradient to x
-            go = self._gradSource(eo)
-            gx, ax = self._gradTarget(x, ex)
-            self._check(self.lib.gt_rope_bwd(self.ctx, T, H, hd, float(base), posOffset, go, gx, ax))
+        return self._record(out, needs, self._ropeBackward, x, ex, eo, T, H, hd, base, posOffset)
 
-        return self._record(out, needs, _bw)
+    def _ropeBackward(self, x, ex, eo, T, H, hd, base, posOffset):
+        self._ensureBackwardBegun()
+        if eo.ropeFused and not (eo.gradLive or eo.copyFrom or eo.pendingDx is not None):
+            return                       # attention's backward already delivered this gradient to x
+        go = self._gradSource(eo)
+        gx, ax = self._gradTarget(x, ex)
+        self._check(self.lib.gt_rope_bwd(self.ctx, T, H, hd, float(base), posOffset, go, gx, ax))
 
     def attention(self, q: Tensor, k: Tensor, v: Tensor, T: int, Hq: int, Hkv: int, hd: int, window: int) -> Tensor:
         """webgpu.ts:1125-1192."""
@@ -1471,7 +1476,7 @@ class CudaBackend:
             data, lse, _n = rec["saved"][rec["pos"]]
             rec["pos"] += 1
             out = Tensor.output([T, Hq * hd], T * Hq * hd, [q, k, v])
-            eo = _Entry(self._uid, data, 0, nbytes, False, out.size)
+            eo = _Entry(self._uid, data, nbytes, out.size)
             eo.needs, eo.region = needs, self._regionStack[-1][0]
             out._needs, out._dev = needs, eo
         else:
@@ -1481,30 +1486,30 @@ class CudaBackend:
             if rec is not None and not rec["replay"]:
                 rec["saved"].append((eo.data, lse, nbytes))
 
-        def _bw():
-            self._ensureBackwardBegun()
-            go = self._gradSource(eo)
-            rq, rk = eq.ropeOf, ek.ropeOf
-            fresh = lambda e: not (e.gradLive or e.copyFrom or e.pendingDx is not None)
-            if (self.fuseRope and rq is not None and rk is not None and eq is not ek and rq[3:] == rk[3:] and rq[3] == hd
-                    and rq[2] == Hq and rk[2] == Hkv and hd in (64, 128) and T >= 64 and self.precision == "tf32"
-                    and fresh(eq) and fresh(ek)):
-                # q and k came out of rotary embeddings and nothing else has written their gradients: the kernels rotate
-                # dQ and dK back as they store them, into the gradients of the embeddings' inputs
-                gq, aq = self._gradTarget(rq[0], rq[1])
-                gk, ak = self._gradTarget(rk[0], rk[1])
-                gv, av = self._gradTarget(v, ev)
-                self._check(self.lib.gt_attention_bwd_rope(self.ctx, T, Hq, Hkv, hd, window, eq.data, ek.data, ev.data, eo.data,
-                                                           lse, go, gq, aq, gk, ak, gv, av, float(rq[4]), rq[5]))
-                eq.ropeFused = ek.ropeFused = True
-                return
-            gq, aq = self._gradTarget(q, eq)
-            gk, ak = self._gradTarget(k, ek)
-            gv, av = self._gradTarget(v, ev)
-            self._check(self.lib.gt_attention_bwd(self.ctx, T, Hq, Hkv, hd, window, eq.data, ek.data, ev.data, eo.data,
-                                                  lse, go, gq, aq, gk, ak, gv, av))
+        return self._record(out, needs, self._attentionBackward, q, eq, k, ek, v, ev, eo, lse, T, Hq, Hkv, hd, window)
 
-        return self._record(out, needs, _bw)
+    def _attentionBackward(self, q, eq, k, ek, v, ev, eo, lse, T, Hq, Hkv, hd, window):
+        self._ensureBackwardBegun()
+        go = self._gradSource(eo)
+        rq, rk = eq.ropeOf, ek.ropeOf
+        fresh = lambda e: not (e.gradLive or e.copyFrom or e.pendingDx is not None)
+        if (self.fuseRope and rq is not None and rk is not None and eq is not ek and rq[3:] == rk[3:] and rq[3] == hd
+                and rq[2] == Hq and rk[2] == Hkv and hd in (64, 128) and T >= 64 and self.precision == "tf32"
+                and fresh(eq) and fresh(ek)):
+            # q and k came out of rotary embeddings and nothing else has written their gradients: the kernels rotate
+            # dQ and dK back as they store them, into the gradients of the embeddings' inputs
+            gq, aq = self._gradTarget(rq[0], rq[1])
+            gk, ak = self._gradTarget(rk[0], rk[1])
+            gv, av = self._gradTarget(v, ev)
+            self._check(self.lib.gt_attention_bwd_rope(self.ctx, T, Hq, Hkv, hd, window, eq.data, ek.data, ev.data, eo.data,
+                                                       lse, go, gq, aq, gk, ak, gv, av, float(rq[4]), rq[5]))
+            eq.ropeFused = ek.ropeFused = True
+            return
+        gq, aq = self._gradTarget(q, eq)
+        gk, ak = self._gradTarget(k, ek)
+        gv, av = self._gradTarget(v, ev)
+        self._check(self.lib.gt_attention_bwd(self.ctx, T, Hq, Hkv, hd, window, eq.data, ek.data, ev.data, eo.data,
+                                              lse, go, gq, aq, gk, ak, gv, av))
 
     def _nseq(self) -> int:
         return self._batch[0] if self._batch[0] else 1
@@ -1513,7 +1518,7 @@ class CudaBackend:
         """The scalar loss tensor plus its device-side companions: [1+nseq] losses and [nseq] 1/kept."""
         nseq = self._nseq()
         loss = Tensor.output([1], 1, list(prev))
-        e = _Entry(self._uid, self._acquireRecycled((1 + nseq) * 4), 0, 4, False, 1)
+        e = _Entry(self._uid, self._acquireRecycled((1 + nseq) * 4), 4, 1)
         e.needs = loss._needs = needs
         e.region = self._regionStack[-1][0] if self._regionStack else 0
         loss._dev = e
