@@ -11,7 +11,10 @@
 // the host checks at the next sync, skips its stores, releases its TMEM and exits.
 #include <cuda.h>
 
+#include <string.h>
+
 #include <mutex>
+#include <unordered_map>
 
 #include "common.cuh"
 #include "tc_common.cuh"
@@ -976,6 +979,36 @@ EncodeTiledFn encode_fn() {
 // kmajor: the tile's rows are K runs (128-byte swizzle); else its rows are MN runs (128-byte swizzle, 32-byte atoms).
 }  // namespace
 
+namespace {
+// Encoded maps are a pure function of their arguments, and a training or decoding loop asks for the same ones again and
+// again (weights stay where they are, recycled activations come back to the same blocks): a few thousand are kept per thread.
+struct MapKey {
+  uint64_t v[8];
+  bool operator==(const MapKey& o) const { return memcmp(v, o.v, sizeof v) == 0; }
+};
+struct WordsHash {
+  template <typename K>
+  size_t operator()(const K& k) const {
+    uint64_t h = 0x9e3779b97f4a7c15ull;
+    for (auto x : k.v) h = (h ^ (uint64_t)x) * 0xff51afd7ed558ccdull, h ^= h >> 29;
+    return (size_t)h;
+  }
+};
+template <typename F>
+bool cached_map(CUtensorMap* map, const MapKey& key, F encode) {
+  thread_local std::unordered_map<MapKey, CUtensorMap, WordsHash> maps;
+  auto it = maps.find(key);
+  if (it == maps.end()) {
+    if (!encode(map)) return false;
+    if (maps.size() >= 4096) maps.clear();
+    maps.emplace(key, *map);
+    return true;
+  }
+  *map = it->second;
+  return true;
+}
+}  // namespace
+
 bool tc::make_map_3d(CUtensorMap* map, const float* ptr, uint64_t inner, uint64_t outer, uint64_t batch, uint64_t row_pitch_elems,
                      uint64_t batch_stride_elems, uint32_t box_outer, bool kmajor) {
   EncodeTiledFn enc = encode_fn();
@@ -984,8 +1017,8 @@ bool tc::make_map_3d(CUtensorMap* map, const float* ptr, uint64_t inner, uint64_
   cuuint64_t strides[2] = {row_pitch_elems * sizeof(float), batch_stride_elems * sizeof(float)};
   cuuint32_t box[3] = {32, box_outer, 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             kmajor ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return cached_map(map, {{(uint64_t)(uintptr_t)ptr, inner, outer, batch, row_pitch_elems, batch_stride_elems, box_outer, kmajor ? 1ull : 2ull}}, [&](CUtensorMap* map) { return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             kmajor ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS; });
 }
 
 bool tc::make_map_atoms(CUtensorMap* map, const float* ptr, uint64_t inner, uint64_t outer, uint64_t row_pitch_elems,
@@ -996,8 +1029,8 @@ bool tc::make_map_atoms(CUtensorMap* map, const float* ptr, uint64_t inner, uint
   cuuint64_t strides[2] = {row_pitch_elems * sizeof(float), 32 * sizeof(float)};
   cuuint32_t box[3] = {32, box_outer, atoms};
   cuuint32_t estr[3] = {1, 1, 1};
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             kmajor ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return cached_map(map, {{(uint64_t)(uintptr_t)ptr, inner, outer, atoms, row_pitch_elems, 0, box_outer, kmajor ? 3ull : 4ull}}, [&](CUtensorMap* map) { return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             kmajor ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS; });
 }
 
 bool tc::make_map_2d(CUtensorMap* map, const float* ptr, uint64_t inner, uint64_t outer, uint64_t row_pitch_elems,
@@ -1057,30 +1090,21 @@ gt_status gt_gemm_tc_answer(gt_ctx* ctx, int code) {
   return gt_fail(ctx, GT_ERR_CUDA, "tensor-core kernel: a pipeline wait expired (code %d); results of that launch are invalid", code);
 }
 
-// `batch` independent products of the same shape, matrix i of each operand `M*K`, `N*K`, `M*N` elements after matrix i-1.
-// With nparts > 1 (batch 1 only): c (+)= sum_p op(a_p).op(b_p), every product of the same kind, K_p deep.
-static gt_status gemm_tc_dispatch(gt_ctx* ctx, int kind, int accum, int M, int N, int nparts, const int* Ks, const float* const* as,
-                                  const float* const* bs, float* c, int batch, float alpha, bool* handled) {
-  *handled = false;
-  if (batch < 1 || nparts < 1 || nparts > MAX_PARTS || (nparts > 1 && batch != 1)) return GT_OK;
-  // Small or oddly aligned products stay on the f32 kernel: TMA needs 16-byte row pitches and bases.
-  const bool a_k = kind != GT_GEMM_TN, b_k = kind == GT_GEMM_NT;
-  if (M < 16 || N < 16 || Ks[0] < 16) return GT_OK;   // (rows of a tile past M or N are zero-filled by TMA and clipped on store)
-  if (((uintptr_t)c) & 15) return GT_OK;
-  int kblocks = 0;
-  for (int p = 0; p < nparts; p++) {
-    const int a_inner = a_k ? Ks[p] : M, b_inner = b_k ? Ks[p] : N;
-    if (Ks[p] < 1 || (a_inner & 3) || (b_inner & 3) || ((((uintptr_t)as[p]) | ((uintptr_t)bs[p])) & 15)) return GT_OK;
-    kblocks += gt_cdiv(Ks[p], BK);
-  }
-  if (ctx->device < 0 || ctx->device >= 64) return GT_OK;
-  if (!device_flag(ctx)) return GT_OK;
+struct Plan { int mt = 0, bn = 0, ks = 1; bool small = false; };   // mt 0: not for the tensor cores
+struct PlanKey {
+  int v[8 + MAX_PARTS] = {};
+  bool operator==(const PlanKey& o) const { return memcmp(v, o.v, sizeof v) == 0; }
+};
+static std::unordered_map<PlanKey, Plan, WordsHash>& plan_cache() {
+  thread_local std::unordered_map<PlanKey, Plan, WordsHash> plans;
+  if (plans.size() > 4096) plans.clear();
+  return plans;
+}
+static Plan choose_plan(gt_ctx* ctx, int accum, int M, int N, int nparts, int kblocks, int batch, const char* force, const char* ds) {
   // Tile shape and split-K factor: the cheapest of the four shapes under a small cost model (cycles of the CTA with
   // the most work: waves x (K blocks x cycles per K block + epilogue)), calibrated on in-kernel cycle counts.
   struct Cfg { int mt, bn; };   // mt 1, 2: 128 / 256 rows on one CTA; mt 3: 256 rows on a CTA pair
   static const Cfg cfgs[6] = {{1, 192}, {1, 128}, {2, 256}, {2, 192}, {3, 192}, {3, 256}};
-  const char* force = getenv("GT_GEMM_TILE");   // "mt,bn": forces one tile shape (read per call so tests can switch it); mt 0: one tile per CTA
-  const char* ds = getenv("GT_GEMM_DEEP_SPLIT");   // "0": never cut a product that already fills the SMs along K (for comparison)
   const bool deep_split = !(ds && ds[0] == '0');
   const int npairs = max(0, pair_capacity(ctx) - (ctx->sm_reserved + 1) / 2);
   int best = 0, ksplit = 1;
@@ -1141,9 +1165,45 @@ static gt_status gemm_tc_dispatch(gt_ctx* ctx, int kind, int accum, int M, int N
   if (fm <= 0)
     small = pick_small(ctx, kblocks, [&](int b) { return (fm == 0 && fb && b != fb) ? 1l << 40 : (long)gt_cdiv(N, b) * gt_cdiv(M, BM1) * batch; }, 32);
   const bool use_small = small.bn && small.cost < best_cost;
-  if (best_cost >= 1e30 && !use_small) return GT_OK;
-  if (use_small) ksplit = small.ks;
-  const int mt = use_small ? 1 : cfgs[best].mt, bn = use_small ? small.bn : cfgs[best].bn;
+  if (best_cost >= 1e30 && !use_small) return {};
+  if (use_small) return {1, small.bn, small.ks, true};
+  return {cfgs[best].mt, cfgs[best].bn, ksplit, false};
+}
+
+// `batch` independent products of the same shape, matrix i of each operand `M*K`, `N*K`, `M*N` elements after matrix i-1.
+// With nparts > 1 (batch 1 only): c (+)= sum_p op(a_p).op(b_p), every product of the same kind, K_p deep.
+static gt_status gemm_tc_dispatch(gt_ctx* ctx, int kind, int accum, int M, int N, int nparts, const int* Ks, const float* const* as,
+                                  const float* const* bs, float* c, int batch, float alpha, bool* handled) {
+  *handled = false;
+  if (batch < 1 || nparts < 1 || nparts > MAX_PARTS || (nparts > 1 && batch != 1)) return GT_OK;
+  // Small or oddly aligned products stay on the f32 kernel: TMA needs 16-byte row pitches and bases.
+  const bool a_k = kind != GT_GEMM_TN, b_k = kind == GT_GEMM_NT;
+  if (M < 16 || N < 16 || Ks[0] < 16) return GT_OK;   // (rows of a tile past M or N are zero-filled by TMA and clipped on store)
+  if (((uintptr_t)c) & 15) return GT_OK;
+  int kblocks = 0;
+  for (int p = 0; p < nparts; p++) {
+    const int a_inner = a_k ? Ks[p] : M, b_inner = b_k ? Ks[p] : N;
+    if (Ks[p] < 1 || (a_inner & 3) || (b_inner & 3) || ((((uintptr_t)as[p]) | ((uintptr_t)bs[p])) & 15)) return GT_OK;
+    kblocks += gt_cdiv(Ks[p], BK);
+  }
+  if (ctx->device < 0 || ctx->device >= 64) return GT_OK;
+  if (!device_flag(ctx)) return GT_OK;
+  const char* force = getenv("GT_GEMM_TILE");   // "mt,bn": forces one tile shape (read per call so tests can switch it); mt 0: one tile per CTA
+  const char* ds = getenv("GT_GEMM_DEEP_SPLIT");   // "0": never cut a product that already fills the SMs along K (for comparison)
+  // the choice is made once per shape
+  Plan plan;
+  PlanKey key = {{kind, accum ? 1 : 0, M, N, batch, ctx->device, ctx->sm_reserved, nparts}};
+  for (int p = 0; p < nparts; p++) key.v[8 + p] = Ks[p];
+  auto& plans = plan_cache();
+  auto found = force || ds ? plans.end() : plans.find(key);
+  if (found != plans.end()) plan = found->second;
+  else {
+    plan = choose_plan(ctx, accum, M, N, nparts, kblocks, batch, force, ds);
+    if (!force && !ds) plans.emplace(key, plan);
+  }
+  if (!plan.mt) return GT_OK;
+  const bool use_small = plan.small;
+  const int ksplit = plan.ks, mt = plan.mt, bn = plan.bn;
   const int a_box = mt == 2 ? 2 * BM1 : BM1, b_box = mt == 3 ? bn / 2 : bn;   // rows one TMA copy brings
   PartMaps maps;
   maps.nparts = nparts;
@@ -1180,6 +1240,7 @@ static gt_status gemm_tc_dispatch(gt_ctx* ctx, int kind, int accum, int M, int N
   const int K0 = Ks[0];
   const long ntiles = (long)gt_cdiv(N, bn) * gt_cdiv(M, mt == 1 ? BM1 : 2 * BM1) * ksplit * batch;
   gt_status s;
+  const int npairs = max(0, pair_capacity(ctx) - (ctx->sm_reserved + 1) / 2);
   if (mt == 3 && bn == 192) s = launch_pair_kind<192>(ctx, kind, maps.a[0], maps.b[0], maps.c[0], tma_store, c, M, N, K0, accum, ksplit, batch, npairs, out_scale);
   else if (mt == 3) s = launch_pair_kind<256>(ctx, kind, maps.a[0], maps.b[0], maps.c[0], tma_store, c, M, N, K0, accum, ksplit, batch, npairs, out_scale);
   else if (mt == 1 && bn == 192) s = launch_kind<192, 1>(ctx, kind, maps, ntiles, tma_store, c, M, N, accum, ksplit, batch, out_scale);
@@ -1191,28 +1252,17 @@ static gt_status gemm_tc_dispatch(gt_ctx* ctx, int kind, int accum, int M, int N
   return GT_OK;
 }
 
-// ngroups independent products of one layout and one K, each with its own operands, extents and accumulate flag, as
-// ONE launch: the weight gradients dW_g = dY_g^T.X_g of several projections (K = rows for all of them). Their tiles
-// are so few per product that each would need its own split-K launch with its own tail; together they fill the SMs.
-static gt_status gemm_tc_grouped(gt_ctx* ctx, int kind, int ngroups, const int* Ms, const int* Ns, int K, const float* const* as,
-                                 const float* const* bs, float* const* cs, const int* accums, const int* ropes, const float2* rope_tab,
-                                 int rope_period, float alpha, bool* handled) {
-  *handled = false;
-  if (ngroups < 2 || ngroups > MAX_PARTS || K < 16) return GT_OK;
-  bool any_rope = false;
-  for (int g = 0; ropes && g < ngroups; g++) {
-    if (!ropes[g]) continue;
-    if (kind != GT_GEMM_NT || (Ns[g] & 63) || !rope_tab || rope_period <= 0) return GT_OK;
-    any_rope = true;
-  }
-  const bool a_k = kind != GT_GEMM_TN, b_k = kind == GT_GEMM_NT;
-  for (int g = 0; g < ngroups; g++) {
-    const int a_inner = a_k ? K : Ms[g], b_inner = b_k ? K : Ns[g];
-    if (Ms[g] < 16 || Ns[g] < 16 || (a_inner & 3) || (b_inner & 3) || (Ns[g] & 3)) return GT_OK;
-    if ((((uintptr_t)as[g]) | ((uintptr_t)bs[g]) | ((uintptr_t)cs[g])) & 15) return GT_OK;
-  }
-  if (ctx->device < 0 || ctx->device >= 64 || !device_flag(ctx)) return GT_OK;
-  const int kblocks = gt_cdiv(K, BK);
+struct GroupKey {
+  int v[6 + 3 * MAX_PARTS] = {};
+  bool operator==(const GroupKey& o) const { return memcmp(v, o.v, sizeof v) == 0; }
+};
+static std::unordered_map<GroupKey, Plan, WordsHash>& group_cache() {
+  thread_local std::unordered_map<GroupKey, Plan, WordsHash> plans;
+  if (plans.size() > 4096) plans.clear();
+  return plans;
+}
+static Plan choose_group_plan(gt_ctx* ctx, int kind, int ngroups, const int* Ms, const int* Ns, int kblocks, const int* accums, bool any_rope,
+                              const char* force) {
   const long workers = ctx->sm_count - ctx->sm_reserved;
   int clears = 0;      // (one clear per product that does not accumulate)
   for (int g = 0; g < ngroups; g++) clears += !accums[g];
@@ -1220,7 +1270,6 @@ static gt_status gemm_tc_grouped(gt_ctx* ctx, int kind, int ngroups, const int* 
   // among those that leave a slice at least 8 K blocks and add at most 8 partial sums per output element
   int best_mt = 1, best_ks = 1;
   double best_cost = 1e30;
-  const char* force = getenv("GT_GEMM_TILE");
   for (int mt = 1; mt <= 2; mt++) {
     if (force) { int fm = 0, fb = 0; if (sscanf(force, "%d,%d", &fm, &fb) == 2 && (fm != mt || fb != 192)) continue; }
     long tiles = 0;
@@ -1248,8 +1297,46 @@ static gt_status gemm_tc_grouped(gt_ctx* ctx, int kind, int ngroups, const int* 
       return n;
     }, any_rope || heads64 ? 64 : 32);
   const bool use_small = small.bn && small.cost < best_cost;
-  if (best_cost >= 1e30 && !use_small) return GT_OK;
-  const int mt = use_small ? 1 : best_mt, ksplit = use_small ? small.ks : best_ks, bm = mt * BM1, bn = use_small ? small.bn : 192;
+  if (best_cost >= 1e30 && !use_small) return {};
+  return use_small ? Plan{1, small.bn, small.ks, true} : Plan{best_mt, 192, best_ks, false};
+}
+
+// ngroups independent products of one layout and one K, each with its own operands, extents and accumulate flag, as
+// ONE launch: the weight gradients dW_g = dY_g^T.X_g of several projections (K = rows for all of them). Their tiles
+// are so few per product that each would need its own split-K launch with its own tail; together they fill the SMs.
+static gt_status gemm_tc_grouped(gt_ctx* ctx, int kind, int ngroups, const int* Ms, const int* Ns, int K, const float* const* as,
+                                 const float* const* bs, float* const* cs, const int* accums, const int* ropes, const float2* rope_tab,
+                                 int rope_period, float alpha, bool* handled) {
+  *handled = false;
+  if (ngroups < 2 || ngroups > MAX_PARTS || K < 16) return GT_OK;
+  bool any_rope = false;
+  for (int g = 0; ropes && g < ngroups; g++) {
+    if (!ropes[g]) continue;
+    if (kind != GT_GEMM_NT || (Ns[g] & 63) || !rope_tab || rope_period <= 0) return GT_OK;
+    any_rope = true;
+  }
+  const bool a_k = kind != GT_GEMM_TN, b_k = kind == GT_GEMM_NT;
+  for (int g = 0; g < ngroups; g++) {
+    const int a_inner = a_k ? K : Ms[g], b_inner = b_k ? K : Ns[g];
+    if (Ms[g] < 16 || Ns[g] < 16 || (a_inner & 3) || (b_inner & 3) || (Ns[g] & 3)) return GT_OK;
+    if ((((uintptr_t)as[g]) | ((uintptr_t)bs[g]) | ((uintptr_t)cs[g])) & 15) return GT_OK;
+  }
+  if (ctx->device < 0 || ctx->device >= 64 || !device_flag(ctx)) return GT_OK;
+  const int kblocks = gt_cdiv(K, BK);
+  const char* force = getenv("GT_GEMM_TILE");
+  GroupKey key = {{kind, K, ngroups, any_rope ? 1 : 0, ctx->device, ctx->sm_reserved}};
+  for (int g = 0; g < ngroups; g++) { key.v[6 + 3 * g] = Ms[g]; key.v[7 + 3 * g] = Ns[g]; key.v[8 + 3 * g] = accums[g] ? 1 : 0; }
+  auto& plans = group_cache();
+  auto found = force ? plans.end() : plans.find(key);
+  Plan plan;
+  if (found != plans.end()) plan = found->second;
+  else {
+    plan = choose_group_plan(ctx, kind, ngroups, Ms, Ns, kblocks, accums, any_rope, force);
+    if (!force) plans.emplace(key, plan);
+  }
+  if (!plan.mt) return GT_OK;
+  const bool use_small = plan.small;
+  const int mt = plan.mt, ksplit = plan.ks, bm = mt * BM1, bn = plan.bn;
   PartMaps maps;
   maps.nparts = 1;
   maps.ngroups = ngroups;
