@@ -395,6 +395,20 @@ class CudaBackend:
         self._check(self.lib.gt_read(self.ctx, addr, out.ctypes.data, out.nbytes))
         self._readback += out.nbytes
 
+    def _readMany(self, wanted):
+        """[(address, host array)] as one read."""
+        n = len(wanted)
+        many = getattr(self.lib, "gt_read_many", None)      # (a stand-in for the library need not have it)
+        if n < 2 or many is None:
+            for addr, out in wanted:
+                self._read(addr, out)
+            return
+        assert all(a.flags["C_CONTIGUOUS"] for _addr, a in wanted)
+        nbytes = [a.nbytes for _addr, a in wanted]
+        self._check(many(self.ctx, n, (C.c_uint64 * n)(*[addr for addr, _a in wanted]), (C.c_void_p * n)(*[a.ctypes.data for _addr, a in wanted]),
+                         (C.c_uint64 * n)(*nbytes)))
+        self._readback += sum(nbytes)
+
     def _uploadU32(self, values, role: Optional[str] = None, bound: int = 0) -> int:
         if hasattr(values, "addr") and hasattr(values, "bound"):
             return int(values.addr)          # already on the device (ingest.DeviceInts): nothing to upload or replay-patch
@@ -772,6 +786,7 @@ class CudaBackend:
         self._pendingAct.clear()
         self._pendingAdd.clear()
         seen = set()
+        wanted = []                            # (address, host array)
         for t in reads:
             if id(t) in seen:
                 continue
@@ -781,7 +796,7 @@ class CudaBackend:
                 continue
             if e.lazy is not None:
                 self._materializeLazy(e)
-            self._read(e.data, t.dataForReading())
+            wanted.append((e.data, t.dataForReading()))
         for t in self._touched:
             e = self._find(t)
             if e is None:
@@ -793,9 +808,10 @@ class CudaBackend:
                     self._check(self.lib.gt_zero(self.ctx, e.grad, e.bytes))
                     self.gradClearsIssued += 1
                 if t not in self._keptOnDevice:
-                    self._read(e.grad, t.gradForReading())
+                    wanted.append((e.grad, t.gradForReading()))
             if e.gradLive:
                 e.gradLive = False   # the next graph's first writer overwrites (the deferred clear)
+        self._readMany(wanted)
         self._check(self.lib.gt_sync(self.ctx))
         self.lastSyncReadbackBytes = self._readback
         for blocks in (self._transients, self._regionFree, self._outer):

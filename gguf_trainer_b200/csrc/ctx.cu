@@ -5,6 +5,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -26,12 +27,15 @@ static inline void cpu_pause() {
 // the next blocks arrive. A copy straight into pageable memory is staged by the driver on one thread, 14 GB/s: 39 ms for
 // the 540 MB of weights that end a training call; the ring keeps the bus busy.
 struct GtHostCopy {
-  static constexpr int SLOTS = 8, THREADS = 4;
-  static constexpr uint64_t BLOCK = 1 << 20;
-  struct Job { void* dst; int slot; uint64_t bytes; };
+  static constexpr int SLOTS = 32, THREADS = 6;
+  static constexpr uint64_t BLOCK = 512 << 10;
+  static constexpr int LAG = 8;           // copies in flight ahead of the block that is being waited for
+  struct Piece { void* dst; uint64_t off, bytes; };    // part of a block, and where it goes
+  struct Job { int slot; };
   char* ring = nullptr;
   cudaEvent_t landed[SLOTS] = {};
   std::atomic<int> busy[SLOTS];          // 1 from the copy's launch until a thread has emptied the block
+  std::vector<Piece> pieces[SLOTS];
   std::mutex m;
   std::condition_variable cv;
   std::deque<Job> jobs;
@@ -49,7 +53,7 @@ struct GtHostCopy {
     return true;
   }
   void empty(const Job& j) {
-    memcpy(j.dst, ring + (uint64_t)j.slot * BLOCK, j.bytes);
+    for (const Piece& p : pieces[j.slot]) memcpy(p.dst, ring + (uint64_t)j.slot * BLOCK + p.off, p.bytes);
     busy[j.slot].store(0, std::memory_order_release);
   }
   void put(const Job& j) {
@@ -318,9 +322,17 @@ gt_status gt_write(gt_ctx* ctx, gt_buf dst, const void* host, uint64_t bytes) {
   return GT_OK;
 }
 
-gt_status gt_read(gt_ctx* ctx, gt_buf src, void* host, uint64_t bytes) {
-  if (bytes == 0) return GT_OK;
-  GT_REQUIRE(ctx, src && host, "gt_read: null argument");
+gt_status gt_read(gt_ctx* ctx, gt_buf src, void* host, uint64_t bytes) { return gt_read_many(ctx, 1, &src, &host, &bytes); }
+
+gt_status gt_read_many(gt_ctx* ctx, int32_t n, const gt_buf* srcs, void* const* hosts, const uint64_t* sizes) {
+  GT_REQUIRE(ctx, n >= 0 && (n == 0 || (srcs && hosts && sizes)), "gt_read_many: null argument");
+  uint64_t total = 0;
+  for (int i = 0; i < n; i++) {
+    if (sizes[i] == 0) continue;
+    GT_REQUIRE(ctx, srcs[i] && hosts[i], "gt_read: null argument");
+    total += sizes[i];
+  }
+  if (total == 0) return GT_OK;
   if (ctx->capturing) return gt_fail(ctx, GT_ERR_STATE, "gt_read inside a graph capture");
   if (!ctx->host_copy) {
     GtHostCopy* hc = new GtHostCopy();
@@ -329,43 +341,56 @@ gt_status gt_read(gt_ctx* ctx, gt_buf src, void* host, uint64_t bytes) {
     ctx->host_copy = hc;
   }
   GtHostCopy& hc = *ctx->host_copy;
-  if (bytes <= 64 * 1024) {                 // (every slot is empty between calls)
-    GT_CUDA(ctx, cudaMemcpyAsync(hc.ring, gt_ptr<void>(src), bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    GT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    memcpy(host, hc.ring, bytes);
-    ctx->readback_bytes += bytes;
-    return GT_OK;
-  }
-  // Blocks of an eighth of the read between 128 KB and 1 MB, so that a read of a few megabytes keeps every thread busy too.
-  // This thread alone talks to the driver (waits in several threads would queue up behind its launches): it keeps LAG
-  // copies ahead of the block it waits for and hands over what has landed.
-  constexpr uint64_t LAG = 5;
-  uint64_t block = (bytes / 8 + 4095) / 4096 * 4096;
+  // Blocks of an eighth of the whole between 128 and 512 KB, so that a read of a few megabytes keeps every thread busy too;
+  // small arrays share one. This thread alone talks to the driver (waits in several threads would queue up behind its
+  // launches): it keeps LAG copies ahead of the block it waits for and hands over what has landed.
+  uint64_t block = (total / 8 + 4095) / 4096 * 4096;
   block = block < (128u << 10) ? (128u << 10) : block > GtHostCopy::BLOCK ? GtHostCopy::BLOCK : block;
-  const uint64_t n = (bytes + block - 1) / block;
   cudaError_t err = cudaSuccess;
-  auto len = [&](uint64_t i) { return i + 1 < n ? block : bytes - i * block; };
-  for (uint64_t i = 0; i < n + LAG && err == cudaSuccess; i++) {
-    if (i < n) {
-      const int slot = (int)(i % GtHostCopy::SLOTS);
+  int item = 0;
+  uint64_t off = 0;                         // what follows is byte `off` of array `item`
+  long issued = 0, handed = 0;
+  for (bool more = true; err == cudaSuccess && (more || handed < issued);) {
+    while (item < n && off == sizes[item]) { item++; off = 0; }
+    more = item < n;
+    if (more) {
+      const int slot = (int)(issued % GtHostCopy::SLOTS);
       while (hc.busy[slot].load(std::memory_order_acquire)) cpu_pause();
-      err = cudaMemcpyAsync(hc.ring + (uint64_t)slot * GtHostCopy::BLOCK, (char*)gt_ptr<void>(src) + i * block, len(i), cudaMemcpyDeviceToHost, ctx->stream);
+      auto& pieces = hc.pieces[slot];
+      pieces.clear();
+      uint64_t fill = 0;
+      while (item < n && fill < block && err == cudaSuccess) {
+        const uint64_t len = std::min(sizes[item] - off, block - fill);
+        if (len) {
+          err = cudaMemcpyAsync(hc.ring + (uint64_t)slot * GtHostCopy::BLOCK + fill, gt_ptr<char>(srcs[item]) + off, len, cudaMemcpyDeviceToHost, ctx->stream);
+          pieces.push_back({(char*)hosts[item] + off, fill, len});
+        }
+        fill += (len + 63) / 64 * 64;
+        off += len;
+        if (off == sizes[item]) { item++; off = 0; }
+      }
       if (err == cudaSuccess) err = cudaEventRecord(hc.landed[slot], ctx->stream);
-      if (err == cudaSuccess) hc.busy[slot].store(1, std::memory_order_relaxed);
+      if (err == cudaSuccess) { hc.busy[slot].store(1, std::memory_order_relaxed); issued++; }
     }
-    if (i >= LAG && i - LAG < n && err == cudaSuccess) {
-      const int slot = (int)((i - LAG) % GtHostCopy::SLOTS);
+    if (err == cudaSuccess && handed < issued && (issued - handed > GtHostCopy::LAG || item >= n)) {
+      const int slot = (int)(handed % GtHostCopy::SLOTS);
       err = cudaEventSynchronize(hc.landed[slot]);
-      if (err == cudaSuccess) hc.put({(char*)host + (i - LAG) * block, slot, len(i - LAG)});
+      if (err == cudaSuccess) {
+        if (issued == 1) hc.empty({slot});  // a single block: no hand-over
+        else hc.put({slot});
+        handed++;
+      }
     }
   }
   for (GtHostCopy::Job j; hc.take(j);) hc.empty(j);
-  for (auto& b : hc.busy) {
-    if (err != cudaSuccess) b = 0;           // (blocks that were never handed over)
-    while (b.load(std::memory_order_acquire)) cpu_pause();
+  if (err != cudaSuccess) {
+    cudaStreamSynchronize(ctx->stream);
+    for (; handed < issued; handed++) hc.busy[handed % GtHostCopy::SLOTS] = 0;   // (blocks that were never handed over)
   }
+  for (auto& b : hc.busy)
+    while (b.load(std::memory_order_acquire)) cpu_pause();
   if (err != cudaSuccess) return gt_check_cuda(ctx, err, "gt_read");
-  ctx->readback_bytes += bytes;
+  ctx->readback_bytes += total;
   return GT_OK;
 }
 

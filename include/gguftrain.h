@@ -60,6 +60,9 @@ gt_status gt_alloc_state(gt_ctx* ctx, uint64_t bytes, gt_buf* out); /* zero-fill
 gt_status gt_free(gt_ctx* ctx, gt_buf buf);                         /* back to the pool */
 gt_status gt_write(gt_ctx* ctx, gt_buf dst, const void* host, uint64_t bytes);
 gt_status gt_read(gt_ctx* ctx, gt_buf src, void* host, uint64_t bytes); /* blocks until the data is on the host */
+/* n such reads as one: array i of bytes[i] bytes at srcs[i] to hosts[i] (the parameters of a model after a training run: their
+ * copies and the hand-over to pageable memory overlap across arrays) */
+gt_status gt_read_many(gt_ctx* ctx, int32_t n, const gt_buf* srcs, void* const* hosts, const uint64_t* bytes);
 /* The same read without blocking the caller or the compute stream (checkpoints taken while training goes on:
  * MuonGpu.syncWeightsToHost / exportState, src/backend/muon-gpu.ts:440-470, built on readStateBuffer,
  * src/backend/webgpu.ts:1492-1503). gt_read_async snapshots `bytes` at `src` as of the work enqueued so far into

@@ -9,10 +9,10 @@ from gguf_trainer_b200 import _lib  # noqa: E402  (only its header parser is use
 
 FFI = {"gt_ctx*": "pointer", "gt_ctx**": "buffer", "gt_buf": "u64", "gt_buf*": "buffer", "const gt_buf*": "buffer", "int32_t": "i32",
        "int32_t*": "buffer", "const int32_t*": "buffer", "uint64_t": "u64", "uint64_t*": "buffer", "const uint64_t*": "buffer",
-       "float": "f32", "float*": "buffer", "double": "f64", "const void*": "buffer", "void*": "buffer", "char*": "buffer",
+       "float": "f32", "float*": "buffer", "double": "f64", "void* const*": "buffer", "const void*": "buffer", "void*": "buffer", "char*": "buffer",
        "const uint8_t*": "buffer", "uint8_t*": "buffer", "uint32_t*": "buffer"}
 # calls that wait for the device: declared nonblocking so they return Promises
-BLOCKING = {"gt_sync", "gt_read", "gt_read_finish", "gt_graph_end", "gt_event_elapsed_ms", "gt_dp_wait_host", "gt_tokens_max", "gt_dp_init"}
+BLOCKING = {"gt_sync", "gt_read", "gt_read_many", "gt_read_finish", "gt_graph_end", "gt_event_elapsed_ms", "gt_dp_wait_host", "gt_tokens_max", "gt_dp_init"}
 
 
 def table() -> str:

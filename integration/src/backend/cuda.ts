@@ -39,6 +39,7 @@ const SYMBOLS = {
   gt_free: { parameters: ["pointer", "u64"], result: "i32" },
   gt_write: { parameters: ["pointer", "u64", "buffer", "u64"], result: "i32" },
   gt_read: { parameters: ["pointer", "u64", "buffer", "u64"], result: "i32", nonblocking: true },
+  gt_read_many: { parameters: ["pointer", "i32", "buffer", "buffer", "buffer"], result: "i32", nonblocking: true },
   gt_read_async: { parameters: ["pointer", "u64", "u64", "buffer"], result: "i32" },
   gt_read_fence: { parameters: ["pointer"], result: "i32" },
   gt_read_finish: { parameters: ["pointer", "u64", "buffer", "u64"], result: "i32", nonblocking: true },
