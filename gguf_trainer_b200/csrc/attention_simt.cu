@@ -140,6 +140,7 @@ __global__ void __launch_bounds__(G::NT) attn_fwd_f32_kernel(int rows, int T, in
                                                              const float* __restrict__ q, const float* __restrict__ k,
                                                              const float* __restrict__ v, float* __restrict__ out,
                                                              float* __restrict__ lse, int vec) {
+  pdl_wait();
   extern __shared__ __align__(16) float sm[];
   constexpr int R = G::R, C = G::C, TR = G::TR, TX = G::TX;
   float* Qs = sm;
@@ -222,6 +223,7 @@ __global__ void __launch_bounds__(G::NT) attn_fwd_f32_kernel(int rows, int T, in
 // D[h,row] = sum_d dO*O   (srcAttnBwdD)
 __global__ void attn_bwd_d_kernel(int rows, int Hq, int hd, const float* __restrict__ go, const float* __restrict__ o,
                                   float* __restrict__ D) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long w = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (w >= (long)rows * Hq) return;
@@ -417,6 +419,7 @@ __device__ void bwd_dkv(const BwdArgs& p, float* sm, int item) {
 // One launch for both: the dK/dV tiles first (the longer ones), then the dQ tiles.
 template <class G>
 __global__ void __launch_bounds__(G::NT) attn_bwd_f32_kernel(const __grid_constant__ BwdArgs p) {
+  pdl_wait();
   extern __shared__ __align__(16) float sm[];
   const int dkv = (int)gridDim.x - p.dq_ctas;
   if ((int)blockIdx.x < dkv) bwd_dkv<G>(p, sm, blockIdx.x);
@@ -432,7 +435,7 @@ gt_status launch_fwd(gt_ctx* ctx, int rows, int T, int Hq, int Hkv, int hd, int 
     done[ctx->device] = true;
   }
   const float scale2 = 1.4426950408889634f / sqrtf((float)hd);
-  attn_fwd_f32_kernel<G><<<dim3(Hq * (rows / T), gt_cdiv(T, G::R)), G::NT, G::FWD_SMEM, ctx->stream>>>(rows, T, Hq, Hkv, hd, window, scale2, q, k, v, out, lse, vec);
+  GT_CUDA(ctx, gt_launch(ctx, 1, attn_fwd_f32_kernel<G>, dim3(Hq * (rows / T), gt_cdiv(T, G::R)), G::NT, G::FWD_SMEM, rows, T, Hq, Hkv, hd, window, scale2, q, k, v, out, lse, vec));
   GT_LAUNCHED(ctx, "attn_fwd_f32_kernel");
   return GT_OK;
 }
@@ -452,18 +455,7 @@ gt_status launch_bwd(gt_ctx* ctx, BwdArgs p) {
       if (group % c == 0) p.cs = c;
   const long dkv = p.gk || p.gv ? (long)p.ntiles * p.Hkv * nseq * p.cs : 0;
   p.dq_ctas = p.gq ? p.ntiles * p.Hq * nseq : 0;           // (a multiple of cs: Hq is)
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(dkv + p.dq_ctas), 1, 1);
-  cfg.blockDim = dim3(G::NT, 1, 1);
-  cfg.dynamicSmemBytes = G::BWD_SMEM;
-  cfg.stream = ctx->stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = p.cs;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = p.cs > 1 ? 1 : 0;
-  GT_CUDA(ctx, cudaLaunchKernelEx(&cfg, attn_bwd_f32_kernel<G>, p));
+  GT_CUDA(ctx, gt_launch(ctx, p.cs, attn_bwd_f32_kernel<G>, dim3((unsigned)(dkv + p.dq_ctas)), G::NT, G::BWD_SMEM, p));
   GT_LAUNCHED(ctx, "attn_bwd_f32_kernel");
   return GT_OK;
 }
@@ -509,7 +501,7 @@ gt_status gt_attention_bwd_simt_scratch(gt_ctx* ctx, float* D, int rows, int T, 
                                         int accum_v) {
   GT_REQUIRE(ctx, ctx->device >= 0 && ctx->device < 64, "gt_attention_bwd: device index %d out of range", ctx->device);
   const long warps = (long)rows * Hq;
-  attn_bwd_d_kernel<<<gt_cdiv(warps * 32, 256), 256, 0, ctx->stream>>>(rows, Hq, hd, go, out, D);
+  GT_CUDA(ctx, gt_launch(ctx, 1, attn_bwd_d_kernel, gt_cdiv(warps * 32, 256), 256, 0, rows, Hq, hd, go, out, D));
   GT_LAUNCHED(ctx, "attn_bwd_d_kernel");
   BwdArgs p = {};
   p.rows = rows; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.hd = hd; p.window = window;

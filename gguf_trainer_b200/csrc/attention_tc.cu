@@ -230,6 +230,7 @@ __global__ void __launch_bounds__(FWD_THREADS, HD <= 64 ? 2 : 1)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                    const __grid_constant__ CUtensorMap mapV, float* __restrict__ out, float* __restrict__ lse, int rows, int T,
                    int Hq, int Hkv, int window, float scale2, int* __restrict__ flag) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   using S = FwdSmem<HD, SPLIT>;
   constexpr int ATOMS = HD / 32, HH = HD / 2, HDF = HD * SPLIT;
@@ -424,6 +425,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
 template <int HD>
 __global__ void attn_bwd_d_tc_kernel(long nitems, float scale, const float* __restrict__ go, const float* __restrict__ o,
                                      float* __restrict__ D, int rows, int Hq) {
+  pdl_wait();
   constexpr int L = HD / 4 < 32 ? HD / 4 : 32;   // lanes per item: 8, 16 or 32
   constexpr int PER = HD / 4 / L;                // 16-byte loads per lane and tensor (2 at HD 256)
   const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -476,6 +478,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_co
                        const float* __restrict__ lse, const float* __restrict__ Ds, float* gk, int accum_k, float* gv, int accum_v,
                        int rows, int T, int Hq, int Hkv, int window, float scale2, float dp_scale, const float2* __restrict__ rope,
                        const int* __restrict__ order, int hs, int* __restrict__ flag) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   using S = DkvSmem<HD, NQ, KBUF, MBUF, SPLIT>;
   constexpr int ATOMS = HD / 32, NH = NQ / 2, HH = HD / 2, HDF = HD * SPLIT;
@@ -822,6 +825,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                       const __grid_constant__ CUtensorMap mapKm, const float* __restrict__ lse, const float* __restrict__ Ds,
                       float* gq, int accum_q, int rows, int T, int Hq, int Hkv, int window, float scale2, float dp_scale, const float2* __restrict__ rope,
                       int* __restrict__ flag) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   using S = DqSmem<HD, NK, KBUF, SB, SPLIT>;
   constexpr int ATOMS = HD / 32, NH = NK / 2, HH = HD / 2, HDF = HD * SPLIT;
@@ -1043,24 +1047,6 @@ gt_status set_smem(gt_ctx* ctx, K kern, int bytes, bool* done) {
   return GT_OK;
 }
 
-// <<<grid, threads, smem, stream>>> with the grid's x axis grouped into clusters of `split` CTAs
-template <typename... KA, typename... A>
-cudaError_t launch_split(void (*kern)(KA...), dim3 grid, int threads, int smem, cudaStream_t stream, int split, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = split;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = split > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
-}
-
 template <int HD, int SPLIT>
 gt_status launch_fwd(gt_ctx* ctx, int rows, int T, int Hq, int Hkv, int window, const float* q, const float* k, const float* v,
                      float* out, float* lse, int* flag) {
@@ -1077,8 +1063,7 @@ gt_status launch_fwd(gt_ctx* ctx, int rows, int T, int Hq, int Hkv, int window, 
   // the S product's truncation bias is folded into the score scale
   const float scale2 = 1.4426950408889634f / sqrtf((float)(HD * SPLIT)) * TRUNC_COMP;
   dim3 grid(Hq * (rows / T) * SPLIT, gt_cdiv(T, ROWS), 1);
-  if (SPLIT == 1) kern<<<grid, FWD_THREADS, SM::TOTAL, ctx->stream>>>(mq, mk, mv, out, lse, rows, T, Hq, Hkv, window, scale2, flag);
-  else GT_CUDA(ctx, launch_split(kern, grid, FWD_THREADS, SM::TOTAL, ctx->stream, SPLIT, mq, mk, mv, out, lse, rows, T, Hq, Hkv, window, scale2, flag));
+  GT_CUDA(ctx, gt_launch(ctx, SPLIT, kern, grid, FWD_THREADS, SM::TOTAL, mq, mk, mv, out, lse, rows, T, Hq, Hkv, window, scale2, flag));
   GT_LAUNCHED(ctx, "attn_fwd_tc_kernel");
   return GT_OK;
 }
@@ -1181,7 +1166,7 @@ gt_status launch_bwd(gt_ctx* ctx, int rows, int T, int Hq, int Hkv, int window, 
   constexpr int HDF = HD * SPLIT;
   const float scale = 1.f / sqrtf((float)HDF);
   const long nitems = (long)rows * Hq;
-  attn_bwd_d_tc_kernel<HDF><<<(unsigned)gt_cdiv(nitems * (HDF / 4 < 32 ? HDF / 4 : 32), 256l), 256, 0, ctx->stream>>>(nitems, scale, go, out, D, rows, Hq);
+  GT_CUDA(ctx, gt_launch(ctx, 1, attn_bwd_d_tc_kernel<HDF>, (unsigned)gt_cdiv(nitems * (HDF / 4 < 32 ? HDF / 4 : 32), 256l), 256, 0, nitems, scale, go, out, D, rows, Hq));
   GT_LAUNCHED(ctx, "attn_bwd_d_tc_kernel");
   const float scale2 = 1.4426950408889634f * scale * TRUNC_COMP;
   const float dp_scale = scale * TRUNC_COMP;
@@ -1206,7 +1191,7 @@ gt_status launch_bwd(gt_ctx* ctx, int rows, int T, int Hq, int Hkv, int window, 
       st = attn_dkv_order(ctx, (int)grid.y, (int)grid.x, Hq / Hkv, T, NQ, window, &order);
       if (st) return st;
     }
-    GT_CUDA(ctx, launch_split(kern, grid, THREADS, SM::TOTAL, ctx->stream, SPLIT * hs, mK, mV, mQk, mQm, mGk, mGm, lse, D, gk, accum_k, gv, accum_v,
+    GT_CUDA(ctx, gt_launch(ctx, SPLIT * hs, kern, grid, THREADS, SM::TOTAL, mK, mV, mQk, mQm, mGk, mGm, lse, D, gk, accum_k, gv, accum_v,
                               rows, T, Hq, Hkv, window, scale2, dp_scale, rope, order, hs, flag));
     GT_LAUNCHED(ctx, "attn_bwd_dkv_tc_kernel");
   }
@@ -1222,10 +1207,7 @@ gt_status launch_bwd(gt_ctx* ctx, int rows, int T, int Hq, int Hkv, int window, 
     st = set_smem(ctx, kern, SM::TOTAL, done);
     if (st) return st;
     dim3 grid(Hq * nseq * SPLIT, gt_cdiv(T, ROWS), 1);
-    if (SPLIT == 1)
-      kern<<<grid, THREADS, SM::TOTAL, ctx->stream>>>(mQ, mG, mKk, mVk, mKm, lse, D, gq, accum_q, rows, T, Hq, Hkv, window, scale2, dp_scale, rope, flag);
-    else
-      GT_CUDA(ctx, launch_split(kern, grid, THREADS, SM::TOTAL, ctx->stream, SPLIT, mQ, mG, mKk, mVk, mKm, lse, D, gq, accum_q, rows, T, Hq, Hkv,
+    GT_CUDA(ctx, gt_launch(ctx, SPLIT, kern, grid, THREADS, SM::TOTAL, mQ, mG, mKk, mVk, mKm, lse, D, gq, accum_q, rows, T, Hq, Hkv,
                                 window, scale2, dp_scale, rope, flag));
     GT_LAUNCHED(ctx, "attn_bwd_dq_tc_kernel");
   }

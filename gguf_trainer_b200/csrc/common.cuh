@@ -95,6 +95,33 @@ enum { GT_FLAG_WINDOW = 0, GT_FLAG_TOKEN_MAX = 1, GT_FLAG_NORM_COUNTER = 8 };
     if (!(cond)) return gt_fail(ctx, GT_ERR_ARG, __VA_ARGS__);          \
   } while (0)
 
+// Every kernel launched through gt_launch starts with pdl_wait(): the next kernel in the stream is then brought onto the
+// chip while the last CTAs of this one finish (programmatic stream serialisation), which takes 0.4 us off the gap between
+// two kernels: 348 -> 326 us for a recorded step of 60 small kernels, 6270 -> 6130 us for one of 400. The wait returns when
+// everything earlier in the stream is complete and visible; nothing global may be read or written before it. No kernel
+// lets its successor start before it ends: an early start puts the successor's CTAs wherever there is room at that
+// moment, two on one SM and none on another, and measured 10 % slower over a whole step.
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_wait() { cudaGridDependencySynchronize(); }
+#endif
+template <typename... KA, typename... A>
+static inline cudaError_t gt_launch(gt_ctx* ctx, int cluster, void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = cluster;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
+}
+
 template <typename T>
 static inline T* gt_ptr(gt_buf b) { return reinterpret_cast<T*>(static_cast<uintptr_t>(b)); }
 static inline int gt_cdiv(long a, long b) { return (int)((a + b - 1) / b); }

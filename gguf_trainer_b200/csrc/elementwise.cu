@@ -42,6 +42,7 @@ __device__ __forceinline__ float ew_da(float a, float b, float c) {
 template <int OP>
 __global__ void ew_fwd_kernel(size_t n, const float* __restrict__ a, const float* __restrict__ b, float c,
                               float* __restrict__ out) {
+  pdl_wait();
   constexpr bool BIN = (OP == GT_EW_ADD || OP == GT_EW_MUL);
   size_t n4 = n / 4;
   size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -62,6 +63,7 @@ __global__ void ew_fwd_kernel(size_t n, const float* __restrict__ a, const float
 template <int OP>
 __global__ void ew_bwd_kernel(size_t n, const float* __restrict__ a, const float* __restrict__ b, float c,
                               const float* __restrict__ g, float* ga, int acc_a, float* gb, int acc_b) {
+  pdl_wait();
   constexpr bool BIN = (OP == GT_EW_ADD || OP == GT_EW_MUL);
   const bool alias = BIN && ga && ga == gb;
   size_t n4 = n / 4;
@@ -110,6 +112,7 @@ __global__ void ew_bwd_kernel(size_t n, const float* __restrict__ a, const float
 // touches HBM: forward 12 B/element instead of 20, backward 20 instead of 32.
 template <int OP>
 __global__ void glu_fwd_kernel(size_t n, const float* __restrict__ x, const float* __restrict__ u, float* __restrict__ out) {
+  pdl_wait();
   size_t n4 = n / 4, stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
     float4 a = ((const float4*)x)[i], b = ((const float4*)u)[i], r;
@@ -124,6 +127,7 @@ __global__ void glu_fwd_kernel(size_t n, const float* __restrict__ x, const floa
 template <int OP>
 __global__ void glu_bwd_kernel(size_t n, const float* __restrict__ x, const float* __restrict__ u, const float* __restrict__ g,
                                float* gx, int acc_x, float* gu, int acc_u) {
+  pdl_wait();
   size_t n4 = n / 4, stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
     const float4 a = ((const float4*)x)[i], b = ((const float4*)u)[i], go = ((const float4*)g)[i];
@@ -166,11 +170,11 @@ gt_status gt_ew_fwd(gt_ctx* ctx, int32_t op, uint64_t n, gt_buf a, gt_buf b, flo
   GT_REQUIRE(ctx, pa && po && aligned16(pa) && aligned16(po) && aligned16(pb), "gt_ew_fwd: operands must be non-null and 16-byte aligned");
   int grid = ew_grid(ctx, n);
   switch (op) {
-    case GT_EW_ADD: GT_REQUIRE(ctx, pb, "gt_ew_fwd: add needs b"); ew_fwd_kernel<GT_EW_ADD><<<grid, 256, 0, ctx->stream>>>(n, pa, pb, c, po); break;
-    case GT_EW_MUL: GT_REQUIRE(ctx, pb, "gt_ew_fwd: mul needs b"); ew_fwd_kernel<GT_EW_MUL><<<grid, 256, 0, ctx->stream>>>(n, pa, pb, c, po); break;
-    case GT_EW_SILU: ew_fwd_kernel<GT_EW_SILU><<<grid, 256, 0, ctx->stream>>>(n, pa, pb, c, po); break;
-    case GT_EW_GELU: ew_fwd_kernel<GT_EW_GELU><<<grid, 256, 0, ctx->stream>>>(n, pa, pb, c, po); break;
-    case GT_EW_SCALE: ew_fwd_kernel<GT_EW_SCALE><<<grid, 256, 0, ctx->stream>>>(n, pa, pb, c, po); break;
+    case GT_EW_ADD: GT_REQUIRE(ctx, pb, "gt_ew_fwd: add needs b"); GT_CUDA(ctx, gt_launch(ctx, 1, ew_fwd_kernel<GT_EW_ADD>, grid, 256, 0, n, pa, pb, c, po)); break;
+    case GT_EW_MUL: GT_REQUIRE(ctx, pb, "gt_ew_fwd: mul needs b"); GT_CUDA(ctx, gt_launch(ctx, 1, ew_fwd_kernel<GT_EW_MUL>, grid, 256, 0, n, pa, pb, c, po)); break;
+    case GT_EW_SILU: GT_CUDA(ctx, gt_launch(ctx, 1, ew_fwd_kernel<GT_EW_SILU>, grid, 256, 0, n, pa, pb, c, po)); break;
+    case GT_EW_GELU: GT_CUDA(ctx, gt_launch(ctx, 1, ew_fwd_kernel<GT_EW_GELU>, grid, 256, 0, n, pa, pb, c, po)); break;
+    case GT_EW_SCALE: GT_CUDA(ctx, gt_launch(ctx, 1, ew_fwd_kernel<GT_EW_SCALE>, grid, 256, 0, n, pa, pb, c, po)); break;
     default: return gt_fail(ctx, GT_ERR_ARG, "gt_ew_fwd: unknown op %d", op);
   }
   GT_LAUNCHED(ctx, "ew_fwd_kernel");
@@ -188,11 +192,11 @@ gt_status gt_ew_bwd(gt_ctx* ctx, int32_t op, uint64_t n, gt_buf a, gt_buf b, flo
   GT_REQUIRE(ctx, pg && aligned16(pa) && aligned16(pb) && aligned16(pg) && aligned16(pga) && aligned16(pgb), "gt_ew_bwd: operands must be 16-byte aligned");
   int grid = ew_grid(ctx, n);
   switch (op) {
-    case GT_EW_ADD: ew_bwd_kernel<GT_EW_ADD><<<grid, 256, 0, ctx->stream>>>(n, pa, pb, c, pg, pga, accum_a, pgb, accum_b); break;
-    case GT_EW_MUL: GT_REQUIRE(ctx, pa && pb, "gt_ew_bwd: mul needs a and b"); ew_bwd_kernel<GT_EW_MUL><<<grid, 256, 0, ctx->stream>>>(n, pa, pb, c, pg, pga, accum_a, pgb, accum_b); break;
-    case GT_EW_SILU: GT_REQUIRE(ctx, pa, "gt_ew_bwd: silu needs a"); ew_bwd_kernel<GT_EW_SILU><<<grid, 256, 0, ctx->stream>>>(n, pa, pb, c, pg, pga, accum_a, pgb, accum_b); break;
-    case GT_EW_GELU: GT_REQUIRE(ctx, pa, "gt_ew_bwd: gelu needs a"); ew_bwd_kernel<GT_EW_GELU><<<grid, 256, 0, ctx->stream>>>(n, pa, pb, c, pg, pga, accum_a, pgb, accum_b); break;
-    case GT_EW_SCALE: ew_bwd_kernel<GT_EW_SCALE><<<grid, 256, 0, ctx->stream>>>(n, pa, pb, c, pg, pga, accum_a, pgb, accum_b); break;
+    case GT_EW_ADD: GT_CUDA(ctx, gt_launch(ctx, 1, ew_bwd_kernel<GT_EW_ADD>, grid, 256, 0, n, pa, pb, c, pg, pga, accum_a, pgb, accum_b)); break;
+    case GT_EW_MUL: GT_REQUIRE(ctx, pa && pb, "gt_ew_bwd: mul needs a and b"); GT_CUDA(ctx, gt_launch(ctx, 1, ew_bwd_kernel<GT_EW_MUL>, grid, 256, 0, n, pa, pb, c, pg, pga, accum_a, pgb, accum_b)); break;
+    case GT_EW_SILU: GT_REQUIRE(ctx, pa, "gt_ew_bwd: silu needs a"); GT_CUDA(ctx, gt_launch(ctx, 1, ew_bwd_kernel<GT_EW_SILU>, grid, 256, 0, n, pa, pb, c, pg, pga, accum_a, pgb, accum_b)); break;
+    case GT_EW_GELU: GT_REQUIRE(ctx, pa, "gt_ew_bwd: gelu needs a"); GT_CUDA(ctx, gt_launch(ctx, 1, ew_bwd_kernel<GT_EW_GELU>, grid, 256, 0, n, pa, pb, c, pg, pga, accum_a, pgb, accum_b)); break;
+    case GT_EW_SCALE: GT_CUDA(ctx, gt_launch(ctx, 1, ew_bwd_kernel<GT_EW_SCALE>, grid, 256, 0, n, pa, pb, c, pg, pga, accum_a, pgb, accum_b)); break;
     default: return gt_fail(ctx, GT_ERR_ARG, "gt_ew_bwd: unknown op %d", op);
   }
   GT_LAUNCHED(ctx, "ew_bwd_kernel");
@@ -205,8 +209,8 @@ gt_status gt_glu_fwd(gt_ctx* ctx, int32_t op, uint64_t n, gt_buf x, gt_buf u, gt
   GT_REQUIRE(ctx, px && pu && po && aligned16(px) && aligned16(pu) && aligned16(po), "gt_glu_fwd: operands must be non-null and 16-byte aligned");
   GT_REQUIRE(ctx, op == GT_EW_SILU || op == GT_EW_GELU, "gt_glu_fwd: the gate activation must be silu or gelu, got op %d", op);
   int grid = ew_grid(ctx, n);
-  if (op == GT_EW_SILU) glu_fwd_kernel<GT_EW_SILU><<<grid, 256, 0, ctx->stream>>>(n, px, pu, po);
-  else glu_fwd_kernel<GT_EW_GELU><<<grid, 256, 0, ctx->stream>>>(n, px, pu, po);
+  if (op == GT_EW_SILU) GT_CUDA(ctx, gt_launch(ctx, 1, glu_fwd_kernel<GT_EW_SILU>, grid, 256, 0, n, px, pu, po));
+  else GT_CUDA(ctx, gt_launch(ctx, 1, glu_fwd_kernel<GT_EW_GELU>, grid, 256, 0, n, px, pu, po));
   GT_LAUNCHED(ctx, "glu_fwd_kernel");
   return GT_OK;
 }
@@ -239,8 +243,8 @@ gt_status gt_glu_bwd(gt_ctx* ctx, int32_t op, uint64_t n, gt_buf x, gt_buf u, gt
   GT_REQUIRE(ctx, op == GT_EW_SILU || op == GT_EW_GELU, "gt_glu_bwd: the gate activation must be silu or gelu, got op %d", op);
   GT_REQUIRE(ctx, !pgx || pgx != pgu, "gt_glu_bwd: the two gradient outputs alias");
   int grid = ew_grid(ctx, n);
-  if (op == GT_EW_SILU) glu_bwd_kernel<GT_EW_SILU><<<grid, 256, 0, ctx->stream>>>(n, px, pu, pg, pgx, accum_x, pgu, accum_u);
-  else glu_bwd_kernel<GT_EW_GELU><<<grid, 256, 0, ctx->stream>>>(n, px, pu, pg, pgx, accum_x, pgu, accum_u);
+  if (op == GT_EW_SILU) GT_CUDA(ctx, gt_launch(ctx, 1, glu_bwd_kernel<GT_EW_SILU>, grid, 256, 0, n, px, pu, pg, pgx, accum_x, pgu, accum_u));
+  else GT_CUDA(ctx, gt_launch(ctx, 1, glu_bwd_kernel<GT_EW_GELU>, grid, 256, 0, n, px, pu, pg, pgx, accum_x, pgu, accum_u));
   GT_LAUNCHED(ctx, "glu_bwd_kernel");
   return GT_OK;
 }

@@ -113,6 +113,7 @@ __device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a
 // gridDim.x = tiles x ksplit, the ksplit CTAs of a tile adjacent and, when there are several, one cluster.
 template <class T, bool A_K, bool B_K, bool VEC>
 __global__ void __launch_bounds__(T::THREADS) gemm_f32_kernel(const __grid_constant__ F32Args p, int ksplit) {
+  pdl_wait();
   extern __shared__ __align__(16) float sm[];
   constexpr int BM = T::BM, BN = T::BN, BK = T::BK, TM = T::TM, TN = T::TN;
   constexpr int TX = BN / TN, TY = BM / TM;
@@ -242,18 +243,7 @@ gt_status launch(gt_ctx* ctx, const F32Args& p, long tiles, int ksplit) {
     GT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM));
     attr_set[ctx->device] = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(tiles * ksplit), 1, 1);
-  cfg.blockDim = dim3(T::THREADS, 1, 1);
-  cfg.dynamicSmemBytes = T::SMEM;
-  cfg.stream = ctx->stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = ksplit;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = ksplit > 1 ? 1 : 0;
-  GT_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, p, ksplit));
+  GT_CUDA(ctx, gt_launch(ctx, ksplit, kern, dim3((unsigned)(tiles * ksplit)), T::THREADS, T::SMEM, p, ksplit));
   GT_LAUNCHED(ctx, "gemm_f32_kernel");
   return GT_OK;
 }

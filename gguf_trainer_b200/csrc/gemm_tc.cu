@@ -92,6 +92,7 @@ template <bool A_K, bool B_K, int BN, int MT, int GLU = 0>
 __global__ void __launch_bounds__(Smem<BN, MT, EpiSub<MT, GLU>::N>::THREADS, 1)
 gemm_tf32_kernel(const __grid_constant__ PartMaps maps, float* __restrict__ C, int M_, int N_,
                  int accum_, int ksplit, int use_tma_store, int batch, float out_scale, int* __restrict__ flag) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   constexpr int SUB = EpiSub<MT, GLU>::N;
   using S = Smem<BN, MT, SUB>;
@@ -422,6 +423,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SmemPair<BN>::THREAD
 gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                       const __grid_constant__ CUtensorMap mapC, float* __restrict__ C, int M, int N, int K, int accum, int ksplit,
                       int use_tma_store, int batch, float out_scale, int* __restrict__ flag) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   using S = SmemPair<BN>;
   constexpr int STAGES = S::STAGES, BM = 2 * BM1;
@@ -603,6 +605,7 @@ struct SmallSmem {
 template <bool A_K, bool B_K, int BN, int EPI>
 __global__ void __launch_bounds__(SmallSmem<BN>::THREADS)
 gemm_tf32_small_kernel(const __grid_constant__ PartMaps maps, int M_, int N_, int accum_, int ksplit, float out_scale, int* __restrict__ flag) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   using S = SmallSmem<BN>;
   constexpr int STAGES = S::STAGES;
@@ -801,18 +804,7 @@ gt_status launch_small(gt_ctx* ctx, const PartMaps& maps, long tiles, int M, int
     GT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL));
     attr_set[ctx->device] = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(tiles * ksplit), 1, 1);
-  cfg.blockDim = dim3(S::THREADS, 1, 1);
-  cfg.dynamicSmemBytes = S::TOTAL;
-  cfg.stream = ctx->stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = ksplit;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = ksplit > 1 ? 1 : 0;
-  GT_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, maps, M, N, accum, ksplit, out_scale, g_flag[ctx->device]));
+  GT_CUDA(ctx, gt_launch(ctx, ksplit, kern, dim3((unsigned)(tiles * ksplit)), S::THREADS, S::TOTAL, maps, M, N, accum, ksplit, out_scale, g_flag[ctx->device]));
   GT_LAUNCHED(ctx, "gemm_tf32_small_kernel");
   return GT_OK;
 }
@@ -895,7 +887,7 @@ gt_status launch(gt_ctx* ctx, const PartMaps& maps, long ntiles, int tma_store, 
     attr_set[ctx->device] = true;
   }
   dim3 grid((unsigned)min((long)(ctx->sm_count - ctx->sm_reserved), ntiles), 1, 1);
-  kern<<<grid, S::THREADS, S::TOTAL, ctx->stream>>>(maps, c, M, N, accum, ksplit, tma_store, batch, out_scale, g_flag[ctx->device]);
+  GT_CUDA(ctx, gt_launch(ctx, 1, kern, grid, S::THREADS, S::TOTAL, maps, c, M, N, accum, ksplit, tma_store, batch, out_scale, g_flag[ctx->device]));
   GT_LAUNCHED(ctx, "gemm_tf32_kernel");
   return GT_OK;
 }
@@ -912,7 +904,7 @@ gt_status launch_pair(gt_ctx* ctx, const CUtensorMap& ma, const CUtensorMap& mb,
   }
   const long ntiles = (long)gt_cdiv(N, BN) * gt_cdiv(M, 2 * BM1) * ksplit * batch;
   dim3 grid(2u * (unsigned)min((long)npairs, ntiles), 1, 1);
-  kern<<<grid, S::THREADS, S::TOTAL, ctx->stream>>>(ma, mb, mc, c, M, N, K, accum, ksplit, tma_store, batch, out_scale, g_flag[ctx->device]);
+  GT_CUDA(ctx, gt_launch(ctx, 1, kern, grid, S::THREADS, S::TOTAL, ma, mb, mc, c, M, N, K, accum, ksplit, tma_store, batch, out_scale, g_flag[ctx->device]));
   GT_LAUNCHED(ctx, "gemm_tf32_pair_kernel");
   return GT_OK;
 }

@@ -12,6 +12,7 @@ template <typename TOK>
 __global__ void gather_windows_kernel(const TOK* __restrict__ tokens, const TOK* __restrict__ mask, unsigned long long count,
                                       const unsigned long long* __restrict__ starts, int B, int T, uint32_t* __restrict__ ids,
                                       uint32_t* __restrict__ targets, int* __restrict__ bad) {
+  pdl_wait();
   const long n = (long)B * T;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const int b = (int)(i / T), t = (int)(i % T);
@@ -74,11 +75,11 @@ gt_status gt_gather_windows(gt_ctx* ctx, gt_buf tokens, gt_buf mask, int32_t byt
   const int grid = (int)min((long)ctx->sm_count * 4, (n + 255) / 256);
   const unsigned long long* st = gt_ptr<const unsigned long long>(starts);
   if (bytes_per_token == 2)
-    gather_windows_kernel<uint16_t><<<grid, 256, 0, ctx->stream>>>(gt_ptr<const uint16_t>(tokens), gt_ptr<const uint16_t>(mask), count, st, B, T,
-                                                                   gt_ptr<uint32_t>(ids), gt_ptr<uint32_t>(targets), bad);
+    GT_CUDA(ctx, gt_launch(ctx, 1, gather_windows_kernel<uint16_t>, grid, 256, 0, gt_ptr<const uint16_t>(tokens), gt_ptr<const uint16_t>(mask), count, st, B, T,
+                                                                   gt_ptr<uint32_t>(ids), gt_ptr<uint32_t>(targets), bad));
   else
-    gather_windows_kernel<uint32_t><<<grid, 256, 0, ctx->stream>>>(gt_ptr<const uint32_t>(tokens), gt_ptr<const uint32_t>(mask), count, st, B, T,
-                                                                   gt_ptr<uint32_t>(ids), gt_ptr<uint32_t>(targets), bad);
+    GT_CUDA(ctx, gt_launch(ctx, 1, gather_windows_kernel<uint32_t>, grid, 256, 0, gt_ptr<const uint32_t>(tokens), gt_ptr<const uint32_t>(mask), count, st, B, T,
+                                                                   gt_ptr<uint32_t>(ids), gt_ptr<uint32_t>(targets), bad));
   GT_LAUNCHED(ctx, "gather_windows_kernel");
   return GT_OK;
 }

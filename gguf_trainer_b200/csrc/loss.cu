@@ -56,6 +56,7 @@ __device__ __forceinline__ MS row_ms(const float* __restrict__ z, int V) {
 // stats[row] = (max, 1/sum, row loss, unused)
 __global__ void __launch_bounds__(ROWT) ce_fwd_kernel(int V, const float* __restrict__ logits,
                                                       const uint32_t* __restrict__ targets, float4* __restrict__ stats) {
+  pdl_wait();
   __shared__ MS sh[ROWT / 32];
   const int row = blockIdx.x;
   const float* z = logits + (size_t)row * V;
@@ -73,6 +74,7 @@ template <int MODE>  // 0: stats float4 .z ; 1: run float3 -> log(sum)+max-tl
 __global__ void __launch_bounds__(1024) loss_reduce_kernel(int rows, int T, int nseq, const float* __restrict__ src,
                                                            const uint32_t* __restrict__ targets, int tstride,
                                                            float* __restrict__ loss, float* __restrict__ inv_kept) {
+  pdl_wait();
   __shared__ float ssum[32];
   __shared__ int scnt[32];
   __shared__ float total;
@@ -110,6 +112,7 @@ __global__ void __launch_bounds__(ROWT) ce_bwd_kernel(int V, int T, int nseq, co
                                                       const uint32_t* __restrict__ targets, const float4* __restrict__ stats,
                                                       const float* __restrict__ inv_kept, const float* __restrict__ gloss,
                                                       float* glogits, int accum) {
+  pdl_wait();
   const int row = blockIdx.x;
   const uint32_t tg = targets[row];
   float* g = glogits + (size_t)row * V;
@@ -143,6 +146,7 @@ __global__ void __launch_bounds__(ROWT) ce_bwd_kernel(int V, int T, int nseq, co
 // run[row] = (max, sum, target logit), updated with chunk columns [v0, v0+n)
 __global__ void __launch_bounds__(ROWT) ce_chunk_stats_kernel(int n, int v0, int first, const float* __restrict__ chunk,
                                                               const uint32_t* __restrict__ targets, float* __restrict__ run) {
+  pdl_wait();
   __shared__ MS sh[ROWT / 32];
   const int row = blockIdx.x;
   const float* z = chunk + (size_t)row * n;
@@ -163,6 +167,7 @@ __global__ void __launch_bounds__(ROWT) ce_chunk_stats_kernel(int n, int v0, int
 __global__ void __launch_bounds__(ROWT) ce_chunk_grad_kernel(int n, int v0, int T, int nseq, float* chunk,
                                                              const uint32_t* __restrict__ targets, const float* __restrict__ run,
                                                              const float* __restrict__ inv_kept, const float* __restrict__ gloss) {
+  pdl_wait();
   const int row = blockIdx.x;
   float* z = chunk + (size_t)row * n;
   const uint32_t tg = targets[row];
@@ -180,6 +185,7 @@ __global__ void __launch_bounds__(ROWT) ce_chunk_grad_kernel(int n, int v0, int 
 __global__ void __launch_bounds__(ROWT) soft_ce_fwd_kernel(int V, int k, const float* __restrict__ logits,
                                                            const uint32_t* __restrict__ tids, const float* __restrict__ tprobs,
                                                            float4* __restrict__ stats) {
+  pdl_wait();
   __shared__ MS sh[ROWT / 32];
   const int row = blockIdx.x;
   const float* z = logits + (size_t)row * V;
@@ -203,6 +209,7 @@ __global__ void __launch_bounds__(ROWT) soft_ce_bwd_kernel(int V, int k, int T, 
                                                            const uint32_t* __restrict__ tids, const float* __restrict__ tprobs,
                                                            const float4* __restrict__ stats, const float* __restrict__ inv_kept,
                                                            const float* __restrict__ gloss, float* glogits, int accum) {
+  pdl_wait();
   const int row = blockIdx.x;
   float* g = glogits + (size_t)row * V;
   if (tids[(size_t)row * k] == IGNORE) {
@@ -234,9 +241,9 @@ gt_status gt_ce_fwd(gt_ctx* ctx, int32_t rows, int32_t V, gt_buf logits, gt_buf 
   GT_REQUIRE(ctx, rows > 0 && V > 0 && logits && targets && stats && loss && inv_kept, "gt_ce_fwd: bad argument");
   int T, nseq; seq_shape(ctx, rows, &T, &nseq);
   GT_REQUIRE(ctx, rows == T * nseq, "gt_ce_fwd: %d rows but the batch is %d x %d", rows, nseq, T);
-  ce_fwd_kernel<<<rows, ROWT, 0, ctx->stream>>>(V, gt_ptr<const float>(logits), gt_ptr<const uint32_t>(targets), gt_ptr<float4>(stats));
+  GT_CUDA(ctx, gt_launch(ctx, 1, ce_fwd_kernel, rows, ROWT, 0, V, gt_ptr<const float>(logits), gt_ptr<const uint32_t>(targets), gt_ptr<float4>(stats)));
   GT_LAUNCHED(ctx, "ce_fwd_kernel");
-  loss_reduce_kernel<0><<<1, 1024, 0, ctx->stream>>>(rows, T, nseq, gt_ptr<const float>(stats), gt_ptr<const uint32_t>(targets), 1, gt_ptr<float>(loss), gt_ptr<float>(inv_kept));
+  GT_CUDA(ctx, gt_launch(ctx, 1, loss_reduce_kernel<0>, 1, 1024, 0, rows, T, nseq, gt_ptr<const float>(stats), gt_ptr<const uint32_t>(targets), 1, gt_ptr<float>(loss), gt_ptr<float>(inv_kept)));
   GT_LAUNCHED(ctx, "loss_reduce_kernel");
   return GT_OK;
 }
@@ -245,15 +252,15 @@ gt_status gt_ce_bwd(gt_ctx* ctx, int32_t rows, int32_t V, gt_buf logits, gt_buf 
   if (!glogits) return GT_OK;
   GT_REQUIRE(ctx, rows > 0 && V > 0 && logits && targets && stats && inv_kept && gloss, "gt_ce_bwd: bad argument");
   int T, nseq; seq_shape(ctx, rows, &T, &nseq);
-  ce_bwd_kernel<<<rows, ROWT, 0, ctx->stream>>>(V, T, nseq, gt_ptr<const float>(logits), gt_ptr<const uint32_t>(targets), gt_ptr<const float4>(stats),
-                                                gt_ptr<const float>(inv_kept), gt_ptr<const float>(gloss), gt_ptr<float>(glogits), accum);
+  GT_CUDA(ctx, gt_launch(ctx, 1, ce_bwd_kernel, rows, ROWT, 0, V, T, nseq, gt_ptr<const float>(logits), gt_ptr<const uint32_t>(targets), gt_ptr<const float4>(stats),
+                                                gt_ptr<const float>(inv_kept), gt_ptr<const float>(gloss), gt_ptr<float>(glogits), accum));
   GT_LAUNCHED(ctx, "ce_bwd_kernel");
   return GT_OK;
 }
 
 gt_status gt_ce_chunk_stats(gt_ctx* ctx, int32_t rows, int32_t n, int32_t v0, int32_t first, gt_buf chunk, gt_buf targets, gt_buf run) {
   GT_REQUIRE(ctx, rows > 0 && n > 0 && v0 >= 0 && chunk && targets && run, "gt_ce_chunk_stats: bad argument");
-  ce_chunk_stats_kernel<<<rows, ROWT, 0, ctx->stream>>>(n, v0, first, gt_ptr<const float>(chunk), gt_ptr<const uint32_t>(targets), gt_ptr<float>(run));
+  GT_CUDA(ctx, gt_launch(ctx, 1, ce_chunk_stats_kernel, rows, ROWT, 0, n, v0, first, gt_ptr<const float>(chunk), gt_ptr<const uint32_t>(targets), gt_ptr<float>(run)));
   GT_LAUNCHED(ctx, "ce_chunk_stats_kernel");
   return GT_OK;
 }
@@ -262,7 +269,7 @@ gt_status gt_ce_loss_from_stats(gt_ctx* ctx, int32_t rows, gt_buf run, gt_buf ta
   GT_REQUIRE(ctx, rows > 0 && run && targets && loss && inv_kept, "gt_ce_loss_from_stats: bad argument");
   int T, nseq; seq_shape(ctx, rows, &T, &nseq);
   GT_REQUIRE(ctx, rows == T * nseq, "gt_ce_loss_from_stats: %d rows but the batch is %d x %d", rows, nseq, T);
-  loss_reduce_kernel<1><<<1, 1024, 0, ctx->stream>>>(rows, T, nseq, gt_ptr<const float>(run), gt_ptr<const uint32_t>(targets), 1, gt_ptr<float>(loss), gt_ptr<float>(inv_kept));
+  GT_CUDA(ctx, gt_launch(ctx, 1, loss_reduce_kernel<1>, 1, 1024, 0, rows, T, nseq, gt_ptr<const float>(run), gt_ptr<const uint32_t>(targets), 1, gt_ptr<float>(loss), gt_ptr<float>(inv_kept)));
   GT_LAUNCHED(ctx, "loss_reduce_kernel");
   return GT_OK;
 }
@@ -270,8 +277,8 @@ gt_status gt_ce_loss_from_stats(gt_ctx* ctx, int32_t rows, gt_buf run, gt_buf ta
 gt_status gt_ce_chunk_grad(gt_ctx* ctx, int32_t rows, int32_t n, int32_t v0, gt_buf chunk, gt_buf targets, gt_buf run, gt_buf inv_kept, gt_buf gloss) {
   GT_REQUIRE(ctx, rows > 0 && n > 0 && chunk && targets && run && inv_kept && gloss, "gt_ce_chunk_grad: bad argument");
   int T, nseq; seq_shape(ctx, rows, &T, &nseq);
-  ce_chunk_grad_kernel<<<rows, ROWT, 0, ctx->stream>>>(n, v0, T, nseq, gt_ptr<float>(chunk), gt_ptr<const uint32_t>(targets), gt_ptr<const float>(run),
-                                                       gt_ptr<const float>(inv_kept), gt_ptr<const float>(gloss));
+  GT_CUDA(ctx, gt_launch(ctx, 1, ce_chunk_grad_kernel, rows, ROWT, 0, n, v0, T, nseq, gt_ptr<float>(chunk), gt_ptr<const uint32_t>(targets), gt_ptr<const float>(run),
+                                                       gt_ptr<const float>(inv_kept), gt_ptr<const float>(gloss)));
   GT_LAUNCHED(ctx, "ce_chunk_grad_kernel");
   return GT_OK;
 }
@@ -280,9 +287,9 @@ gt_status gt_soft_ce_fwd(gt_ctx* ctx, int32_t rows, int32_t V, int32_t k, gt_buf
   GT_REQUIRE(ctx, rows > 0 && V > 0 && k > 0 && logits && tids && tprobs && stats && loss && inv_kept, "gt_soft_ce_fwd: bad argument");
   int T, nseq; seq_shape(ctx, rows, &T, &nseq);
   GT_REQUIRE(ctx, rows == T * nseq, "gt_soft_ce_fwd: %d rows but the batch is %d x %d", rows, nseq, T);
-  soft_ce_fwd_kernel<<<rows, ROWT, 0, ctx->stream>>>(V, k, gt_ptr<const float>(logits), gt_ptr<const uint32_t>(tids), gt_ptr<const float>(tprobs), gt_ptr<float4>(stats));
+  GT_CUDA(ctx, gt_launch(ctx, 1, soft_ce_fwd_kernel, rows, ROWT, 0, V, k, gt_ptr<const float>(logits), gt_ptr<const uint32_t>(tids), gt_ptr<const float>(tprobs), gt_ptr<float4>(stats)));
   GT_LAUNCHED(ctx, "soft_ce_fwd_kernel");
-  loss_reduce_kernel<0><<<1, 1024, 0, ctx->stream>>>(rows, T, nseq, gt_ptr<const float>(stats), gt_ptr<const uint32_t>(tids), k, gt_ptr<float>(loss), gt_ptr<float>(inv_kept));
+  GT_CUDA(ctx, gt_launch(ctx, 1, loss_reduce_kernel<0>, 1, 1024, 0, rows, T, nseq, gt_ptr<const float>(stats), gt_ptr<const uint32_t>(tids), k, gt_ptr<float>(loss), gt_ptr<float>(inv_kept)));
   GT_LAUNCHED(ctx, "loss_reduce_kernel");
   return GT_OK;
 }
@@ -291,8 +298,8 @@ gt_status gt_soft_ce_bwd(gt_ctx* ctx, int32_t rows, int32_t V, int32_t k, gt_buf
   if (!glogits) return GT_OK;
   GT_REQUIRE(ctx, rows > 0 && V > 0 && k > 0 && logits && tids && tprobs && stats && inv_kept && gloss, "gt_soft_ce_bwd: bad argument");
   int T, nseq; seq_shape(ctx, rows, &T, &nseq);
-  soft_ce_bwd_kernel<<<rows, ROWT, 0, ctx->stream>>>(V, k, T, nseq, gt_ptr<const float>(logits), gt_ptr<const uint32_t>(tids), gt_ptr<const float>(tprobs),
-                                                     gt_ptr<const float4>(stats), gt_ptr<const float>(inv_kept), gt_ptr<const float>(gloss), gt_ptr<float>(glogits), accum);
+  GT_CUDA(ctx, gt_launch(ctx, 1, soft_ce_bwd_kernel, rows, ROWT, 0, V, k, T, nseq, gt_ptr<const float>(logits), gt_ptr<const uint32_t>(tids), gt_ptr<const float>(tprobs),
+                                                     gt_ptr<const float4>(stats), gt_ptr<const float>(inv_kept), gt_ptr<const float>(gloss), gt_ptr<float>(glogits), accum));
   GT_LAUNCHED(ctx, "soft_ce_bwd_kernel");
   return GT_OK;
 }

@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(int rows, int d, const
                                                           const float* __restrict__ w, float eps,
                                                           float* __restrict__ y, float* __restrict__ rinv,
                                                           const float2* __restrict__ rope, int H, int period) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -130,6 +131,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_vec_kernel(int rows, int d, c
                                                               const float* __restrict__ w, float eps,
                                                               float* __restrict__ y, float* __restrict__ rinv,
                                                               const float2* __restrict__ rope, int H, int period) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -198,6 +200,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(int rows, int d, const
                                                           const float* __restrict__ w, const float* __restrict__ rinv,
                                                           const float* __restrict__ g, const float* gadd, float* gx, int accum_x,
                                                           float* gw, int accum_w, int warp_rows, float* part, int* counter) {
+  pdl_wait();
   extern __shared__ float sdw[];  // column sums: [warps][d], or [d]
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -254,6 +257,7 @@ __global__ void __launch_bounds__(TH) rmsnorm_bwd_vec_kernel(int rows, int d, co
                                                               const float* __restrict__ rinv, const float* __restrict__ g,
                                                               const float* gadd, float* gx, int accum_x, float* gw, int accum_w,
                                                               int warp_rows, float* part, int* counter) {
+  pdl_wait();
   extern __shared__ __align__(16) float sdw[];
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -359,7 +363,7 @@ gt_status launch_bwd_vec(gt_ctx* ctx, int rows, int d, const float* x, const flo
     if (s) return s;
   }
   const int wr = warp_rows_fit(TH, d);
-  rmsnorm_bwd_vec_kernel<V4, TH><<<blocks, TH, sizeof(float) * d * max(wr, 1), ctx->stream>>>(rows, d, x, w, rinv, g, gadd, gx, accum_x, gw, accum_w, wr, part, counter);
+  GT_CUDA(ctx, gt_launch(ctx, 1, rmsnorm_bwd_vec_kernel<V4, TH>, blocks, TH, sizeof(float) * d * max(wr, 1), rows, d, x, w, rinv, g, gadd, gx, accum_x, gw, accum_w, wr, part, counter));
   GT_LAUNCHED(ctx, "rmsnorm_bwd_vec_kernel");
   return GT_OK;
 }
@@ -368,7 +372,7 @@ template <int NPL>
 gt_status launch_fwd(gt_ctx* ctx, int rows, int d, const float* x, const float* xb, float* sum, const float* w, float eps, float* y,
                      float* rinv, const float2* rope = nullptr, int H = 1, int period = 1) {
   int blocks = min(gt_cdiv(rows, 8), ctx->sm_count * 8);
-  rmsnorm_fwd_kernel<NPL><<<blocks, 256, 0, ctx->stream>>>(rows, d, x, xb, sum, w, eps, y, rinv, rope, H, period);
+  GT_CUDA(ctx, gt_launch(ctx, 1, rmsnorm_fwd_kernel<NPL>, blocks, 256, 0, rows, d, x, xb, sum, w, eps, y, rinv, rope, H, period));
   GT_LAUNCHED(ctx, "rmsnorm_fwd_kernel");
   return GT_OK;
 }
@@ -376,7 +380,7 @@ template <int V4>
 gt_status launch_fwd_vec(gt_ctx* ctx, int rows, int d, const float* x, const float* xb, float* sum, const float* w, float eps, float* y,
                          float* rinv, const float2* rope, int H, int period) {
   int blocks = min(gt_cdiv(rows, 8), ctx->sm_count * 8);
-  rmsnorm_fwd_vec_kernel<V4><<<blocks, 256, 0, ctx->stream>>>(rows, d, x, xb, sum, w, eps, y, rinv, rope, H, period);
+  GT_CUDA(ctx, gt_launch(ctx, 1, rmsnorm_fwd_vec_kernel<V4>, blocks, 256, 0, rows, d, x, xb, sum, w, eps, y, rinv, rope, H, period));
   GT_LAUNCHED(ctx, "rmsnorm_fwd_vec_kernel");
   return GT_OK;
 }
@@ -392,7 +396,7 @@ gt_status launch_bwd(gt_ctx* ctx, int rows, int d, const float* x, const float* 
     if (s) return s;
   }
   const int wr = warp_rows_fit(256, d);
-  rmsnorm_bwd_kernel<NPL><<<blocks, 256, sizeof(float) * d * max(wr, 1), ctx->stream>>>(rows, d, x, w, rinv, g, gadd, gx, accum_x, gw, accum_w, wr, part, counter);
+  GT_CUDA(ctx, gt_launch(ctx, 1, rmsnorm_bwd_kernel<NPL>, blocks, 256, sizeof(float) * d * max(wr, 1), rows, d, x, w, rinv, g, gadd, gx, accum_x, gw, accum_w, wr, part, counter));
   GT_LAUNCHED(ctx, "rmsnorm_bwd_kernel");
   return GT_OK;
 }

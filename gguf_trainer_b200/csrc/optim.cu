@@ -30,6 +30,7 @@ __device__ __forceinline__ float block_sum(float v, float* sh) {
 
 __global__ void __launch_bounds__(OT) sumsq_partial_kernel(const Chunk* __restrict__ chunks, float* const* __restrict__ grads,
                                                            float* __restrict__ partials) {
+  pdl_wait();
   __shared__ float sh[OT / 32];
   const Chunk c = chunks[blockIdx.x];
   const float* g = grads[c.tensor] + c.start;
@@ -46,6 +47,7 @@ __global__ void __launch_bounds__(OT) sumsq_partial_kernel(const Chunk* __restri
 
 // same reduction over one plain array; CTA b covers elements [b*CHUNK, (b+1)*CHUNK)
 __global__ void __launch_bounds__(OT) sumsq_direct_kernel(const float* __restrict__ g, size_t n, float* __restrict__ partials) {
+  pdl_wait();
   __shared__ float sh[OT / 32];
   size_t start = (size_t)blockIdx.x * CHUNK;
   size_t end = start + CHUNK < n ? start + CHUNK : n;
@@ -59,6 +61,7 @@ __global__ void __launch_bounds__(OT) sumsq_direct_kernel(const float* __restric
 // mode 1: out[0] = 1/(sqrt(sum)+1e-7)                                  (muon.ts:140-141)
 __global__ void __launch_bounds__(1024) sumsq_final_kernel(int n, const float* __restrict__ partials, int mode, float clip,
                                                            float* __restrict__ out) {
+  pdl_wait();
   __shared__ double sh[32];
   double s = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += (double)partials[i];
@@ -79,6 +82,7 @@ __global__ void __launch_bounds__(OT) adamw_kernel(const Chunk* __restrict__ chu
                                                    float* const* __restrict__ grads, float* const* __restrict__ ms,
                                                    float* const* __restrict__ vs, const float* __restrict__ scale_p, float lr,
                                                    float bc1, float bc2, float b1, float b2, float eps, float wd) {
+  pdl_wait();
   const Chunk c = chunks[blockIdx.x];
   float* w = datas[c.tensor] + c.start;
   const float* g = grads[c.tensor] + c.start;
@@ -112,6 +116,7 @@ __global__ void __launch_bounds__(OT) adamw_kernel(const Chunk* __restrict__ chu
 // X[r,c] = (flip ? U^T : U) * inv[0], U is [m,n]   (srcNormalize muon-gpu.ts:100-135)
 __global__ void muon_normalize_kernel(int m, int n, int flip, const float* __restrict__ U, const float* __restrict__ inv,
                                       float* __restrict__ X) {
+  pdl_wait();
   size_t total = (size_t)m * n, stride = (size_t)gridDim.x * blockDim.x;
   const float s = inv[0];
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -121,11 +126,13 @@ __global__ void muon_normalize_kernel(int m, int n, int flip, const float* __res
 }
 // out = ca*a + cb*b
 __global__ void axpby_kernel(size_t n, float ca, const float* __restrict__ a, float cb, const float* __restrict__ b, float* out) {
+  pdl_wait();
   size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = ca * a[i] + cb * b[i];
 }
 // W[m,n] -= lr*scale * (flip ? X^T : X)    (srcApply muon-gpu.ts:173-190)
 __global__ void muon_apply_kernel(int m, int n, int flip, float f, const float* __restrict__ X, float* __restrict__ W) {
+  pdl_wait();
   size_t total = (size_t)m * n, stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
     float o;
@@ -138,6 +145,7 @@ __global__ void muon_apply_kernel(int m, int n, int flip, float f, const float* 
 // ---- the same pieces over a group of same-shape matrices: blockIdx.y = matrix, workspaces are [nb, rows, cols] ----
 __global__ void muon_momentum_batched_kernel(size_t el, float* const* __restrict__ grads, float* const* __restrict__ bufs,
                                              float* __restrict__ U, float mu, int nesterov) {
+  pdl_wait();
   const int b = blockIdx.y;
   const float* g = grads[b];
   float* buf = bufs[b];
@@ -153,6 +161,7 @@ __global__ void muon_momentum_batched_kernel(size_t el, float* const* __restrict
 // Newton-Schulz products are issued in the layout the matrix is stored in (see gt_muon_step).
 __global__ void muon_momentum_batched_v4_kernel(size_t el4, float* const* __restrict__ grads, float* const* __restrict__ bufs,
                                                 float* __restrict__ U, float mu, int nesterov) {
+  pdl_wait();
   const int b = blockIdx.y;
   const float4* g = reinterpret_cast<const float4*>(grads[b]);
   float4* buf = reinterpret_cast<float4*>(bufs[b]);
@@ -168,6 +177,7 @@ __global__ void muon_momentum_batched_v4_kernel(size_t el4, float* const* __rest
 }
 // X = U * inv[matrix]
 __global__ void muon_scale_batched_v4_kernel(size_t el4, const float* __restrict__ U, const float* __restrict__ inv, float* __restrict__ X) {
+  pdl_wait();
   const int b = blockIdx.y;
   const float s = inv[b];
   const float4* u = reinterpret_cast<const float4*>(U) + (size_t)b * el4;
@@ -180,6 +190,7 @@ __global__ void muon_scale_batched_v4_kernel(size_t el4, const float* __restrict
 }
 // W -= f * X
 __global__ void muon_apply_batched_v4_kernel(size_t el4, float f, const float* __restrict__ X, float* const* __restrict__ datas) {
+  pdl_wait();
   const int b = blockIdx.y;
   const float4* x = reinterpret_cast<const float4*>(X) + (size_t)b * el4;
   float4* w = reinterpret_cast<float4*>(datas[b]);
@@ -193,6 +204,7 @@ __global__ void muon_apply_batched_v4_kernel(size_t el4, float f, const float* _
 }
 // B' = ca*I + cb*A + cc*AA over nb matrices of r x r, written over AA: then a*X + (b*A + c*A.A).X is the one product B'.X
 __global__ void ns_poly_batched_kernel(size_t n, int r, float ca, float cb, const float* __restrict__ A, float cc, float* AA) {
+  pdl_wait();
   size_t stride = (size_t)gridDim.x * blockDim.x;
   const size_t rr = (size_t)r * r;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -201,6 +213,7 @@ __global__ void ns_poly_batched_kernel(size_t n, int r, float ca, float cb, cons
   }
 }
 __global__ void __launch_bounds__(OT) sumsq_batched_kernel(const float* __restrict__ U, size_t el, int nch, float* __restrict__ partials) {
+  pdl_wait();
   __shared__ float sh[OT / 32];
   const int b = blockIdx.y;
   const float* g = U + (size_t)b * el;
@@ -212,6 +225,7 @@ __global__ void __launch_bounds__(OT) sumsq_batched_kernel(const float* __restri
   if (threadIdx.x == 0) partials[(size_t)b * nch + blockIdx.x] = s;
 }
 __global__ void frob_inv_batched_kernel(int nch, const float* __restrict__ partials, float* __restrict__ inv) {
+  pdl_wait();
   // one small CTA per matrix, fixed order
   const int b = blockIdx.x;
   if (threadIdx.x == 0) {
@@ -222,6 +236,7 @@ __global__ void frob_inv_batched_kernel(int nch, const float* __restrict__ parti
 }
 __global__ void muon_normalize_batched_kernel(int m, int n, int flip, const float* __restrict__ U, const float* __restrict__ inv,
                                               float* __restrict__ X) {
+  pdl_wait();
   const int b = blockIdx.y;
   size_t total = (size_t)m * n, stride = (size_t)gridDim.x * blockDim.x;
   const float s = inv[b];
@@ -233,6 +248,7 @@ __global__ void muon_normalize_batched_kernel(int m, int n, int flip, const floa
   }
 }
 __global__ void muon_apply_batched_kernel(int m, int n, int flip, float f, const float* __restrict__ X, float* const* __restrict__ datas) {
+  pdl_wait();
   const int b = blockIdx.y;
   size_t total = (size_t)m * n, stride = (size_t)gridDim.x * blockDim.x;
   const float* x = X + (size_t)b * total;
@@ -304,11 +320,11 @@ static gt_status ns_iterations(gt_ctx* ctx, int r, int c, int steps, float* X, f
     if (st) return st;
     st = gt_gemm(ctx, GT_GEMM_NN, 0, r, r, r, (gt_buf)(uintptr_t)A, (gt_buf)(uintptr_t)A, (gt_buf)(uintptr_t)AA);
     if (st) return st;
-    axpby_kernel<<<egrid(ctx, (size_t)r * r), 256, 0, ctx->stream>>>((size_t)r * r, -4.7750f, A, 2.0315f, AA, AA);
+    GT_CUDA(ctx, gt_launch(ctx, 1, axpby_kernel, egrid(ctx, (size_t)r * r), 256, 0, (size_t)r * r, -4.7750f, A, 2.0315f, AA, AA));
     GT_LAUNCHED(ctx, "axpby_kernel");
     st = gt_gemm(ctx, GT_GEMM_NN, 0, r, c, r, (gt_buf)(uintptr_t)AA, (gt_buf)(uintptr_t)X, (gt_buf)(uintptr_t)BX);
     if (st) return st;
-    axpby_kernel<<<egrid(ctx, (size_t)r * c), 256, 0, ctx->stream>>>((size_t)r * c, 3.4445f, X, 1.f, BX, X);
+    GT_CUDA(ctx, gt_launch(ctx, 1, axpby_kernel, egrid(ctx, (size_t)r * c), 256, 0, (size_t)r * c, 3.4445f, X, 1.f, BX, X));
     GT_LAUNCHED(ctx, "axpby_kernel");
   }
   return GT_OK;
@@ -317,9 +333,9 @@ static gt_status ns_iterations(gt_ctx* ctx, int r, int c, int steps, float* X, f
 // inv[0] = 1/(||U||_F + 1e-7) for one array of n elements, using `partials` (>= ceil(n/CHUNK) floats)
 static gt_status frob_inv(gt_ctx* ctx, const float* U, size_t n, float* partials, float* inv) {
   int nch = gt_cdiv((long)n, CHUNK);
-  sumsq_direct_kernel<<<nch, OT, 0, ctx->stream>>>(U, n, partials);
+  GT_CUDA(ctx, gt_launch(ctx, 1, sumsq_direct_kernel, nch, OT, 0, U, n, partials));
   GT_LAUNCHED(ctx, "sumsq_direct_kernel");
-  sumsq_final_kernel<<<1, 1024, 0, ctx->stream>>>(nch, partials, 1, 0.f, inv);
+  GT_CUDA(ctx, gt_launch(ctx, 1, sumsq_final_kernel, 1, 1024, 0, nch, partials, 1, 0.f, inv));
   GT_LAUNCHED(ctx, "sumsq_final_kernel");
   return GT_OK;
 }
@@ -415,16 +431,16 @@ gt_status gt_adamw_step(gt_ctx* ctx, uint64_t h) {
   float** P = a->d_ptrs;
   const float* scale = nullptr;
   if (a->clip > 0.f) {
-    sumsq_partial_kernel<<<a->nchunks, OT, 0, ctx->stream>>>(a->d_chunks, P + a->n, a->d_partials);
+    GT_CUDA(ctx, gt_launch(ctx, 1, sumsq_partial_kernel, a->nchunks, OT, 0, a->d_chunks, P + a->n, a->d_partials));
     GT_LAUNCHED(ctx, "sumsq_partial_kernel");
-    sumsq_final_kernel<<<1, 1024, 0, ctx->stream>>>(a->nchunks, a->d_partials, 0, a->clip, a->d_scale);
+    GT_CUDA(ctx, gt_launch(ctx, 1, sumsq_final_kernel, 1, 1024, 0, a->nchunks, a->d_partials, 0, a->clip, a->d_scale));
     GT_LAUNCHED(ctx, "sumsq_final_kernel");
     scale = a->d_scale;
   }
   float bc1 = (float)(1.0 - pow((double)a->b1, (double)a->t));
   float bc2 = (float)(1.0 - pow((double)a->b2, (double)a->t));
-  adamw_kernel<<<a->nchunks, OT, 0, ctx->stream>>>(a->d_chunks, P, P + a->n, P + 2 * a->n, P + 3 * a->n, scale, a->lr, bc1, bc2,
-                                                   a->b1, a->b2, a->eps, a->wd);
+  GT_CUDA(ctx, gt_launch(ctx, 1, adamw_kernel, a->nchunks, OT, 0, a->d_chunks, P, P + a->n, P + 2 * a->n, P + 3 * a->n, scale, a->lr, bc1, bc2,
+                                                   a->b1, a->b2, a->eps, a->wd));
   GT_LAUNCHED(ctx, "adamw_kernel");
   return GT_OK;
 }
@@ -570,14 +586,14 @@ gt_status gt_muon_step(gt_ctx* ctx, uint64_t h) {
       // update X.B'^T (an NT product), so no transposed copy is made. And a*X + (b*A + c*A.A).X is formed as ONE
       // product B'.X with B' = a*I + b*A + c*A.A, into the other of two buffers, instead of a product and a pass.
       const size_t el4 = el / 4;
-      muon_momentum_batched_v4_kernel<<<eg, 256, 0, ctx->stream>>>(el4, P, P + nb, g.U, m->mu, m->nesterov);
+      GT_CUDA(ctx, gt_launch(ctx, 1, muon_momentum_batched_v4_kernel, eg, 256, 0, el4, P, P + nb, g.U, m->mu, m->nesterov));
       GT_LAUNCHED(ctx, "muon_momentum_batched_v4_kernel");
-      sumsq_batched_kernel<<<dim3(nch, nb), OT, 0, ctx->stream>>>(g.U, el, nch, g.partials);
+      GT_CUDA(ctx, gt_launch(ctx, 1, sumsq_batched_kernel, dim3(nch, nb), OT, 0, g.U, el, nch, g.partials));
       GT_LAUNCHED(ctx, "sumsq_batched_kernel");
-      frob_inv_batched_kernel<<<nb, 32, 0, ctx->stream>>>(nch, g.partials, g.inv);
+      GT_CUDA(ctx, gt_launch(ctx, 1, frob_inv_batched_kernel, nb, 32, 0, nch, g.partials, g.inv));
       GT_LAUNCHED(ctx, "frob_inv_batched_kernel");
       float *X = g.X, *Y = g.BX;
-      muon_scale_batched_v4_kernel<<<eg, 256, 0, ctx->stream>>>(el4, g.U, g.inv, X);
+      GT_CUDA(ctx, gt_launch(ctx, 1, muon_scale_batched_v4_kernel, eg, 256, 0, el4, g.U, g.inv, X));
       GT_LAUNCHED(ctx, "muon_scale_batched_v4_kernel");
       // this rank's share of the group's matrices: all of them, or its slice when the work is sharded
       const int slice = gt_cdiv(nb, dp_world);
@@ -592,7 +608,7 @@ gt_status gt_muon_step(gt_ctx* ctx, uint64_t h) {
           st = gt_gemm_batched(ctx, GT_GEMM_NN, 0, r, r, r, g.A, g.A, g.AA, mine);
           if (st) return st;
           const size_t rr = (size_t)r * r * mine;
-          ns_poly_batched_kernel<<<egrid(ctx, rr), 256, 0, ctx->stream>>>(rr, r, 3.4445f, -4.7750f, g.A, 2.0315f, g.AA);
+          GT_CUDA(ctx, gt_launch(ctx, 1, ns_poly_batched_kernel, egrid(ctx, rr), 256, 0, rr, r, 3.4445f, -4.7750f, g.A, 2.0315f, g.AA));
           GT_LAUNCHED(ctx, "ns_poly_batched_kernel");
           st = flip ? gt_gemm_batched(ctx, GT_GEMM_NT, 0, c, r, r, Xs, g.AA, Ys, mine)             // [c, r] = X.B'^T
                     : gt_gemm_batched(ctx, GT_GEMM_NN, 0, r, c, r, g.AA, Xs, Ys, mine);            // [r, c] = B'.X
@@ -604,17 +620,17 @@ gt_status gt_muon_step(gt_ctx* ctx, uint64_t h) {
         gt_status st = gt_dp_allgather(ctx, X, (size_t)slice * el);
         if (st) return st;
       }
-      muon_apply_batched_v4_kernel<<<eg, 256, 0, ctx->stream>>>(el4, f, X, P + 2 * nb);
+      GT_CUDA(ctx, gt_launch(ctx, 1, muon_apply_batched_v4_kernel, eg, 256, 0, el4, f, X, P + 2 * nb));
       GT_LAUNCHED(ctx, "muon_apply_batched_v4_kernel");
       continue;
     }
-    muon_momentum_batched_kernel<<<eg, 256, 0, ctx->stream>>>(el, P, P + nb, g.U, m->mu, m->nesterov);
+    GT_CUDA(ctx, gt_launch(ctx, 1, muon_momentum_batched_kernel, eg, 256, 0, el, P, P + nb, g.U, m->mu, m->nesterov));
     GT_LAUNCHED(ctx, "muon_momentum_batched_kernel");
-    sumsq_batched_kernel<<<dim3(nch, nb), OT, 0, ctx->stream>>>(g.U, el, nch, g.partials);
+    GT_CUDA(ctx, gt_launch(ctx, 1, sumsq_batched_kernel, dim3(nch, nb), OT, 0, g.U, el, nch, g.partials));
     GT_LAUNCHED(ctx, "sumsq_batched_kernel");
-    frob_inv_batched_kernel<<<nb, 32, 0, ctx->stream>>>(nch, g.partials, g.inv);
+    GT_CUDA(ctx, gt_launch(ctx, 1, frob_inv_batched_kernel, nb, 32, 0, nch, g.partials, g.inv));
     GT_LAUNCHED(ctx, "frob_inv_batched_kernel");
-    muon_normalize_batched_kernel<<<eg, 256, 0, ctx->stream>>>(rows, cols, flip, g.U, g.inv, g.X);
+    GT_CUDA(ctx, gt_launch(ctx, 1, muon_normalize_batched_kernel, eg, 256, 0, rows, cols, flip, g.U, g.inv, g.X));
     GT_LAUNCHED(ctx, "muon_normalize_batched_kernel");
     for (int it = 0; it < m->ns; it++) {   // A = X.X^T ; AA = A.A ; B = b*A + c*AA ; X = a*X + B.X   (muon.ts:143-155)
       gt_status st = gt_gemm_batched(ctx, GT_GEMM_NT, 0, r, r, c, g.X, g.X, g.A, nb);
@@ -622,14 +638,14 @@ gt_status gt_muon_step(gt_ctx* ctx, uint64_t h) {
       st = gt_gemm_batched(ctx, GT_GEMM_NN, 0, r, r, r, g.A, g.A, g.AA, nb);
       if (st) return st;
       const size_t rr = (size_t)r * r * nb;
-      axpby_kernel<<<egrid(ctx, rr), 256, 0, ctx->stream>>>(rr, -4.7750f, g.A, 2.0315f, g.AA, g.AA);
+      GT_CUDA(ctx, gt_launch(ctx, 1, axpby_kernel, egrid(ctx, rr), 256, 0, rr, -4.7750f, g.A, 2.0315f, g.AA, g.AA));
       GT_LAUNCHED(ctx, "axpby_kernel");
       st = gt_gemm_batched(ctx, GT_GEMM_NN, 0, r, c, r, g.AA, g.X, g.BX, nb);
       if (st) return st;
-      axpby_kernel<<<egrid(ctx, el * nb), 256, 0, ctx->stream>>>(el * nb, 3.4445f, g.X, 1.f, g.BX, g.X);
+      GT_CUDA(ctx, gt_launch(ctx, 1, axpby_kernel, egrid(ctx, el * nb), 256, 0, el * nb, 3.4445f, g.X, 1.f, g.BX, g.X));
       GT_LAUNCHED(ctx, "axpby_kernel");
     }
-    muon_apply_batched_kernel<<<eg, 256, 0, ctx->stream>>>(rows, cols, flip, f, g.X, P + 2 * nb);
+    GT_CUDA(ctx, gt_launch(ctx, 1, muon_apply_batched_kernel, eg, 256, 0, rows, cols, flip, f, g.X, P + 2 * nb));
     GT_LAUNCHED(ctx, "muon_apply_batched_kernel");
   }
   return GT_OK;
@@ -654,14 +670,14 @@ gt_status gt_newton_schulz(gt_ctx* ctx, int32_t mm, int32_t nn, int32_t steps, g
   GT_CUDA(ctx, cudaMalloc(&partials, sizeof(float) * (el / CHUNK + 2))); GT_CUDA(ctx, cudaMalloc(&inv, 256));
   gt_status s = frob_inv(ctx, gt_ptr<const float>(g), el, partials, inv);
   if (!s) {
-    muon_normalize_kernel<<<egrid(ctx, el), 256, 0, ctx->stream>>>(mm, nn, flip, gt_ptr<const float>(g), inv, X);
+    GT_CUDA(ctx, gt_launch(ctx, 1, muon_normalize_kernel, egrid(ctx, el), 256, 0, mm, nn, flip, gt_ptr<const float>(g), inv, X));
     ctx->launches++;
     s = ns_iterations(ctx, r, c, steps, X, A, AA, BX);
   }
   if (!s) {
     // out = 0 - (-1) * (flip ? X^T : X): the apply kernel with factor -1 into a zeroed tensor (muon-gpu.ts:270-279)
     cudaMemsetAsync(gt_ptr<float>(out), 0, sizeof(float) * el, ctx->stream);
-    muon_apply_kernel<<<egrid(ctx, el), 256, 0, ctx->stream>>>(mm, nn, flip, -1.f, X, gt_ptr<float>(out));
+    GT_CUDA(ctx, gt_launch(ctx, 1, muon_apply_kernel, egrid(ctx, el), 256, 0, mm, nn, flip, -1.f, X, gt_ptr<float>(out)));
     ctx->launches++;
   }
   cudaStreamSynchronize(ctx->stream);

@@ -19,7 +19,8 @@ __global__ void rope_table_kernel(int T, int half, int hd, double base, int pos_
 // one thread per (row, head, pair); pairs are the fastest index so loads coalesce
 template <bool BWD>
 __global__ void rope_kernel(long npairs, int H, int hd, int period, const float2* __restrict__ tab,
-                            const float* in, float* out, int accum) {   // in == out is allowed: a thread reads its pair before it writes it
+                            const float* in, float* out, int accum) {
+  pdl_wait();   // in == out is allowed: a thread reads its pair before it writes it
   const int half = hd >> 1;
   long stride = (long)gridDim.x * blockDim.x;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < npairs; i += stride) {
@@ -42,7 +43,8 @@ __global__ void rope_kernel(long npairs, int H, int hd, int period, const float2
 // the row, two of the table, two 16-byte stores, 32-bit index arithmetic.
 template <bool BWD>
 __global__ void rope_vec_kernel(unsigned nvec, int H, int hd, int period, const float2* __restrict__ tab,
-                                const float* in, float* out, int accum) {   // in == out is allowed, as above
+                                const float* in, float* out, int accum) {
+  pdl_wait();   // in == out is allowed, as above
   const unsigned half = hd >> 1, hv = half >> 2;
   const unsigned stride = gridDim.x * blockDim.x;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += stride) {
@@ -74,6 +76,7 @@ __global__ void rope_vec_kernel(unsigned nvec, int H, int hd, int period, const 
 
 __global__ void embedding_fwd_kernel(long n, int d, const float* __restrict__ w, const uint32_t* __restrict__ ids,
                                      float* __restrict__ out) {
+  pdl_wait();
   long stride = (long)gridDim.x * blockDim.x;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     long t = i / d;
@@ -86,6 +89,7 @@ __global__ void embedding_fwd_kernel(long n, int d, const float* __restrict__ w,
 // rows for every element of the table. Summation order across duplicate ids is not fixed.
 __global__ void embedding_bwd_kernel(long n, int d, const float* __restrict__ g, const uint32_t* __restrict__ ids,
                                      float* gw) {
+  pdl_wait();
   long stride = (long)gridDim.x * blockDim.x;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     long t = i / d;
@@ -117,6 +121,7 @@ gt_status rope_table(gt_ctx* ctx, int T, int hd, double base, int pos_offset, co
 // reference's rule (one owner per gradient element, src/backend/webgpu.ts:21-26) without its O(V) scan.
 __global__ void __launch_bounds__(128) embedding_bwd_ordered_kernel(int rows, int d, const float* __restrict__ g,
                                                                     const uint32_t* __restrict__ ids, float* gw) {
+  pdl_wait();
   extern __shared__ uint32_t bits[];   // one bit per position
   const int t = blockIdx.x;
   const uint32_t id = ids[t];
@@ -172,12 +177,12 @@ gt_status rope_run(gt_ctx* ctx, int rows, int H, int hd, double base, int pos_of
   if (hd % 8 == 0 && npairs < (1l << 31) && ((((uintptr_t)in) | ((uintptr_t)out)) & 15) == 0) {
     const long nvec = npairs / 4;
     int grid = (int)min((long)ctx->sm_count * 8, (nvec + 255) / 256);
-    rope_vec_kernel<BWD><<<grid, 256, 0, ctx->stream>>>((unsigned)nvec, H, hd, period, tab, in, out, accum);
+    GT_CUDA(ctx, gt_launch(ctx, 1, rope_vec_kernel<BWD>, grid, 256, 0, (unsigned)nvec, H, hd, period, tab, in, out, accum));
     GT_LAUNCHED(ctx, "rope_vec_kernel");
     return GT_OK;
   }
   int grid = (int)min((long)ctx->sm_count * 16, (npairs + 255) / 256);
-  rope_kernel<BWD><<<grid, 256, 0, ctx->stream>>>(npairs, H, hd, period, tab, in, out, accum);
+  GT_CUDA(ctx, gt_launch(ctx, 1, rope_kernel<BWD>, grid, 256, 0, npairs, H, hd, period, tab, in, out, accum));
   GT_LAUNCHED(ctx, "rope_kernel");
   return GT_OK;
 }
@@ -212,7 +217,7 @@ gt_status gt_embedding_fwd(gt_ctx* ctx, int32_t rows, int32_t d, gt_buf w, gt_bu
   GT_REQUIRE(ctx, rows > 0 && d > 0 && w && ids && out, "gt_embedding_fwd: bad argument");
   long n = (long)rows * d;
   int grid = (int)min((long)ctx->sm_count * 16, (n + 255) / 256);
-  embedding_fwd_kernel<<<grid, 256, 0, ctx->stream>>>(n, d, gt_ptr<const float>(w), gt_ptr<const uint32_t>(ids), gt_ptr<float>(out));
+  GT_CUDA(ctx, gt_launch(ctx, 1, embedding_fwd_kernel, grid, 256, 0, n, d, gt_ptr<const float>(w), gt_ptr<const uint32_t>(ids), gt_ptr<float>(out)));
   GT_LAUNCHED(ctx, "embedding_fwd_kernel");
   return GT_OK;
 }
@@ -221,14 +226,14 @@ gt_status gt_embedding_bwd(gt_ctx* ctx, int32_t rows, int32_t d, gt_buf gy, gt_b
   if (!gw) return GT_OK;
   GT_REQUIRE(ctx, rows > 0 && d > 0 && gy && ids, "gt_embedding_bwd: bad argument");
   if (ctx->precision == GT_PREC_FP32 && rows <= 8 * 40960) {   // (the bitmap fits the default shared-memory limit)
-    embedding_bwd_ordered_kernel<<<rows, 128, sizeof(uint32_t) * ((rows + 31) / 32), ctx->stream>>>(rows, d, gt_ptr<const float>(gy),
-                                                                                                  gt_ptr<const uint32_t>(ids), gt_ptr<float>(gw));
+    GT_CUDA(ctx, gt_launch(ctx, 1, embedding_bwd_ordered_kernel, rows, 128, sizeof(uint32_t) * ((rows + 31) / 32), rows, d, gt_ptr<const float>(gy),
+                                                                                                  gt_ptr<const uint32_t>(ids), gt_ptr<float>(gw)));
     GT_LAUNCHED(ctx, "embedding_bwd_ordered_kernel");
     return GT_OK;
   }
   long n = (long)rows * d;
   int grid = (int)min((long)ctx->sm_count * 16, (n + 255) / 256);
-  embedding_bwd_kernel<<<grid, 256, 0, ctx->stream>>>(n, d, gt_ptr<const float>(gy), gt_ptr<const uint32_t>(ids), gt_ptr<float>(gw));
+  GT_CUDA(ctx, gt_launch(ctx, 1, embedding_bwd_kernel, grid, 256, 0, n, d, gt_ptr<const float>(gy), gt_ptr<const uint32_t>(ids), gt_ptr<float>(gw)));
   GT_LAUNCHED(ctx, "embedding_bwd_kernel");
   return GT_OK;
 }
