@@ -1585,10 +1585,15 @@ class CudaBackend:
         ch = self._acquireRecycled(T * width * 4)
         needs = self._flows(hidden, eh) or self._flows(w, ew)
         loss, eo, invKept = self._lossOut([hidden, w], needs)
+        # the product of a span with its statistics or its gradient in one call (a library without these makes two of it)
+        fusedStats, fusedGrad = (getattr(self.lib, name, None) for name in ("gt_readout_ce_stats", "gt_readout_ce_grad"))
         for v0 in range(0, V, chunk):
             n = min(chunk, V - v0)
-            self._gemm("NT", 0, T, n, H, eh.data, ew.data + v0 * H * 4, ch)
-            self._check(self.lib.gt_ce_chunk_stats(self.ctx, T, n, v0, 1 if v0 == 0 else 0, ch, tgt, run))
+            if fusedStats is not None:
+                self._check(fusedStats(self.ctx, T, n, H, v0, 1 if v0 == 0 else 0, eh.data, ew.data + v0 * H * 4, ch, tgt, run))
+            else:
+                self._gemm("NT", 0, T, n, H, eh.data, ew.data + v0 * H * 4, ch)
+                self._check(self.lib.gt_ce_chunk_stats(self.ctx, T, n, v0, 1 if v0 == 0 else 0, ch, tgt, run))
         self._check(self.lib.gt_ce_loss_from_stats(self.ctx, T, run, tgt, eo.data, invKept))
 
         def _bw():
@@ -1598,8 +1603,11 @@ class CudaBackend:
             gw, aw = self._gradTarget(w, ew)
             for v0 in range(0, V, chunk):
                 n = min(chunk, V - v0)
-                self._gemm("NT", 0, T, n, H, eh.data, ew.data + v0 * H * 4, ch)
-                self._check(self.lib.gt_ce_chunk_grad(self.ctx, T, n, v0, ch, tgt, run, invKept, seed))
+                if fusedGrad is not None:
+                    self._check(fusedGrad(self.ctx, T, n, H, v0, eh.data, ew.data + v0 * H * 4, ch, tgt, run, invKept, seed))
+                else:
+                    self._gemm("NT", 0, T, n, H, eh.data, ew.data + v0 * H * 4, ch)
+                    self._check(self.lib.gt_ce_chunk_grad(self.ctx, T, n, v0, ch, tgt, run, invKept, seed))
                 if gh:
                     self._gemm("NN", ah, T, H, n, ch, ew.data + v0 * H * 4, gh)
                     ah = 1

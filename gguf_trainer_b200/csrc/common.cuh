@@ -128,6 +128,17 @@ static inline int gt_cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 
 // internal cross-file entry points
 gt_status gt_gemm_simt(gt_ctx* ctx, int kind, int accum, int M, int N, int K, const float* a, const float* b, float* c, float alpha);
+// what the readout forms of the tensor-core product need of the loss (gt_readout_tc)
+struct CeArgs {
+  const uint32_t* targets;       // [rows], 0xffffffff: row ignored
+  float* run;                    // [rows, 3] running (max, sum, target logit)
+  const float* inv_kept;         // [nseq]
+  const float* gloss;
+  float2* part;                  // statistics: (max, sum) per row and column strip, strip-major
+  int v0, T, nseq;
+};
+gt_status gt_readout_tc(gt_ctx* ctx, bool grad, int rows, int n, int h, const float* hidden, const float* w, float* chunk, const CeArgs& ce,
+                        int* parts, bool* handled);
 gt_status gt_gemm_tc(gt_ctx* ctx, int kind, int accum, int M, int N, int K, const float* a, const float* b, float* c, float alpha,
                      bool* handled);
 gt_status gt_gemm_tc_batched(gt_ctx* ctx, int kind, int accum, int M, int N, int K, const float* a, const float* b, float* c,

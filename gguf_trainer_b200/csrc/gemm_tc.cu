@@ -73,8 +73,10 @@ struct PartMaps {
   float* cp[MAX_PARTS];     // the outputs themselves (gemm_tf32_small_kernel stores without a tensor map)
   const float2* rope_tab;   // [rope_period][32] (cos, sin) of the 32 pairs of a 64-wide head
   int rope_period;          // positions per sequence: row r is position r % rope_period
+  CeArgs ce;                // readout forms (EPI_CE_STATS, EPI_CE_GRAD)
 };
-constexpr int EPI_ROPE = 8;   // a value of the kernel's GLU argument that is neither activation
+constexpr int EPI_ROPE = 8;   // values of the kernel's GLU argument that are neither activation
+constexpr int EPI_CE_STATS = 16, EPI_CE_GRAD = 32;
 
 // GLU != 0 (GT_EW_SILU or GT_EW_GELU; NT layout, BN = 192 only): the gated unit of the FFN in the projection that
 // feeds it. B is two weight matrices: the tile's first 96 columns are rows [n0/2, n0/2 + 96) of b[0] (gate), the other 96
@@ -86,6 +88,11 @@ constexpr int EPI_ROPE = 8;   // a value of the kernel's GLU argument that is ne
 // 192-column tile is three whole heads; the thread that owns a row loads the two 32-column halves of a head, rotates
 // pair (j, j + 32) by the angle of (row's position, j) from the table, and both halves go out as they would have.
 // The unrotated projection is never written.
+// GLU == EPI_CE_STATS, EPI_CE_GRAD (NT layout, one product, no split): the logits of one vocabulary span of the chunked
+// readout loss. STATS keeps, per row, the maximum and the sum of exponentials of the tile's columns (one pair per epilogue
+// thread, merged by ce_merge_kernel) and the target's logit, and writes no logits at all; GRAD turns the logits into the
+// loss's gradient on their way out. The passes over [rows, span] that did this (a read; a read and a write) are bound by
+// HBM: at 8192 x 32768 157 and 552 us beside a product of 1.3 ms.
 template <int MT, int GLU>
 struct EpiSub { static constexpr int N = MT == 1 && GLU != 0 ? 3 : 1; };
 template <bool A_K, bool B_K, int BN, int MT, int GLU = 0>
@@ -241,10 +248,47 @@ gemm_tf32_kernel(const __grid_constant__ PartMaps maps, float* __restrict__ C, i
       const int b = slot_of(tl, half);
       const bool have = z * per < kblocks;     // an empty split-K slice issues no MMA and contributes nothing
       const int row = m0 + q * 32 + lane;
+      uint32_t ce_tg = 0xffffffffu;              // readout forms: what the row needs, fetched while the tile is being made
+      float ce_m = 0.f, ce_inv = 0.f, ce_sc = 0.f;
+      if ((GLU == EPI_CE_STATS || GLU == EPI_CE_GRAD) && row < M) {
+        ce_tg = __ldg(maps.ce.targets + row);
+        if (GLU == EPI_CE_GRAD) {
+          ce_m = __ldg(maps.ce.run + (size_t)row * 3);
+          ce_inv = 1.f / __ldg(maps.ce.run + (size_t)row * 3 + 1);
+          ce_sc = __ldg(maps.ce.gloss) * __ldg(maps.ce.inv_kept + row / maps.ce.T) / (float)maps.ce.nseq;
+        }
+      }
       if (have) wait(acc_full(b), par_of(tl), 3);
       dead = __any_sync(0xffffffffu, dead);
       tc_fence_after();
-      if (IS_GLU && have) {
+      if (GLU == EPI_CE_STATS && have) {
+        float m = -3.0e38f, s = 0.f;
+        const uint32_t tcol = ce_tg - (uint32_t)maps.ce.v0;   // the target's column of the span, if it is below N
+#pragma unroll 1
+        for (int c = sub; c < BN / 32; c += SUB) {
+          const int col0 = n0 + c * 32;
+          if (col0 >= N) break;   // uniform across the warp
+          float v[32];
+          tmem_ld32(tmem + b * BN + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32), v);
+          float mb = m;
+#pragma unroll
+          for (int j = 0; j < 32; j++) {
+            v[j] = col0 + j < N ? v[j] * out_scale : -3.0e38f;
+            mb = fmaxf(mb, v[j]);
+          }
+          float t[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int j = 0; j < 32; j++) t[j & 3] += __expf(v[j] - mb);
+          s = s * __expf(m - mb) + ((t[0] + t[1]) + (t[2] + t[3]));
+          m = mb;
+          if (ce_tg != 0xffffffffu && tcol - (uint32_t)col0 < 32u && tcol < (uint32_t)N && !dead) {
+#pragma unroll
+            for (int j = 0; j < 32; j++)
+              if (tcol == (uint32_t)(col0 + j)) maps.ce.run[(size_t)row * 3 + 2] = v[j];
+          }
+        }
+        if (row < M && !dead) maps.ce.part[(size_t)((n0 / BN) * SUB + sub) * M + row] = make_float2(m, s);
+      } else if (IS_GLU && have) {
         // gate | up halves of the accumulator: three outputs per 32-column block, each through its own tensor map
         auto put = [&](const float* v, const CUtensorMap* map, int col0) {
           const uint32_t tile = epi + (uint32_t)(ew * S::EPI_TILES + (nst % S::EPI_TILES)) * 4096u;
@@ -333,6 +377,14 @@ gemm_tf32_kernel(const __grid_constant__ PartMaps maps, float* __restrict__ C, i
           tmem_ld32(tmem + b * BN + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32), v);
 #pragma unroll
           for (int j = 0; j < 32; j++) v[j] *= out_scale;   // the caller's factor times the truncation compensation
+          if (GLU == EPI_CE_GRAD) {
+            const uint32_t tcol = ce_tg - (uint32_t)(maps.ce.v0 + col0);
+#pragma unroll
+            for (int j = 0; j < 32; j++) {
+              const float g = ce_sc * (__expf(v[j] - ce_m) * ce_inv - (tcol == (uint32_t)j ? 1.f : 0.f));
+              v[j] = ce_tg == 0xffffffffu ? 0.f : g;
+            }
+          }
           if (use_tma_store) {
             // Stage the warp's 32x32 block in shared memory (128-byte rows, 16-byte chunks XOR (row mod 8), the layout
             // the store's tensor map expects) and let TMA write it: whole 128-byte rows, clipped at M and N, as a
@@ -1435,6 +1487,51 @@ gt_status gt_glu_linear_tc(gt_ctx* ctx, int op, int rows, int ffn, int in, const
   gt_status s = op == GT_EW_SILU
                     ? launch<true, true, BN, 1, GT_EW_SILU>(ctx, maps, ntiles, 1, out, rows, N2, 0, 1, 1, TRUNC_COMP)
                     : launch<true, true, BN, 1, GT_EW_GELU>(ctx, maps, ntiles, 1, out, rows, N2, 0, 1, 1, TRUNC_COMP);
+  if (s) return s;
+  *handled = true;
+  return GT_OK;
+}
+
+// One vocabulary span of the chunked readout loss: logits = hidden.w^T with their statistics or their gradient taken in
+// the epilogue (see the kernel). `parts` is the number of (max, sum) pairs per row that the statistics form leaves in
+// ce.part, which lies in the span's logits buffer: nothing else is written there.
+gt_status gt_readout_tc(gt_ctx* ctx, bool grad, int rows, int n, int h, const float* hidden, const float* w, float* chunk, const CeArgs& ce,
+                        int* parts, bool* handled) {
+  *handled = false;
+  if (rows < 16 || n < 192 || h < 16 || (h & 3) || (grad && (n & 3))) return GT_OK;
+  if ((((uintptr_t)hidden) | ((uintptr_t)w) | ((uintptr_t)chunk)) & 15) return GT_OK;
+  if (ctx->device < 0 || ctx->device >= 64 || !device_flag(ctx)) return GT_OK;
+  const int kblocks = gt_cdiv(h, BK);
+  const long workers = ctx->sm_count - ctx->sm_reserved;
+  const long t1 = (long)gt_cdiv(n, 192) * gt_cdiv(rows, BM1), t2 = (long)gt_cdiv(n, 256) * gt_cdiv(rows, 2 * BM1);
+  // Spans with few tiles go through the product that cuts its contraction, and a pass that then finds them in L2.
+  if (2 * t1 < workers) return GT_OK;
+  // 128 x 192 tiles hide their epilogue, 256 x 256 ones move fewer bytes per product (choose_plan's cycle counts)
+  const double c1 = (double)gt_cdiv(t1, workers) * (kblocks * 0.92 * 2.0 * (BM1 + 192) + 1500.0);
+  const double c2 = (double)gt_cdiv(t2, workers) * (kblocks * 0.92 * (512.0 + 2.0 * (BM1 + 256)) + 14.0 * 256 + 900.0 + 1500.0);
+  int mt = c2 < c1 ? 2 : 1;
+  if (const char* force = getenv("GT_GEMM_TILE")) {
+    if (!strcmp(force, "1,192")) mt = 1;
+    else if (!strcmp(force, "2,256")) mt = 2;
+    else return GT_OK;
+  }
+  const int bn = mt == 2 ? 256 : 192, bm = mt * BM1;
+  PartMaps maps;
+  maps.nparts = maps.ngroups = 1;
+  if (!make_map_3d(&maps.a[0], hidden, h, rows, 1, h, (uint64_t)rows * h, bm, true) ||
+      !make_map_3d(&maps.b[0], w, h, n, 1, h, (uint64_t)n * h, bn, true))
+    return GT_OK;
+  maps.c[0] = maps.a[0];
+  if (grad && !make_map_3d(&maps.c[0], chunk, n, rows, 1, n, (uint64_t)rows * n, 32, true)) return GT_OK;
+  maps.kb_end[0] = kblocks;
+  maps.ce = ce;
+  *parts = gt_cdiv(n, bn) * (mt == 1 ? EpiSub<1, EPI_CE_STATS>::N : 1);
+  const long tiles = mt == 2 ? t2 : t1;
+  gt_status s;
+  if (grad) s = mt == 2 ? launch<true, true, 256, 2, EPI_CE_GRAD>(ctx, maps, tiles, 1, chunk, rows, n, 0, 1, 1, TRUNC_COMP)
+                        : launch<true, true, 192, 1, EPI_CE_GRAD>(ctx, maps, tiles, 1, chunk, rows, n, 0, 1, 1, TRUNC_COMP);
+  else s = mt == 2 ? launch<true, true, 256, 2, EPI_CE_STATS>(ctx, maps, tiles, 0, chunk, rows, n, 0, 1, 1, TRUNC_COMP)
+                   : launch<true, true, 192, 1, EPI_CE_STATS>(ctx, maps, tiles, 0, chunk, rows, n, 0, 1, 1, TRUNC_COMP);
   if (s) return s;
   *handled = true;
   return GT_OK;

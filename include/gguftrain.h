@@ -209,6 +209,12 @@ gt_status gt_ce_chunk_stats(gt_ctx* ctx, int32_t rows, int32_t n, int32_t v0, in
 gt_status gt_ce_loss_from_stats(gt_ctx* ctx, int32_t rows, gt_buf run, gt_buf targets, gt_buf loss, gt_buf inv_kept);
 gt_status gt_ce_chunk_grad(gt_ctx* ctx, int32_t rows, int32_t n, int32_t v0, gt_buf chunk, gt_buf targets,
                            gt_buf run, gt_buf inv_kept, gt_buf gloss);
+/* the same with the product that makes the span's logits, hidden [rows, h] . w [n, h]^T: one launch on the tensor cores,
+ * whose epilogue takes the statistics (chunk is then workspace, its contents undefined) or writes the gradient */
+gt_status gt_readout_ce_stats(gt_ctx* ctx, int32_t rows, int32_t n, int32_t h, int32_t v0, int32_t first, gt_buf hidden,
+                              gt_buf w, gt_buf chunk, gt_buf targets, gt_buf run);
+gt_status gt_readout_ce_grad(gt_ctx* ctx, int32_t rows, int32_t n, int32_t h, int32_t v0, gt_buf hidden, gt_buf w,
+                             gt_buf chunk, gt_buf targets, gt_buf run, gt_buf inv_kept, gt_buf gloss);
 /* sparse-teacher soft CE (webgpu.ts:1331-1378; srcSoftCeFwd/BwdP/BwdQ wgsl.ts:1004-1110).
  * tids/tprobs: [rows, k]; a row whose first id is 0xffffffff is ignored. */
 gt_status gt_soft_ce_fwd(gt_ctx* ctx, int32_t rows, int32_t V, int32_t k, gt_buf logits, gt_buf tids, gt_buf tprobs,
