@@ -93,8 +93,201 @@ constexpr int EPI_CE_STATS = 16, EPI_CE_GRAD = 32;
 // thread, merged by ce_merge_kernel) and the target's logit, and writes no logits at all; GRAD turns the logits into the
 // loss's gradient on their way out. The passes over [rows, span] that did this (a read; a read and a write) are bound by
 // HBM: at 8192 x 32768 157 and 552 us beside a product of 1.3 ms.
+// (epilogue warps per lane quadrant: three where the epilogue computes and runs beside the main loop)
 template <int MT, int GLU>
 struct EpiSub { static constexpr int N = MT == 1 && GLU != 0 ? 3 : 1; };
+// What one epilogue warp does with its share of a finished accumulator: 32 rows (a TMEM lane quadrant), every SUB-th column
+// block. Outputs are staged as 32x32 blocks in shared memory (128-byte rows, 16-byte chunks XOR (row mod 8), the layout the
+// store's tensor map expects) and written by TMA: whole 128-byte rows, clipped at M and N, as a plain store or, when
+// accumulating or combining split-K slices, as an f32 reduce-add performed in L2. Shared by the kernels below.
+struct CeRow { uint32_t tg; float m, inv, sc; };   // readout forms: what the row needs of the loss
+template <int GLU>
+__device__ __forceinline__ CeRow ce_row(const PartMaps& maps, int row, int M) {
+  CeRow r = {0xffffffffu, 0.f, 0.f, 0.f};
+  if ((GLU == EPI_CE_STATS || GLU == EPI_CE_GRAD) && row < M) {
+    r.tg = __ldg(maps.ce.targets + row);
+    if (GLU == EPI_CE_GRAD) {
+      r.m = __ldg(maps.ce.run + (size_t)row * 3);
+      r.inv = 1.f / __ldg(maps.ce.run + (size_t)row * 3 + 1);
+      r.sc = __ldg(maps.ce.gloss) * __ldg(maps.ce.inv_kept + row / maps.ce.T) / (float)maps.ce.nseq;
+    }
+  }
+  return r;
+}
+struct Drain {           // of one tile
+  const CUtensorMap* mapC;
+  float* C;
+  int bi, g, n0, row0, M, N, ksplit, accum, use_tma_store;   // row0: first row of this warp's 32
+  float out_scale;
+  bool dead;             // a wait has expired: nothing is stored
+};
+template <int BN, int GLU, int SUB, int TILES>
+__device__ __forceinline__ void drain_tile(const PartMaps& maps, const Drain& d, const CeRow& ce, uint8_t* smem_raw, uint32_t stage,
+                                           uint32_t tacc, int sub, int lane, uint32_t& nst) {
+  constexpr bool IS_GLU = GLU == GT_EW_SILU || GLU == GT_EW_GELU;
+  const int M = d.M, N = d.N, n0 = d.n0, row = d.row0 + lane;
+  auto put = [&](const float* v, const CUtensorMap* map, int col0) {
+    const uint32_t tile = stage + (nst % TILES) * 4096u;
+    if (nst >= TILES) tma_wait_read<TILES - 1>();   // the tile's previous contents have been read out
+    __syncwarp();
+    uint8_t* tp = smem_raw + (tile - smem_u32(smem_raw)) + lane * 128;
+#pragma unroll
+    for (int c4 = 0; c4 < 8; c4++)
+      *reinterpret_cast<float4*>(tp + ((c4 ^ (lane & 7)) * 16)) = make_float4(v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
+    fence_async_smem();
+    __syncwarp();
+    if (lane == 0 && !d.dead && d.row0 < M) {
+      if (!IS_GLU && (d.ksplit > 1 || d.accum)) tma_reduce_add_3d(map, tile, col0, d.row0, d.bi);
+      else tma_store_3d(map, tile, col0, d.row0, d.bi);
+    }
+    if (lane == 0) tma_commit_group();
+    nst++;
+  };
+  if (GLU == EPI_CE_STATS) {
+    float m = -3.0e38f, s = 0.f;
+    const uint32_t tcol = ce.tg - (uint32_t)maps.ce.v0;   // the target's column of the span, if it is below N
+#pragma unroll 1
+    for (int c = sub; c < BN / 32; c += SUB) {
+      const int col0 = n0 + c * 32;
+      if (col0 >= N) break;   // uniform across the warp
+      float v[32];
+      tmem_ld32(tacc + (uint32_t)(c * 32), v);
+      float mb = m;
+#pragma unroll
+      for (int j = 0; j < 32; j++) {
+        v[j] = col0 + j < N ? v[j] * d.out_scale : -3.0e38f;
+        mb = fmaxf(mb, v[j]);
+      }
+      float t[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 32; j++) t[j & 3] += __expf(v[j] - mb);
+      s = s * __expf(m - mb) + ((t[0] + t[1]) + (t[2] + t[3]));
+      m = mb;
+      if (ce.tg != 0xffffffffu && tcol - (uint32_t)col0 < 32u && tcol < (uint32_t)N && !d.dead) {
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+          if (tcol == (uint32_t)(col0 + j)) maps.ce.run[(size_t)row * 3 + 2] = v[j];
+      }
+    }
+    if (row < M && !d.dead) maps.ce.part[(size_t)((n0 / BN) * SUB + sub) * M + row] = make_float2(m, s);
+  } else if (IS_GLU) {
+    // gate | up halves of the accumulator: three outputs per 32-column block, each through its own tensor map
+#pragma unroll 1
+    for (int c = sub; c < BN / 64; c += SUB) {
+      const int col0 = (n0 >> 1) + c * 32;
+      if (col0 >= (N >> 1)) break;   // uniform across the warp
+      float vg[32], vu[32];
+      tmem_ld32_issue(tacc + (uint32_t)(c * 32), vg);
+      tmem_ld32_issue(tacc + (uint32_t)(c * 32) + BN / 2, vu);
+      tmem_wait_ld();
+#pragma unroll
+      for (int j = 0; j < 32; j++) { vg[j] *= d.out_scale; vu[j] *= d.out_scale; }
+      put(vg, &maps.c[0], col0);
+      put(vu, &maps.c[1], col0);
+#pragma unroll
+      for (int j = 0; j < 32; j++) {
+        const float a = vg[j];
+        float act;
+        if (GLU == GT_EW_SILU) act = a / (1.f + __expf(-a));
+        else act = 0.5f * a * (1.f + tanhf(0.7978845608028654f * (a + 0.044715f * a * a * a)));
+        vg[j] = act * vu[j];
+      }
+      put(vg, &maps.c[2], col0);
+    }
+  } else if (GLU == EPI_ROPE && maps.g_rope[d.g]) {
+    // (cos, sin) of this row's position, pairs 0..31; rows past M are clipped by the store and read row M - 1's.
+    // (adding into the output is allowed: a rotation is linear)
+    const float4* tab4 = reinterpret_cast<const float4*>(maps.rope_tab + (size_t)((row < M ? row : M - 1) % maps.rope_period) * 32);
+#pragma unroll 1
+    for (int c = sub; c < BN / 64; c += SUB) {
+      const int col0 = n0 + c * 64;
+      if (col0 >= N) break;   // uniform across the warp
+      float v0[32], v1[32];
+      tmem_ld32_issue(tacc + (uint32_t)(c * 64), v0);
+      tmem_ld32_issue(tacc + (uint32_t)(c * 64) + 32, v1);
+      tmem_wait_ld();
+#pragma unroll
+      for (int j = 0; j < 32; j += 2) {
+        const float4 cs = __ldg(tab4 + (j >> 1));   // cos, sin of pair j; cos, sin of pair j + 1
+        const float a0 = v0[j] * d.out_scale, a1 = v1[j] * d.out_scale, b0 = v0[j + 1] * d.out_scale, b1 = v1[j + 1] * d.out_scale;
+        v0[j] = a0 * cs.x - a1 * cs.y;
+        v1[j] = a0 * cs.y + a1 * cs.x;
+        v0[j + 1] = b0 * cs.z - b1 * cs.w;
+        v1[j + 1] = b0 * cs.w + b1 * cs.z;
+      }
+      put(v0, d.mapC, col0);
+      put(v1, d.mapC, col0 + 32);
+    }
+  } else {
+    const bool vec = (N & 3) == 0;
+#pragma unroll 1
+    for (int c = sub; c < BN / 32; c += SUB) {
+      const int col0 = n0 + c * 32;
+      if (col0 >= N) break;   // uniform across the warp
+      float v[32];
+      tmem_ld32(tacc + (uint32_t)(c * 32), v);
+#pragma unroll
+      for (int j = 0; j < 32; j++) v[j] *= d.out_scale;   // the caller's factor times the truncation compensation
+      if (GLU == EPI_CE_GRAD) {
+        const uint32_t tcol = ce.tg - (uint32_t)(maps.ce.v0 + col0);
+#pragma unroll
+        for (int j = 0; j < 32; j++) {
+          const float g = ce.sc * (__expf(v[j] - ce.m) * ce.inv - (tcol == (uint32_t)j ? 1.f : 0.f));
+          v[j] = ce.tg == 0xffffffffu ? 0.f : g;
+        }
+      }
+      if (d.use_tma_store) {
+        put(v, d.mapC, col0);
+      } else if (row < M && !d.dead) {
+        float* dst = d.C + (size_t)d.bi * M * N + (size_t)row * N + col0;
+        if (vec && col0 + 32 <= N) {
+          if (d.ksplit > 1) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) atomicAdd(reinterpret_cast<float4*>(dst + j), make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]));
+          } else if (d.accum) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              float4 o = *reinterpret_cast<float4*>(dst + j);
+              o.x += v[j]; o.y += v[j + 1]; o.z += v[j + 2]; o.w += v[j + 3];
+              *reinterpret_cast<float4*>(dst + j) = o;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; j++) {
+            if (col0 + j < N) {
+              if (d.ksplit > 1) atomicAdd(dst + j, v[j]);
+              else dst[j] = d.accum ? dst[j] + v[j] : v[j];
+            }
+          }
+        }
+      }
+    }
+  }
+}
+
+// Where tile t of a launch lies: batch matrix (or group), first column, first row, K slice (n fastest, then m, then the slice).
+struct Where { int bi, g, n0, m0, z; };
+template <int BM, int BN>
+__device__ __forceinline__ Where tile_at(const PartMaps& maps, int t, int tiles_n, int tiles_m, int per_mat) {
+  Where w;
+  if (maps.ngroups > 1) {
+    int g = 0;
+    while (t >= maps.unit_end[g]) g++;
+    const int tt = t - (g ? maps.unit_end[g - 1] : 0);
+    const int tn = (maps.gN[g] + BN - 1) / BN, tmn = tn * ((maps.gM[g] + BM - 1) / BM);
+    const int rem = tt % tmn;
+    w.bi = 0; w.g = g; w.z = tt / tmn; w.n0 = (rem % tn) * BN; w.m0 = (rem / tn) * BM;
+  } else {
+    const int tt = t % per_mat;
+    w.bi = t / per_mat; w.g = 0; w.n0 = (tt % tiles_n) * BN; w.m0 = ((tt / tiles_n) % tiles_m) * BM; w.z = tt / (tiles_n * tiles_m);
+  }
+  return w;
+}
+
 template <bool A_K, bool B_K, int BN, int MT, int GLU = 0>
 __global__ void __launch_bounds__(Smem<BN, MT, EpiSub<MT, GLU>::N>::THREADS, 1)
 gemm_tf32_kernel(const __grid_constant__ PartMaps maps, float* __restrict__ C, int M_, int N_,
@@ -121,23 +314,7 @@ gemm_tf32_kernel(const __grid_constant__ PartMaps maps, float* __restrict__ C, i
   const int per_mat = tiles_n * tiles_m * ksplit;
   const int ngroups = maps.ngroups;
   const int ntiles = ngroups > 1 ? maps.unit_end[ngroups - 1] : per_mat * batch;   // the matrices of a batch are just more tiles
-  // where tile t lies: batch matrix (or group), first column, first row (of the 256-row tile when MT = 2), K slice
-  struct Where { int bi, g, n0, m0, z; };
-  auto where = [&](int t) {
-    Where w;
-    if (ngroups > 1) {
-      int g = 0;
-      while (t >= maps.unit_end[g]) g++;
-      const int tt = t - (g ? maps.unit_end[g - 1] : 0);
-      const int tn = (maps.gN[g] + BN - 1) / BN, tmn = tn * ((maps.gM[g] + BM - 1) / BM);
-      const int rem = tt % tmn;
-      w.bi = 0; w.g = g; w.z = tt / tmn; w.n0 = (rem % tn) * BN; w.m0 = (rem / tn) * BM;
-    } else {
-      const int tt = t % per_mat;
-      w.bi = t / per_mat; w.g = 0; w.n0 = (tt % tiles_n) * BN; w.m0 = ((tt / tiles_n) % tiles_m) * BM; w.z = tt / (tiles_n * tiles_m);
-    }
-    return w;
-  };
+  auto where = [&](int t) { return tile_at<BM, BN>(maps, t, tiles_n, tiles_m, per_mat); };
   // Further products of the same layout are accumulated into the same tiles: their K blocks simply follow those of
   // the first in the main loop, read through their own tensor maps.
   const int kblocks = maps.kb_end[maps.nparts - 1];
@@ -237,201 +414,20 @@ gemm_tf32_kernel(const __grid_constant__ PartMaps maps, float* __restrict__ C, i
   } else {
     // ---- epilogue: warp w may touch TMEM lanes [32*(w%4), 32*(w%4)+32) ----
     const int q = warp & 3, ew = warp - 2, half = MT == 2 ? ew >> 2 : 0, sub = MT == 2 ? 0 : ew >> 2;
-    const bool vec = (N & 3) == 0;
     uint32_t tl = 0, nst = 0;   // nst: TMA stores issued by this warp
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, tl++) {
       const Where wh = where(t);
-      const int bi = wh.bi, n0 = wh.n0, m0 = wh.m0 + half * BM1, z = wh.z;
       const int M = ngroups > 1 ? maps.gM[wh.g] : M_, N = ngroups > 1 ? maps.gN[wh.g] : N_;
-      const int accum = ngroups > 1 ? maps.g_accum[wh.g] : accum_;
-      const CUtensorMap* mapC = &maps.c[wh.g];
-      const int b = slot_of(tl, half);
-      const bool have = z * per < kblocks;     // an empty split-K slice issues no MMA and contributes nothing
-      const int row = m0 + q * 32 + lane;
-      uint32_t ce_tg = 0xffffffffu;              // readout forms: what the row needs, fetched while the tile is being made
-      float ce_m = 0.f, ce_inv = 0.f, ce_sc = 0.f;
-      if ((GLU == EPI_CE_STATS || GLU == EPI_CE_GRAD) && row < M) {
-        ce_tg = __ldg(maps.ce.targets + row);
-        if (GLU == EPI_CE_GRAD) {
-          ce_m = __ldg(maps.ce.run + (size_t)row * 3);
-          ce_inv = 1.f / __ldg(maps.ce.run + (size_t)row * 3 + 1);
-          ce_sc = __ldg(maps.ce.gloss) * __ldg(maps.ce.inv_kept + row / maps.ce.T) / (float)maps.ce.nseq;
-        }
-      }
+      const int b = slot_of(tl, half), row0 = wh.m0 + half * BM1 + q * 32;
+      const CeRow ce = ce_row<GLU>(maps, row0 + lane, M);   // (fetched while the tile is being made)
+      const bool have = wh.z * per < kblocks;     // an empty split-K slice issues no MMA and contributes nothing
       if (have) wait(acc_full(b), par_of(tl), 3);
       dead = __any_sync(0xffffffffu, dead);
       tc_fence_after();
-      if (GLU == EPI_CE_STATS && have) {
-        float m = -3.0e38f, s = 0.f;
-        const uint32_t tcol = ce_tg - (uint32_t)maps.ce.v0;   // the target's column of the span, if it is below N
-#pragma unroll 1
-        for (int c = sub; c < BN / 32; c += SUB) {
-          const int col0 = n0 + c * 32;
-          if (col0 >= N) break;   // uniform across the warp
-          float v[32];
-          tmem_ld32(tmem + b * BN + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32), v);
-          float mb = m;
-#pragma unroll
-          for (int j = 0; j < 32; j++) {
-            v[j] = col0 + j < N ? v[j] * out_scale : -3.0e38f;
-            mb = fmaxf(mb, v[j]);
-          }
-          float t[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-          for (int j = 0; j < 32; j++) t[j & 3] += __expf(v[j] - mb);
-          s = s * __expf(m - mb) + ((t[0] + t[1]) + (t[2] + t[3]));
-          m = mb;
-          if (ce_tg != 0xffffffffu && tcol - (uint32_t)col0 < 32u && tcol < (uint32_t)N && !dead) {
-#pragma unroll
-            for (int j = 0; j < 32; j++)
-              if (tcol == (uint32_t)(col0 + j)) maps.ce.run[(size_t)row * 3 + 2] = v[j];
-          }
-        }
-        if (row < M && !dead) maps.ce.part[(size_t)((n0 / BN) * SUB + sub) * M + row] = make_float2(m, s);
-      } else if (IS_GLU && have) {
-        // gate | up halves of the accumulator: three outputs per 32-column block, each through its own tensor map
-        auto put = [&](const float* v, const CUtensorMap* map, int col0) {
-          const uint32_t tile = epi + (uint32_t)(ew * S::EPI_TILES + (nst % S::EPI_TILES)) * 4096u;
-          if (nst >= S::EPI_TILES) tma_wait_read<S::EPI_TILES - 1>();
-          __syncwarp();
-          uint8_t* tp = smem_raw + (tile - smem_u32(smem_raw)) + lane * 128;
-#pragma unroll
-          for (int c4 = 0; c4 < 8; c4++)
-            *reinterpret_cast<float4*>(tp + ((c4 ^ (lane & 7)) * 16)) = make_float4(v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
-          fence_async_smem();
-          __syncwarp();
-          if (lane == 0 && !dead && m0 + q * 32 < M) tma_store_3d(map, tile, col0, m0 + q * 32, bi);
-          if (lane == 0) tma_commit_group();
-          nst++;
-        };
-#pragma unroll 1
-        for (int c = sub; c < BN / 64; c += SUB) {
-          const int col0 = (n0 >> 1) + c * 32;
-          if (col0 >= (N >> 1)) break;   // uniform across the warp
-          float vg[32], vu[32];
-          const uint32_t ta = tmem + b * BN + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32);
-          tmem_ld32_issue(ta, vg);
-          tmem_ld32_issue(ta + BN / 2, vu);
-          tmem_wait_ld();
-#pragma unroll
-          for (int j = 0; j < 32; j++) { vg[j] *= out_scale; vu[j] *= out_scale; }
-          put(vg, &maps.c[0], col0);
-          put(vu, &maps.c[1], col0);
-#pragma unroll
-          for (int j = 0; j < 32; j++) {
-            const float a = vg[j];
-            float act;
-            if (GLU == GT_EW_SILU) act = a / (1.f + __expf(-a));
-            else act = 0.5f * a * (1.f + tanhf(0.7978845608028654f * (a + 0.044715f * a * a * a)));
-            vg[j] = act * vu[j];
-          }
-          put(vg, &maps.c[2], col0);
-        }
-      } else if (GLU == EPI_ROPE && have && maps.g_rope[wh.g]) {
-        auto put = [&](const float* v, int col0) {
-          const uint32_t tile = epi + (uint32_t)(ew * S::EPI_TILES + (nst % S::EPI_TILES)) * 4096u;
-          if (nst >= S::EPI_TILES) tma_wait_read<S::EPI_TILES - 1>();
-          __syncwarp();
-          uint8_t* tp = smem_raw + (tile - smem_u32(smem_raw)) + lane * 128;
-#pragma unroll
-          for (int c4 = 0; c4 < 8; c4++)
-            *reinterpret_cast<float4*>(tp + ((c4 ^ (lane & 7)) * 16)) = make_float4(v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
-          fence_async_smem();
-          __syncwarp();
-          if (lane == 0 && !dead && m0 + q * 32 < M) {
-            if (ksplit > 1 || accum) tma_reduce_add_3d(mapC, tile, col0, m0 + q * 32, bi);   // (a rotation is linear)
-            else tma_store_3d(mapC, tile, col0, m0 + q * 32, bi);
-          }
-          if (lane == 0) tma_commit_group();
-          nst++;
-        };
-        // (cos, sin) of this row's position, pairs 0..31; rows past M are clipped by the store and read row M - 1's
-        const float4* tab4 = reinterpret_cast<const float4*>(maps.rope_tab + (size_t)((row < M ? row : M - 1) % maps.rope_period) * 32);
-#pragma unroll 1
-        for (int c = sub; c < BN / 64; c += SUB) {
-          const int col0 = n0 + c * 64;
-          if (col0 >= N) break;   // uniform across the warp
-          float v0[32], v1[32];
-          const uint32_t ta = tmem + b * BN + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 64);
-          tmem_ld32_issue(ta, v0);
-          tmem_ld32_issue(ta + 32, v1);
-          tmem_wait_ld();
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float4 cs = __ldg(tab4 + (j >> 1));   // cos, sin of pair j; cos, sin of pair j + 1
-            const float a0 = v0[j] * out_scale, a1 = v1[j] * out_scale, b0 = v0[j + 1] * out_scale, b1 = v1[j + 1] * out_scale;
-            v0[j] = a0 * cs.x - a1 * cs.y;
-            v1[j] = a0 * cs.y + a1 * cs.x;
-            v0[j + 1] = b0 * cs.z - b1 * cs.w;
-            v1[j + 1] = b0 * cs.w + b1 * cs.z;
-          }
-          put(v0, col0);
-          put(v1, col0 + 32);
-        }
-      } else if (have) {
-#pragma unroll 1
-        for (int c = sub; c < BN / 32; c += SUB) {
-          const int col0 = n0 + c * 32;
-          if (col0 >= N) break;   // uniform across the warp
-          float v[32];
-          tmem_ld32(tmem + b * BN + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32), v);
-#pragma unroll
-          for (int j = 0; j < 32; j++) v[j] *= out_scale;   // the caller's factor times the truncation compensation
-          if (GLU == EPI_CE_GRAD) {
-            const uint32_t tcol = ce_tg - (uint32_t)(maps.ce.v0 + col0);
-#pragma unroll
-            for (int j = 0; j < 32; j++) {
-              const float g = ce_sc * (__expf(v[j] - ce_m) * ce_inv - (tcol == (uint32_t)j ? 1.f : 0.f));
-              v[j] = ce_tg == 0xffffffffu ? 0.f : g;
-            }
-          }
-          if (use_tma_store) {
-            // Stage the warp's 32x32 block in shared memory (128-byte rows, 16-byte chunks XOR (row mod 8), the layout
-            // the store's tensor map expects) and let TMA write it: whole 128-byte rows, clipped at M and N, as a
-            // plain store or, when accumulating or combining split-K slices, as an f32 reduce-add performed in L2.
-            const uint32_t tile = epi + (uint32_t)(ew * S::EPI_TILES + (nst % S::EPI_TILES)) * 4096u;
-            if (nst >= S::EPI_TILES) tma_wait_read<S::EPI_TILES - 1>();   // the tile's previous contents have been read out
-            __syncwarp();
-            uint8_t* tp = smem_raw + (tile - smem_u32(smem_raw)) + lane * 128;
-#pragma unroll
-            for (int c4 = 0; c4 < 8; c4++)
-              *reinterpret_cast<float4*>(tp + ((c4 ^ (lane & 7)) * 16)) = make_float4(v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0 && !dead && m0 + q * 32 < M) {
-              if (ksplit > 1 || accum) tma_reduce_add_3d(mapC, tile, col0, m0 + q * 32, bi);
-              else tma_store_3d(mapC, tile, col0, m0 + q * 32, bi);
-            }
-            if (lane == 0) tma_commit_group();
-            nst++;
-          } else if (row < M && !dead) {
-            float* dst = C + (size_t)bi * M * N + (size_t)row * N + col0;
-            if (vec && col0 + 32 <= N) {
-              if (ksplit > 1) {
-#pragma unroll
-                for (int j = 0; j < 32; j += 4) atomicAdd(reinterpret_cast<float4*>(dst + j), make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]));
-              } else if (accum) {
-#pragma unroll
-                for (int j = 0; j < 32; j += 4) {
-                  float4 o = *reinterpret_cast<float4*>(dst + j);
-                  o.x += v[j]; o.y += v[j + 1]; o.z += v[j + 2]; o.w += v[j + 3];
-                  *reinterpret_cast<float4*>(dst + j) = o;
-                }
-              } else {
-#pragma unroll
-                for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; j++) {
-                if (col0 + j < N) {
-                  if (ksplit > 1) atomicAdd(dst + j, v[j]);
-                  else dst[j] = accum ? dst[j] + v[j] : v[j];
-                }
-              }
-            }
-          }
-        }
+      if (have) {
+        const Drain d = {&maps.c[wh.g], C, wh.bi, wh.g, wh.n0, row0, M, N, ksplit, ngroups > 1 ? maps.g_accum[wh.g] : accum_, use_tma_store, out_scale, dead};
+        drain_tile<BN, GLU, SUB, S::EPI_TILES>(maps, d, ce, smem_raw, epi + (uint32_t)(ew * S::EPI_TILES) * 4096u,
+                                               tmem + b * BN + ((uint32_t)(q * 32) << 16), sub, lane, nst);
       }
       tc_fence_before();
       mbar_arrive(acc_empty(b));
@@ -456,28 +452,35 @@ gemm_tf32_kernel(const __grid_constant__ PartMaps maps, float* __restrict__ C, i
 // their bytes on the even CTA's `full`; `empty` and `acc_full` receive the MMA completions in both CTAs (multicast
 // commit); the epilogue threads of both CTAs arrive on the even CTA's `acc_empty`.
 // ---------------------------------------------------------------------------------------------
-template <int BN>
+// A 256 wide tile holds four blocks of a gated unit or four heads, a 192 wide one three: the computing epilogues have a warp
+// per lane quadrant for each (two per quadrant instead of four: 241 against 173 us for gate, up and the unit at
+// 16384 x 640 x 2*2048, where a block waits for its stores and then computes). The readout forms have eight blocks and two.
+template <int BN, int GLU>
+struct PairSub { static constexpr int N = GLU == 0 ? 1 : GLU >= EPI_CE_STATS ? 2 : BN / 64; };
+template <int BN, int GLU = 0>
 struct SmemPair {
   static constexpr int BH = BN / 2;                 // rows of the B tile staged by each CTA
   static constexpr int A_BYTES = BM1 * BK * 4;      // 16 KB
   static constexpr int B_BYTES = BH * BK * 4;
   static constexpr int STAGE = A_BYTES + B_BYTES;
-  static constexpr int EPI_BYTES = 4 * 2 * 4096;
-  static constexpr int STAGES = (232448 - EPI_BYTES - 1024 - 256) / STAGE;   // 6 for BN = 256 and 192
+  static constexpr int SUB = PairSub<BN, GLU>::N;
+  static constexpr int EPI_TILES = SUB == 1 ? 2 : 1;
+  static constexpr int EPI_BYTES = 4 * SUB * EPI_TILES * 4096;
+  static constexpr int STAGES = (232448 - EPI_BYTES - 1024 - 256) / STAGE;   // 6 (7 for BN = 192)
   static constexpr int TOTAL = STAGES * STAGE + EPI_BYTES + 1024 + 256;
   static constexpr uint32_t TMEM_COLS = 2 * BN <= 256 ? 256 : 512;
-  static constexpr int THREADS = 192;
+  static constexpr int THREADS = 64 + 128 * SUB;
   static_assert(BH % 32 == 0 && STAGES >= 3 && 8 * (2 * STAGES + 5) <= 256, "tile");
 };
 
-template <bool A_K, bool B_K, int BN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SmemPair<BN>::THREADS, 1)
-gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-                      const __grid_constant__ CUtensorMap mapC, float* __restrict__ C, int M, int N, int K, int accum, int ksplit,
+template <bool A_K, bool B_K, int BN, int GLU = 0>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SmemPair<BN, GLU>::THREADS, 1)
+gemm_tf32_pair_kernel(const __grid_constant__ PartMaps maps, float* __restrict__ C, int M_, int N_, int accum_, int ksplit,
                       int use_tma_store, int batch, float out_scale, int* __restrict__ flag) {
   pdl_wait();
   extern __shared__ uint8_t smem_raw[];
-  using S = SmemPair<BN>;
+  using S = SmemPair<BN, GLU>;
+  constexpr bool IS_GLU = GLU == GT_EW_SILU || GLU == GT_EW_GELU;
   constexpr int STAGES = S::STAGES, BM = 2 * BM1;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t epi = base + STAGES * S::STAGE;
@@ -492,15 +495,17 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank();          // 0: issues the MMAs; both stage operands and drain their rows
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
-  const int tiles_n = (N + BN - 1) / BN, tiles_m = (M + BM - 1) / BM;
+  const int tiles_n = (N_ + BN - 1) / BN, tiles_m = (M_ + BM - 1) / BM;
   const int per_mat = tiles_n * tiles_m * ksplit;
-  const int ntiles = per_mat * batch;
-  const int kblocks = (K + BK - 1) / BK;
+  const int ngroups = maps.ngroups;
+  const int ntiles = ngroups > 1 ? maps.unit_end[ngroups - 1] : per_mat * batch;
+  auto where = [&](int t) { return tile_at<BM, BN>(maps, t, tiles_n, tiles_m, per_mat); };
+  const int kblocks = maps.kb_end[maps.nparts - 1];
   const int per = (kblocks + ksplit - 1) / ksplit;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 256); }   // 128 epilogue threads per CTA
+    for (int b = 0; b < 2; b++) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 256 * S::SUB); }   // the epilogue threads of both CTAs
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc_pair(tmem_slot, S::TMEM_COLS);
@@ -520,21 +525,25 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
       // ---- TMA producer (both CTAs) ----
       uint32_t it = 0;
       for (int t = pair; t < ntiles; t += npairs) {
-        const int bi = t / per_mat, tt = t % per_mat;
-        const int n0 = (tt % tiles_n) * BN + rank * S::BH, m0 = ((tt / tiles_n) % tiles_m) * BM + rank * BM1, z = tt / (tiles_n * tiles_m);
-        const int kb0 = z * per, kb1 = min(kblocks, kb0 + per);
+        const Where wh = where(t);
+        const int bi = wh.bi, n0 = wh.n0 + rank * S::BH, m0 = wh.m0 + rank * BM1;
+        const int kb0 = wh.z * per, kb1 = min(kblocks, kb0 + per);
+        int part = wh.g;
         for (int kb = kb0; kb < kb1; kb++, it++) {
           const int s = it % STAGES;
           wait(empty_bar(s), ((it / STAGES) & 1) ^ 1, 1);
           const uint32_t a_dst = base + s * S::STAGE, b_dst = a_dst + S::A_BYTES;
-          const int k0 = kb * BK;
+          if (ngroups == 1) while (kb >= maps.kb_end[part]) part++;
+          const CUtensorMap* pa = &maps.a[part];
+          const CUtensorMap* pb = &maps.b[IS_GLU ? rank : part];   // (gated unit: the even CTA stages the gate's rows, the odd one up's)
+          const int k0 = (ngroups == 1 ? kb - (part ? maps.kb_end[part - 1] : 0) : kb) * BK;
           if (rank == 0) mbar_expect_tx(full_bar(s), 2 * S::STAGE);   // both CTAs' stages
-          if (A_K) tma_load_3d_pair(a_dst, &mapA, k0, m0, bi, full_bar(s));
+          if (A_K) tma_load_3d_pair(a_dst, pa, k0, m0, bi, full_bar(s));
           else
-            for (int c = 0; c < BM1 / 32; c++) tma_load_3d_pair(a_dst + c * 4096, &mapA, m0 + 32 * c, k0, bi, full_bar(s));
-          if (B_K) tma_load_3d_pair(b_dst, &mapB, k0, n0, bi, full_bar(s));
+            for (int c = 0; c < BM1 / 32; c++) tma_load_3d_pair(a_dst + c * 4096, pa, m0 + 32 * c, k0, bi, full_bar(s));
+          if (B_K) tma_load_3d_pair(b_dst, pb, k0, IS_GLU ? wh.n0 >> 1 : n0, bi, full_bar(s));
           else
-            for (int c = 0; c < S::BH / 32; c++) tma_load_3d_pair(b_dst + c * 4096, &mapB, n0 + 32 * c, k0, bi, full_bar(s));
+            for (int c = 0; c < S::BH / 32; c++) tma_load_3d_pair(b_dst + c * 4096, pb, n0 + 32 * c, k0, bi, full_bar(s));
         }
       }
     }
@@ -547,7 +556,7 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
       constexpr uint32_t A_STEP = A_K ? 32 : 1024, B_STEP = B_K ? 32 : 1024;
       uint32_t it = 0, tl = 0;
       for (int t = pair; t < ntiles; t += npairs, tl++) {
-        const int z = (t % per_mat) / (tiles_n * tiles_m);
+        const int z = where(t).z;
         const int kb0 = z * per, kb1 = min(kblocks, kb0 + per);
         const int b = tl & 1;
         wait(acc_empty(b), ((tl >> 1) & 1) ^ 1, 4);   // both CTAs have drained this accumulator
@@ -569,53 +578,21 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
     }
   } else {
     // ---- epilogue (both CTAs): this CTA's 128 rows ----
-    const int q = warp & 3;
+    const int q = warp & 3, ew = warp - 2, sub = ew >> 2;
     uint32_t tl = 0, nst = 0;
     for (int t = pair; t < ntiles; t += npairs, tl++) {
-      const int bi = t / per_mat, tt = t % per_mat;
-      const int n0 = (tt % tiles_n) * BN, m0 = ((tt / tiles_n) % tiles_m) * BM + rank * BM1, z = tt / (tiles_n * tiles_m);
-      const int b = tl & 1;
-      const bool have = z * per < kblocks;
-      const int row = m0 + q * 32 + lane;
+      const Where wh = where(t);
+      const int M = ngroups > 1 ? maps.gM[wh.g] : M_, N = ngroups > 1 ? maps.gN[wh.g] : N_;
+      const int b = tl & 1, row0 = wh.m0 + rank * BM1 + q * 32;
+      const CeRow ce = ce_row<GLU>(maps, row0 + lane, M);
+      const bool have = wh.z * per < kblocks;
       if (have) wait(acc_full(b), (tl >> 1) & 1, 3);
       dead = __any_sync(0xffffffffu, dead);
       tc_fence_after();
       if (have) {
-#pragma unroll 1
-        for (int c = 0; c < BN / 32; c++) {
-          const int col0 = n0 + c * 32;
-          if (col0 >= N) break;
-          float v[32];
-          tmem_ld32(tmem + b * BN + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32), v);
-#pragma unroll
-          for (int j = 0; j < 32; j++) v[j] *= out_scale;   // the caller's factor times the truncation compensation
-          if (use_tma_store) {
-            const uint32_t tile = epi + (uint32_t)(q * 2 + (nst & 1)) * 4096u;
-            if (nst >= 2) tma_wait_read<1>();
-            __syncwarp();
-            uint8_t* tp = smem_raw + (tile - smem_u32(smem_raw)) + lane * 128;
-#pragma unroll
-            for (int c4 = 0; c4 < 8; c4++)
-              *reinterpret_cast<float4*>(tp + ((c4 ^ (lane & 7)) * 16)) = make_float4(v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0 && !dead && m0 + q * 32 < M) {
-              if (ksplit > 1 || accum) tma_reduce_add_3d(&mapC, tile, col0, m0 + q * 32, bi);
-              else tma_store_3d(&mapC, tile, col0, m0 + q * 32, bi);
-            }
-            if (lane == 0) tma_commit_group();
-            nst++;
-          } else if (row < M && !dead) {
-            float* dst = C + (size_t)bi * M * N + (size_t)row * N + col0;
-#pragma unroll
-            for (int j = 0; j < 32; j++) {
-              if (col0 + j < N) {
-                if (ksplit > 1) atomicAdd(dst + j, v[j]);
-                else dst[j] = accum ? dst[j] + v[j] : v[j];
-              }
-            }
-          }
-        }
+        const Drain d = {&maps.c[wh.g], C, wh.bi, wh.g, wh.n0, row0, M, N, ksplit, ngroups > 1 ? maps.g_accum[wh.g] : accum_, use_tma_store, out_scale, dead};
+        drain_tile<BN, GLU, S::SUB, S::EPI_TILES>(maps, d, ce, smem_raw, epi + (uint32_t)(ew * S::EPI_TILES) * 4096u,
+                                                  tmem + b * BN + ((uint32_t)(q * 32) << 16), sub, lane, nst);
       }
       tc_fence_before();
       mbar_arrive_leader(acc_empty(b));
@@ -900,33 +877,44 @@ int cluster_room(gt_ctx* ctx, int c) {
   return r;
 }
 
-// The best shape of the one-tile-per-CTA kernel for `tiles(bn)` tiles of 128 x bn and its predicted cycles, on the scale of
-// the persistent kernel's cost model. A K block costs its shared-memory traffic (the stage written and read once at
-// 128 B/clk); resident CTAs of an SM share that.
-constexpr double SMALL_FIXED = 10500.0, SMALL_WAVE = 8500.0;
+// Predicted times in microseconds, fitted to 919 launches of 154 products (16 to 16384 rows, outputs 576 to 49152 wide, depths
+// 576 to 49152; the fit's rms error is 4 %): a launch costs a fixed part and, per wave of tiles, its K blocks and what of
+// the epilogue is not hidden. A K block costs the larger of its shared-memory traffic (written once by TMA, read once per 128-row half by the MMAs,
+// 128 B/clk for all of it) and its MMAs; MN-major operands cost CTA pairs more than that.
+struct Shape { int mt, bn; double per_kb[3], epilogue; };   // mt 1, 2: 128 / 256 rows on one CTA; mt 3: 256 rows on a CTA pair; per_kb by layout
+constexpr Shape SHAPES[6] = {{1, 192, {0.345, 0.400, 0.465}, 1.67}, {1, 128, {0.312, 0.358, 0.429}, 0.76}, {2, 256, {0.651, 0.631, 0.638}, 5.35},
+                             {2, 192, {0.550, 0.543, 0.621}, 3.90}, {3, 192, {0.330, 0.392, 0.502}, 0.89}, {3, 256, {0.334, 0.428, 0.529}, 1.75}};
+constexpr double FIXED = 4.3, FIXED_PAIR = 6.1;   // what a launch costs beside its tiles
+constexpr double SLICE = 0.52;                    // per wave when slices of K are added up in L2
+constexpr double CLEAR = 3.4;                     // the clear before a launch whose slices meet in L2, and the gap before it
+double shape_cost(const Shape& h, int kind, long units, long workers, int kblocks, int ks) {
+  return (h.mt == 3 ? FIXED_PAIR : FIXED) + gt_cdiv(units, workers) * (gt_cdiv(kblocks, ks) * h.per_kb[kind] + h.epilogue + (ks > 1 ? SLICE : 0.0));
+}
+
+// The best shape of the one-tile-per-CTA kernel for `tiles(bn)` tiles of 128 x bn and its predicted time. A K block costs
+// its shared-memory traffic; resident CTAs of an SM share that. (Measured in cycles, CYCLE us each.)
+constexpr double SMALL_FIXED = 10500.0, SMALL_WAVE = 8500.0, CYCLE = 0.00067;
 struct SmallPick { int bn = 0, ks = 1; double cost = 1e30; };
 template <typename F>
-SmallPick pick_small(gt_ctx* ctx, int kblocks, F tiles, int min_bn) {
+SmallPick pick_small(gt_ctx* ctx, int kind, int kblocks, F tiles, int min_bn) {
   const long workers = ctx->sm_count - ctx->sm_reserved;
   SmallPick p;
   for (int bn = min_bn; bn <= 128; bn *= 2) {
     const long n = tiles(bn);
     if (n > 4 * workers) continue;
-    const double per_kb = 2.0 * (BM1 + bn) * BK * 4 / 128.0;
+    const double per_kb = 2.0 * (BM1 + bn) * BK * 4 / 128.0 * (kind == GT_GEMM_NT ? 1.0 : 1.25);   // (MN-major stages come in more copies)
     for (int ks = 1; ks <= 8 && ks <= kblocks; ks++) {
       const int per = gt_cdiv(kblocks, ks);
       if ((long)(ks - 1) * per >= kblocks) continue;   // (an empty slice)
       const long room = ks == 1 ? workers : max((long)ks, (long)cluster_room(ctx, ks) - ctx->sm_reserved);   // two CTAs of up to 64 columns share an SM
       const double share = n * ks > room && bn <= 64 ? 2.0 : 1.0;
       const double waves = ceil((double)(n * ks) / (room * share));
-      const double cost = waves * (per * per_kb * share + SMALL_WAVE) + (SMALL_FIXED - SMALL_WAVE) + (share > 1.0 ? 5000.0 : 0.0) + 6.0 * bn;
-      if (cost < p.cost) { p.cost = cost; p.bn = bn; p.ks = ks; }
+      const double cost = waves * (per * per_kb * share + SMALL_WAVE) + (SMALL_FIXED - SMALL_WAVE) + (share > 1.0 ? 5000.0 : 0.0) + 6.0 * bn + (ks > 1 ? 2000.0 : 0.0);
+      if (cost * CYCLE < p.cost) { p.cost = cost * CYCLE; p.bn = bn; p.ks = ks; }
     }
   }
   return p;
 }
-// what a launch of the persistent kernel costs beside its tiles, and the clear before one whose slices meet in L2
-constexpr double PERSISTENT_FIXED = 9500.0, CLEAR_FIXED = 2800.0;
 
 template <bool A_K, bool B_K, int BN, int MT, int GLU = 0>
 gt_status launch(gt_ctx* ctx, const PartMaps& maps, long ntiles, int tma_store, float* c, int M, int N, int accum, int ksplit,
@@ -944,29 +932,28 @@ gt_status launch(gt_ctx* ctx, const PartMaps& maps, long ntiles, int tma_store, 
   return GT_OK;
 }
 
-template <bool A_K, bool B_K, int BN>
-gt_status launch_pair(gt_ctx* ctx, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, int tma_store, float* c, int M, int N,
-                      int K, int accum, int ksplit, int batch, int npairs, float out_scale) {
-  auto kern = gemm_tf32_pair_kernel<A_K, B_K, BN>;
-  using S = SmemPair<BN>;
+template <bool A_K, bool B_K, int BN, int GLU = 0>
+gt_status launch_pair(gt_ctx* ctx, const PartMaps& maps, long ntiles, int tma_store, float* c, int M, int N, int accum, int ksplit,
+                      int batch, int npairs, float out_scale) {
+  auto kern = gemm_tf32_pair_kernel<A_K, B_K, BN, GLU>;
+  using S = SmemPair<BN, GLU>;
   static bool attr_set[64] = {};
   if (!attr_set[ctx->device]) {
     GT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL));
     attr_set[ctx->device] = true;
   }
-  const long ntiles = (long)gt_cdiv(N, BN) * gt_cdiv(M, 2 * BM1) * ksplit * batch;
   dim3 grid(2u * (unsigned)min((long)npairs, ntiles), 1, 1);
-  GT_CUDA(ctx, gt_launch(ctx, 1, kern, grid, S::THREADS, S::TOTAL, ma, mb, mc, c, M, N, K, accum, ksplit, tma_store, batch, out_scale, g_flag[ctx->device]));
+  GT_CUDA(ctx, gt_launch(ctx, 1, kern, grid, S::THREADS, S::TOTAL, maps, c, M, N, accum, ksplit, tma_store, batch, out_scale, g_flag[ctx->device]));
   GT_LAUNCHED(ctx, "gemm_tf32_pair_kernel");
   return GT_OK;
 }
 
 template <int BN>
-gt_status launch_pair_kind(gt_ctx* ctx, int kind, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, int tma_store,
-                           float* c, int M, int N, int K, int accum, int ksplit, int batch, int npairs, float out_scale) {
-  if (kind == GT_GEMM_NT) return launch_pair<true, true, BN>(ctx, ma, mb, mc, tma_store, c, M, N, K, accum, ksplit, batch, npairs, out_scale);
-  if (kind == GT_GEMM_NN) return launch_pair<true, false, BN>(ctx, ma, mb, mc, tma_store, c, M, N, K, accum, ksplit, batch, npairs, out_scale);
-  return launch_pair<false, false, BN>(ctx, ma, mb, mc, tma_store, c, M, N, K, accum, ksplit, batch, npairs, out_scale);
+gt_status launch_pair_kind(gt_ctx* ctx, int kind, const PartMaps& maps, long ntiles, int tma_store, float* c, int M, int N, int accum,
+                           int ksplit, int batch, int npairs, float out_scale) {
+  if (kind == GT_GEMM_NT) return launch_pair<true, true, BN>(ctx, maps, ntiles, tma_store, c, M, N, accum, ksplit, batch, npairs, out_scale);
+  if (kind == GT_GEMM_NN) return launch_pair<true, false, BN>(ctx, maps, ntiles, tma_store, c, M, N, accum, ksplit, batch, npairs, out_scale);
+  return launch_pair<false, false, BN>(ctx, maps, ntiles, tma_store, c, M, N, accum, ksplit, batch, npairs, out_scale);
 }
 
 // CTA pairs that can be resident at once (two neighbouring SMs each); 0 when the device cannot run the pair kernel.
@@ -991,6 +978,8 @@ int pair_capacity(gt_ctx* ctx) {
   }
   return cap[ctx->device];
 }
+
+int pair_workers(gt_ctx* ctx) { return max(0, pair_capacity(ctx) - (ctx->sm_reserved + 1) / 2); }
 
 template <int BN, int MT>
 gt_status launch_kind(gt_ctx* ctx, int kind, const PartMaps& maps, long ntiles, int tma_store, float* c, int M, int N, int accum,
@@ -1144,44 +1133,31 @@ static std::unordered_map<PlanKey, Plan, WordsHash>& plan_cache() {
   if (plans.size() > 4096) plans.clear();
   return plans;
 }
-static Plan choose_plan(gt_ctx* ctx, int accum, int M, int N, int nparts, int kblocks, int batch, const char* force, const char* ds) {
-  // Tile shape and split-K factor: the cheapest of the four shapes under a small cost model (cycles of the CTA with
-  // the most work: waves x (K blocks x cycles per K block + epilogue)), calibrated on in-kernel cycle counts.
-  struct Cfg { int mt, bn; };   // mt 1, 2: 128 / 256 rows on one CTA; mt 3: 256 rows on a CTA pair
-  static const Cfg cfgs[6] = {{1, 192}, {1, 128}, {2, 256}, {2, 192}, {3, 192}, {3, 256}};
+static Plan choose_plan(gt_ctx* ctx, int kind, int accum, int M, int N, int kblocks, int batch, const char* force, const char* ds) {
+  // Tile shape and split-K factor: the cheapest under the model above.
   const bool deep_split = !(ds && ds[0] == '0');
-  const int npairs = max(0, pair_capacity(ctx) - (ctx->sm_reserved + 1) / 2);
-  int best = 0, ksplit = 1;
+  const int npairs = pair_workers(ctx);
+  int best = -1, ksplit = 1;
   double best_cost = 1e30;
   int best_deep = 0, ks_deep = 1;      // the best choice that also cuts a product with enough tiles along K (see below)
   double cost_deep = 1e30;
   for (int i = 0; i < 6; i++) {
-    const int mt = cfgs[i].mt, bn = cfgs[i].bn, bm = mt == 1 ? BM1 : 2 * BM1;
-    if (mt == 3 && (npairs < 8 || nparts > 1)) continue;   // (the pair kernel takes one product)
+    const Shape& h = SHAPES[i];
+    const int bm = h.mt == 1 ? BM1 : 2 * BM1;
+    if (h.mt == 3 && npairs < 8) continue;
     if (force) {
       int fm = 0, fb = 0;
-      if (sscanf(force, "%d,%d", &fm, &fb) == 2 && (fm != mt || fb != bn)) continue;
+      if (sscanf(force, "%d,%d", &fm, &fb) == 2 && (fm != h.mt || fb != h.bn)) continue;
     }
-    const long workers = mt == 3 ? npairs : ctx->sm_count - ctx->sm_reserved;
-    const long tiles = (long)gt_cdiv(N, bn) * gt_cdiv(M, bm) * batch;
+    const long workers = h.mt == 3 ? npairs : ctx->sm_count - ctx->sm_reserved;
+    const long tiles = (long)gt_cdiv(N, h.bn) * gt_cdiv(M, bm) * batch;
     // split K when the output has few tiles and K is deep (dW: K = rows); partial sums meet in L2 with f32 adds
     int ks = 1;
     if (tiles < workers && kblocks >= 16) {
       ks = (int)min((long)(workers / tiles), (long)(kblocks / 8));
       if (ks < 1) ks = 1;
     }
-    // One K block costs the slower of its MMAs (N/2 cycles each) and its shared-memory traffic at 128 B/clk: the stage
-    // is written once by TMA and read once per 128-row half by the MMAs (measured: 0.9 of that bound). The epilogue
-    // of a 256-row tile is exposed, that of a 128-row tile mostly hidden.
-    // A CTA of a pair stages 128 rows of A and half of the B tile but still serves both halves of B to the pair's
-    // tensor cores: measured 640 (BN 192) and 720 (BN 256) cycles per K block, little better per flop than one CTA
-    // with a 256-row tile; what the pair adds is the second accumulator (hidden epilogue) and a deeper pipeline.
-    const double tensor = (mt == 2 ? 2 : 1) * 4.0 * (bn / 2);
-    const double smem = mt == 3 ? (bn == 192 ? 640.0 : 720.0)
-                                : 0.92 * ((bm * 128.0 + bn * 128.0) + mt * (BM1 * 128.0 + bn * 128.0)) / 128.0;
-    const double per_kb = tensor > smem ? tensor : smem;
-    const double epilogue = mt == 2 ? 14.0 * bn + 900.0 : 1500.0;
-    const double cost = gt_cdiv(tiles * ks, workers) * ((double)gt_cdiv(kblocks, ks) * per_kb + epilogue) + PERSISTENT_FIXED + (ks > 1 && !accum ? CLEAR_FIXED : 0.0);
+    const double cost = shape_cost(h, kind, tiles * ks, workers, kblocks, ks) + (ks > 1 && !accum ? CLEAR : 0.0);
     if (cost < best_cost) { best_cost = cost; best = i; ksplit = ks; }
     // A deep product whose tiles fill the SMs unevenly (the readout's dX: 384 tiles of 128 x 192 on 148 SMs are 2.6
     // waves, run as 3) may be cut along K as well when that evens the waves out: as 192 tiles of 256 x 192 in three
@@ -1189,7 +1165,7 @@ static Plan choose_plan(gt_ctx* ctx, int accum, int M, int N, int nparts, int kb
     // charged; the candidate is taken after the loop only if it is predicted well ahead. Measured at rows 16384: the
     // readout's dX (K 49152) 1890 -> 1292 us, dX of gate and up (K 3072) 128 -> 106 us; at K 1536 the same choice
     // measured slower (60.5 -> 67.9 us), hence the depth limit of 64 K blocks.
-    if (ks == 1 && tiles >= workers && kblocks >= 64 && deep_split && mt != 3) {
+    if (ks == 1 && tiles >= workers && kblocks >= 64 && deep_split) {
       double best_w = (double)gt_cdiv(tiles, workers);
       int k2best = 1;
       for (int k2 = 2; k2 <= 4; k2++) {
@@ -1197,7 +1173,7 @@ static Plan choose_plan(gt_ctx* ctx, int accum, int M, int N, int nparts, int kb
         if (w2 < best_w - 0.05) { best_w = w2; k2best = k2; }
       }
       if (k2best > 1) {
-        const double c2 = gt_cdiv(tiles * k2best, workers) * ((double)gt_cdiv(kblocks, k2best) * per_kb + epilogue + 600.0) + 8000.0 + PERSISTENT_FIXED;
+        const double c2 = shape_cost(h, kind, tiles * k2best, workers, kblocks, k2best) + CLEAR + 2.0;
         if (c2 < cost_deep) { cost_deep = c2; best_deep = i; ks_deep = k2best; }
       }
     }
@@ -1207,11 +1183,11 @@ static Plan choose_plan(gt_ctx* ctx, int accum, int M, int N, int nparts, int kb
   if (force && sscanf(force, "%d,%d", &fm, &fb) < 1) fm = -1;
   SmallPick small;
   if (fm <= 0)
-    small = pick_small(ctx, kblocks, [&](int b) { return (fm == 0 && fb && b != fb) ? 1l << 40 : (long)gt_cdiv(N, b) * gt_cdiv(M, BM1) * batch; }, 32);
+    small = pick_small(ctx, kind, kblocks, [&](int b) { return (fm == 0 && fb && b != fb) ? 1l << 40 : (long)gt_cdiv(N, b) * gt_cdiv(M, BM1) * batch; }, 32);
   const bool use_small = small.bn && small.cost < best_cost;
-  if (best_cost >= 1e30 && !use_small) return {};
+  if (best < 0 && !use_small) return {};
   if (use_small) return {1, small.bn, small.ks, true};
-  return {cfgs[best].mt, cfgs[best].bn, ksplit, false};
+  return {SHAPES[best].mt, SHAPES[best].bn, ksplit, false};
 }
 
 // `batch` independent products of the same shape, matrix i of each operand `M*K`, `N*K`, `M*N` elements after matrix i-1.
@@ -1242,7 +1218,7 @@ static gt_status gemm_tc_dispatch(gt_ctx* ctx, int kind, int accum, int M, int N
   auto found = force || ds ? plans.end() : plans.find(key);
   if (found != plans.end()) plan = found->second;
   else {
-    plan = choose_plan(ctx, accum, M, N, nparts, kblocks, batch, force, ds);
+    plan = choose_plan(ctx, kind, accum, M, N, kblocks, batch, force, ds);
     if (!force && !ds) plans.emplace(key, plan);
   }
   if (!plan.mt) return GT_OK;
@@ -1281,12 +1257,11 @@ static gt_status gemm_tc_dispatch(gt_ctx* ctx, int kind, int accum, int M, int N
   for (int p = 0; p < MAX_PARTS; p++) { maps.gM[p] = M; maps.gN[p] = N; maps.g_accum[p] = accum; maps.unit_end[p] = 0; }
   if (ksplit > 1 && !accum) GT_CUDA(ctx, cudaMemsetAsync(c, 0, sizeof(float) * (size_t)M * N * batch, ctx->stream));
   const float out_scale = alpha * TRUNC_COMP;
-  const int K0 = Ks[0];
   const long ntiles = (long)gt_cdiv(N, bn) * gt_cdiv(M, mt == 1 ? BM1 : 2 * BM1) * ksplit * batch;
   gt_status s;
-  const int npairs = max(0, pair_capacity(ctx) - (ctx->sm_reserved + 1) / 2);
-  if (mt == 3 && bn == 192) s = launch_pair_kind<192>(ctx, kind, maps.a[0], maps.b[0], maps.c[0], tma_store, c, M, N, K0, accum, ksplit, batch, npairs, out_scale);
-  else if (mt == 3) s = launch_pair_kind<256>(ctx, kind, maps.a[0], maps.b[0], maps.c[0], tma_store, c, M, N, K0, accum, ksplit, batch, npairs, out_scale);
+  const int npairs = pair_workers(ctx);
+  if (mt == 3 && bn == 192) s = launch_pair_kind<192>(ctx, kind, maps, ntiles, tma_store, c, M, N, accum, ksplit, batch, npairs, out_scale);
+  else if (mt == 3) s = launch_pair_kind<256>(ctx, kind, maps, ntiles, tma_store, c, M, N, accum, ksplit, batch, npairs, out_scale);
   else if (mt == 1 && bn == 192) s = launch_kind<192, 1>(ctx, kind, maps, ntiles, tma_store, c, M, N, accum, ksplit, batch, out_scale);
   else if (mt == 1) s = launch_kind<128, 1>(ctx, kind, maps, ntiles, tma_store, c, M, N, accum, ksplit, batch, out_scale);
   else if (bn == 256) s = launch_kind<256, 2>(ctx, kind, maps, ntiles, tma_store, c, M, N, accum, ksplit, batch, out_scale);
@@ -1307,23 +1282,23 @@ static std::unordered_map<GroupKey, Plan, WordsHash>& group_cache() {
 }
 static Plan choose_group_plan(gt_ctx* ctx, int kind, int ngroups, const int* Ms, const int* Ns, int kblocks, const int* accums, bool any_rope,
                               const char* force) {
-  const long workers = ctx->sm_count - ctx->sm_reserved;
   int clears = 0;      // (one clear per product that does not accumulate)
   for (int g = 0; g < ngroups; g++) clears += !accums[g];
-  // 256 x 192 or 128 x 192 tiles; the split-K factor (one for the whole launch) that wastes least of the last wave,
-  // among those that leave a slice at least 8 K blocks and add at most 8 partial sums per output element
-  int best_mt = 1, best_ks = 1;
+  // The tile shape and the split-K factor (one for the whole launch) with the least predicted time, among slices of at
+  // least 8 K blocks and at most 8 partial sums per output element.
+  int best = -1, best_ks = 1;
   double best_cost = 1e30;
-  for (int mt = 1; mt <= 2; mt++) {
-    if (force) { int fm = 0, fb = 0; if (sscanf(force, "%d,%d", &fm, &fb) == 2 && (fm != mt || fb != 192)) continue; }
+  const int npairs = pair_workers(ctx);
+  for (int i = 0; i < 6; i++) {
+    const Shape& h = SHAPES[i];
+    if ((h.mt == 3 && npairs < 8) || h.bn == 128 || (any_rope && h.mt == 2)) continue;
+    if (force) { int fm = 0, fb = 0; if (sscanf(force, "%d,%d", &fm, &fb) == 2 && (fm != h.mt || fb != h.bn)) continue; }
     long tiles = 0;
-    for (int g = 0; g < ngroups; g++) tiles += (long)gt_cdiv(Ns[g], 192) * gt_cdiv(Ms[g], mt * BM1);
-    const double per_kb = 0.92 * ((mt * BM1 * 128.0 + 192 * 128.0) + mt * (BM1 * 128.0 + 192 * 128.0)) / 128.0;
-    const double epilogue = mt == 2 ? 14.0 * 192 + 900.0 : 1500.0;
+    for (int g = 0; g < ngroups; g++) tiles += (long)gt_cdiv(Ns[g], h.bn) * gt_cdiv(Ms[g], h.mt == 1 ? BM1 : 2 * BM1);
+    const long workers = h.mt == 3 ? npairs : ctx->sm_count - ctx->sm_reserved;
     for (int ks = 1; ks <= 8 && (ks == 1 || kblocks / ks >= 8); ks++) {
-      const long waves = gt_cdiv(tiles * ks, workers);
-      const double cost = waves * (gt_cdiv(kblocks, ks) * per_kb + epilogue + (ks > 1 ? 600.0 : 0.0)) + PERSISTENT_FIXED + (ks > 1 ? clears * CLEAR_FIXED : 0.0);
-      if (cost < best_cost) { best_cost = cost; best_mt = mt; best_ks = ks; }
+      const double cost = shape_cost(h, kind, tiles * ks, workers, kblocks, ks) + (ks > 1 ? clears * CLEAR : 0.0);
+      if (cost < best_cost) { best_cost = cost; best = i; best_ks = ks; }
     }
   }
   int fm = -1, fb = 0;
@@ -1334,15 +1309,15 @@ static Plan choose_group_plan(gt_ctx* ctx, int kind, int ngroups, const int* Ms,
   for (int g = 0; g < ngroups; g++) heads64 = heads64 && (Ns[g] & 63) == 0;
   SmallPick small;
   if (fm <= 0)
-    small = pick_small(ctx, kblocks, [&](int b) {
+    small = pick_small(ctx, kind, kblocks, [&](int b) {
       if (fm == 0 && fb && b != fb) return 1l << 40;
       long n = 0;
       for (int g = 0; g < ngroups; g++) n += (long)gt_cdiv(Ns[g], b) * gt_cdiv(Ms[g], BM1);
       return n;
     }, any_rope || heads64 ? 64 : 32);
   const bool use_small = small.bn && small.cost < best_cost;
-  if (best_cost >= 1e30 && !use_small) return {};
-  return use_small ? Plan{1, small.bn, small.ks, true} : Plan{best_mt, 192, best_ks, false};
+  if (best < 0 && !use_small) return {};
+  return use_small ? Plan{1, small.bn, small.ks, true} : Plan{SHAPES[best].mt, SHAPES[best].bn, best_ks, false};
 }
 
 // ngroups independent products of one layout and one K, each with its own operands, extents and accumulate flag, as
@@ -1380,15 +1355,16 @@ static gt_status gemm_tc_grouped(gt_ctx* ctx, int kind, int ngroups, const int* 
   }
   if (!plan.mt) return GT_OK;
   const bool use_small = plan.small;
-  const int mt = plan.mt, ksplit = plan.ks, bm = mt * BM1, bn = plan.bn;
+  const int mt = plan.mt, ksplit = plan.ks, bm = mt == 1 ? BM1 : 2 * BM1, bn = plan.bn;
+  const int a_box = mt == 2 ? 2 * BM1 : BM1, b_box = mt == 3 ? bn / 2 : bn;   // rows one TMA copy brings
   PartMaps maps;
   maps.nparts = 1;
   maps.ngroups = ngroups;
   int units = 0;
   for (int g = 0; g < ngroups; g++) {
     const int M = Ms[g], N = Ns[g];
-    const bool oka = a_k ? make_map_3d(&maps.a[g], as[g], K, M, 1, K, (uint64_t)M * K, bm, true) : make_map_3d(&maps.a[g], as[g], M, K, 1, M, (uint64_t)M * K, BK, false);
-    const bool okb = b_k ? make_map_3d(&maps.b[g], bs[g], K, N, 1, K, (uint64_t)N * K, bn, true) : make_map_3d(&maps.b[g], bs[g], N, K, 1, N, (uint64_t)N * K, BK, false);
+    const bool oka = a_k ? make_map_3d(&maps.a[g], as[g], K, M, 1, K, (uint64_t)M * K, a_box, true) : make_map_3d(&maps.a[g], as[g], M, K, 1, M, (uint64_t)M * K, BK, false);
+    const bool okb = b_k ? make_map_3d(&maps.b[g], bs[g], K, N, 1, K, (uint64_t)N * K, b_box, true) : make_map_3d(&maps.b[g], bs[g], N, K, 1, N, (uint64_t)N * K, BK, false);
     const bool okc = use_small || make_map_3d(&maps.c[g], cs[g], N, M, 1, N, (uint64_t)M * N, 32, true);
     if (!oka || !okb || !okc) return GT_OK;
     maps.cp[g] = cs[g];
@@ -1420,12 +1396,18 @@ static gt_status gemm_tc_grouped(gt_ctx* ctx, int kind, int ngroups, const int* 
     for (int g = 0; g < ngroups; g++)
       if (!accums[g]) GT_CUDA(ctx, cudaMemsetAsync(cs[g], 0, sizeof(float) * (size_t)Ms[g] * Ns[g], ctx->stream));
   gt_status s;
+  const float scale = alpha * TRUNC_COMP;
+  const int npairs = pair_workers(ctx);
   if (any_rope)
-    s = mt == 1 ? launch<true, true, 192, 1, EPI_ROPE>(ctx, maps, units, 1, cs[0], Ms[0], Ns[0], accums[0], ksplit, 1, alpha * TRUNC_COMP)
-                : launch<true, true, 192, 2, EPI_ROPE>(ctx, maps, units, 1, cs[0], Ms[0], Ns[0], accums[0], ksplit, 1, alpha * TRUNC_COMP);
+    s = mt == 1 ? launch<true, true, 192, 1, EPI_ROPE>(ctx, maps, units, 1, cs[0], Ms[0], Ns[0], accums[0], ksplit, 1, scale)
+        : bn == 192 ? launch_pair<true, true, 192, EPI_ROPE>(ctx, maps, units, 1, cs[0], Ms[0], Ns[0], accums[0], ksplit, 1, npairs, scale)
+                    : launch_pair<true, true, 256, EPI_ROPE>(ctx, maps, units, 1, cs[0], Ms[0], Ns[0], accums[0], ksplit, 1, npairs, scale);
   else
-    s = mt == 1 ? launch_kind<192, 1>(ctx, kind, maps, units, 1, cs[0], Ms[0], Ns[0], accums[0], ksplit, 1, alpha * TRUNC_COMP)
-                : launch_kind<192, 2>(ctx, kind, maps, units, 1, cs[0], Ms[0], Ns[0], accums[0], ksplit, 1, alpha * TRUNC_COMP);
+    s = mt == 1 ? launch_kind<192, 1>(ctx, kind, maps, units, 1, cs[0], Ms[0], Ns[0], accums[0], ksplit, 1, scale)
+        : mt == 2 && bn == 256 ? launch_kind<256, 2>(ctx, kind, maps, units, 1, cs[0], Ms[0], Ns[0], accums[0], ksplit, 1, scale)
+        : mt == 2 ? launch_kind<192, 2>(ctx, kind, maps, units, 1, cs[0], Ms[0], Ns[0], accums[0], ksplit, 1, scale)
+        : bn == 192 ? launch_pair_kind<192>(ctx, kind, maps, units, 1, cs[0], Ms[0], Ns[0], accums[0], ksplit, 1, npairs, scale)
+                    : launch_pair_kind<256>(ctx, kind, maps, units, 1, cs[0], Ms[0], Ns[0], accums[0], ksplit, 1, npairs, scale);
   if (s) return s;
   *handled = true;
   return GT_OK;
@@ -1438,14 +1420,19 @@ gt_status gt_glu_linear_tc(gt_ctx* ctx, int op, int rows, int ffn, int in, const
   if (rows < 16 || ffn < 96 || in < 16 || (in & 3) || (ffn & 3)) return GT_OK;
   if ((((uintptr_t)x) | ((uintptr_t)wg) | ((uintptr_t)wu) | ((uintptr_t)gate) | ((uintptr_t)up) | ((uintptr_t)out)) & 15) return GT_OK;
   if (ctx->device < 0 || ctx->device >= 64 || !device_flag(ctx)) return GT_OK;
-  constexpr int BN = 192;
   PartMaps maps;
   maps.nparts = 1;
   maps.ngroups = 1;
   const int kblocks = gt_cdiv(in, BK);
   const long workers = ctx->sm_count - ctx->sm_reserved;
-  const double cost = (double)gt_cdiv((long)gt_cdiv(ffn, BN / 2) * gt_cdiv(rows, BM1), workers) * (kblocks * 0.92 * 2.0 * (BM1 + BN) + 1500.0) + PERSISTENT_FIXED;
-  const SmallPick small = pick_small(ctx, kblocks, [&](int b) { return (long)gt_cdiv(ffn, b / 2) * gt_cdiv(rows, BM1); }, 32);
+  const int npairs = pair_workers(ctx);
+  // (the unit's epilogue is not hidden: 3 us a 192 wide tile, 6.5 us a 256 wide pair of them)
+  const Shape s1 = {1, 192, {SHAPES[0].per_kb[0]}, 5.0}, s3 = {3, 256, {SHAPES[5].per_kb[0]}, 5.5};
+  double cost = shape_cost(s1, 0, (long)gt_cdiv(ffn, 96) * gt_cdiv(rows, BM1), workers, kblocks, 1);
+  const double cost_pair = npairs < 8 ? 1e30 : shape_cost(s3, 0, (long)gt_cdiv(ffn, 128) * gt_cdiv(rows, 2 * BM1), npairs, kblocks, 1);
+  bool pair = cost_pair < cost;
+  cost = min(cost, cost_pair);
+  const SmallPick small = pick_small(ctx, GT_GEMM_NT, kblocks, [&](int b) { return (long)gt_cdiv(ffn, b / 2) * gt_cdiv(rows, BM1); }, 32);
   const char* force = getenv("GT_GEMM_TILE");
   if (small.bn && small.cost < cost && (!force || force[0] == '0')) {
     const int bn = small.bn;
@@ -1469,9 +1456,12 @@ gt_status gt_glu_linear_tc(gt_ctx* ctx, int op, int rows, int ffn, int in, const
     *handled = true;
     return GT_OK;
   }
+  if (force && !strcmp(force, "1,192")) pair = false;
+  if (force && !strcmp(force, "3,256") && npairs >= 8) pair = true;
+  const int bn = pair ? 256 : 192, bm = pair ? 2 * BM1 : BM1;
   bool ok = make_map_3d(&maps.a[0], x, in, rows, 1, in, (uint64_t)rows * in, BM1, true);
-  ok = ok && make_map_3d(&maps.b[0], wg, in, ffn, 1, in, (uint64_t)ffn * in, BN / 2, true);
-  ok = ok && make_map_3d(&maps.b[1], wu, in, ffn, 1, in, (uint64_t)ffn * in, BN / 2, true);
+  ok = ok && make_map_3d(&maps.b[0], wg, in, ffn, 1, in, (uint64_t)ffn * in, bn / 2, true);
+  ok = ok && make_map_3d(&maps.b[1], wu, in, ffn, 1, in, (uint64_t)ffn * in, bn / 2, true);
   ok = ok && make_map_3d(&maps.c[0], gate, ffn, rows, 1, ffn, (uint64_t)rows * ffn, 32, true);
   ok = ok && make_map_3d(&maps.c[1], up, ffn, rows, 1, ffn, (uint64_t)rows * ffn, 32, true);
   ok = ok && make_map_3d(&maps.c[2], out, ffn, rows, 1, ffn, (uint64_t)rows * ffn, 32, true);
@@ -1482,11 +1472,13 @@ gt_status gt_glu_linear_tc(gt_ctx* ctx, int op, int rows, int ffn, int in, const
     if (p > 2) maps.c[p] = maps.c[0];
     maps.kb_end[p] = kblocks; maps.gM[p] = rows; maps.gN[p] = 2 * ffn; maps.g_accum[p] = 0; maps.unit_end[p] = 0;
   }
-  const int N2 = 2 * gt_cdiv(ffn, BN / 2) * (BN / 2);   // whole tiles of 96 + 96 columns; the maps clip at ffn
-  const long ntiles = (long)gt_cdiv(N2, BN) * gt_cdiv(rows, BM1);
-  gt_status s = op == GT_EW_SILU
-                    ? launch<true, true, BN, 1, GT_EW_SILU>(ctx, maps, ntiles, 1, out, rows, N2, 0, 1, 1, TRUNC_COMP)
-                    : launch<true, true, BN, 1, GT_EW_GELU>(ctx, maps, ntiles, 1, out, rows, N2, 0, 1, 1, TRUNC_COMP);
+  const int N2 = 2 * gt_cdiv(ffn, bn / 2) * (bn / 2);   // whole tiles of two halves; the maps clip at ffn
+  const long ntiles = (long)gt_cdiv(N2, bn) * gt_cdiv(rows, bm);
+  gt_status s;
+  if (pair) s = op == GT_EW_SILU ? launch_pair<true, true, 256, GT_EW_SILU>(ctx, maps, ntiles, 1, out, rows, N2, 0, 1, 1, npairs, TRUNC_COMP)
+                                 : launch_pair<true, true, 256, GT_EW_GELU>(ctx, maps, ntiles, 1, out, rows, N2, 0, 1, 1, npairs, TRUNC_COMP);
+  else s = op == GT_EW_SILU ? launch<true, true, 192, 1, GT_EW_SILU>(ctx, maps, ntiles, 1, out, rows, N2, 0, 1, 1, TRUNC_COMP)
+                            : launch<true, true, 192, 1, GT_EW_GELU>(ctx, maps, ntiles, 1, out, rows, N2, 0, 1, 1, TRUNC_COMP);
   if (s) return s;
   *handled = true;
   return GT_OK;
@@ -1498,40 +1490,30 @@ gt_status gt_glu_linear_tc(gt_ctx* ctx, int op, int rows, int ffn, int in, const
 gt_status gt_readout_tc(gt_ctx* ctx, bool grad, int rows, int n, int h, const float* hidden, const float* w, float* chunk, const CeArgs& ce,
                         int* parts, bool* handled) {
   *handled = false;
-  if (rows < 16 || n < 192 || h < 16 || (h & 3) || (grad && (n & 3))) return GT_OK;
+  if (rows < 16 || n < 256 || h < 16 || (h & 3) || (grad && (n & 3))) return GT_OK;
   if ((((uintptr_t)hidden) | ((uintptr_t)w) | ((uintptr_t)chunk)) & 15) return GT_OK;
   if (ctx->device < 0 || ctx->device >= 64 || !device_flag(ctx)) return GT_OK;
   const int kblocks = gt_cdiv(h, BK);
-  const long workers = ctx->sm_count - ctx->sm_reserved;
-  const long t1 = (long)gt_cdiv(n, 192) * gt_cdiv(rows, BM1), t2 = (long)gt_cdiv(n, 256) * gt_cdiv(rows, 2 * BM1);
-  // Spans with few tiles go through the product that cuts its contraction, and a pass that then finds them in L2.
-  if (2 * t1 < workers) return GT_OK;
-  // 128 x 192 tiles hide their epilogue, 256 x 256 ones move fewer bytes per product (choose_plan's cycle counts)
-  const double c1 = (double)gt_cdiv(t1, workers) * (kblocks * 0.92 * 2.0 * (BM1 + 192) + 1500.0);
-  const double c2 = (double)gt_cdiv(t2, workers) * (kblocks * 0.92 * (512.0 + 2.0 * (BM1 + 256)) + 14.0 * 256 + 900.0 + 1500.0);
-  int mt = c2 < c1 ? 2 : 1;
-  if (const char* force = getenv("GT_GEMM_TILE")) {
-    if (!strcmp(force, "1,192")) mt = 1;
-    else if (!strcmp(force, "2,256")) mt = 2;
-    else return GT_OK;
-  }
-  const int bn = mt == 2 ? 256 : 192, bm = mt * BM1;
+  const int npairs = pair_workers(ctx);
+  // Spans with few tiles go through the product that cuts its contraction, and a pass that then finds them in L2. The CTA
+  // pair hides most of this epilogue: 665 (statistics) and 763 us (gradient) at 8192 x 32768 x 1024, against 731 and 893 on
+  // 256-row tiles of one CTA.
+  const long tiles = (long)gt_cdiv(n, 256) * gt_cdiv(rows, 2 * BM1);
+  if (npairs < 8 || 2 * tiles < npairs) return GT_OK;
+  const char* force = getenv("GT_GEMM_TILE");
+  if (force && strcmp(force, "3,256")) return GT_OK;
   PartMaps maps;
   maps.nparts = maps.ngroups = 1;
-  if (!make_map_3d(&maps.a[0], hidden, h, rows, 1, h, (uint64_t)rows * h, bm, true) ||
-      !make_map_3d(&maps.b[0], w, h, n, 1, h, (uint64_t)n * h, bn, true))
+  if (!make_map_3d(&maps.a[0], hidden, h, rows, 1, h, (uint64_t)rows * h, BM1, true) ||
+      !make_map_3d(&maps.b[0], w, h, n, 1, h, (uint64_t)n * h, 128, true))
     return GT_OK;
   maps.c[0] = maps.a[0];
   if (grad && !make_map_3d(&maps.c[0], chunk, n, rows, 1, n, (uint64_t)rows * n, 32, true)) return GT_OK;
   maps.kb_end[0] = kblocks;
   maps.ce = ce;
-  *parts = gt_cdiv(n, bn) * (mt == 1 ? EpiSub<1, EPI_CE_STATS>::N : 1);
-  const long tiles = mt == 2 ? t2 : t1;
-  gt_status s;
-  if (grad) s = mt == 2 ? launch<true, true, 256, 2, EPI_CE_GRAD>(ctx, maps, tiles, 1, chunk, rows, n, 0, 1, 1, TRUNC_COMP)
-                        : launch<true, true, 192, 1, EPI_CE_GRAD>(ctx, maps, tiles, 1, chunk, rows, n, 0, 1, 1, TRUNC_COMP);
-  else s = mt == 2 ? launch<true, true, 256, 2, EPI_CE_STATS>(ctx, maps, tiles, 0, chunk, rows, n, 0, 1, 1, TRUNC_COMP)
-                   : launch<true, true, 192, 1, EPI_CE_STATS>(ctx, maps, tiles, 0, chunk, rows, n, 0, 1, 1, TRUNC_COMP);
+  *parts = gt_cdiv(n, 256) * PairSub<256, EPI_CE_STATS>::N;
+  gt_status s = grad ? launch_pair<true, true, 256, EPI_CE_GRAD>(ctx, maps, tiles, 1, chunk, rows, n, 0, 1, 1, npairs, TRUNC_COMP)
+                     : launch_pair<true, true, 256, EPI_CE_STATS>(ctx, maps, tiles, 0, chunk, rows, n, 0, 1, 1, npairs, TRUNC_COMP);
   if (s) return s;
   *handled = true;
   return GT_OK;
