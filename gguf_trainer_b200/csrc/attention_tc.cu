@@ -1130,7 +1130,7 @@ gt_status attn_dkv_order(gt_ctx* ctx, int nkb, int ntx, int group, int T, int NQ
 // tokens of 9/3 heads of 64 27.6 -> 14.3 us, 2 x 500 of 16/8 of 128 58 -> 35, 3 x 400 of 4/1 of 256 148 -> 45; at 8 x 2048
 // of 4/1 of 256 one CTA per tile stays ahead, 709 against 906.
 int dkv_head_split(gt_ctx* ctx, int Hkv, int group, int nseq, int T, int NQ, int window, int split) {
-  const char* force = getenv("GT_ATTN_HEAD_SPLIT");
+  const char* force = gt_env("GT_ATTN_HEAD_SPLIT");
   double total = 0.0, longest = 0.0;
   const int nkb = gt_cdiv(T, ROWS), tiles = nkb * Hkv * nseq;
   for (int kb = 0; kb < nkb; kb++) {
@@ -1187,7 +1187,7 @@ gt_status launch_bwd(gt_ctx* ctx, int rows, int T, int Hq, int Hkv, int window, 
     const int hs = dkv_head_split(ctx, Hkv, Hq / Hkv, nseq, T, NQ, window, SPLIT);
     dim3 grid(Hkv * nseq * SPLIT * hs, gt_cdiv(T, ROWS), 1);
     const int* order = nullptr;
-    if (SPLIT == 1 && hs == 1 && (int)(grid.x * grid.y) > ctx->sm_count && !getenv("GT_ATTN_INDEX_ORDER")) {   // (the variable keeps index order, for comparison)
+    if (SPLIT == 1 && hs == 1 && (int)(grid.x * grid.y) > ctx->sm_count && !gt_env("GT_ATTN_INDEX_ORDER")) {   // (the variable keeps index order, for comparison)
       st = attn_dkv_order(ctx, (int)grid.y, (int)grid.x, Hq / Hkv, T, NQ, window, &order);
       if (st) return st;
     }

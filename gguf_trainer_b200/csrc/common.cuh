@@ -8,11 +8,15 @@
 #include <unordered_map>
 #include <vector>
 
+#ifndef GT_QUEUE_FRONT
+#include "queue_names.h"
+#endif
 #include "../../include/gguftrain.h"
 
 struct GtAdamW;
 struct GtMuon;
 struct GtDp;
+struct GtQueue;      // launch queue (queue.cu)
 struct GtHostCopy;   // staging ring and copy threads of gt_read (ctx.cu)
 
 struct gt_ctx {
@@ -51,6 +55,7 @@ struct gt_ctx {
   // staging
   void* pinned = nullptr;
   uint64_t pinned_bytes = 0, pinned_cursor = 0;
+  GtQueue* queue = nullptr;
   GtHostCopy* host_copy = nullptr;
   int* flag_words = nullptr;   // pinned: the latched device words as gt_sync last saw them
   bool capturing = false;
@@ -69,6 +74,17 @@ struct gt_ctx {
   uint64_t next_ticket = 1;
 };
 
+// Waits until every queued op has been launched; the status of one that could not be, once. First statement of every entry
+// point that is not queued itself and touches the stream or what the ops keep in the context.
+gt_status gt_drain(gt_ctx* ctx);
+void gt_queue_destroy(gt_ctx* ctx);
+std::string& gt_error_text(gt_ctx* ctx);   // where a failing call of this thread leaves its message
+const char* gt_env(const char* name);      // getenv, but null on the thread that launches (the variables may change beside it)
+#define GT_DRAIN(ctx)                                                   \
+  do {                                                                  \
+    const gt_status _s = gt_drain(ctx);                                 \
+    if (_s) return _s;                                                  \
+  } while (0)
 gt_status gt_fail(gt_ctx* ctx, gt_status code, const char* fmt, ...);
 gt_status gt_check_cuda(gt_ctx* ctx, cudaError_t e, const char* what);
 // scratch of at least `bytes` (grows outside graph capture only)

@@ -108,7 +108,7 @@ gt_status gt_fail(gt_ctx* ctx, gt_status code, const char* fmt, ...) {
   va_start(ap, fmt);
   vsnprintf(buf, sizeof buf, fmt, ap);
   va_end(ap);
-  if (ctx) ctx->err = buf; else g_init_error = buf;
+  if (ctx) gt_error_text(ctx) = buf; else g_init_error = buf;
   return code;
 }
 
@@ -169,6 +169,8 @@ gt_status gt_init(int32_t device, gt_ctx** out) {
 
 gt_status gt_destroy(gt_ctx* ctx) {
   if (!ctx) return GT_OK;
+  gt_drain(ctx);
+  gt_queue_destroy(ctx);
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
   gt_dp_teardown(ctx);
@@ -207,6 +209,7 @@ gt_status gt_device_name(gt_ctx* ctx, char* out, int32_t cap) {
 }
 
 gt_status gt_set_precision(gt_ctx* ctx, int32_t mode) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, mode >= GT_PREC_FP32 && mode <= GT_PREC_BF16, "gt_set_precision: unknown mode %d", mode);
   if (mode == GT_PREC_BF16)
     return gt_fail(ctx, GT_ERR_UNSUPPORTED, "gt_set_precision: there are no BF16 kernels in this library (a single BF16 product is 1.6e-3 off in "
@@ -216,6 +219,7 @@ gt_status gt_set_precision(gt_ctx* ctx, int32_t mode) {
 }
 
 gt_status gt_set_batch(gt_ctx* ctx, int32_t batch, int32_t seq_len) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, batch >= 0 && (batch == 0 || seq_len > 0), "gt_set_batch: batch %d seq_len %d", batch, seq_len);
   ctx->batch = batch;
   ctx->seq_len = batch ? seq_len : 0;
@@ -248,6 +252,7 @@ gt_status gt_alloc(gt_ctx* ctx, uint64_t bytes, gt_buf* out) {
 }
 
 gt_status gt_alloc_state(gt_ctx* ctx, uint64_t bytes, gt_buf* out) {
+  GT_DRAIN(ctx);
   if (ctx->capturing) return gt_fail(ctx, GT_ERR_STATE, "gt_alloc_state inside a graph capture");
   uint64_t size = bucket(bytes);
   void* p = nullptr;
@@ -270,6 +275,7 @@ gt_status gt_free(gt_ctx* ctx, gt_buf buf) {
     auto st = ctx->state.find(p);
     if (st == ctx->state.end()) return gt_fail(ctx, GT_ERR_ARG, "gt_free: %p is not a live allocation of this context", p);
     // state buffers are not pooled; stream order makes the free safe
+    GT_DRAIN(ctx);
     GT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     cudaFree(p);
     ctx->state_bytes -= st->second;
@@ -325,6 +331,7 @@ gt_status gt_write(gt_ctx* ctx, gt_buf dst, const void* host, uint64_t bytes) {
 gt_status gt_read(gt_ctx* ctx, gt_buf src, void* host, uint64_t bytes) { return gt_read_many(ctx, 1, &src, &host, &bytes); }
 
 gt_status gt_read_many(gt_ctx* ctx, int32_t n, const gt_buf* srcs, void* const* hosts, const uint64_t* sizes) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, n >= 0 && (n == 0 || (srcs && hosts && sizes)), "gt_read_many: null argument");
   uint64_t total = 0;
   for (int i = 0; i < n; i++) {
@@ -407,6 +414,7 @@ gt_status gt_copy(gt_ctx* ctx, gt_buf dst, gt_buf src, uint64_t bytes) {
 }
 
 gt_status gt_sync(gt_ctx* ctx) {
+  GT_DRAIN(ctx);
   if (ctx->capturing) return gt_fail(ctx, GT_ERR_STATE, "gt_sync inside a graph capture");
   // the latched words ride on the same wait
   if (!ctx->flag_words) GT_CUDA(ctx, cudaMallocHost(&ctx->flag_words, 2 * sizeof(int)));
@@ -440,6 +448,7 @@ static gt_status copy_stream_ready(gt_ctx* ctx) {
 }
 
 gt_status gt_read_async(gt_ctx* ctx, gt_buf src, uint64_t bytes, uint64_t* out_ticket) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, src && bytes > 0 && out_ticket, "gt_read_async: null argument");
   if (ctx->capturing) return gt_fail(ctx, GT_ERR_STATE, "gt_read_async inside a graph capture");
   gt_status s = copy_stream_ready(ctx);
@@ -470,6 +479,7 @@ gt_status gt_read_async(gt_ctx* ctx, gt_buf src, uint64_t bytes, uint64_t* out_t
 }
 
 gt_status gt_read_fence(gt_ctx* ctx) {
+  GT_DRAIN(ctx);
   if (!ctx->copy_pending) return GT_OK;
   if (ctx->capturing) return gt_fail(ctx, GT_ERR_STATE, "gt_read_fence inside a graph capture");
   GT_CUDA(ctx, cudaEventRecord(ctx->copy_done, ctx->copy_stream));
@@ -479,6 +489,7 @@ gt_status gt_read_fence(gt_ctx* ctx) {
 }
 
 gt_status gt_read_finish(gt_ctx* ctx, uint64_t ticket, void* host, uint64_t bytes) {
+  GT_DRAIN(ctx);
   auto it = ctx->async_reads.find(ticket);
   if (it == ctx->async_reads.end()) return gt_fail(ctx, GT_ERR_ARG, "gt_read_finish: unknown ticket %llu", (unsigned long long)ticket);
   GT_REQUIRE(ctx, host && bytes <= it->second.bytes, "gt_read_finish: %llu bytes asked of a %llu-byte read", (unsigned long long)bytes,
@@ -493,6 +504,7 @@ gt_status gt_read_finish(gt_ctx* ctx, uint64_t ticket, void* host, uint64_t byte
 }
 
 gt_status gt_stats(gt_ctx* ctx, uint64_t* out4) {
+  GT_DRAIN(ctx);
   out4[0] = ctx->pool_bytes;
   out4[1] = ctx->state_bytes;
   out4[2] = ctx->readback_bytes;
@@ -502,6 +514,7 @@ gt_status gt_stats(gt_ctx* ctx, uint64_t* out4) {
 
 // ---- graphs ----
 gt_status gt_graph_begin(gt_ctx* ctx) {
+  GT_DRAIN(ctx);
   if (ctx->capturing) return gt_fail(ctx, GT_ERR_STATE, "gt_graph_begin: already capturing");
   GT_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   ctx->capturing = true;
@@ -509,6 +522,7 @@ gt_status gt_graph_begin(gt_ctx* ctx) {
 }
 
 gt_status gt_graph_end(gt_ctx* ctx, uint64_t* out_graph) {
+  GT_DRAIN(ctx);
   if (!ctx->capturing) return gt_fail(ctx, GT_ERR_STATE, "gt_graph_end: not capturing");
   ctx->capturing = false;
   cudaGraph_t g = nullptr;
@@ -523,12 +537,14 @@ gt_status gt_graph_end(gt_ctx* ctx, uint64_t* out_graph) {
 }
 
 gt_status gt_graph_launch(gt_ctx* ctx, uint64_t graph) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, graph >= 1 && graph <= ctx->graphs.size() && ctx->graphs[graph - 1], "gt_graph_launch: bad handle %llu", (unsigned long long)graph);
   GT_CUDA(ctx, cudaGraphLaunch(ctx->graphs[graph - 1], ctx->stream));
   return GT_OK;
 }
 
 gt_status gt_graph_destroy(gt_ctx* ctx, uint64_t graph) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, graph >= 1 && graph <= ctx->graphs.size() && ctx->graphs[graph - 1], "gt_graph_destroy: bad handle %llu", (unsigned long long)graph);
   GT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   cudaGraphExecDestroy(ctx->graphs[graph - 1]);
@@ -538,6 +554,7 @@ gt_status gt_graph_destroy(gt_ctx* ctx, uint64_t graph) {
 
 // ---- events ----
 gt_status gt_event_record(gt_ctx* ctx, int32_t slot) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, slot >= 0 && slot < 64, "gt_event_record: slot %d", slot);
   if (!ctx->events[slot]) GT_CUDA(ctx, cudaEventCreate(&ctx->events[slot]));
   GT_CUDA(ctx, cudaEventRecord(ctx->events[slot], ctx->stream));
@@ -545,6 +562,7 @@ gt_status gt_event_record(gt_ctx* ctx, int32_t slot) {
 }
 
 gt_status gt_event_elapsed_ms(gt_ctx* ctx, int32_t a, int32_t b, float* ms) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, a >= 0 && a < 64 && b >= 0 && b < 64 && ctx->events[a] && ctx->events[b], "gt_event_elapsed_ms: slots %d,%d not recorded", a, b);
   GT_CUDA(ctx, cudaEventSynchronize(ctx->events[b]));
   GT_CUDA(ctx, cudaEventElapsedTime(ms, ctx->events[a], ctx->events[b]));

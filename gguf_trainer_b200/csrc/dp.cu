@@ -90,6 +90,7 @@ gt_status gt_dp_unique_id(uint8_t* out128) {
 }
 
 gt_status gt_dp_init(gt_ctx* ctx, int32_t rank, int32_t world, const uint8_t* id128) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, world >= 1 && rank >= 0 && rank < world && id128, "gt_dp_init: rank %d of %d", rank, world);
   if (ctx->dp) return gt_fail(ctx, GT_ERR_STATE, "gt_dp_init: already initialised");
   if (!load_nccl()) return gt_fail(ctx, GT_ERR_NCCL, "%s", g_nccl_err.c_str());
@@ -108,6 +109,7 @@ gt_status gt_dp_init(gt_ctx* ctx, int32_t rank, int32_t world, const uint8_t* id
 }
 
 gt_status gt_dp_allreduce_start(gt_ctx* ctx, gt_buf buf, uint64_t count) {
+  GT_DRAIN(ctx);
   GtDp* d = ctx->dp;
   if (!d) return gt_fail(ctx, GT_ERR_STATE, "gt_dp_allreduce_start: gt_dp_init has not run");
   if (!d->comm) return gt_fail(ctx, GT_ERR_NCCL, "gt_dp_allreduce_start: the communicator was aborted; gt_dp_destroy and gt_dp_init again");
@@ -122,6 +124,7 @@ gt_status gt_dp_allreduce_start(gt_ctx* ctx, gt_buf buf, uint64_t count) {
 }
 
 gt_status gt_dp_wait(gt_ctx* ctx) {
+  GT_DRAIN(ctx);
   GtDp* d = ctx->dp;
   if (!d) return gt_fail(ctx, GT_ERR_STATE, "gt_dp_wait: gt_dp_init has not run");
   if (!d->pending) return GT_OK;
@@ -140,6 +143,7 @@ gt_status gt_dp_wait(gt_ctx* ctx) {
 // otherwise wait for the missing rank for ever) and the status is GT_ERR_NCCL; the context itself stays usable for
 // single-GPU work and gt_dp_init may be called again after gt_dp_destroy.
 gt_status gt_dp_wait_host(gt_ctx* ctx, int32_t timeout_ms) {
+  GT_DRAIN(ctx);
   GtDp* d = ctx->dp;
   if (!d) return gt_fail(ctx, GT_ERR_STATE, "gt_dp_wait_host: gt_dp_init has not run");
   GT_REQUIRE(ctx, timeout_ms > 0, "gt_dp_wait_host: timeout %d ms", timeout_ms);
@@ -176,12 +180,14 @@ gt_status gt_dp_wait_host(gt_ctx* ctx, int32_t timeout_ms) {
 // per SM of the whole device then has CTAs that only start when others finish: its last wave doubles. Reserving those
 // SMs makes the persistent matrix-product kernels size their grids (and choose their tiles) for what is left.
 gt_status gt_dp_reserve_sms(gt_ctx* ctx, int32_t n) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, n >= 0 && n < ctx->sm_count, "gt_dp_reserve_sms: %d of %d SMs", n, ctx->sm_count);
   ctx->sm_reserved = n;
   return GT_OK;
 }
 
 gt_status gt_dp_destroy(gt_ctx* ctx) {
+  GT_DRAIN(ctx);
   gt_dp_teardown(ctx);
   return GT_OK;
 }

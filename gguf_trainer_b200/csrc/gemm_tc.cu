@@ -872,7 +872,7 @@ int cluster_room(gt_ctx* ctx, int c) {
       n = 0;
     }
     r = n > 0 ? n * c : c;
-    if (getenv("GT_GEMM_TILE")) fprintf(stderr, "[gguftrain] resident CTAs in clusters of %d: %d\n", c, r);
+    if (gt_env("GT_GEMM_TILE")) fprintf(stderr, "[gguftrain] resident CTAs in clusters of %d: %d\n", c, r);
   }
   return r;
 }
@@ -974,7 +974,7 @@ int pair_capacity(gt_ctx* ctx) {
     }
     cap[ctx->device] = n;
     known[ctx->device] = true;
-    if (getenv("GT_GEMM_TILE")) fprintf(stderr, "[gguftrain] resident CTA pairs: %d\n", n);
+    if (gt_env("GT_GEMM_TILE")) fprintf(stderr, "[gguftrain] resident CTA pairs: %d\n", n);
   }
   return cap[ctx->device];
 }
@@ -1106,6 +1106,7 @@ __global__ void bounded_wait_selftest_kernel(unsigned long long limit_ns, int* _
 }
 
 extern "C" gt_status gt_selftest_bounded_wait(gt_ctx* ctx, int32_t limit_us) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, limit_us >= 1 && limit_us <= 1000000, "gt_selftest_bounded_wait: limit %d us (1..1000000)", limit_us);
   if (ctx->capturing) return gt_fail(ctx, GT_ERR_STATE, "gt_selftest_bounded_wait inside a graph capture");
   int* flag = device_flag(ctx);
@@ -1208,8 +1209,8 @@ static gt_status gemm_tc_dispatch(gt_ctx* ctx, int kind, int accum, int M, int N
   }
   if (ctx->device < 0 || ctx->device >= 64) return GT_OK;
   if (!device_flag(ctx)) return GT_OK;
-  const char* force = getenv("GT_GEMM_TILE");   // "mt,bn": forces one tile shape (read per call so tests can switch it); mt 0: one tile per CTA
-  const char* ds = getenv("GT_GEMM_DEEP_SPLIT");   // "0": never cut a product that already fills the SMs along K (for comparison)
+  const char* force = gt_env("GT_GEMM_TILE");   // "mt,bn": forces one tile shape (read per call so tests can switch it); mt 0: one tile per CTA
+  const char* ds = gt_env("GT_GEMM_DEEP_SPLIT");   // "0": never cut a product that already fills the SMs along K (for comparison)
   // the choice is made once per shape
   Plan plan;
   PlanKey key = {{kind, accum ? 1 : 0, M, N, batch, ctx->device, ctx->sm_reserved, nparts}};
@@ -1342,7 +1343,7 @@ static gt_status gemm_tc_grouped(gt_ctx* ctx, int kind, int ngroups, const int* 
   }
   if (ctx->device < 0 || ctx->device >= 64 || !device_flag(ctx)) return GT_OK;
   const int kblocks = gt_cdiv(K, BK);
-  const char* force = getenv("GT_GEMM_TILE");
+  const char* force = gt_env("GT_GEMM_TILE");
   GroupKey key = {{kind, K, ngroups, any_rope ? 1 : 0, ctx->device, ctx->sm_reserved}};
   for (int g = 0; g < ngroups; g++) { key.v[6 + 3 * g] = Ms[g]; key.v[7 + 3 * g] = Ns[g]; key.v[8 + 3 * g] = accums[g] ? 1 : 0; }
   auto& plans = group_cache();
@@ -1433,7 +1434,7 @@ gt_status gt_glu_linear_tc(gt_ctx* ctx, int op, int rows, int ffn, int in, const
   bool pair = cost_pair < cost;
   cost = min(cost, cost_pair);
   const SmallPick small = pick_small(ctx, GT_GEMM_NT, kblocks, [&](int b) { return (long)gt_cdiv(ffn, b / 2) * gt_cdiv(rows, BM1); }, 32);
-  const char* force = getenv("GT_GEMM_TILE");
+  const char* force = gt_env("GT_GEMM_TILE");
   if (small.bn && small.cost < cost && (!force || force[0] == '0')) {
     const int bn = small.bn;
     if (!make_map_3d(&maps.a[0], x, in, rows, 1, in, (uint64_t)rows * in, BM1, true) ||
@@ -1500,7 +1501,7 @@ gt_status gt_readout_tc(gt_ctx* ctx, bool grad, int rows, int n, int h, const fl
   // 256-row tiles of one CTA.
   const long tiles = (long)gt_cdiv(n, 256) * gt_cdiv(rows, 2 * BM1);
   if (npairs < 8 || 2 * tiles < npairs) return GT_OK;
-  const char* force = getenv("GT_GEMM_TILE");
+  const char* force = gt_env("GT_GEMM_TILE");
   if (force && strcmp(force, "3,256")) return GT_OK;
   PartMaps maps;
   maps.nparts = maps.ngroups = 1;

@@ -46,6 +46,7 @@ __global__ void token_max_kernel(const TOK* __restrict__ tokens, unsigned long l
 extern "C" {
 
 gt_status gt_tokens_max(gt_ctx* ctx, gt_buf tokens, int32_t bytes_per_token, uint64_t count, uint32_t* out_max) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, tokens && out_max && count > 0 && (bytes_per_token == 2 || bytes_per_token == 4),
              "gt_tokens_max: tokens %p count %llu bytes_per_token %d (2 or 4)", gt_ptr<void>(tokens), (unsigned long long)count, bytes_per_token);
   if (ctx->capturing) return gt_fail(ctx, GT_ERR_STATE, "gt_tokens_max inside a graph capture");
@@ -64,6 +65,7 @@ gt_status gt_tokens_max(gt_ctx* ctx, gt_buf tokens, int32_t bytes_per_token, uin
 
 gt_status gt_gather_windows(gt_ctx* ctx, gt_buf tokens, gt_buf mask, int32_t bytes_per_token, uint64_t count, gt_buf starts,
                             int32_t B, int32_t T, gt_buf ids, gt_buf targets) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, tokens && starts && ids && targets, "gt_gather_windows: null operand");
   GT_REQUIRE(ctx, B > 0 && T > 0 && (bytes_per_token == 2 || bytes_per_token == 4) && count >= (uint64_t)T + 1,
              "gt_gather_windows: B %d T %d bytes_per_token %d corpus %llu tokens (a window needs T+1)", B, T, bytes_per_token,

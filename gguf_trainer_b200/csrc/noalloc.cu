@@ -31,6 +31,7 @@ extern "C" gt_status gt_attention_bwd_static(gt_ctx* ctx, int32_t rows, int32_t 
                                              gt_buf q, gt_buf k, gt_buf v, gt_buf out, gt_buf lse, gt_buf gout, gt_buf gq,
                                              int32_t accum_q, gt_buf gk, int32_t accum_k, gt_buf gv, int32_t accum_v) {
   if (!ctx) return gt_fail(nullptr, GT_ERR_ARG, "gt_attention_bwd_static: null context");
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, rows > 0 && Hq > 0 && Hkv > 0 && hd > 0 && hd <= 256 && window >= 0,
              "gt_attention_bwd_static: rows %d Hq %d Hkv %d hd %d window %d (hd must be in 1..256)", rows, Hq, Hkv, hd, window);
   GT_REQUIRE(ctx, Hq % Hkv == 0, "gt_attention_bwd_static: %d KV heads do not divide %d query heads", Hkv, Hq);

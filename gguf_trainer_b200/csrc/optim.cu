@@ -363,6 +363,7 @@ extern "C" {
 
 gt_status gt_adamw_create(gt_ctx* ctx, int32_t n, const gt_buf* data, const gt_buf* grad, const uint64_t* sizes, float lr,
                           float beta1, float beta2, float eps, float weight_decay, float clip, uint64_t* out_handle) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, n >= 0 && out_handle, "gt_adamw_create: bad argument");
   if (ctx->capturing) return gt_fail(ctx, GT_ERR_STATE, "gt_adamw_create inside a graph capture");
   GtAdamW* a = new GtAdamW();
@@ -417,6 +418,7 @@ static GtAdamW* adamw_of(gt_ctx* ctx, uint64_t h) {
 }
 
 gt_status gt_adamw_set_lr(gt_ctx* ctx, uint64_t h, float lr) {
+  GT_DRAIN(ctx);
   GtAdamW* a = adamw_of(ctx, h);
   GT_REQUIRE(ctx, a, "gt_adamw_set_lr: bad handle");
   a->lr = lr;
@@ -424,6 +426,7 @@ gt_status gt_adamw_set_lr(gt_ctx* ctx, uint64_t h, float lr) {
 }
 
 gt_status gt_adamw_step(gt_ctx* ctx, uint64_t h) {
+  GT_DRAIN(ctx);
   GtAdamW* a = adamw_of(ctx, h);
   GT_REQUIRE(ctx, a, "gt_adamw_step: bad handle");
   a->t += 1;
@@ -446,6 +449,7 @@ gt_status gt_adamw_step(gt_ctx* ctx, uint64_t h) {
 }
 
 gt_status gt_adamw_state(gt_ctx* ctx, uint64_t h, int32_t i, gt_buf* m, gt_buf* v) {
+  GT_DRAIN(ctx);
   GtAdamW* a = adamw_of(ctx, h);
   GT_REQUIRE(ctx, a && i >= 0 && i < a->n, "gt_adamw_state: bad handle or index");
   *m = (gt_buf)(uintptr_t)a->m[i];
@@ -453,12 +457,14 @@ gt_status gt_adamw_state(gt_ctx* ctx, uint64_t h, int32_t i, gt_buf* m, gt_buf* 
   return GT_OK;
 }
 gt_status gt_adamw_get_t(gt_ctx* ctx, uint64_t h, int32_t* t) {
+  GT_DRAIN(ctx);
   GtAdamW* a = adamw_of(ctx, h);
   GT_REQUIRE(ctx, a, "gt_adamw_get_t: bad handle");
   *t = a->t;
   return GT_OK;
 }
 gt_status gt_adamw_set_t(gt_ctx* ctx, uint64_t h, int32_t t) {
+  GT_DRAIN(ctx);
   GtAdamW* a = adamw_of(ctx, h);
   GT_REQUIRE(ctx, a && t >= 0, "gt_adamw_set_t: bad handle or step");
   a->t = t;
@@ -467,6 +473,7 @@ gt_status gt_adamw_set_t(gt_ctx* ctx, uint64_t h, int32_t t) {
 
 gt_status gt_muon_create(gt_ctx* ctx, int32_t n, const gt_buf* data, const gt_buf* grad, const int32_t* rows, const int32_t* cols,
                          float lr, float momentum, int32_t nesterov, int32_t ns_steps, uint64_t* out_handle) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, n >= 0 && out_handle && ns_steps >= 0, "gt_muon_create: bad argument");
   if (ctx->capturing) return gt_fail(ctx, GT_ERR_STATE, "gt_muon_create inside a graph capture");
   GtMuon* m = new GtMuon();
@@ -526,6 +533,7 @@ static GtMuon* muon_of(gt_ctx* ctx, uint64_t h) {
 }
 
 gt_status gt_muon_set_lr(gt_ctx* ctx, uint64_t h, float lr) {
+  GT_DRAIN(ctx);
   GtMuon* m = muon_of(ctx, h);
   GT_REQUIRE(ctx, m, "gt_muon_set_lr: bad handle");
   m->lr = lr;
@@ -538,6 +546,7 @@ gt_status gt_muon_set_lr(gt_ctx* ctx, uint64_t h, float lr) {
 // products cost 1/world per rank; momentum and the apply pass stay replicated (they are what keeps state and weights
 // identical everywhere). The group's two iteration buffers are re-made with room for world*slice matrices.
 gt_status gt_muon_set_sharded(gt_ctx* ctx, uint64_t h, int32_t on) {
+  GT_DRAIN(ctx);
   GtMuon* m = muon_of(ctx, h);
   GT_REQUIRE(ctx, m, "gt_muon_set_sharded: bad handle");
   if (ctx->capturing) return gt_fail(ctx, GT_ERR_STATE, "gt_muon_set_sharded inside a graph capture");
@@ -564,6 +573,7 @@ gt_status gt_muon_set_sharded(gt_ctx* ctx, uint64_t h, int32_t on) {
 }
 
 gt_status gt_muon_step(gt_ctx* ctx, uint64_t h) {
+  GT_DRAIN(ctx);
   GtMuon* m = muon_of(ctx, h);
   GT_REQUIRE(ctx, m, "gt_muon_step: bad handle");
   int dp_rank = 0, dp_world = 1;
@@ -652,6 +662,7 @@ gt_status gt_muon_step(gt_ctx* ctx, uint64_t h) {
 }
 
 gt_status gt_muon_state(gt_ctx* ctx, uint64_t h, int32_t i, gt_buf* momentum) {
+  GT_DRAIN(ctx);
   GtMuon* m = muon_of(ctx, h);
   GT_REQUIRE(ctx, m && i >= 0 && i < m->n, "gt_muon_state: bad handle or index");
   *momentum = (gt_buf)(uintptr_t)m->buf[i];
@@ -659,6 +670,7 @@ gt_status gt_muon_state(gt_ctx* ctx, uint64_t h, int32_t i, gt_buf* momentum) {
 }
 
 gt_status gt_newton_schulz(gt_ctx* ctx, int32_t mm, int32_t nn, int32_t steps, gt_buf g, gt_buf out) {
+  GT_DRAIN(ctx);
   GT_REQUIRE(ctx, mm > 0 && nn > 0 && steps >= 0 && g && out, "gt_newton_schulz: bad argument");
   if (ctx->capturing) return gt_fail(ctx, GT_ERR_STATE, "gt_newton_schulz inside a graph capture");
   const size_t el = (size_t)mm * nn;
