@@ -66,5 +66,16 @@ def load():
         fn = getattr(lib, name)
         fn.restype = C.c_char_p if ret.startswith("const char") else C.c_int32
         fn.argtypes = [_TYPES[t] for t in types]
+    # The ops a training or decoding loop calls thousands of times a second, without ctypes' conversion of their arguments
+    # (built with the library; an interpreter of another version keeps the ctypes functions).
+    try:
+        from . import _calls
+    except ImportError:
+        pass
+    else:
+        names = [n for n in dir(_calls) if n.startswith("gt_")]
+        _calls.bind(lib._handle, {n: getattr(lib, n) for n in names})
+        for n in names:
+            setattr(lib, n, getattr(_calls, n))
     _lib = lib
     return lib

@@ -5,9 +5,11 @@ Usage: python build.py [--force] [--verbose]   (also imported by __graft_entry__
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 OUT = os.path.join(HERE, "libgguftrain_cuda.so")
+CALLS = os.path.join(HERE, "..", "_calls" + sysconfig.get_config_var("EXT_SUFFIX"))   # CPython functions of the hot entry points
 SOURCES = ["ctx.cu", "gemm_simt.cu", "gemm_tc.cu", "elementwise.cu", "norm.cu", "rope_embed.cu", "attention.cu",
            "attention_simt.cu", "attention_tc.cu", "loss.cu", "optim.cu", "dp.cu", "noalloc.cu", "ingest.cu", "queue.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
@@ -21,10 +23,10 @@ def sources():
 
 
 def stale():
-    if not os.path.exists(OUT):
+    if not os.path.exists(OUT) or not os.path.exists(CALLS):
         return True
-    t = os.path.getmtime(OUT)
-    deps = sources() + ["common.cuh", "queue_names.h", "../../include/gguftrain.h", "build.py"] + \
+    t = min(os.path.getmtime(OUT), os.path.getmtime(CALLS))
+    deps = sources() + ["common.cuh", "queue_names.h", "pycalls.cpp", "../../include/gguftrain.h", "build.py"] + \
         [f for f in os.listdir(HERE) if f.endswith(".cuh")]
     return any(os.path.getmtime(os.path.join(HERE, d)) > t for d in deps)
 
@@ -39,13 +41,16 @@ def build(force=False, verbose=False):
         o = os.path.join(HERE, "build", s.replace(".cu", ".o"))
         objs.append(o)
         src = os.path.join(HERE, s)
-        hdr_t = max(os.path.getmtime(os.path.join(HERE, h)) for h in os.listdir(HERE) if h.endswith(".cuh"))
+        hdr_t = max(os.path.getmtime(os.path.join(HERE, h)) for h in os.listdir(HERE) if h.endswith((".cuh", ".h")))
         hdr_t = max(hdr_t, os.path.getmtime(os.path.join(HERE, "../../include/gguftrain.h")))
         if not force and os.path.exists(o) and os.path.getmtime(o) > max(os.path.getmtime(src), hdr_t):
             continue
         cmd = [NVCC] + [f for f in FLAGS if f != "--use_fast_math=false"] + (["-Xptxas", "-v"] if verbose else []) + \
             ["-c", src, "-o", o]
         procs.append((s, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"],
+           os.path.join(HERE, "pycalls.cpp"), "-o", CALLS, "-ldl"]
+    procs.append(("pycalls.cpp", subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     failed = False
     for s, p in procs:
         out, _ = p.communicate()
@@ -53,7 +58,7 @@ def build(force=False, verbose=False):
             sys.stderr.write(f"--- {s} ---\n{out}\n")
         failed |= p.returncode != 0
     if failed:
-        raise RuntimeError("nvcc failed")
+        raise RuntimeError("compilation failed")
     subprocess.check_call([NVCC, "-shared", "-o", OUT] + objs + ["-ldl"])
     return OUT
 

@@ -3,7 +3,8 @@
 // A launch costs the host 4 to 5 us in the driver, and the code that records the ops (a training loop outside a graph,
 // scoring, decoding) spends about as long again on each of them. Done by one thread the two add up, and at model sizes
 // where a kernel takes 5 us that sum is what a step takes; on two threads the longer of them is.
-//   Recording 30 layers of 576 for 4 tokens of decoding 12.6 -> 8.1 ms, two sequences of 512 scored 3.1 -> 1.9 ms.
+// Measured: 4 tokens decoded by 30 layers of 576 13.1 -> 9.9 ms, two sequences of 512 scored by 15 layers 3.1 -> 2.4 ms, a
+// loop over micro-batches of a tiny model 7.4 -> 5.7 ms.
 //
 // What the public names of these ops do: check the arguments, copy them (arrays included) into a ring of records and
 // return. Every other entry point waits for the ring to be empty first (gt_drain), so reads, waits, graph recordings and
@@ -169,180 +170,180 @@ bool aligned(A... a) { return ((a | ...) & 15) == 0; }
   return s_ ? s_ : __VA_ARGS__
 
 extern "C" {
-decltype(gt_gemm) gt_gemm_now;
-decltype(gt_gemm_scaled) gt_gemm_scaled_now;
-decltype(gt_gemm2) gt_gemm2_now;
-decltype(gt_ew_fwd) gt_ew_fwd_now;
-decltype(gt_ew_bwd) gt_ew_bwd_now;
-decltype(gt_glu_fwd) gt_glu_fwd_now;
-decltype(gt_glu_linear_fwd) gt_glu_linear_fwd_now;
-decltype(gt_glu_bwd) gt_glu_bwd_now;
-decltype(gt_rmsnorm_fwd) gt_rmsnorm_fwd_now;
-decltype(gt_add_rmsnorm_fwd) gt_add_rmsnorm_fwd_now;
-decltype(gt_rmsnorm_heads_rope_fwd) gt_rmsnorm_heads_rope_fwd_now;
-decltype(gt_rmsnorm_bwd) gt_rmsnorm_bwd_now;
-decltype(gt_rmsnorm_bwd_add) gt_rmsnorm_bwd_add_now;
-decltype(gt_embedding_fwd) gt_embedding_fwd_now;
-decltype(gt_embedding_bwd) gt_embedding_bwd_now;
-decltype(gt_rope_fwd) gt_rope_fwd_now;
-decltype(gt_rope_bwd) gt_rope_bwd_now;
-decltype(gt_attention_fwd) gt_attention_fwd_now;
-decltype(gt_attention_bwd) gt_attention_bwd_now;
-decltype(gt_attention_bwd_rope) gt_attention_bwd_rope_now;
-decltype(gt_ce_fwd) gt_ce_fwd_now;
-decltype(gt_ce_bwd) gt_ce_bwd_now;
-decltype(gt_ce_chunk_stats) gt_ce_chunk_stats_now;
-decltype(gt_ce_loss_from_stats) gt_ce_loss_from_stats_now;
-decltype(gt_ce_chunk_grad) gt_ce_chunk_grad_now;
-decltype(gt_readout_ce_stats) gt_readout_ce_stats_now;
-decltype(gt_readout_ce_grad) gt_readout_ce_grad_now;
-decltype(gt_soft_ce_fwd) gt_soft_ce_fwd_now;
-decltype(gt_soft_ce_bwd) gt_soft_ce_bwd_now;
-decltype(gt_zero) gt_zero_now;
-decltype(gt_copy) gt_copy_now;
-decltype(gt_gemm_multi) gt_gemm_multi_now;
-decltype(gt_gemm_grouped) gt_gemm_grouped_now;
-decltype(gt_gemm_grouped_scaled) gt_gemm_grouped_scaled_now;
-decltype(gt_linear_rope_grouped) gt_linear_rope_grouped_now;
-decltype(gt_write) gt_write_now;
+decltype(gt_gemm) now_gt_gemm;
+decltype(gt_gemm_scaled) now_gt_gemm_scaled;
+decltype(gt_gemm2) now_gt_gemm2;
+decltype(gt_ew_fwd) now_gt_ew_fwd;
+decltype(gt_ew_bwd) now_gt_ew_bwd;
+decltype(gt_glu_fwd) now_gt_glu_fwd;
+decltype(gt_glu_linear_fwd) now_gt_glu_linear_fwd;
+decltype(gt_glu_bwd) now_gt_glu_bwd;
+decltype(gt_rmsnorm_fwd) now_gt_rmsnorm_fwd;
+decltype(gt_add_rmsnorm_fwd) now_gt_add_rmsnorm_fwd;
+decltype(gt_rmsnorm_heads_rope_fwd) now_gt_rmsnorm_heads_rope_fwd;
+decltype(gt_rmsnorm_bwd) now_gt_rmsnorm_bwd;
+decltype(gt_rmsnorm_bwd_add) now_gt_rmsnorm_bwd_add;
+decltype(gt_embedding_fwd) now_gt_embedding_fwd;
+decltype(gt_embedding_bwd) now_gt_embedding_bwd;
+decltype(gt_rope_fwd) now_gt_rope_fwd;
+decltype(gt_rope_bwd) now_gt_rope_bwd;
+decltype(gt_attention_fwd) now_gt_attention_fwd;
+decltype(gt_attention_bwd) now_gt_attention_bwd;
+decltype(gt_attention_bwd_rope) now_gt_attention_bwd_rope;
+decltype(gt_ce_fwd) now_gt_ce_fwd;
+decltype(gt_ce_bwd) now_gt_ce_bwd;
+decltype(gt_ce_chunk_stats) now_gt_ce_chunk_stats;
+decltype(gt_ce_loss_from_stats) now_gt_ce_loss_from_stats;
+decltype(gt_ce_chunk_grad) now_gt_ce_chunk_grad;
+decltype(gt_readout_ce_stats) now_gt_readout_ce_stats;
+decltype(gt_readout_ce_grad) now_gt_readout_ce_grad;
+decltype(gt_soft_ce_fwd) now_gt_soft_ce_fwd;
+decltype(gt_soft_ce_bwd) now_gt_soft_ce_bwd;
+decltype(gt_zero) now_gt_zero;
+decltype(gt_copy) now_gt_copy;
+decltype(gt_gemm_multi) now_gt_gemm_multi;
+decltype(gt_gemm_grouped) now_gt_gemm_grouped;
+decltype(gt_gemm_grouped_scaled) now_gt_gemm_grouped_scaled;
+decltype(gt_linear_rope_grouped) now_gt_linear_rope_grouped;
+decltype(gt_write) now_gt_write;
 
 gt_status gt_gemm(gt_ctx* ctx, int32_t kind, int32_t accum, int32_t M, int32_t N, int32_t K, gt_buf a, gt_buf b, gt_buf c) {
-  GT_QUEUED(ctx, M > 0 && N > 0 && K > 0 && a && b && c, gt_gemm_now(ctx, kind, accum, M, N, K, a, b, c));
+  GT_QUEUED(ctx, M > 0 && N > 0 && K > 0 && a && b && c, now_gt_gemm(ctx, kind, accum, M, N, K, a, b, c));
 }
 gt_status gt_gemm_scaled(gt_ctx* ctx, int32_t kind, int32_t accum, int32_t M, int32_t N, int32_t K, gt_buf a, gt_buf b, gt_buf c,
             float alpha) {
-  GT_QUEUED(ctx, M > 0 && N > 0 && K > 0 && a && b && c, gt_gemm_scaled_now(ctx, kind, accum, M, N, K, a, b, c, alpha));
+  GT_QUEUED(ctx, M > 0 && N > 0 && K > 0 && a && b && c, now_gt_gemm_scaled(ctx, kind, accum, M, N, K, a, b, c, alpha));
 }
 gt_status gt_gemm2(gt_ctx* ctx, int32_t kind, int32_t accum, int32_t M, int32_t N, int32_t K, gt_buf a, gt_buf b, int32_t K2, gt_buf a2,
             gt_buf b2, gt_buf c) {
-  GT_QUEUED(ctx, M > 0 && N > 0 && K > 0 && K2 > 0 && a && b && a2 && b2 && c, gt_gemm2_now(ctx, kind, accum, M, N, K, a, b, K2, a2, b2,
+  GT_QUEUED(ctx, M > 0 && N > 0 && K > 0 && K2 > 0 && a && b && a2 && b2 && c, now_gt_gemm2(ctx, kind, accum, M, N, K, a, b, K2, a2, b2,
             c));
 }
 gt_status gt_ew_fwd(gt_ctx* ctx, int32_t op, uint64_t n, gt_buf a, gt_buf b, float c, gt_buf out) {
-  GT_QUEUED(ctx, a && out && aligned(a, b, out) && op >= GT_EW_ADD && op <= GT_EW_SCALE && (b || op > GT_EW_MUL), gt_ew_fwd_now(ctx, op, n,
+  GT_QUEUED(ctx, a && out && aligned(a, b, out) && op >= GT_EW_ADD && op <= GT_EW_SCALE && (b || op > GT_EW_MUL), now_gt_ew_fwd(ctx, op, n,
             a, b, c, out));
 }
 gt_status gt_ew_bwd(gt_ctx* ctx, int32_t op, uint64_t n, gt_buf a, gt_buf b, float c, gt_buf gout, gt_buf ga, int32_t accum_a, gt_buf gb,
             int32_t accum_b) {
   GT_QUEUED(ctx, gout && aligned(a, b, gout, ga, gb) && op >= GT_EW_ADD && op <= GT_EW_SCALE &&
-            (a || op == GT_EW_ADD || op == GT_EW_SCALE) && (b || op != GT_EW_MUL), gt_ew_bwd_now(ctx, op, n, a, b, c, gout, ga, accum_a,
+            (a || op == GT_EW_ADD || op == GT_EW_SCALE) && (b || op != GT_EW_MUL), now_gt_ew_bwd(ctx, op, n, a, b, c, gout, ga, accum_a,
             gb, accum_b));
 }
 gt_status gt_glu_fwd(gt_ctx* ctx, int32_t op, uint64_t n, gt_buf x, gt_buf u, gt_buf out) {
-  GT_QUEUED(ctx, x && u && out && aligned(x, u, out) && unit(op), gt_glu_fwd_now(ctx, op, n, x, u, out));
+  GT_QUEUED(ctx, x && u && out && aligned(x, u, out) && unit(op), now_gt_glu_fwd(ctx, op, n, x, u, out));
 }
 gt_status gt_glu_linear_fwd(gt_ctx* ctx, int32_t op, int32_t rows, int32_t ffn, int32_t in, gt_buf x, gt_buf wg, gt_buf wu, gt_buf gate,
             gt_buf up, gt_buf out) {
-  GT_QUEUED(ctx, rows > 0 && ffn > 0 && in > 0 && x && wg && wu && gate && up && out && unit(op), gt_glu_linear_fwd_now(ctx, op, rows, ffn,
+  GT_QUEUED(ctx, rows > 0 && ffn > 0 && in > 0 && x && wg && wu && gate && up && out && unit(op), now_gt_glu_linear_fwd(ctx, op, rows, ffn,
             in, x, wg, wu, gate, up, out));
 }
 gt_status gt_glu_bwd(gt_ctx* ctx, int32_t op, uint64_t n, gt_buf x, gt_buf u, gt_buf gout, gt_buf gx, int32_t accum_x, gt_buf gu,
             int32_t accum_u) {
-  GT_QUEUED(ctx, x && u && gout && aligned(x, u, gout, gx, gu) && unit(op) && (!gx || gx != gu), gt_glu_bwd_now(ctx, op, n, x, u, gout, gx,
+  GT_QUEUED(ctx, x && u && gout && aligned(x, u, gout, gx, gu) && unit(op) && (!gx || gx != gu), now_gt_glu_bwd(ctx, op, n, x, u, gout, gx,
             accum_x, gu, accum_u));
 }
 gt_status gt_rmsnorm_fwd(gt_ctx* ctx, int32_t rows, int32_t d, gt_buf x, gt_buf w, float eps, gt_buf y, gt_buf rinv) {
-  GT_QUEUED(ctx, rows > 0 && d > 0 && d <= 2048 && x && w && y && rinv, gt_rmsnorm_fwd_now(ctx, rows, d, x, w, eps, y, rinv));
+  GT_QUEUED(ctx, rows > 0 && d > 0 && d <= 2048 && x && w && y && rinv, now_gt_rmsnorm_fwd(ctx, rows, d, x, w, eps, y, rinv));
 }
 gt_status gt_add_rmsnorm_fwd(gt_ctx* ctx, int32_t rows, int32_t d, gt_buf a, gt_buf b, gt_buf w, float eps, gt_buf sum, gt_buf y,
             gt_buf rinv) {
-  GT_QUEUED(ctx, rows > 0 && d > 0 && d <= 2048 && a && b && w && sum && y && rinv, gt_add_rmsnorm_fwd_now(ctx, rows, d, a, b, w, eps, sum,
+  GT_QUEUED(ctx, rows > 0 && d > 0 && d <= 2048 && a && b && w && sum && y && rinv, now_gt_add_rmsnorm_fwd(ctx, rows, d, a, b, w, eps, sum,
             y, rinv));
 }
 gt_status gt_rmsnorm_heads_rope_fwd(gt_ctx* ctx, int32_t rows, int32_t H, int32_t hd, gt_buf x, gt_buf w, float eps, gt_buf y, gt_buf rinv,
             double base, int32_t pos_offset) {
   GT_QUEUED(ctx, rows > 0 && H > 0 && hd > 0 && hd <= 2048 && hd % 2 == 0 && x && w && y && rinv && in_batch(ctx, rows),
-            gt_rmsnorm_heads_rope_fwd_now(ctx, rows, H, hd, x, w, eps, y, rinv, base, pos_offset));
+            now_gt_rmsnorm_heads_rope_fwd(ctx, rows, H, hd, x, w, eps, y, rinv, base, pos_offset));
 }
 gt_status gt_rmsnorm_bwd(gt_ctx* ctx, int32_t rows, int32_t d, gt_buf x, gt_buf w, gt_buf rinv, gt_buf gy, gt_buf gx, int32_t accum_x,
             gt_buf gw, int32_t accum_w) {
-  GT_QUEUED(ctx, rows > 0 && d > 0 && d <= 2048 && x && w && rinv && gy, gt_rmsnorm_bwd_now(ctx, rows, d, x, w, rinv, gy, gx, accum_x, gw,
+  GT_QUEUED(ctx, rows > 0 && d > 0 && d <= 2048 && x && w && rinv && gy, now_gt_rmsnorm_bwd(ctx, rows, d, x, w, rinv, gy, gx, accum_x, gw,
             accum_w));
 }
 gt_status gt_rmsnorm_bwd_add(gt_ctx* ctx, int32_t rows, int32_t d, gt_buf x, gt_buf w, gt_buf rinv, gt_buf gy, gt_buf gadd, gt_buf gx,
             gt_buf gw, int32_t accum_w) {
-  GT_QUEUED(ctx, rows > 0 && d > 0 && d <= 2048 && x && w && rinv && gy && gadd && gx, gt_rmsnorm_bwd_add_now(ctx, rows, d, x, w, rinv, gy,
+  GT_QUEUED(ctx, rows > 0 && d > 0 && d <= 2048 && x && w && rinv && gy && gadd && gx, now_gt_rmsnorm_bwd_add(ctx, rows, d, x, w, rinv, gy,
             gadd, gx, gw, accum_w));
 }
 gt_status gt_embedding_fwd(gt_ctx* ctx, int32_t rows, int32_t d, gt_buf w, gt_buf ids, gt_buf out) {
-  GT_QUEUED(ctx, rows > 0 && d > 0 && w && ids && out, gt_embedding_fwd_now(ctx, rows, d, w, ids, out));
+  GT_QUEUED(ctx, rows > 0 && d > 0 && w && ids && out, now_gt_embedding_fwd(ctx, rows, d, w, ids, out));
 }
 gt_status gt_embedding_bwd(gt_ctx* ctx, int32_t rows, int32_t d, gt_buf gy, gt_buf ids, gt_buf gw) {
-  GT_QUEUED(ctx, rows > 0 && d > 0 && gy && ids, gt_embedding_bwd_now(ctx, rows, d, gy, ids, gw));
+  GT_QUEUED(ctx, rows > 0 && d > 0 && gy && ids, now_gt_embedding_bwd(ctx, rows, d, gy, ids, gw));
 }
 gt_status gt_rope_fwd(gt_ctx* ctx, int32_t rows, int32_t H, int32_t hd, double base, int32_t pos_offset, gt_buf x, gt_buf y) {
-  GT_QUEUED(ctx, rows > 0 && H > 0 && hd > 0 && hd % 2 == 0 && x && y && in_batch(ctx, rows), gt_rope_fwd_now(ctx, rows, H, hd, base,
+  GT_QUEUED(ctx, rows > 0 && H > 0 && hd > 0 && hd % 2 == 0 && x && y && in_batch(ctx, rows), now_gt_rope_fwd(ctx, rows, H, hd, base,
             pos_offset, x, y));
 }
 gt_status gt_rope_bwd(gt_ctx* ctx, int32_t rows, int32_t H, int32_t hd, double base, int32_t pos_offset, gt_buf gy, gt_buf gx,
             int32_t accum) {
-  GT_QUEUED(ctx, rows > 0 && H > 0 && hd > 0 && hd % 2 == 0 && gy && gx && in_batch(ctx, rows), gt_rope_bwd_now(ctx, rows, H, hd, base,
+  GT_QUEUED(ctx, rows > 0 && H > 0 && hd > 0 && hd % 2 == 0 && gy && gx && in_batch(ctx, rows), now_gt_rope_bwd(ctx, rows, H, hd, base,
             pos_offset, gy, gx, accum));
 }
 gt_status gt_attention_fwd(gt_ctx* ctx, int32_t rows, int32_t Hq, int32_t Hkv, int32_t hd, int32_t window, gt_buf q, gt_buf k, gt_buf v,
             gt_buf out, gt_buf lse) {
-  GT_QUEUED(ctx, heads(rows, Hq, Hkv, hd, window) && in_batch(ctx, rows) && q && k && v && out && lse, gt_attention_fwd_now(ctx, rows, Hq,
+  GT_QUEUED(ctx, heads(rows, Hq, Hkv, hd, window) && in_batch(ctx, rows) && q && k && v && out && lse, now_gt_attention_fwd(ctx, rows, Hq,
             Hkv, hd, window, q, k, v, out, lse));
 }
 gt_status gt_attention_bwd(gt_ctx* ctx, int32_t rows, int32_t Hq, int32_t Hkv, int32_t hd, int32_t window, gt_buf q, gt_buf k, gt_buf v,
             gt_buf out, gt_buf lse, gt_buf gout, gt_buf gq, int32_t accum_q, gt_buf gk, int32_t accum_k, gt_buf gv, int32_t accum_v) {
-  GT_QUEUED(ctx, heads(rows, Hq, Hkv, hd, window) && in_batch(ctx, rows) && q && k && v && out && lse && gout, gt_attention_bwd_now(ctx,
+  GT_QUEUED(ctx, heads(rows, Hq, Hkv, hd, window) && in_batch(ctx, rows) && q && k && v && out && lse && gout, now_gt_attention_bwd(ctx,
             rows, Hq, Hkv, hd, window, q, k, v, out, lse, gout, gq, accum_q, gk, accum_k, gv, accum_v));
 }
 gt_status gt_attention_bwd_rope(gt_ctx* ctx, int32_t rows, int32_t Hq, int32_t Hkv, int32_t hd, int32_t window, gt_buf q, gt_buf k,
             gt_buf v, gt_buf out, gt_buf lse, gt_buf gout, gt_buf gq, int32_t accum_q, gt_buf gk, int32_t accum_k, gt_buf gv,
             int32_t accum_v, double base, int32_t pos_offset) {
   GT_QUEUED(ctx, heads(rows, Hq, Hkv, hd, window) && hd % 2 == 0 && in_batch(ctx, rows) && q && k && v && out && lse && gout,
-            gt_attention_bwd_rope_now(ctx, rows, Hq, Hkv, hd, window, q, k, v, out, lse, gout, gq, accum_q, gk, accum_k, gv, accum_v, base,
+            now_gt_attention_bwd_rope(ctx, rows, Hq, Hkv, hd, window, q, k, v, out, lse, gout, gq, accum_q, gk, accum_k, gv, accum_v, base,
             pos_offset));
 }
 gt_status gt_ce_fwd(gt_ctx* ctx, int32_t rows, int32_t V, gt_buf logits, gt_buf targets, gt_buf stats, gt_buf loss, gt_buf inv_kept) {
-  GT_QUEUED(ctx, rows > 0 && V > 0 && in_batch(ctx, rows) && logits && targets && stats && loss && inv_kept, gt_ce_fwd_now(ctx, rows, V,
+  GT_QUEUED(ctx, rows > 0 && V > 0 && in_batch(ctx, rows) && logits && targets && stats && loss && inv_kept, now_gt_ce_fwd(ctx, rows, V,
             logits, targets, stats, loss, inv_kept));
 }
 gt_status gt_ce_bwd(gt_ctx* ctx, int32_t rows, int32_t V, gt_buf logits, gt_buf targets, gt_buf stats, gt_buf inv_kept, gt_buf gloss,
             gt_buf glogits, int32_t accum) {
-  GT_QUEUED(ctx, rows > 0 && V > 0 && logits && targets && stats && inv_kept && gloss, gt_ce_bwd_now(ctx, rows, V, logits, targets, stats,
+  GT_QUEUED(ctx, rows > 0 && V > 0 && logits && targets && stats && inv_kept && gloss, now_gt_ce_bwd(ctx, rows, V, logits, targets, stats,
             inv_kept, gloss, glogits, accum));
 }
 gt_status gt_ce_chunk_stats(gt_ctx* ctx, int32_t rows, int32_t n, int32_t v0, int32_t first, gt_buf chunk, gt_buf targets, gt_buf run) {
-  GT_QUEUED(ctx, rows > 0 && n > 0 && v0 >= 0 && chunk && targets && run, gt_ce_chunk_stats_now(ctx, rows, n, v0, first, chunk, targets,
+  GT_QUEUED(ctx, rows > 0 && n > 0 && v0 >= 0 && chunk && targets && run, now_gt_ce_chunk_stats(ctx, rows, n, v0, first, chunk, targets,
             run));
 }
 gt_status gt_ce_loss_from_stats(gt_ctx* ctx, int32_t rows, gt_buf run, gt_buf targets, gt_buf loss, gt_buf inv_kept) {
-  GT_QUEUED(ctx, rows > 0 && in_batch(ctx, rows) && run && targets && loss && inv_kept, gt_ce_loss_from_stats_now(ctx, rows, run, targets,
+  GT_QUEUED(ctx, rows > 0 && in_batch(ctx, rows) && run && targets && loss && inv_kept, now_gt_ce_loss_from_stats(ctx, rows, run, targets,
             loss, inv_kept));
 }
 gt_status gt_ce_chunk_grad(gt_ctx* ctx, int32_t rows, int32_t n, int32_t v0, gt_buf chunk, gt_buf targets, gt_buf run, gt_buf inv_kept,
             gt_buf gloss) {
-  GT_QUEUED(ctx, rows > 0 && n > 0 && chunk && targets && run && inv_kept && gloss, gt_ce_chunk_grad_now(ctx, rows, n, v0, chunk, targets,
+  GT_QUEUED(ctx, rows > 0 && n > 0 && chunk && targets && run && inv_kept && gloss, now_gt_ce_chunk_grad(ctx, rows, n, v0, chunk, targets,
             run, inv_kept, gloss));
 }
 gt_status gt_readout_ce_stats(gt_ctx* ctx, int32_t rows, int32_t n, int32_t h, int32_t v0, int32_t first, gt_buf hidden, gt_buf w,
             gt_buf chunk, gt_buf targets, gt_buf run) {
-  GT_QUEUED(ctx, rows > 0 && n > 0 && h > 0 && v0 >= 0 && hidden && w && chunk && targets && run, gt_readout_ce_stats_now(ctx, rows, n, h,
+  GT_QUEUED(ctx, rows > 0 && n > 0 && h > 0 && v0 >= 0 && hidden && w && chunk && targets && run, now_gt_readout_ce_stats(ctx, rows, n, h,
             v0, first, hidden, w, chunk, targets, run));
 }
 gt_status gt_readout_ce_grad(gt_ctx* ctx, int32_t rows, int32_t n, int32_t h, int32_t v0, gt_buf hidden, gt_buf w, gt_buf chunk,
             gt_buf targets, gt_buf run, gt_buf inv_kept, gt_buf gloss) {
   GT_QUEUED(ctx, rows > 0 && n > 0 && h > 0 && v0 >= 0 && hidden && w && chunk && targets && run && inv_kept && gloss,
-            gt_readout_ce_grad_now(ctx, rows, n, h, v0, hidden, w, chunk, targets, run, inv_kept, gloss));
+            now_gt_readout_ce_grad(ctx, rows, n, h, v0, hidden, w, chunk, targets, run, inv_kept, gloss));
 }
 gt_status gt_soft_ce_fwd(gt_ctx* ctx, int32_t rows, int32_t V, int32_t k, gt_buf logits, gt_buf tids, gt_buf tprobs, gt_buf stats,
             gt_buf loss, gt_buf inv_kept) {
   GT_QUEUED(ctx, rows > 0 && V > 0 && k > 0 && in_batch(ctx, rows) && logits && tids && tprobs && stats && loss && inv_kept,
-            gt_soft_ce_fwd_now(ctx, rows, V, k, logits, tids, tprobs, stats, loss, inv_kept));
+            now_gt_soft_ce_fwd(ctx, rows, V, k, logits, tids, tprobs, stats, loss, inv_kept));
 }
 gt_status gt_soft_ce_bwd(gt_ctx* ctx, int32_t rows, int32_t V, int32_t k, gt_buf logits, gt_buf tids, gt_buf tprobs, gt_buf stats,
             gt_buf inv_kept, gt_buf gloss, gt_buf glogits, int32_t accum) {
-  GT_QUEUED(ctx, rows > 0 && V > 0 && k > 0 && logits && tids && tprobs && stats && inv_kept && gloss, gt_soft_ce_bwd_now(ctx, rows, V, k,
+  GT_QUEUED(ctx, rows > 0 && V > 0 && k > 0 && logits && tids && tprobs && stats && inv_kept && gloss, now_gt_soft_ce_bwd(ctx, rows, V, k,
             logits, tids, tprobs, stats, inv_kept, gloss, glogits, accum));
 }
 gt_status gt_zero(gt_ctx* ctx, gt_buf buf, uint64_t bytes) {
-  GT_QUEUED(ctx, true, gt_zero_now(ctx, buf, bytes));
+  GT_QUEUED(ctx, true, now_gt_zero(ctx, buf, bytes));
 }
 gt_status gt_copy(gt_ctx* ctx, gt_buf dst, gt_buf src, uint64_t bytes) {
-  GT_QUEUED(ctx, true, gt_copy_now(ctx, dst, src, bytes));
+  GT_QUEUED(ctx, true, now_gt_copy(ctx, dst, src, bytes));
 }
 
 // ---- entry points with arrays: copied into the record ----
@@ -356,9 +357,9 @@ gt_status gt_gemm_multi(gt_ctx* ctx, int32_t kind, int32_t accum, int32_t M, int
   }
   if (!ok) {
     const gt_status s = gt_drain(ctx);
-    return s ? s : gt_gemm_multi_now(ctx, kind, accum, M, N, nparts, Ks, as, bs, c);
+    return s ? s : now_gt_gemm_multi(ctx, kind, accum, M, N, nparts, Ks, as, bs, c);
   }
-  GT_QUEUED(ctx, true, gt_gemm_multi_now(ctx, kind, accum, M, N, nparts, v.k, v.a, v.b, c));
+  GT_QUEUED(ctx, true, now_gt_gemm_multi(ctx, kind, accum, M, N, nparts, v.k, v.a, v.b, c));
 }
 gt_status gt_gemm_grouped_scaled(gt_ctx* ctx, int32_t kind, int32_t ngroups, const int32_t* Ms, const int32_t* Ns, int32_t K, const gt_buf* as,
                                  const gt_buf* bs, const gt_buf* cs, const int32_t* accums, float alpha) {
@@ -370,9 +371,9 @@ gt_status gt_gemm_grouped_scaled(gt_ctx* ctx, int32_t kind, int32_t ngroups, con
   }
   if (!ok) {
     const gt_status s = gt_drain(ctx);
-    return s ? s : gt_gemm_grouped_scaled_now(ctx, kind, ngroups, Ms, Ns, K, as, bs, cs, accums, alpha);
+    return s ? s : now_gt_gemm_grouped_scaled(ctx, kind, ngroups, Ms, Ns, K, as, bs, cs, accums, alpha);
   }
-  GT_QUEUED(ctx, true, gt_gemm_grouped_scaled_now(ctx, kind, ngroups, v.m, v.n, K, v.a, v.b, v.c, v.acc, alpha));
+  GT_QUEUED(ctx, true, now_gt_gemm_grouped_scaled(ctx, kind, ngroups, v.m, v.n, K, v.a, v.b, v.c, v.acc, alpha));
 }
 gt_status gt_gemm_grouped(gt_ctx* ctx, int32_t kind, int32_t ngroups, const int32_t* Ms, const int32_t* Ns, int32_t K, const gt_buf* as,
                           const gt_buf* bs, const gt_buf* cs, const int32_t* accums) {
@@ -388,9 +389,9 @@ gt_status gt_linear_rope_grouped(gt_ctx* ctx, int32_t ngroups, int32_t rows, int
   }
   if (!ok) {
     const gt_status s = gt_drain(ctx);
-    return s ? s : gt_linear_rope_grouped_now(ctx, ngroups, rows, K, x, Ns, ws, ys, hs, hd, base, pos_offset);
+    return s ? s : now_gt_linear_rope_grouped(ctx, ngroups, rows, K, x, Ns, ws, ys, hs, hd, base, pos_offset);
   }
-  GT_QUEUED(ctx, true, gt_linear_rope_grouped_now(ctx, ngroups, rows, K, x, v.n, v.w, v.y, v.h, hd, base, pos_offset));
+  GT_QUEUED(ctx, true, now_gt_linear_rope_grouped(ctx, ngroups, rows, K, x, v.n, v.w, v.y, v.h, hd, base, pos_offset));
 }
 // Small writes (token ids, targets) keep their place among the ops through a copy of their own; large ones are made at once.
 gt_status gt_write(gt_ctx* ctx, gt_buf dst, const void* host, uint64_t bytes) {
@@ -398,11 +399,11 @@ gt_status gt_write(gt_ctx* ctx, gt_buf dst, const void* host, uint64_t bytes) {
   char* copy = q && !q->failed.load(std::memory_order_relaxed) ? (char*)malloc(bytes) : nullptr;
   if (!copy) {
     const gt_status s = gt_drain(ctx);
-    return s ? s : gt_write_now(ctx, dst, host, bytes);
+    return s ? s : now_gt_write(ctx, dst, host, bytes);
   }
   memcpy(copy, host, bytes);
   return q->put([=]() -> gt_status {
-    const gt_status s = gt_skip_queued(ctx) ? GT_OK : gt_write_now(ctx, dst, copy, bytes);
+    const gt_status s = gt_skip_queued(ctx) ? GT_OK : now_gt_write(ctx, dst, copy, bytes);
     free(copy);
     return s;
   });
