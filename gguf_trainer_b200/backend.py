@@ -1555,14 +1555,27 @@ class CudaBackend:
     def crossEntropy(self, logits: Tensor, targets, kept: int) -> Tensor:
         """webgpu.ts:1295-1329. `kept` was counted above the dispatch; the device derives the same
         count from the uploaded targets, so nothing host-computed is baked into a replayable graph."""
-        self._beginForwardOp()
+        # The readout that makes the logits usually waits to be launched: then it takes the loss's statistics as it writes them.
+        readout = None
+        fused = getattr(self.lib, "gt_readout_ce_fwd", None)    # (a stand-in for the library need not have it)
+        pend = self._pendingFwd
+        if (fused is not None and len(pend) == 1 and logits._dev is pend[0]["eo"] and logits._dev.owner == self._uid
+                and not ("rope" in pend[0] or "lora" in pend[0] or "norm" in pend[0])):
+            readout = pend[0]
+        self._beginForwardOp(keepPending=readout is not None)
         T, V = logits.shape
-        el = self._entryFor(logits)
         tgt = self._uploadU32(targets, "targets", V)
+        if readout is not None:
+            self._pendingFwd = []
+            readout["eo"].pendingFwd = False
+        el = self._entryFor(logits)
         stats = self._acquireRecycled(T * 16)
         needs = self._flows(logits, el)
         loss, eo, invKept = self._lossOut([logits], needs)
-        self._check(self.lib.gt_ce_fwd(self.ctx, T, V, el.data, tgt, stats, eo.data, invKept))
+        if readout is not None:
+            self._check(fused(self.ctx, T, V, readout["inDim"], readout["ex"].data, readout["ew"].data, el.data, tgt, stats, eo.data, invKept))
+        else:
+            self._check(self.lib.gt_ce_fwd(self.ctx, T, V, el.data, tgt, stats, eo.data, invKept))
 
         def _bw():
             self._ensureBackwardBegun()

@@ -153,7 +153,8 @@ struct CeArgs {
   float2* part;                  // statistics: (max, sum) per row and column strip, strip-major
   int v0, T, nseq;
 };
-gt_status gt_readout_tc(gt_ctx* ctx, bool grad, int rows, int n, int h, const float* hidden, const float* w, float* chunk, const CeArgs& ce,
+enum { GT_READOUT_STATS, GT_READOUT_GRAD, GT_READOUT_BOTH };   // statistics alone, the gradient, the logits and their statistics
+gt_status gt_readout_tc(gt_ctx* ctx, int form, int rows, int n, int h, const float* hidden, const float* w, float* chunk, const CeArgs& ce,
                         int* parts, bool* handled);
 gt_status gt_gemm_tc(gt_ctx* ctx, int kind, int accum, int M, int N, int K, const float* a, const float* b, float* c, float alpha,
                      bool* handled);

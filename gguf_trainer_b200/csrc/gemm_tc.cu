@@ -76,7 +76,7 @@ struct PartMaps {
   CeArgs ce;                // readout forms (EPI_CE_STATS, EPI_CE_GRAD)
 };
 constexpr int EPI_ROPE = 8;   // values of the kernel's GLU argument that are neither activation
-constexpr int EPI_CE_STATS = 16, EPI_CE_GRAD = 32;
+constexpr int EPI_CE_STATS = 16, EPI_CE_GRAD = 32, EPI_CE_BOTH = 64;
 
 // GLU != 0 (GT_EW_SILU or GT_EW_GELU; NT layout, BN = 192 only): the gated unit of the FFN in the projection that
 // feeds it. B is two weight matrices: the tile's first 96 columns are rows [n0/2, n0/2 + 96) of b[0] (gate), the other 96
@@ -93,6 +93,8 @@ constexpr int EPI_CE_STATS = 16, EPI_CE_GRAD = 32;
 // thread, merged by ce_merge_kernel) and the target's logit, and writes no logits at all; GRAD turns the logits into the
 // loss's gradient on their way out. The passes over [rows, span] that did this (a read; a read and a write) are bound by
 // HBM: at 8192 x 32768 157 and 552 us beside a product of 1.3 ms.
+// EPI_CE_BOTH writes the logits of a whole vocabulary and takes their statistics (the loss that keeps its logits): the pass
+// over them costs 239 us at 8192 x 49152.
 // (epilogue warps per lane quadrant: three where the epilogue computes and runs beside the main loop)
 template <int MT, int GLU>
 struct EpiSub { static constexpr int N = MT == 1 && GLU != 0 ? 3 : 1; };
@@ -104,7 +106,7 @@ struct CeRow { uint32_t tg; float m, inv, sc; };   // readout forms: what the ro
 template <int GLU>
 __device__ __forceinline__ CeRow ce_row(const PartMaps& maps, int row, int M) {
   CeRow r = {0xffffffffu, 0.f, 0.f, 0.f};
-  if ((GLU == EPI_CE_STATS || GLU == EPI_CE_GRAD) && row < M) {
+  if (GLU >= EPI_CE_STATS && row < M) {
     r.tg = __ldg(maps.ce.targets + row);
     if (GLU == EPI_CE_GRAD) {
       r.m = __ldg(maps.ce.run + (size_t)row * 3);
@@ -143,7 +145,7 @@ __device__ __forceinline__ void drain_tile(const PartMaps& maps, const Drain& d,
     if (lane == 0) tma_commit_group();
     nst++;
   };
-  if (GLU == EPI_CE_STATS) {
+  if (GLU == EPI_CE_STATS || GLU == EPI_CE_BOTH) {
     float m = -3.0e38f, s = 0.f;
     const uint32_t tcol = ce.tg - (uint32_t)maps.ce.v0;   // the target's column of the span, if it is below N
 #pragma unroll 1
@@ -158,6 +160,7 @@ __device__ __forceinline__ void drain_tile(const PartMaps& maps, const Drain& d,
         v[j] = col0 + j < N ? v[j] * d.out_scale : -3.0e38f;
         mb = fmaxf(mb, v[j]);
       }
+      if (GLU == EPI_CE_BOTH) put(v, d.mapC, col0);
       float t[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int j = 0; j < 32; j++) t[j & 3] += __expf(v[j] - mb);
@@ -1487,11 +1490,12 @@ gt_status gt_glu_linear_tc(gt_ctx* ctx, int op, int rows, int ffn, int in, const
 
 // One vocabulary span of the chunked readout loss: logits = hidden.w^T with their statistics or their gradient taken in
 // the epilogue (see the kernel). `parts` is the number of (max, sum) pairs per row that the statistics form leaves in
-// ce.part, which lies in the span's logits buffer: nothing else is written there.
-gt_status gt_readout_tc(gt_ctx* ctx, bool grad, int rows, int n, int h, const float* hidden, const float* w, float* chunk, const CeArgs& ce,
+// ce.part (two per 256 columns, or part of a tile of them).
+gt_status gt_readout_tc(gt_ctx* ctx, int form, int rows, int n, int h, const float* hidden, const float* w, float* chunk, const CeArgs& ce,
                         int* parts, bool* handled) {
   *handled = false;
-  if (rows < 16 || n < 256 || h < 16 || (h & 3) || (grad && (n & 3))) return GT_OK;
+  const bool store = form != GT_READOUT_STATS;
+  if (rows < 16 || n < 256 || h < 16 || (h & 3) || (store && (n & 3))) return GT_OK;
   if ((((uintptr_t)hidden) | ((uintptr_t)w) | ((uintptr_t)chunk)) & 15) return GT_OK;
   if (ctx->device < 0 || ctx->device >= 64 || !device_flag(ctx)) return GT_OK;
   const int kblocks = gt_cdiv(h, BK);
@@ -1509,11 +1513,12 @@ gt_status gt_readout_tc(gt_ctx* ctx, bool grad, int rows, int n, int h, const fl
       !make_map_3d(&maps.b[0], w, h, n, 1, h, (uint64_t)n * h, 128, true))
     return GT_OK;
   maps.c[0] = maps.a[0];
-  if (grad && !make_map_3d(&maps.c[0], chunk, n, rows, 1, n, (uint64_t)rows * n, 32, true)) return GT_OK;
+  if (store && !make_map_3d(&maps.c[0], chunk, n, rows, 1, n, (uint64_t)rows * n, 32, true)) return GT_OK;
   maps.kb_end[0] = kblocks;
   maps.ce = ce;
   *parts = gt_cdiv(n, 256) * PairSub<256, EPI_CE_STATS>::N;
-  gt_status s = grad ? launch_pair<true, true, 256, EPI_CE_GRAD>(ctx, maps, tiles, 1, chunk, rows, n, 0, 1, 1, npairs, TRUNC_COMP)
+  gt_status s = form == GT_READOUT_GRAD ? launch_pair<true, true, 256, EPI_CE_GRAD>(ctx, maps, tiles, 1, chunk, rows, n, 0, 1, 1, npairs, TRUNC_COMP)
+                : form == GT_READOUT_BOTH ? launch_pair<true, true, 256, EPI_CE_BOTH>(ctx, maps, tiles, 1, chunk, rows, n, 0, 1, 1, npairs, TRUNC_COMP)
                      : launch_pair<true, true, 256, EPI_CE_STATS>(ctx, maps, tiles, 0, chunk, rows, n, 0, 1, 1, npairs, TRUNC_COMP);
   if (s) return s;
   *handled = true;

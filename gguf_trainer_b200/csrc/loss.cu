@@ -195,8 +195,9 @@ __global__ void __launch_bounds__(ROWT) ce_chunk_grad_kernel(int n, int v0, int 
 
 // run[row] merged with the `parts` (max, sum) pairs per row that the readout product left (strip-major): 32 rows a CTA, one
 // per lane, the strips dealt out to the warps. The product has already written the target logits that lie in its span.
+// stats != null: the span is the whole vocabulary and what the loss over kept logits wants (see ce_fwd_kernel) goes there instead.
 __global__ void __launch_bounds__(ROWT) ce_merge_kernel(int rows, int n, int v0, int first, int parts, const float2* __restrict__ part,
-                                                        const uint32_t* __restrict__ targets, float* __restrict__ run) {
+                                                        const uint32_t* __restrict__ targets, float* __restrict__ run, float4* __restrict__ stats) {
   pdl_wait();
   __shared__ MS sh[ROWT / 32][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, row = blockIdx.x * 32 + lane;
@@ -212,9 +213,13 @@ __global__ void __launch_bounds__(ROWT) ce_merge_kernel(int rows, int n, int v0,
   float* rr = run + (size_t)row * 3;
   MS r = first ? MS{NEG, 0.f} : MS{rr[0], rr[1]};
   for (int i = 0; i < ROWT / 32; i++) r = ms_merge(r, sh[i][lane]);
+  const uint32_t t = targets[row];
+  if (stats) {
+    stats[row] = make_float4(r.m, 1.f / r.s, t != IGNORE ? logf(r.s) + r.m - rr[2] : 0.f, 0.f);
+    return;
+  }
   rr[0] = r.m;
   rr[1] = r.s;
-  const uint32_t t = targets[row];
   if (first && !(t != IGNORE && t >= (uint32_t)v0 && t < (uint32_t)(v0 + n))) rr[2] = 0.f;
 }
 
@@ -328,10 +333,10 @@ gt_status gt_readout_ce_stats(gt_ctx* ctx, int32_t rows, int32_t n, int32_t h, i
     const CeArgs ce = {gt_ptr<const uint32_t>(targets), gt_ptr<float>(run), nullptr, nullptr, gt_ptr<float2>(chunk), v0, rows, 1};
     bool handled = false;
     int parts = 0;
-    gt_status s = gt_readout_tc(ctx, false, rows, n, h, gt_ptr<const float>(hidden), gt_ptr<const float>(w), gt_ptr<float>(chunk), ce, &parts, &handled);
+    gt_status s = gt_readout_tc(ctx, GT_READOUT_STATS, rows, n, h, gt_ptr<const float>(hidden), gt_ptr<const float>(w), gt_ptr<float>(chunk), ce, &parts, &handled);
     if (s) return s;
     if (handled) {
-      GT_CUDA(ctx, gt_launch(ctx, 1, ce_merge_kernel, gt_cdiv(rows, 32), ROWT, 0, rows, n, v0, first, parts, gt_ptr<const float2>(chunk), gt_ptr<const uint32_t>(targets), gt_ptr<float>(run)));
+      GT_CUDA(ctx, gt_launch(ctx, 1, ce_merge_kernel, gt_cdiv(rows, 32), ROWT, 0, rows, n, v0, first, parts, gt_ptr<const float2>(chunk), gt_ptr<const uint32_t>(targets), gt_ptr<float>(run), (float4*)nullptr));
       GT_LAUNCHED(ctx, "ce_merge_kernel");
       return GT_OK;
     }
@@ -347,11 +352,39 @@ gt_status gt_readout_ce_grad(gt_ctx* ctx, int32_t rows, int32_t n, int32_t h, in
     const CeArgs ce = {gt_ptr<const uint32_t>(targets), gt_ptr<float>(run), gt_ptr<const float>(inv_kept), gt_ptr<const float>(gloss), nullptr, v0, T, nseq};
     bool handled = false;
     int parts = 0;
-    gt_status s = gt_readout_tc(ctx, true, rows, n, h, gt_ptr<const float>(hidden), gt_ptr<const float>(w), gt_ptr<float>(chunk), ce, &parts, &handled);
+    gt_status s = gt_readout_tc(ctx, GT_READOUT_GRAD, rows, n, h, gt_ptr<const float>(hidden), gt_ptr<const float>(w), gt_ptr<float>(chunk), ce, &parts, &handled);
     if (s || handled) return s;
   }
   gt_status s = gt_gemm(ctx, GT_GEMM_NT, 0, rows, n, h, hidden, w, chunk);
   return s ? s : gt_ce_chunk_grad(ctx, rows, n, v0, chunk, targets, run, inv_kept, gloss);
+}
+
+gt_status gt_readout_ce_fwd(gt_ctx* ctx, int32_t rows, int32_t V, int32_t h, gt_buf hidden, gt_buf w, gt_buf logits, gt_buf targets, gt_buf stats, gt_buf loss, gt_buf inv_kept) {
+  GT_REQUIRE(ctx, rows > 0 && V > 0 && h > 0 && hidden && w && logits && targets && stats && loss && inv_kept, "gt_readout_ce_fwd: bad argument");
+  int T, nseq; seq_shape(ctx, rows, &T, &nseq);
+  GT_REQUIRE(ctx, rows == T * nseq, "gt_readout_ce_fwd: %d rows but the batch is %d x %d", rows, nseq, T);
+  if (ctx->precision != GT_PREC_FP32) {
+    const size_t strips = 2 * (size_t)gt_cdiv(V, 256);
+    float* blk = nullptr;      // the pairs, and the target logits where the running form keeps them
+    gt_status s = gt_scratch(ctx, (strips * 2 + 3) * sizeof(float) * (size_t)rows, &blk);
+    if (s) return s;
+    float2* const part = reinterpret_cast<float2*>(blk);
+    float* const run = blk + strips * 2 * (size_t)rows;
+    const CeArgs ce = {gt_ptr<const uint32_t>(targets), run, nullptr, nullptr, part, 0, T, nseq};
+    bool handled = false;
+    int parts = 0;
+    s = gt_readout_tc(ctx, GT_READOUT_BOTH, rows, V, h, gt_ptr<const float>(hidden), gt_ptr<const float>(w), gt_ptr<float>(logits), ce, &parts, &handled);
+    if (s) return s;
+    if (handled) {
+      GT_CUDA(ctx, gt_launch(ctx, 1, ce_merge_kernel, gt_cdiv(rows, 32), ROWT, 0, rows, V, 0, 1, parts, (const float2*)part, gt_ptr<const uint32_t>(targets), run, gt_ptr<float4>(stats)));
+      GT_LAUNCHED(ctx, "ce_merge_kernel");
+      GT_CUDA(ctx, gt_launch(ctx, 1, loss_reduce_kernel<0>, 1, 1024, 0, rows, T, nseq, gt_ptr<const float>(stats), gt_ptr<const uint32_t>(targets), 1, gt_ptr<float>(loss), gt_ptr<float>(inv_kept)));
+      GT_LAUNCHED(ctx, "loss_reduce_kernel");
+      return GT_OK;
+    }
+  }
+  gt_status s = gt_gemm(ctx, GT_GEMM_NT, 0, rows, V, h, hidden, w, logits);
+  return s ? s : gt_ce_fwd(ctx, rows, V, logits, targets, stats, loss, inv_kept);
 }
 
 gt_status gt_soft_ce_fwd(gt_ctx* ctx, int32_t rows, int32_t V, int32_t k, gt_buf logits, gt_buf tids, gt_buf tprobs, gt_buf stats, gt_buf loss, gt_buf inv_kept) {

@@ -84,7 +84,7 @@ PyObject* invoke(gt_status (*fn)(A...), PyObject* slow, PyObject* const* args, P
   X(gt_linear_rope_grouped) X(gt_ew_fwd) X(gt_ew_bwd) X(gt_glu_fwd) X(gt_glu_linear_fwd) X(gt_glu_bwd) X(gt_rmsnorm_fwd)      \
   X(gt_add_rmsnorm_fwd) X(gt_rmsnorm_heads_rope_fwd) X(gt_rmsnorm_bwd) X(gt_rmsnorm_bwd_add) X(gt_embedding_fwd)              \
   X(gt_embedding_bwd) X(gt_rope_fwd) X(gt_rope_bwd) X(gt_attention_fwd) X(gt_attention_bwd) X(gt_attention_bwd_rope)          \
-  X(gt_ce_fwd) X(gt_ce_bwd) X(gt_readout_ce_stats) X(gt_readout_ce_grad) X(gt_ce_loss_from_stats) X(gt_zero) X(gt_copy)
+  X(gt_ce_fwd) X(gt_ce_bwd) X(gt_readout_ce_fwd) X(gt_readout_ce_stats) X(gt_readout_ce_grad) X(gt_ce_loss_from_stats) X(gt_zero) X(gt_copy)
 
 #define X(name)                                                                       \
   decltype(&name) fn_##name = nullptr;                                                \

@@ -195,6 +195,7 @@ decltype(gt_ce_bwd) now_gt_ce_bwd;
 decltype(gt_ce_chunk_stats) now_gt_ce_chunk_stats;
 decltype(gt_ce_loss_from_stats) now_gt_ce_loss_from_stats;
 decltype(gt_ce_chunk_grad) now_gt_ce_chunk_grad;
+decltype(gt_readout_ce_fwd) now_gt_readout_ce_fwd;
 decltype(gt_readout_ce_stats) now_gt_readout_ce_stats;
 decltype(gt_readout_ce_grad) now_gt_readout_ce_grad;
 decltype(gt_soft_ce_fwd) now_gt_soft_ce_fwd;
@@ -318,6 +319,11 @@ gt_status gt_ce_chunk_grad(gt_ctx* ctx, int32_t rows, int32_t n, int32_t v0, gt_
             gt_buf gloss) {
   GT_QUEUED(ctx, rows > 0 && n > 0 && chunk && targets && run && inv_kept && gloss, now_gt_ce_chunk_grad(ctx, rows, n, v0, chunk, targets,
             run, inv_kept, gloss));
+}
+gt_status gt_readout_ce_fwd(gt_ctx* ctx, int32_t rows, int32_t V, int32_t h, gt_buf hidden, gt_buf w, gt_buf logits, gt_buf targets,
+            gt_buf stats, gt_buf loss, gt_buf inv_kept) {
+  GT_QUEUED(ctx, rows > 0 && V > 0 && h > 0 && in_batch(ctx, rows) && hidden && w && logits && targets && stats && loss && inv_kept,
+            now_gt_readout_ce_fwd(ctx, rows, V, h, hidden, w, logits, targets, stats, loss, inv_kept));
 }
 gt_status gt_readout_ce_stats(gt_ctx* ctx, int32_t rows, int32_t n, int32_t h, int32_t v0, int32_t first, gt_buf hidden, gt_buf w,
             gt_buf chunk, gt_buf targets, gt_buf run) {

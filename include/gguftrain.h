@@ -215,6 +215,9 @@ gt_status gt_readout_ce_stats(gt_ctx* ctx, int32_t rows, int32_t n, int32_t h, i
                               gt_buf w, gt_buf chunk, gt_buf targets, gt_buf run);
 gt_status gt_readout_ce_grad(gt_ctx* ctx, int32_t rows, int32_t n, int32_t h, int32_t v0, gt_buf hidden, gt_buf w,
                              gt_buf chunk, gt_buf targets, gt_buf run, gt_buf inv_kept, gt_buf gloss);
+/* gt_ce_fwd with the product that makes its logits, hidden [rows, h] . w [V, h]^T, which are kept */
+gt_status gt_readout_ce_fwd(gt_ctx* ctx, int32_t rows, int32_t V, int32_t h, gt_buf hidden, gt_buf w, gt_buf logits,
+                            gt_buf targets, gt_buf stats, gt_buf loss, gt_buf inv_kept);
 /* sparse-teacher soft CE (webgpu.ts:1331-1378; srcSoftCeFwd/BwdP/BwdQ wgsl.ts:1004-1110).
  * tids/tprobs: [rows, k]; a row whose first id is 0xffffffff is ignored. */
 gt_status gt_soft_ce_fwd(gt_ctx* ctx, int32_t rows, int32_t V, int32_t k, gt_buf logits, gt_buf tids, gt_buf tprobs,

@@ -81,6 +81,7 @@ const SYMBOLS = {
   gt_ce_chunk_grad: { parameters: ["pointer", "i32", "i32", "i32", "u64", "u64", "u64", "u64", "u64"], result: "i32" },
   gt_readout_ce_stats: { parameters: ["pointer", "i32", "i32", "i32", "i32", "i32", "u64", "u64", "u64", "u64", "u64"], result: "i32" },
   gt_readout_ce_grad: { parameters: ["pointer", "i32", "i32", "i32", "i32", "u64", "u64", "u64", "u64", "u64", "u64", "u64"], result: "i32" },
+  gt_readout_ce_fwd: { parameters: ["pointer", "i32", "i32", "i32", "u64", "u64", "u64", "u64", "u64", "u64", "u64"], result: "i32" },
   gt_soft_ce_fwd: { parameters: ["pointer", "i32", "i32", "i32", "u64", "u64", "u64", "u64", "u64", "u64"], result: "i32" },
   gt_soft_ce_bwd: { parameters: ["pointer", "i32", "i32", "i32", "u64", "u64", "u64", "u64", "u64", "u64", "u64", "i32"], result: "i32" },
   gt_adamw_create: { parameters: ["pointer", "i32", "buffer", "buffer", "buffer", "f32", "f32", "f32", "f32", "f32", "f32", "buffer"], result: "i32" },

@@ -56,6 +56,20 @@ def test_readout_ce(gpu, monkeypatch, tile, rows, h, spans):
         assert (got[~kept] == 0).all()
         assert np.linalg.norm(got - want[:, v0:v0 + n]) <= 5e-3 * np.linalg.norm(want)
         v0 += n
+    # the whole vocabulary at once, logits kept
+    V4 = V - V % 4
+    t4 = np.where(tg < V4, tg, 0xFFFFFFFF).astype(np.uint32)
+    k4 = t4 != 0xFFFFFFFF
+    lg, st, ls, ik, d4 = (gpu.createStateBuffer(n) for n in (rows * V4 * 4, rows * 16, 8, 4, rows * 4))
+    gpu.writeStateBuffer(d4, t4.view(np.float32))
+    gpu._check(gpu.lib.gt_readout_ce_fwd(gpu.ctx, rows, V4, h, dx, dw, lg, d4, st, ls, ik))
+    assert np.linalg.norm(gpu.readStateBuffer(lg, rows * V4).reshape(rows, V4) - z[:, :V4]) <= 2e-3 * np.linalg.norm(z)
+    m4 = z[:, :V4].max(1)
+    lse4 = np.log(np.exp(z[:, :V4] - m4[:, None]).sum(1)) + m4
+    S = gpu.readStateBuffer(st, rows * 4).reshape(rows, 4).astype(np.float64)
+    nll = np.where(k4, lse4 - z[np.arange(rows), np.where(k4, t4, 0)], 0.0)
+    assert np.abs(S[:, 0] - np.log(S[:, 1]) - lse4).max() <= 2e-3 * scale and np.abs(S[:, 2] - nll).max() <= 4e-3 * scale
+    assert abs(gpu.readStateBuffer(ls, 1)[0] - nll.sum() / k4.sum()) <= 2e-3 * scale
     gpu.sync([])
-    for b in (dx, dw, dt, di, dl, run, chunk):
+    for b in (dx, dw, dt, di, dl, run, chunk, lg, st, ls, ik, d4):
         gpu._check(gpu.lib.gt_free(gpu.ctx, b))
