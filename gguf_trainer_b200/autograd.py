@@ -15,7 +15,6 @@ from typing import Callable, Dict, List, Optional, Sequence
 import numpy as np
 
 _tensors_created = itertools.count()
-_new = object.__new__
 
 
 def _noop():
@@ -53,15 +52,7 @@ class Tensor:
     @staticmethod
     def output(shape: List[int], size: int, prev: List["Tensor"]) -> "Tensor":
         """The output of a backend's op: `zeros(shape)` recorded on `prev`, for a backend that has the element count."""
-        t = _new(Tensor)
-        t._data = t._grad = t._dev = None
-        t.requiresGrad = t._needs = False
-        t._backward = _noop
-        t.size = size
-        t.shape = shape
-        t._prev = prev
-        t.seq = next(_tensors_created)
-        return t
+        return _output(shape, size, prev, next(_tensors_created))
 
     @staticmethod
     def zeros(shape: Sequence[int], requiresGrad: bool = False) -> "Tensor":
@@ -103,6 +94,27 @@ class Tensor:
             self._grad.fill(0)
 
 
+def slotMaker(cls, fixed, args):
+    """A function of `args` that makes a `cls` with those slots and the `fixed` ones set: compiled where the extension of the
+    hot calls is there."""
+    try:
+        from ._calls import maker
+        return maker(cls, fixed, args)
+    except ImportError:
+        new = object.__new__
+
+        def make(*values):
+            t = new(cls)
+            for name, v in fixed.items():
+                setattr(t, name, v)
+            for name, v in zip(args, values):
+                setattr(t, name, v)
+            return t
+        return make
+
+
+_output = slotMaker(Tensor, dict(_data=None, _grad=None, _dev=None, requiresGrad=False, _needs=False, _backward=_noop),
+                    ("shape", "size", "_prev", "seq"))
 _by_seq = operator.attrgetter("seq")
 
 

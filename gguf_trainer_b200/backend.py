@@ -41,24 +41,26 @@ class _Entry:
     __slots__ = ("owner", "needs", "region", "data", "grad", "bytes", "external", "gradLive", "size", "pendingDx", "copyFrom", "pendingDw", "pendingFwd",
                  "lazy", "ropeOf", "ropeFused", "touched")
 
-    def __init__(self, owner: int, data: int, nbytes: int, size: int):
-        self.owner = owner        # `_uid` of the backend
-        self.data = data
-        self.grad = 0             # 0 for a frozen external (webgpu.ts frozenGradStub), and for an op's output until written
-        self.needs = False        # an op's output: does a gradient flow through it? (an external: does it have a buffer)
-        self.region = 0           # the recompute region it was made in (0: none): how long a gradient buffer must live
-        self.bytes = nbytes
-        self.external = self.touched = False   # touched: an external listed in _touched
-        self.gradLive = False     # has anything been written to grad in the current graph?
-        self.size = size
-        self.pendingDx = None     # (rows, cols, [(dY address, W address, K)]): input-gradient products not launched yet
-        self.copyFrom = 0         # address whose contents are this gradient's value so far (a copy not made yet)
-        self.pendingDw = False    # a weight-gradient product into this gradient is noted in _pendingDw, not launched yet
-        self.pendingFwd = False   # the projection that produces this tensor is noted in _pendingFwd, not launched yet
-        self.lazy = None          # a launch that fills `data`: set on a projection (or per-head norm) whose only reader took it
-                                  # rotated, so that it was never written; run if someone else asks for it (_materializeLazy)
-        self.ropeOf = None        # for a rotary embedding's output: (input tensor, its entry, H, hd, base, posOffset)
-        self.ropeFused = False    # its gradient went straight to the rotation's input (attention backward applied it)
+    # owner      `_uid` of the backend
+    # data       device address; `bytes` long, `size` elements
+    # grad       0 for a frozen external (webgpu.ts frozenGradStub), and for an op's output until written
+    # needs      an op's output: does a gradient flow through it? (an external: does it have a buffer)
+    # region     the recompute region it was made in (0: none): how long a gradient buffer must live
+    # touched    an external listed in _touched
+    # gradLive   has anything been written to grad in the current graph?
+    # pendingDx  (rows, cols, [(dY address, W address, K)]): input-gradient products not launched yet
+    # copyFrom   address whose contents are this gradient's value so far (a copy not made yet)
+    # pendingDw  a weight-gradient product into this gradient is noted in _pendingDw, not launched yet
+    # pendingFwd the projection that produces this tensor is noted in _pendingFwd, not launched yet
+    # lazy       a launch that fills `data`: set on a projection (or per-head norm) whose only reader took it rotated, so that it
+    #            was never written; run if someone else asks for it (_materializeLazy)
+    # ropeOf     for a rotary embedding's output: (input tensor, its entry, H, hd, base, posOffset)
+    # ropeFused  its gradient went straight to the rotation's input (attention backward applied it)
+
+
+_entry = ag.slotMaker(_Entry, dict(grad=0, needs=False, region=0, external=False, touched=False, gradLive=False, pendingDx=None, copyFrom=0,
+                                   pendingDw=False, pendingFwd=False, lazy=None, ropeOf=None, ropeFused=False),
+                      ("owner", "data", "bytes", "size"))
 
 
 class CapturedGraph:
@@ -438,7 +440,7 @@ class CudaBackend:
         return self._externals.get(t)
 
     def _newExternal(self, t: Tensor, data: int, grad: int) -> _Entry:
-        e = _Entry(self._uid, data, t.size * 4, t.size)
+        e = _entry(self._uid, data, t.size * 4, t.size)
         e.grad, e.needs, e.external = grad, grad != 0, True
         self._externals[t] = e
         t._dev = e
@@ -503,7 +505,7 @@ class CudaBackend:
             self._transients.append((addr, (nbytes + 255) & ~255 if nbytes > 256 else 256))
         else:
             addr = self._acquireRecycled(nbytes)
-        t._dev = e = _Entry(self._uid, addr, nbytes, t.size)
+        t._dev = e = _entry(self._uid, addr, nbytes, t.size)
         if needs:
             e.needs = t._needs = True
         if self._regionStack:
@@ -1492,7 +1494,7 @@ class CudaBackend:
             data, lse, _n = rec["saved"][rec["pos"]]
             rec["pos"] += 1
             out = Tensor.output([T, Hq * hd], T * Hq * hd, [q, k, v])
-            eo = _Entry(self._uid, data, nbytes, out.size)
+            eo = _entry(self._uid, data, nbytes, out.size)
             eo.needs, eo.region = needs, self._regionStack[-1][0]
             out._needs, out._dev = needs, eo
         else:
@@ -1534,7 +1536,7 @@ class CudaBackend:
         """The scalar loss tensor plus its device-side companions: [1+nseq] losses and [nseq] 1/kept."""
         nseq = self._nseq()
         loss = Tensor.output([1], 1, list(prev))
-        e = _Entry(self._uid, self._acquireRecycled((1 + nseq) * 4), 4, 1)
+        e = _entry(self._uid, self._acquireRecycled((1 + nseq) * 4), 4, 1)
         e.needs = loss._needs = needs
         e.region = self._regionStack[-1][0] if self._regionStack else 0
         loss._dev = e

@@ -6,6 +6,7 @@
 #include <Python.h>
 
 #include <dlfcn.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include <tuple>
@@ -113,8 +114,71 @@ PyObject* bind(PyObject*, PyObject* args) {
   Py_RETURN_NONE;
 }
 
+// maker(cls, {slot: value}, (slot, ...)): a callable that makes an instance of a class with __slots__, the named slots taken from
+// its arguments, the others set to the given values. Written in Python the two records that every op makes, a tensor and
+// its device entry, cost 0.9 us of slot stores.
+struct Maker {
+  PyObject_HEAD
+  vectorcallfunc call;
+  PyTypeObject* cls;
+  Py_ssize_t nargs, nfixed;
+  Py_ssize_t arg_at[16], fixed_at[32];
+  PyObject* fixed[32];
+};
+PyObject* make(PyObject* self, PyObject* const* args, size_t nf, PyObject* kw) {
+  Maker* m = reinterpret_cast<Maker*>(self);
+  if (PyVectorcall_NARGS(nf) != m->nargs || (kw && PyTuple_GET_SIZE(kw)))
+    return PyErr_Format(PyExc_TypeError, "%s takes %zd arguments", m->cls->tp_name, m->nargs);
+  PyObject* o = m->cls->tp_alloc(m->cls, 0);       // (slots start out null)
+  if (!o) return nullptr;
+  char* base = reinterpret_cast<char*>(o);
+  for (Py_ssize_t i = 0; i < m->nargs; i++) *reinterpret_cast<PyObject**>(base + m->arg_at[i]) = Py_NewRef(args[i]);
+  for (Py_ssize_t i = 0; i < m->nfixed; i++) *reinterpret_cast<PyObject**>(base + m->fixed_at[i]) = Py_NewRef(m->fixed[i]);
+  return o;
+}
+void maker_dealloc(PyObject* self) {
+  Maker* m = reinterpret_cast<Maker*>(self);
+  for (Py_ssize_t i = 0; i < m->nfixed; i++) Py_DECREF(m->fixed[i]);
+  Py_XDECREF(m->cls);
+  Py_TYPE(self)->tp_free(self);
+}
+PyTypeObject MakerType = {PyVarObject_HEAD_INIT(nullptr, 0) "_calls.maker", sizeof(Maker)};
+Py_ssize_t slot_offset(PyObject* cls, PyObject* name) {
+  PyObject* d = PyObject_GetAttr(cls, name);
+  if (!d) return -1;
+  Py_ssize_t at = -1;
+  if (Py_IS_TYPE(d, &PyMemberDescr_Type) && reinterpret_cast<PyMemberDescrObject*>(d)->d_common.d_type == reinterpret_cast<PyTypeObject*>(cls))
+    at = reinterpret_cast<PyMemberDescrObject*>(d)->d_member->offset;
+  Py_DECREF(d);
+  if (at < 0) PyErr_Format(PyExc_TypeError, "%R is no slot of %R", name, cls);
+  return at;
+}
+PyObject* maker(PyObject*, PyObject* args) {
+  PyObject *cls, *fixed, *names;
+  if (!PyArg_ParseTuple(args, "O!O!O!", &PyType_Type, &cls, &PyDict_Type, &fixed, &PyTuple_Type, &names)) return nullptr;
+  if (PyDict_GET_SIZE(fixed) > 32 || PyTuple_GET_SIZE(names) > 16) return PyErr_Format(PyExc_ValueError, "too many slots");
+  Maker* m = PyObject_New(Maker, &MakerType);
+  if (!m) return nullptr;
+  m->call = make;
+  m->cls = reinterpret_cast<PyTypeObject*>(Py_NewRef(cls));
+  m->nargs = m->nfixed = 0;
+  PyObject *k, *v;
+  Py_ssize_t pos = 0, at;
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(names); i++) {
+    if ((at = slot_offset(cls, PyTuple_GET_ITEM(names, i))) < 0) { Py_DECREF(m); return nullptr; }
+    m->arg_at[m->nargs++] = at;
+  }
+  while (PyDict_Next(fixed, &pos, &k, &v)) {
+    if ((at = slot_offset(cls, k)) < 0) { Py_DECREF(m); return nullptr; }
+    m->fixed_at[m->nfixed] = at;
+    m->fixed[m->nfixed++] = Py_NewRef(v);
+  }
+  return reinterpret_cast<PyObject*>(m);
+}
+
 PyMethodDef methods[] = {
     {"bind", bind, METH_VARARGS, nullptr},
+    {"maker", maker, METH_VARARGS, nullptr},
 #define X(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, nullptr},
     GT_CALLS(X)
 #undef X
@@ -123,4 +187,11 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_calls", nullptr, -1, methods, nul
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__calls(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__calls(void) {
+  MakerType.tp_dealloc = maker_dealloc;
+  MakerType.tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_VECTORCALL;
+  MakerType.tp_vectorcall_offset = offsetof(Maker, call);
+  MakerType.tp_call = PyVectorcall_Call;
+  if (PyType_Ready(&MakerType) < 0) return nullptr;
+  return PyModule_Create(&module);
+}
