@@ -127,3 +127,25 @@ def _attention_f64(q, k, v, T, Hq, Hkv, hd, window, up):
         gq[:, h] = ds @ K[:, n]
         gk[:, n] += ds.T @ Q[:, h]
     return out.reshape(-1), [gq.reshape(-1), gk.reshape(-1), gv.reshape(-1)]
+
+
+@pytest.mark.parametrize("d", [64, 576, 1024])
+@pytest.mark.parametrize("rows", [1, 16, 17, 127, 128, 129, 513])
+def test_norm_backward_few_rows(gpu, d, rows):
+    """dw over one CTA, one cluster (up to 128 rows), and beyond it; overwriting and adding."""
+    rng = np.random.default_rng(rows + d)
+    x, g, gadd = (rng.standard_normal((rows, d), dtype=np.float32) for _ in range(3))
+    w, gw0 = rng.standard_normal(d, dtype=np.float32), rng.standard_normal(d, dtype=np.float32)
+    X = x.astype(np.float64)
+    r = 1.0 / np.sqrt((X * X).mean(1) + 1e-5)
+    rinv = r.astype(np.float32)
+    want_x = w * r[:, None] * g - X * (r ** 3 * (g * w * X).sum(1) / d)[:, None]
+    want_w = (g * X * r[:, None]).sum(0)
+    bufs = dx, dw, dr, dg, da, do, dgw = [_dev(gpu, a) for a in (x, w, rinv, g, gadd, x, gw0)]
+    for acc in (1, 0):
+        gpu._check(gpu.lib.gt_rmsnorm_bwd_add(gpu.ctx, rows, d, dx, dw, dr, dg, da, do, dgw, acc))
+        assert rel_l2(gpu.readStateBuffer(dgw, d), want_w + (gw0 if acc else 0.0)) <= REL_L2_FP32
+        assert rel_l2(gpu.readStateBuffer(do, rows * d), want_x + gadd) <= REL_L2_FP32
+    gpu.sync([])
+    for b in bufs:
+        gpu._check(gpu.lib.gt_free(gpu.ctx, b))
