@@ -889,7 +889,7 @@ constexpr Shape SHAPES[6] = {{1, 192, {0.345, 0.400, 0.465}, 1.67}, {1, 128, {0.
                              {2, 192, {0.550, 0.543, 0.621}, 3.90}, {3, 192, {0.330, 0.392, 0.502}, 0.89}, {3, 256, {0.334, 0.428, 0.529}, 1.75}};
 constexpr double FIXED = 4.3, FIXED_PAIR = 6.1;   // what a launch costs beside its tiles
 constexpr double SLICE = 0.52;                    // per wave when slices of K are added up in L2
-constexpr double CLEAR = 3.4;                     // the clear before a launch whose slices meet in L2, and the gap before it
+constexpr double CLEAR = 4.6;                     // the clear before a launch whose slices meet in L2: itself, and a node that nothing overlaps
 double shape_cost(const Shape& h, int kind, long units, long workers, int kblocks, int ks) {
   return (h.mt == 3 ? FIXED_PAIR : FIXED) + gt_cdiv(units, workers) * (gt_cdiv(kblocks, ks) * h.per_kb[kind] + h.epilogue + (ks > 1 ? SLICE : 0.0));
 }

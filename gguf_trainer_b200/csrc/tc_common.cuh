@@ -29,12 +29,16 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 // false on timeout
+// A wait is given up after WAIT_NS and not before its 4096th look: the wall clock is set now and then, and a step of it (back or
+// forth) must not end a wait that has only begun.
+__device__ __forceinline__ bool expired(uint64_t t0, uint32_t looks) {
+  return looks >= 4096 && ((int64_t)(gtimer() - t0) > (int64_t)WAIT_NS || looks == 0xffffffffu);
+}
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   if (mbar_try(bar, parity)) return true;
   const uint64_t t0 = gtimer();
-  while (!mbar_try(bar, parity)) {
-    if (gtimer() - t0 > WAIT_NS) return false;
-  }
+  for (uint32_t n = 0; !mbar_try(bar, parity); n++)
+    if (expired(t0, n)) return false;
   return true;
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
@@ -217,9 +221,8 @@ __device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity) 
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity) {   // false on timeout
   if (mbar_try_cluster(bar, parity)) return true;
   const uint64_t t0 = gtimer();
-  while (!mbar_try_cluster(bar, parity)) {
-    if (gtimer() - t0 > WAIT_NS) return false;
-  }
+  for (uint32_t n = 0; !mbar_try_cluster(bar, parity); n++)
+    if (expired(t0, n)) return false;
   return true;
 }
 
